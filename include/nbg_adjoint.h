@@ -165,6 +165,40 @@ nbg_status nbg_adjoint_wgrad(const void *a_hi, const void *a_lo, const void *b, 
 nbg_status nbg_adjoint_reduce_add(float *g, const float *part, int split, int64_t count, int64_t stride,
                                   void *stream);
 
+/* FP32 products on the CUDA cores for the shapes the tensor-core path does
+ * not take (any B, N >= 1).  Sums are chains of a few terms per thread and
+ * fixed trees over warps and CTAs: the order depends on the shape alone.
+ *   nbg_transpose   out[c][r] = in[r][c]
+ *   nbg_product_nt  C (M x N) = A (M x K) W^T, W N x K: both contiguous in k
+ *   nbg_lif_forward_step_smooth  the smoothed mode's nbg_lif_forward_step
+ *                   with I = s_prev W_rec + xi, the product in the same launch
+ *                   (w_rec_t = W_rec transposed; s_out another buffer than
+ *                   s_prev)
+ *   nbg_lif_adjoint_step_product  nbg_lif_adjoint_step with g_ext =
+ *                   dI_next W_rec^T in the same launch (dI_next NULL: none;
+ *                   dI another buffer than dI_next)
+ *   nbg_product_tn  part[q] (M x N) = the terms of split q of A^T B, A K x M,
+ *                   B K x N; added by nbg_adjoint_reduce_add.  `split` from
+ *                   nbg_product_tn_split, which needs `split * M * N` floats.
+ * chained != 0 launches a step with programmatic stream serialization: its
+ * W tiles and the operands no step writes (the record, xi, g_read, the
+ * parameters) may be read before the launch before it has ended, so that one
+ * must be a step of the same sweep.  No counterpart in the reference. */
+nbg_status nbg_transpose(const float *in, float *out, int rows, int cols, void *stream);
+nbg_status nbg_product_nt(const float *A, const float *W, float *C, int M, int N, int K, void *stream);
+nbg_status nbg_lif_forward_step_smooth(const float *s_prev, const float *w_rec_t, const float *xi, float *v,
+                                       float *s_out, float *u_rec, uint8_t *m_rec, float *vprev_rec, float *z,
+                                       float c_t, const float *alpha, const float *theta,
+                                       const nbg_lif_grad_params *p, int chained, int B, int N, void *stream);
+nbg_status nbg_lif_adjoint_step_product(const float *dI_next, const float *w_rec, const float *g_read, float c_t,
+                                        const float *u, const float *s, const uint8_t *m, const float *vprev,
+                                        float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
+                                        const float *theta, const nbg_lif_grad_params *p, int chained, int B, int N,
+                                        void *stream);
+int nbg_product_tn_split(int M, int N, int K);
+nbg_status nbg_product_tn(const float *A, const float *B, float *part, int split, int M, int N, int K,
+                          void *stream);
+
 /* C = A B for the readout's small products (B x N by N x O, its transposes):
  * element (r, c) of A at A[r * a_rs + c * a_cs], likewise B; C is M x N row
  * major, FP32 sums.  K < 64: one thread per output, k ascending; K >= 64: one

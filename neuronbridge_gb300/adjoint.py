@@ -18,9 +18,10 @@ backward, off the training step.
   is no GEMM in the forward at all.  The adjoint's recurrent term
   dI_{t+1} W_rec^T and the weight gradients run on tcgen05 in split BF16
   (nbg_adjoint_tc.cu) where the shapes allow (B = 128, N a multiple of
-  128), else as the engine's FP32 CUDA-core product (nbg_small_gemm).
+  128), else in FP32 on the CUDA cores (nbg_adjoint_f32.cu), the recurrent
+  product and the step that consumes it in one launch.
 * Smoothed (sigmoid) mode, the finite-difference test mode: x W_in and
-  s_{t-1} W_rec are that FP32 product too, followed by the fused elementwise
+  s_{t-1} W_rec are such FP32 products too, the recurrent one fused with the
   step.  No cuBLAS kernel runs in either mode.
 * All elementwise work of an adjoint step is one fused kernel.
 
@@ -72,6 +73,14 @@ _SIG = {
                                              _vp]),
     "nbg_small_gemm": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, ctypes.c_int, _vp,
                                       ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp]),
+    "nbg_transpose": (ctypes.c_int, [_vp, _vp, ctypes.c_int, ctypes.c_int, _vp]),
+    "nbg_product_nt": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp]),
+    "nbg_lif_forward_step_smooth": (ctypes.c_int, [_vp] * 9 + [ctypes.c_float, _vp, _vp, ctypes.POINTER(GradParams),
+                                                               ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp]),
+    "nbg_lif_adjoint_step_product": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_float] + [_vp] * 10 +
+                                     [ctypes.POINTER(GradParams), ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp]),
+    "nbg_product_tn_split": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int]),
+    "nbg_product_tn": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp]),
     "nbg_adjoint_wgrad": (ctypes.c_int, [_vp, _vp, _vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp,
                                          ctypes.c_int, _vp, _vp]),
     "nbg_adjoint_reduce_add": (ctypes.c_int, [_vp, _vp, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, _vp]),
@@ -238,7 +247,8 @@ def _forward_body(lib, x, w_in, w_rec, w_out, alpha, theta, p, K, coef, ck_v, ck
     sparse = _sparse_ok(p, N)
     lists = _SpikeLists(B, N, x.device) if sparse else None  # no spikes before step 0
     coef_dev = _coef_device(coef, x.device) if sparse else None
-    I = torch.empty((B, N), device=x.device, dtype=torch.float32)
+    smooth = _Smooth(lib, w_in, w_rec, B, st) if p.smooth else None
+    I = None if sparse or smooth else torch.empty((B, N), device=x.device, dtype=torch.float32)
     for seg, t0 in enumerate(range(0, T, K)):
         t1 = min(T, t0 + K)
         if rec is None:
@@ -256,18 +266,47 @@ def _forward_body(lib, x, w_in, w_rec, w_out, alpha, theta, p, K, coef, ck_v, ck
                                      coef_dev[t0:t1], alpha, theta, p, t1 - t0, B, N, st)
             continue
         xi = torch.empty((t1 - t0, B, N), device=x.device, dtype=torch.float32)
-        _gemm(lib, x[t0:t1], C, 1, w_in, N, 1, xi, (t1 - t0) * B, N, C, st)  # x W_in of the segment
+        if smooth:
+            smooth.inputs(x[t0:t1], xi)
+        else:
+            _gemm(lib, x[t0:t1], C, 1, w_in, N, 1, xi, (t1 - t0) * B, N, C, st)  # x W_in of the segment
         for t in range(t0, t1):
             if rec is None:
                 s, u_t, m_t, vp_t = sbuf[t & 1], None, None, None
             else:
                 s, u_t, m_t, vp_t = rec[1][t + 1], _ptr(rec[0][t]), _ptr(rec[2][t]), _ptr(rec[3][t])
+            if smooth:
+                smooth.step(s_prev, xi[t - t0], v, s, u_t, m_t, vp_t, z, float(coef[t]), alpha, theta, p, t > t0)
+                s_prev = s
+                continue
             _gemm(lib, s_prev, N, 1, w_rec, N, 1, I, B, N, N, st)  # s_{t-1} W_rec, then + x_t W_in
             I.add_(xi[t - t0])
             _lib.check(lib.nbg_lif_forward_step(_ptr(I), _ptr(v), _ptr(ref), _ptr(s), u_t, m_t, vp_t, _ptr(z),
                                                 float(coef[t]), _ptr(alpha), _ptr(theta), ctypes.byref(p), B, N, st))
             s_prev = s
     _readout(lib, z, w_out, out, st)
+
+
+class _Smooth:
+    """The smoothed mode's products: x W_in of a segment, and s_{t-1} W_rec fused with the step that consumes it
+    (nbg_lif_forward_step_smooth), on the transposed weights."""
+
+    def __init__(self, lib, w_in, w_rec, B, st):
+        self.lib, self.B, self.st = lib, B, st
+        self.C, self.N = w_in.shape
+        self.w_in_t = torch.empty((self.N, self.C), device=w_in.device, dtype=torch.float32)
+        self.w_rec_t = torch.empty_like(w_rec)
+        _lib.check(lib.nbg_transpose(_ptr(w_in), _ptr(self.w_in_t), self.C, self.N, st))
+        _lib.check(lib.nbg_transpose(_ptr(w_rec), _ptr(self.w_rec_t), self.N, self.N, st))
+
+    def inputs(self, x, xi) -> None:
+        L = x.shape[0]
+        _lib.check(self.lib.nbg_product_nt(_ptr(x), _ptr(self.w_in_t), _ptr(xi), L * self.B, self.N, self.C, self.st))
+
+    def step(self, s_prev, xi, v, s, u_t, m_t, vp_t, z, c, alpha, theta, p, chained) -> None:
+        _lib.check(self.lib.nbg_lif_forward_step_smooth(
+            _ptr(s_prev), _ptr(self.w_rec_t), _ptr(xi), _ptr(v), _ptr(s), u_t, m_t, vp_t, _ptr(z), c, _ptr(alpha),
+            _ptr(theta), ctypes.byref(p), int(chained), self.B, self.N, self.st))
 
 
 def _gemm(lib, a, a_rs, a_cs, b, b_rs, b_cs, out, M, N, K, st) -> None:
@@ -305,8 +344,6 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
     lam_v = torch.zeros((B, N), device=dev, dtype=torch.float32)
     g_theta = torch.zeros((B, N), device=dev, dtype=torch.float32)
     g_alpha = torch.zeros((B, N), device=dev, dtype=torch.float32)
-    g_ext = torch.empty((B, N), device=dev, dtype=torch.float32)
-    I = torch.empty((B, N), device=dev, dtype=torch.float32)
     L_max = min(K, T)
     if rec is None:  # one segment's replay
         U = torch.empty((L_max, B, N), device=dev, dtype=torch.float32)
@@ -318,13 +355,19 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
     lists = _SpikeLists(B, N, dev) if sparse and rec is None else None
     tc = _tc_ok(p, B, N)
     fused = _fused_ok(p, B, N)
+    # with the state recorded, the weight gradients run once, over every
+    # (step, row) pair of the run
+    whole = rec is not None and (fused or not tc)
+    smooth = _Smooth(lib, w_in, w_rec, B, st) if p.smooth and rec is None else None
+    I = None if sparse or smooth else torch.empty((B, N), device=dev, dtype=torch.float32)
     # the fused step writes dI^T for the weight gradients itself (no FP32 dI,
     # no transpose); the other forms keep dI in FP32
-    dI = None if fused else torch.empty((L_max, B, N), device=dev, dtype=torch.float32)
-    dI_next = None if fused else torch.empty((B, N), device=dev, dtype=torch.float32)
-    if not tc:  # the weight-gradient products of a segment (CUDA cores)
-        tmp_rec = torch.empty((N, N), device=dev, dtype=torch.float32)
-        tmp_in = torch.empty((C, N), device=dev, dtype=torch.float32)
+    dI_all = None if fused else torch.empty((T if whole else L_max, B, N), device=dev, dtype=torch.float32)
+    dI_next = None if fused or whole else torch.empty((B, N), device=dev, dtype=torch.float32)
+    if not tc:  # split-K partials of the weight-gradient products (CUDA cores)
+        kk_max = (T if whole else L_max) * B
+        tn_part = torch.empty(max(lib.nbg_product_tn_split(N, N, kk_max) * N * N,
+                                  lib.nbg_product_tn_split(C, N, kk_max) * C * N), device=dev, dtype=torch.float32)
     if tc:
         w_hi = torch.empty(N * N, device=dev, dtype=torch.bfloat16)
         w_lo = torch.empty(N * N, device=dev, dtype=torch.bfloat16)
@@ -338,9 +381,7 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
         tc_err = torch.zeros(1, device=dev, dtype=torch.int32)
         _lib.check(lib.nbg_adjoint_rec_prepare(_ptr(w_rec), _ptr(w_hi), _ptr(w_lo), N, st))
     # weight gradients on the tensor cores: the product's column operand (S^T,
-    # X^T) is padded with zero rows to a multiple of 256; with the state
-    # recorded they run once, over every (step, row) pair of the run
-    whole = fused and rec is not None
+    # X^T) is padded with zero rows to a multiple of 256
     if tc:
         kk_max = (T if whole else L_max) * B
         N256, C256 = -(-N // 256) * 256, -(-C // 256) * 256
@@ -369,6 +410,13 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
                                          _ptr(w_part), ws, _ptr(tc_err), st))
         _lib.check(lib.nbg_adjoint_reduce_add(_ptr(g_w_in), _ptr(w_part), ws, C * N, C256 * N, st))
 
+    def wgrad_f32(s_rows, x_rows, d_rows, L):
+        """dW_rec += S^T dI and dW_in += X^T dI over L steps on the CUDA cores."""
+        kk = L * B
+        for a, rows, g in ((s_rows, N, g_w_rec), (x_rows, C, g_w_in)):
+            split = lib.nbg_product_tn_split(rows, N, kk)
+            _lib.check(lib.nbg_product_tn(_ptr(a), _ptr(d_rows), _ptr(tn_part), split, rows, N, kk, st))
+            _lib.check(lib.nbg_adjoint_reduce_add(_ptr(g), _ptr(tn_part), split, rows * N, rows * N, st))
 
     segments = list(enumerate(range(0, T, K)))
     for seg, t0 in reversed(segments):
@@ -385,13 +433,21 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
                                      theta, p, L, B, N, st)
             else:
                 xi = torch.empty((L, B, N), device=dev, dtype=torch.float32)
-                _gemm(lib, x[t0:t1], C, 1, w_in, N, 1, xi, L * B, N, C, st)
+                if smooth:
+                    smooth.inputs(x[t0:t1], xi)
+                else:
+                    _gemm(lib, x[t0:t1], C, 1, w_in, N, 1, xi, L * B, N, C, st)
                 for k in range(L):
+                    if smooth:
+                        smooth.step(S[k], xi[k], v, S[k + 1], _ptr(U[k]), _ptr(M[k]), _ptr(VP[k]), None, 0.0, alpha,
+                                    theta, p, k > 0)
+                        continue
                     _gemm(lib, S[k], N, 1, w_rec, N, 1, I, B, N, N, st)
                     I.add_(xi[k])
                     _lib.check(lib.nbg_lif_forward_step(_ptr(I), _ptr(v), _ptr(ref), _ptr(S[k + 1]), _ptr(U[k]),
                                                         _ptr(M[k]), _ptr(VP[k]), None, 0.0, _ptr(alpha),
                                                         _ptr(theta), ctypes.byref(p), B, N, st))
+        dI = None if fused else dI_all[t0:t1] if whole else dI_all
         for k in reversed(range(L)):
             t = t0 + k
             if fused:  # dI_{t+1} W_rec^T (zero at the run's last step) and step t, one launch
@@ -412,14 +468,12 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
                                                     _ptr(g_parts), split, B, N, _ptr(tc_err), st))
                 have_next = True
                 continue
-            ge = None
-            if have_next:  # dL/ds_t from the recurrent path: dI_{t+1} W_rec^T
-                _gemm(lib, dI_next if k == L - 1 else dI[k + 1], N, 1, w_rec, 1, N, g_ext, B, N, N, st)
-                ge = g_ext
-            _lib.check(lib.nbg_lif_adjoint_step(_ptr(ge), _ptr(g_read), float(coef[t]), _ptr(U[k]),
-                                                _ptr(S[k + 1]), _ptr(M[k]), _ptr(VP[k]), _ptr(lam_v),
-                                                _ptr(dI[k]), _ptr(g_theta), _ptr(g_alpha), _ptr(alpha),
-                                                _ptr(theta), ctypes.byref(p), B, N, st))
+            # dL/ds_t from the recurrent path (dI_{t+1} W_rec^T) and the step that consumes it, one launch
+            d_next = (dI[k + 1] if k < L - 1 else dI_all[t1] if whole else dI_next) if have_next else None
+            _lib.check(lib.nbg_lif_adjoint_step_product(
+                _ptr(d_next), _ptr(w_rec), _ptr(g_read), float(coef[t]), _ptr(U[k]), _ptr(S[k + 1]), _ptr(M[k]),
+                _ptr(VP[k]), _ptr(lam_v), _ptr(dI[k]), _ptr(g_theta), _ptr(g_alpha), _ptr(alpha), _ptr(theta),
+                ctypes.byref(p), int(k < L - 1), B, N, st))
             have_next = True
         if whole:
             continue
@@ -429,16 +483,15 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
             transposes(S, x[t0:t1], L)
             wgrad(L)
         else:
-            # S^T dI and X^T dI over the segment's (step, row) pairs
-            _gemm(lib, S, 1, N, dI, N, 1, tmp_rec, N, N, L * B, st)
-            g_w_rec.add_(tmp_rec)
-            _gemm(lib, x[t0:t1], 1, C, dI, N, 1, tmp_in, C, N, L * B, st)
-            g_w_in.add_(tmp_in)
+            wgrad_f32(S, x[t0:t1], dI, L)
         if dI_next is not None:
             dI_next.copy_(dI[0])
     if whole:  # the whole run's weight gradients at once
-        transposes(rec[1], x, T)
-        wgrad(T)
+        if fused:
+            transposes(rec[1], x, T)
+            wgrad(T)
+        else:
+            wgrad_f32(rec[1], x, dI_all, T)
     return g_w_in, g_w_rec, g_w_out, g_alpha.sum(0), g_theta.sum(0), (tc_err if tc else None)
 
 
