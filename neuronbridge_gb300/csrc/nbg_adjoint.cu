@@ -7,6 +7,9 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <type_traits>
+
 #include "nbg_adjoint.h"
 #include "nbg_lif_grad.cuh"
 #include "nbg_common.cuh"
@@ -144,12 +147,10 @@ __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_sparse(
     if (tid == 0) cnt_out[b] = base;
 }
 
-// A whole checkpoint segment of the spike-driven forward: L steps of
-// k_lif_fwd_sparse in one launch.  Rows are independent (row b's input at
-// step t is x_t W_in plus the W_rec rows of row b's own spikes of step t-1),
-// so each CTA runs its row through all L steps with v and ref in registers
-// and the spike list in shared memory: no launch per step and no exchange
-// between CTAs.  The arithmetic is k_lif_fwd_sparse's, in the same order.
+// A whole checkpoint segment of the spike-driven forward for more than
+// kRowsMaxInputs input channels (k_lif_fwd_rows below takes the others, whose
+// inputs fit its shared-memory ring): one CTA per row, the lists of a step's
+// nonzero inputs and of the spikes in shared memory.
 //
 // acc[q] (column tid + q * kSparseThreads) += the rows idx[0..n) of w (N
 // columns), in ascending k, each scaled by val[k] when kScaled.  The rows are
@@ -183,23 +184,18 @@ __device__ __forceinline__ void gather_rows(float (&acc)[kSparseCols], const flo
     }
 }
 
-//
-// kGather: the input term too is a gather instead of a precomputed xi.  At
-// every step the CTA lists row b's nonzero inputs x_t[b][c] (ascending c,
-// with their values) in shared memory and starts the sum from them:
-// I_t = (sum over listed c of x_t[b][c] * W_in[c]) + (the W_rec rows of the
-// previous step's spikes), each term added in ascending order.  With spike
-// inputs (x in {0, 1}) the products are exact and the step costs a few rows
-// of W_in instead of a GEMM of the segment's inputs.
-template <bool kGather>
+// At every step the CTA lists row b's nonzero inputs x_t[b][c] (ascending c,
+// with their values) and starts the sum from them: I_t = (sum over listed c
+// of x_t[b][c] * W_in[c]) + (the W_rec rows of the previous step's spikes),
+// each term added in ascending order.
 __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_segment(
-    const float *__restrict__ xi, const float *__restrict__ x, const float *__restrict__ w_in, int C,
+    const float *__restrict__ x, const float *__restrict__ w_in, int C,
     const float *__restrict__ w, int *__restrict__ spk, int *__restrict__ cnt,
     float *__restrict__ v, int *__restrict__ ref, float *__restrict__ s_out, float *__restrict__ s_last,
     float *__restrict__ u_rec, unsigned char *__restrict__ m_rec, float *__restrict__ vprev_rec,
     float *__restrict__ z, const float *__restrict__ c, const float *__restrict__ alpha,
     const float *__restrict__ theta, nbg_lif_grad_params p, int L, int B, int N) {
-    extern __shared__ int seg_lists[]; // [2][N], then (kGather) in_idx[C], in_val[C]
+    extern __shared__ int seg_lists[]; // [2][N], then in_idx[C], in_val[C]
     __shared__ int warp_base[kSparseThreads / 32 + 1];
     __shared__ int list_cnt[2];
     int *in_idx = seg_lists + 2 * N;
@@ -227,46 +223,37 @@ __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_segment(
     int cur = 0;
     for (int step = 0; step < L; ++step) {
         float acc[kSparseCols];
-        if constexpr (kGather) {
-            // row b's nonzero inputs of this step, ascending
-            const float *xr = x + ((size_t)step * B + b) * C;
-            int nin = 0;
-            for (int c0 = 0; c0 < C; c0 += kSparseThreads) {
-                const int ch = c0 + tid;
-                const float xv = ch < C ? xr[ch] : 0.0f;
-                const bool nz = xv != 0.0f;
-                const unsigned bal = __ballot_sync(0xffffffffu, nz);
-                if (lane == 0) warp_base[wid] = __popc(bal);
-                __syncthreads();
-                if (tid == 0) {
-                    int sum = 0;
-                    for (int k = 0; k < kSparseThreads / 32; ++k) {
-                        const int cc = warp_base[k];
-                        warp_base[k] = sum;
-                        sum += cc;
-                    }
-                    warp_base[kSparseThreads / 32] = sum;
+        // row b's nonzero inputs of this step, ascending
+        const float *xr = x + ((size_t)step * B + b) * C;
+        int nin = 0;
+        for (int c0 = 0; c0 < C; c0 += kSparseThreads) {
+            const int ch = c0 + tid;
+            const float xv = ch < C ? xr[ch] : 0.0f;
+            const bool nz = xv != 0.0f;
+            const unsigned bal = __ballot_sync(0xffffffffu, nz);
+            if (lane == 0) warp_base[wid] = __popc(bal);
+            __syncthreads();
+            if (tid == 0) {
+                int sum = 0;
+                for (int k = 0; k < kSparseThreads / 32; ++k) {
+                    const int cc = warp_base[k];
+                    warp_base[k] = sum;
+                    sum += cc;
                 }
-                __syncthreads();
-                if (nz) {
-                    const int at = nin + warp_base[wid] + __popc(bal & ((1u << lane) - 1u));
-                    in_idx[at] = ch;
-                    in_val[at] = xv;
-                }
-                nin += warp_base[kSparseThreads / 32];
-                __syncthreads();
+                warp_base[kSparseThreads / 32] = sum;
             }
-#pragma unroll
-            for (int q = 0; q < kSparseCols; ++q) acc[q] = 0.0f;
-            gather_rows<true>(acc, w_in, in_idx, in_val, nin, tid, nq, N);
-        } else {
-            const float *xs = xi + (size_t)step * plane + row;
-#pragma unroll
-            for (int q = 0; q < kSparseCols; ++q) {
-                const int j = tid + q * kSparseThreads;
-                acc[q] = (q < nq && j < N) ? xs[j] : 0.0f;
+            __syncthreads();
+            if (nz) {
+                const int at = nin + warp_base[wid] + __popc(bal & ((1u << lane) - 1u));
+                in_idx[at] = ch;
+                in_val[at] = xv;
             }
+            nin += warp_base[kSparseThreads / 32];
+            __syncthreads();
         }
+#pragma unroll
+        for (int q = 0; q < kSparseCols; ++q) acc[q] = 0.0f;
+        gather_rows<true>(acc, w_in, in_idx, in_val, nin, tid, nq, N);
         const int *list = seg_lists + cur * N;
         gather_rows<false>(acc, w, list, nullptr, list_cnt[cur], tid, nq, N);
         int *out_list = seg_lists + (cur ^ 1) * N;
@@ -328,6 +315,424 @@ __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_segment(
     const int nl = list_cnt[cur];
     for (int k = tid; k < nl; k += kSparseThreads) spk[row + k] = seg_lists[cur * N + k];
     if (tid == 0) cnt[b] = nl;
+}
+
+// ------------------------------------------------ rows through a segment
+//
+// The spike-driven forward of a checkpoint segment, one CTA per batch row
+// (rows are independent), for up to kRowsMaxInputs input channels.  Per step:
+//   I = (x_t[c] * W_in[c] over the nonzero inputs c) + (the W_rec rows of the
+//       spikes of step t - 1), every term added in ascending order,
+// then the update of k_lif_fwd_sparse in the same operations.
+//
+// What bounds it: the spikes of a step must be known before the next step's
+// rows (about 28 of 4 KiB at 1,024 neurons firing 2 % of the steps, from L2)
+// can be asked for, so a step is one chain -- spike list, row loads, sums,
+// threshold, list -- and a warp's own instructions on it weigh as much as the
+// loads' latency.  So:
+//   * a thread owns two neighbouring columns (four above 1,024 neurons, single
+//     ones where N or a pointer is not aligned), adds them packed, and has up
+//     to 24 rows in flight; the list holds byte offsets of rows, read four at
+//     a time, padded to whole groups of four;
+//   * the input rows of step t + 1 do not depend on the spikes of step t: they
+//     are requested behind the recurrent rows of step t and summed into the
+//     next step's start value;
+//   * inputs come through a ring of kRing rows in shared memory, copied
+//     asynchronously, and one warp (another each step) lists the nonzero
+//     channels of step t + 2 from it while the rows are in flight;
+//   * the new spikes are ranked by ballots and one exchange of the warps'
+//     counts: two block barriers a step.
+// The kernel before it listed, summed and ranked one after the other with
+// about twenty barriers a step.  Measured, 500 steps of 64 rows, 1,000
+// neurons, 200 inputs, 2.2 % firing: 3.17 -> 1.27 ms (6.3 -> 2.5 us a step;
+// eight warps of four columns each, unpacked, 2.45 ms: 1,506 instructions a
+// warp and step, few of them waiting for memory).  A training step of 128 rows
+// x 1,024 neurons x 1,000 steps: 14.96 -> 11.50 ms.
+constexpr int kRing = 8;
+constexpr int kRowsMaxInputs = 4096;
+constexpr int kRowsMaxNeurons = 2048;
+
+__device__ __forceinline__ void ring_copy(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// A thread's columns of a row, and sums of them: V neighbouring columns (2 or
+// 4, as packed pairs) or NC single ones (V = 1).  Packed or not, every
+// addition and product is rounded once.
+template <int V, int NC> struct Cols {
+    static constexpr int kN = V == 1 ? NC : V / 2;
+    typename std::conditional<V == 1, float, unsigned long long>::type d[kN];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < kN; ++i) d[i] = 0;
+    }
+    // at: byte offsets of this thread's columns (one per column group)
+    __device__ __forceinline__ void load(const float *base, unsigned row, const unsigned (&at)[V == 1 ? NC : 1]) {
+        if constexpr (V == 1) {
+#pragma unroll
+            for (int i = 0; i < NC; ++i) d[i] = __ldg(reinterpret_cast<const float *>((const char *)base + (row + at[i])));
+        } else if constexpr (V == 2) {
+            d[0] = __ldg(reinterpret_cast<const unsigned long long *>((const char *)base + (row + at[0])));
+        } else {
+            const ulonglong2 q = __ldg(reinterpret_cast<const ulonglong2 *>((const char *)base + (row + at[0])));
+            d[0] = q.x;
+            d[1] = q.y;
+        }
+    }
+    __device__ __forceinline__ void add(const Cols &o) {
+#pragma unroll
+        for (int i = 0; i < kN; ++i) {
+            if constexpr (V == 1) d[i] = d[i] + o.d[i];
+            else asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d[i]) : "l"(o.d[i]));
+        }
+    }
+    __device__ __forceinline__ void add_scaled(float x, const Cols &o) {
+#pragma unroll
+        for (int i = 0; i < kN; ++i) {
+            if constexpr (V == 1) {
+                d[i] = d[i] + x * o.d[i];
+            } else {
+                // single products: a packed product and sum would be fused into one rounding
+                unsigned long long q;
+                asm("mov.b64 %0, {%1, %2};" : "=l"(q) : "f"(__fmul_rn(x, o.get(2 * i))), "f"(__fmul_rn(x, o.get(2 * i + 1))));
+                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d[i]) : "l"(q));
+            }
+        }
+    }
+    __device__ __forceinline__ float get(int i) const {
+        if constexpr (V == 1) {
+            return d[i];
+        } else {
+            float x, y;
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(d[i >> 1]));
+            return i & 1 ? y : x;
+        }
+    }
+};
+
+template <bool kGather, int V, int NC, int kMaxThreads>
+__global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
+    const float *__restrict__ xi, const float *__restrict__ x, const float *__restrict__ w_in, int C,
+    const float *__restrict__ w, int *__restrict__ spk, int *__restrict__ cnt, float *__restrict__ v,
+    int *__restrict__ ref, float *__restrict__ s_out, float *__restrict__ s_last, float *__restrict__ u_rec,
+    unsigned char *__restrict__ m_rec, float *__restrict__ vprev_rec, float *__restrict__ z,
+    const float *__restrict__ c, const float *__restrict__ alpha, const float *__restrict__ theta,
+    nbg_lif_grad_params p, int L, int B, int N) {
+    static_assert(V == 1 || NC == V, "a group is the thread's neighbouring columns");
+    constexpr int kGroups = NC == 4 ? 3 : NC == 2 ? 6 : 8; // groups of four rows in flight: 48 registers at most
+    constexpr int kSegs = V == 1 ? NC : 1;                 // segments of the ascending order: (column group, warp)
+    __shared__ __align__(16) unsigned list[kRowsMaxNeurons + 4]; // ascending spikes of the step before: row offsets
+    __shared__ int seg_cnt[64];                                  // spikes per (column group, warp)
+    __shared__ int in_cnt[2];
+    extern __shared__ __align__(16) uint2 rows_smem[]; // kGather: lists [2][C + 4 rounded to even] (row offset, value), ring [kRing][C]
+    const int Cl = (C + 5) & ~1;
+    uint2 *const in_list = rows_smem;
+    float *const ring = reinterpret_cast<float *>(rows_smem + 2 * Cl);
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int T = blockDim.x, nw = T >> 5;
+    const unsigned row_bytes = (unsigned)N * 4u;
+    const size_t row = (size_t)b * N, plane = (size_t)B * N;
+    int col[NC];
+    bool has[NC]; // V > 1: N is a multiple of V, so all or none
+    unsigned at[kSegs]; // a thread without columns reads the row's first ones and drops them
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        col[i] = V == 1 ? i * T + tid : tid * V + i;
+        has[i] = col[i] < N;
+    }
+#pragma unroll
+    for (int i = 0; i < kSegs; ++i) at[i] = has[i] ? (unsigned)col[i] * 4u : 0u;
+    float vv[NC], zz[NC], al[NC], th[NC];
+    int rr[NC];
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        vv[i] = zz[i] = al[i] = th[i] = 0.0f;
+        rr[i] = 0;
+        if (has[i]) {
+            vv[i] = v[row + col[i]];
+            rr[i] = ref[row + col[i]];
+            if (z) zz[i] = z[row + col[i]];
+            al[i] = alpha[col[i]];
+            th[i] = theta[col[i]];
+        }
+    }
+    using Row = Cols<V, NC>;
+    // four rows of the spike list from k on, and their sum in order
+    auto request = [&](Row (&d)[4], int k) {
+        const uint4 o = *reinterpret_cast<const uint4 *>(list + k);
+        d[0].load(w, o.x, at);
+        d[1].load(w, o.y, at);
+        d[2].load(w, o.z, at);
+        d[3].load(w, o.w, at);
+    };
+    auto add = [&](Row &acc, const Row (&d)[4], int left) {
+        acc.add(d[0]);
+        if (left >= 4) {
+            acc.add(d[1]);
+            acc.add(d[2]);
+            acc.add(d[3]);
+        } else {
+            if (left > 1) acc.add(d[1]);
+            if (left > 2) acc.add(d[2]);
+        }
+    };
+    auto request_in = [&](Row (&d)[4], float (&xv)[4], int at_list) {
+        const uint4 p0 = *reinterpret_cast<const uint4 *>(in_list + at_list);
+        const uint4 p1 = *reinterpret_cast<const uint4 *>(in_list + at_list + 2);
+        d[0].load(w_in, p0.x, at);
+        d[1].load(w_in, p0.z, at);
+        d[2].load(w_in, p1.x, at);
+        d[3].load(w_in, p1.z, at);
+        xv[0] = __uint_as_float(p0.y);
+        xv[1] = __uint_as_float(p0.w);
+        xv[2] = __uint_as_float(p1.y);
+        xv[3] = __uint_as_float(p1.w);
+    };
+    auto add_in = [&](Row &acc, const Row (&d)[4], const float (&xv)[4], int left) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (left > r) acc.add_scaled(xv[r], d[r]);
+    };
+    auto ring_load = [&](int step, int slot) {
+        if (step < L) {
+            const float *xr = x + ((size_t)step * B + b) * C;
+            float *d = ring + slot * C;
+            for (int ch = tid; ch < C; ch += T) ring_copy(d + ch, xr + ch);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto list_inputs = [&](int step) { // one warp: the nonzero channels of `step`, ascending
+        const float *xr = ring + (step % kRing) * C;
+        uint2 *const out = in_list + (step & 1) * Cl;
+        int n = 0;
+#pragma unroll 4
+        for (int c0 = 0; c0 < C; c0 += 32) {
+            const float xv = c0 + lane < C ? xr[c0 + lane] : 0.0f;
+            const bool nz = xv != 0.0f;
+            const unsigned bal = __ballot_sync(0xffffffffu, nz);
+            if (nz) out[n + __popc(bal & ((1u << lane) - 1u))] = make_uint2((unsigned)(c0 + lane) * row_bytes, __float_as_uint(xv));
+            n += __popc(bal);
+        }
+        if (lane < 4) out[n + lane] = make_uint2(0u, 0u); // the last group's padding: row 0, not added
+        if (lane == 0) in_cnt[step & 1] = n;
+    };
+    int n_spk = cnt[b];
+    for (int k = tid; k < n_spk + 4; k += T) list[k] = k < n_spk ? (unsigned)spk[row + k] * row_bytes : 0u;
+    if constexpr (kGather) {
+        for (int k = 0; k < kRing; ++k) ring_load(k, k);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (wid == 0) {
+            list_inputs(0);
+            if (L > 1) list_inputs(1);
+        }
+    }
+    __syncthreads();
+    Row start; // the sum the next step starts from: its input term
+    start.zero();
+    if constexpr (kGather) {
+        for (int k = 0; k < in_cnt[0]; k += 4) {
+            Row d[4];
+            float xv[4];
+            request_in(d, xv, k);
+            add_in(start, d, xv, in_cnt[0] - k);
+        }
+        __syncthreads(); // step 0 lists the inputs of step 2 over those of step 0
+    } else {
+        start.load(xi + row, 0u, at);
+    }
+    int lister = 0; // the warp that lists next
+    for (int step = 0; step < L; ++step) {
+        Row acc = start;
+        const float ct = z ? c[step] : 0.0f;
+        const bool more = step + 1 < L;
+        const int slot = (step + 1) & 1;
+        Row d[kGroups][4];
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g)
+            if (4 * g < n_spk) request(d[g], 4 * g);
+        int n_in = 0;
+        Row di[2][4];
+        float xv[2][4];
+        if constexpr (kGather) {
+            if (more) {
+                n_in = in_cnt[slot];
+#pragma unroll
+                for (int g = 0; g < 2; ++g)
+                    if (4 * g < n_in) request_in(di[g], xv[g], slot * Cl + 4 * g);
+            }
+            if (wid == lister && step + 2 < L) list_inputs(step + 2);
+            lister = lister + 1 == nw ? 0 : lister + 1;
+            if (step > 0) ring_load(step + kRing - 1, (step - 1) % kRing); // over the row listed three steps ago
+        } else {
+            if (more) start.load(xi + (size_t)(step + 1) * plane + row, 0u, at);
+        }
+        for (int k = 0;;) {
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g)
+                if (k + 4 * g < n_spk) add(acc, d[g], n_spk - k - 4 * g);
+            k += 4 * kGroups;
+            if (k >= n_spk) break;
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g)
+                if (k + 4 * g < n_spk) request(d[g], k + 4 * g);
+        }
+        float uu[NC], vp[NC];
+        unsigned bal[NC];
+        bool integ[NC], sp[NC];
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+            vp[i] = vv[i];
+            const int rf = rr[i];
+            integ[i] = rf == 0;
+            uu[i] = integ[i] ? vp[i] + al[i] * (p.v_rest - vp[i]) + acc.get(i) : p.v_reset;
+            sp[i] = has[i] && uu[i] > th[i];
+            const float sv = sp[i] ? 1.0f : 0.0f;
+            vv[i] = uu[i] - sv * (uu[i] - p.v_reset);
+            rr[i] = sp[i] ? p.t_ref : (rf > 0 ? rf - 1 : 0);
+            if (z) zz[i] = zz[i] + ct * sv;
+            bal[i] = __ballot_sync(0xffffffffu, sp[i]);
+        }
+        // ranks: within the warp by ballots, across warps by their counts
+        if (lane == 0) {
+            if constexpr (V == 1) {
+#pragma unroll
+                for (int i = 0; i < NC; ++i) seg_cnt[i * nw + wid] = __popc(bal[i]);
+            } else {
+                int k = 0;
+#pragma unroll
+                for (int i = 0; i < NC; ++i) k += __popc(bal[i]);
+                seg_cnt[wid] = k;
+            }
+        }
+        if constexpr (kGather) asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 5) : "memory"); // the row listed next step
+        __syncthreads(); // counts; everyone has read the list
+        const unsigned lt = (1u << lane) - 1u;
+        int total = 0;
+#pragma unroll
+        for (int s = 0; s < kSegs; ++s) {
+            // spikes before segment s * nw + wid (low half) and in all (high half): both at most 2,048
+            unsigned both = 0u;
+#pragma unroll
+            for (int h = 0; h < (kSegs > 1 ? 2 : 1); ++h) {
+                const int k = lane + 32 * h;
+                const unsigned q = k < kSegs * nw ? (unsigned)seg_cnt[k] : 0u;
+                both += q << 16 | (k < s * nw + wid ? q : 0u);
+            }
+            both = __reduce_add_sync(0xffffffffu, both);
+            int pos = (int)(both & 0xffffu);
+            total = (int)(both >> 16);
+            if constexpr (V == 1) {
+                if (sp[s]) list[pos + __popc(bal[s] & lt)] = (unsigned)col[s] * row_bytes;
+            } else {
+#pragma unroll
+                for (int i = 0; i < NC; ++i) pos += __popc(bal[i] & lt);
+#pragma unroll
+                for (int i = 0; i < NC; ++i)
+                    if (sp[i]) list[pos++] = (unsigned)col[i] * row_bytes;
+            }
+        }
+        n_spk = total;
+        if (tid < 4) list[total + tid] = 0u; // the last group's padding: row 0, not added
+        // the record, and the next step's input term, off the spikes' chain
+        {
+            const size_t o = (size_t)step * plane + row;
+            float sv[NC];
+#pragma unroll
+            for (int i = 0; i < NC; ++i) sv[i] = sp[i] ? 1.0f : 0.0f;
+            if constexpr (V == 4) {
+                if (has[0]) {
+                    const size_t q = (o >> 2) + tid; // rows are multiples of four
+                    if (s_out) reinterpret_cast<float4 *>(s_out)[q] = make_float4(sv[0], sv[1], sv[2], sv[3]);
+                    if (s_last && !more)
+                        reinterpret_cast<float4 *>(s_last)[(row >> 2) + tid] = make_float4(sv[0], sv[1], sv[2], sv[3]);
+                    if (u_rec) reinterpret_cast<float4 *>(u_rec)[q] = make_float4(uu[0], uu[1], uu[2], uu[3]);
+                    if (m_rec)
+                        reinterpret_cast<uchar4 *>(m_rec)[q] = make_uchar4(integ[0], integ[1], integ[2], integ[3]);
+                    if (vprev_rec) reinterpret_cast<float4 *>(vprev_rec)[q] = make_float4(vp[0], vp[1], vp[2], vp[3]);
+                }
+            } else if constexpr (V == 2) {
+                if (has[0]) {
+                    const size_t q = (o >> 1) + tid;
+                    if (s_out) reinterpret_cast<float2 *>(s_out)[q] = make_float2(sv[0], sv[1]);
+                    if (s_last && !more) reinterpret_cast<float2 *>(s_last)[(row >> 1) + tid] = make_float2(sv[0], sv[1]);
+                    if (u_rec) reinterpret_cast<float2 *>(u_rec)[q] = make_float2(uu[0], uu[1]);
+                    if (m_rec) reinterpret_cast<uchar2 *>(m_rec)[q] = make_uchar2(integ[0], integ[1]);
+                    if (vprev_rec) reinterpret_cast<float2 *>(vprev_rec)[q] = make_float2(vp[0], vp[1]);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < NC; ++i)
+                    if (has[i]) {
+                        const size_t q = o + col[i];
+                        if (s_out) s_out[q] = sv[i];
+                        if (s_last && !more) s_last[row + col[i]] = sv[i];
+                        if (u_rec) u_rec[q] = uu[i];
+                        if (m_rec) m_rec[q] = integ[i] ? 1 : 0;
+                        if (vprev_rec) vprev_rec[q] = vp[i];
+                    }
+            }
+        }
+        if constexpr (kGather) {
+            start.zero();
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+                if (4 * g < n_in) add_in(start, di[g], xv[g], n_in - 4 * g);
+            for (int k = 8; k < n_in; k += 4) {
+                request_in(di[0], xv[0], slot * Cl + k);
+                add_in(start, di[0], xv[0], n_in - k);
+            }
+        }
+        __syncthreads(); // the list; the input list of step + 2
+    }
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+        if (!has[i]) continue;
+        v[row + col[i]] = vv[i];
+        ref[row + col[i]] = rr[i];
+        if (z) z[row + col[i]] = zz[i];
+    }
+    for (int k = tid; k < n_spk; k += T) spk[row + k] = (int)(list[k] / row_bytes);
+    if (tid == 0) cnt[b] = n_spk;
+}
+
+// Launch k_lif_fwd_rows: neighbouring columns where N is a multiple of their
+// number and every matrix aligned to them, else single columns.  Two a thread
+// up to 1,024 neurons: sixteen warps issue a step's row loads and sums in half
+// the instructions a warp that eight warps of four columns take.
+template <bool kGather>
+nbg_status launch_rows(const float *xi, const float *x, const float *w_in, int C, const float *w, int *spk, int *cnt,
+                       float *v, int *ref, float *s_out, float *s_last, float *u_rec, unsigned char *m_rec,
+                       float *vprev_rec, float *z, const float *c, const float *alpha, const float *theta,
+                       const nbg_lif_grad_params &p, int L, int B, int N, cudaStream_t stream) {
+    using Kernel = void (*)(const float *, const float *, const float *, int, const float *, int *, int *, float *,
+                            int *, float *, float *, float *, unsigned char *, float *, float *, const float *,
+                            const float *, const float *, nbg_lif_grad_params, int, int, int);
+    const uintptr_t bits = (uintptr_t)xi | (uintptr_t)w_in | (uintptr_t)w | (uintptr_t)s_out | (uintptr_t)s_last |
+                           (uintptr_t)u_rec | (uintptr_t)vprev_rec | (uintptr_t)m_rec * 4u;
+    Kernel k;
+    int threads;
+    if (N % 2 == 0 && N <= 1024 && (bits & 7u) == 0) {
+        threads = (N / 2 + 31) & ~31;
+        k = k_lif_fwd_rows<kGather, 2, 2, 512>;
+    } else if (N % 4 == 0 && N > 1024 && (bits & 15u) == 0) {
+        threads = (N / 4 + 31) & ~31;
+        k = k_lif_fwd_rows<kGather, 4, 4, 512>;
+    } else {
+        threads = std::min(512, (N + 31) & ~31);
+        const int nc = (N + threads - 1) / threads;
+        k = nc == 1   ? k_lif_fwd_rows<kGather, 1, 1, 512>
+            : nc == 2 ? k_lif_fwd_rows<kGather, 1, 2, 512>
+                      : k_lif_fwd_rows<kGather, 1, 4, 512>;
+    }
+    const size_t smem = kGather ? 2 * ((size_t)(C + 5) & ~(size_t)1) * sizeof(uint2) + (size_t)kRing * C * sizeof(float) : 0;
+    if (smem > 32 * 1024)
+        NBG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k<<<B, threads, smem, stream>>>(xi, x, w_in, C, w, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec, z, c,
+                                    alpha, theta, p, L, B, N);
+    NBG_CUDA(cudaGetLastError());
+    return NBG_OK;
 }
 
 // Ascending spike list of each row of a 0/1 matrix (segment restarts).
@@ -482,11 +887,8 @@ nbg_status nbg_lif_forward_segment_sparse(const float *xi, const float *w_rec, i
     if (N > kSparseThreads * kSparseCols)
         return nbg_fail(NBG_ERR_UNSUPPORTED, "the spike-driven step supports up to %d neurons",
                         kSparseThreads * kSparseCols);
-    k_lif_fwd_segment<false><<<B, kSparseThreads, 2 * N * sizeof(int), (cudaStream_t)stream>>>(
-        xi, nullptr, nullptr, 0, w_rec, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec, z, c, alpha,
-        theta, *p, L, B, N);
-    NBG_CUDA(cudaGetLastError());
-    return NBG_OK;
+    return launch_rows<false>(xi, nullptr, nullptr, 0, w_rec, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec,
+                              z, c, alpha, theta, *p, L, B, N, (cudaStream_t)stream);
 }
 
 nbg_status nbg_lif_forward_segment_gather(const float *x, const float *w_in, int C, const float *w_rec, int32_t *spk,
@@ -501,13 +903,15 @@ nbg_status nbg_lif_forward_segment_gather(const float *x, const float *w_in, int
     if (N > kSparseThreads * kSparseCols)
         return nbg_fail(NBG_ERR_UNSUPPORTED, "the spike-driven step supports up to %d neurons",
                         kSparseThreads * kSparseCols);
+    if (C <= kRowsMaxInputs)
+        return launch_rows<true>(nullptr, x, w_in, C, w_rec, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec,
+                                 z, c, alpha, theta, *p, L, B, N, (cudaStream_t)stream);
     const size_t smem = (2 * (size_t)N + 2 * (size_t)C) * sizeof(int);
     if (smem > 200 * 1024) return nbg_fail(NBG_ERR_UNSUPPORTED, "too many inputs for the gather form (C = %d)", C);
     if (smem > 48 * 1024)
-        NBG_CUDA(cudaFuncSetAttribute(k_lif_fwd_segment<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-    k_lif_fwd_segment<true><<<B, kSparseThreads, smem, (cudaStream_t)stream>>>(
-        nullptr, x, w_in, C, w_rec, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec, z, c, alpha, theta,
+        NBG_CUDA(cudaFuncSetAttribute(k_lif_fwd_segment, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_lif_fwd_segment<<<B, kSparseThreads, smem, (cudaStream_t)stream>>>(
+        x, w_in, C, w_rec, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec, z, c, alpha, theta,
         *p, L, B, N);
     NBG_CUDA(cudaGetLastError());
     return NBG_OK;
