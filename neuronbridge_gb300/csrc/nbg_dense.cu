@@ -19,7 +19,7 @@
 //     128 CTAs; the two partial sums are added in a fixed order by the update
 //     kernel, so results are deterministic.  At M = 64 instances the GEMM
 //     streams 2 x N^2 BF16 per step and is HBM-bound.
-//   * NBG_DENSE_FP32 -- CUDA cores: each post neuron sums W[i][j] over the
+//   * NBG_DENSE_FP32 -- CUDA cores (k_dense_gather): each post neuron sums W[i][j] over the
 //     spiking pre-synaptic i of its instance in ascending i, in FP32, which is
 //     the exact sequential sum the CPU oracle computes.
 
@@ -215,29 +215,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
 }
 
-// --------------------------------------------------------- FP32 CUDA cores
-
-// cur[b][j] = sum over i ascending with bit i of S_b set of W[i][j]
-__global__ void __launch_bounds__(256) k_dense_fp32(const float *__restrict__ w, const unsigned *__restrict__ sbits,
-                                                    float *__restrict__ cur, int n) {
-    extern __shared__ unsigned bits[];
-    const int b = blockIdx.y;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nw = n / 32;
-    for (int k = threadIdx.x; k < nw; k += blockDim.x) bits[k] = sbits[(size_t)b * nw + k];
-    __syncthreads();
-    float sum = 0.0f;
-    for (int k = 0; k < nw; ++k) {
-        unsigned word = bits[k];
-        while (word) {
-            const int i = k * 32 + __ffs(word) - 1;
-            word &= word - 1u;
-            sum = sum + w[(size_t)i * n + j];
-        }
-    }
-    cur[(size_t)b * n + j] = sum;
-}
-
 // -------------------------------------------------------------- LIF update
 
 struct LifParams {
@@ -245,11 +222,9 @@ struct LifParams {
     int t_ref;
 };
 
-// One update of every (instance, neuron): summed arrival, refractory-gated
-// voltage jump, forward-Euler voltage-jump LIF (TimeDrivenLIF_Voltage_jump.cpp
-// :49-86), spike -> S_t (BF16 0/1 for the tensor path, bit words for FP32).
-// One neuron's update (state vv, ls in registers) given its summed arrival
-// `a`; idx = the element of the instance-major state (the drive's hash index).
+// One neuron's update: summed arrival, refractory-gated voltage jump,
+// forward-Euler voltage-jump LIF (TimeDrivenLIF_Voltage_jump.cpp:49-86),
+// state vv, ls in registers, `a` its summed arrival; idx = the element of the instance-major state (the drive's hash index).
 __device__ __forceinline__ bool lif_apply(const LifParams &P, float a, float &vv, int &ls, int t, int idx) {
     if (t >= 1 && nbg_hash_uniform01(idx, t - 1) < P.drive_p) a = a + P.drive_w;
     if (ls > P.t_ref) vv = vv + a;
@@ -267,11 +242,122 @@ __device__ __forceinline__ bool lif_apply(const LifParams &P, float a, float &vv
     return spk;
 }
 
+// --------------------------------------------------------- FP32 CUDA cores
+
+// One step on the FP32 path: cur[b][j] = the sum over i ascending with bit i
+// of instance b's spike words set of W[i][j] (kLif = false: the result), then
+// the neuron update on it, writing the next step's spike words.
+//
+// What bounds it: every instance reads the rows of its own spikes (131 of 32
+// KiB at 8,192 neurons firing 1.6 % of the steps; 270 MB a step for the 64),
+// so the L2, and below that the latency of dependent loads: the kernel before
+// this one kept one 4-byte load a thread in flight (13.0 us a step at 2,048
+// neurons, 152 at 8,192, and 2.6 more for the update in its own launch).  Here
+// a CTA ranks the instance's spikes into a list once, each thread owns two
+// neighbouring columns and asks for kGatherRows rows before it adds the first.
+// The instances of one column slice are neighbours in the grid, so a row that
+// several of them need is read from memory once.  Measured, update included:
+// 154 -> 32.9 us a step at 8,192 neurons (8.2 TB/s of row reads), 100 steps
+// and their read-out at 2,048 neurons 2.61 -> 0.78 ms.
+constexpr int kGatherThreads = 256;
+constexpr int kGatherCols = 2 * kGatherThreads; // columns of a CTA
+constexpr int kGatherWords = 256;               // spike words listed at a time (8,192 neurons)
+constexpr int kGatherRows = 16;
+
+// bits 0..15 of x to the even bits of the result
+__device__ __forceinline__ unsigned spread16(unsigned x) {
+    x = (x | x << 8) & 0x00ff00ffu;
+    x = (x | x << 4) & 0x0f0f0f0fu;
+    x = (x | x << 2) & 0x33333333u;
+    return (x | x << 1) & 0x55555555u;
+}
+
+template <bool kLif>
+__global__ void __launch_bounds__(kGatherThreads) k_dense_gather(const float *__restrict__ w,
+                                                                 const unsigned *__restrict__ sbits,
+                                                                 float *__restrict__ cur, LifParams P, float *v,
+                                                                 int *last, unsigned *__restrict__ bits_out,
+                                                                 int *__restrict__ counts, int t, int n) {
+    __shared__ __align__(16) int list[kGatherWords * 32 + 4];
+    __shared__ int warp_cnt[kGatherThreads / 32];
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int j = blockIdx.y * kGatherCols + 2 * tid;
+    const bool has = j < n; // n is a multiple of 128: whole warps
+    const float *const col = w + (has ? j : 0);
+    const int nw = n / 32;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory"); // the previous step's spikes, v and last
+    const size_t at = (size_t)b * n + j;
+    float2 vv = make_float2(0.0f, 0.0f);
+    int2 ls = make_int2(0, 0);
+    if (kLif && has) {
+        vv = *reinterpret_cast<const float2 *>(v + at);
+        ls = *reinterpret_cast<const int2 *>(last + at);
+    }
+    float2 sum = make_float2(0.0f, 0.0f);
+    for (int w0 = 0; w0 < nw; w0 += kGatherWords) {
+        // this chunk's spikes, ascending: one word a thread, ranked by a scan
+        unsigned word = tid < kGatherWords && w0 + tid < nw ? __ldcg(sbits + (size_t)b * nw + w0 + tid) : 0u;
+        int incl = __popc(word);
+        const int own = incl;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        __syncthreads(); // the list and the counts of the chunk before have been read
+        if (lane == 31) warp_cnt[wid] = incl;
+        __syncthreads();
+        int pos = incl - own, total = 0;
+#pragma unroll
+        for (int k = 0; k < kGatherThreads / 32; ++k) {
+            const int q = warp_cnt[k];
+            if (k < wid) pos += q;
+            total += q;
+        }
+        for (; word; word &= word - 1u) list[pos++] = (w0 + tid) * 32 + __ffs(word) - 1;
+        if (tid < 4) list[total + tid] = 0; // padding: row 0, not added
+        __syncthreads();
+        for (int k0 = 0; k0 < total; k0 += kGatherRows) {
+            float2 x[kGatherRows];
+#pragma unroll
+            for (int g = 0; g < kGatherRows; g += 4)
+                if (k0 + g < total) {
+                    const int4 q = *reinterpret_cast<const int4 *>(list + k0 + g);
+                    x[g] = __ldg(reinterpret_cast<const float2 *>(col + (size_t)q.x * n));
+                    x[g + 1] = __ldg(reinterpret_cast<const float2 *>(col + (size_t)q.y * n));
+                    x[g + 2] = __ldg(reinterpret_cast<const float2 *>(col + (size_t)q.z * n));
+                    x[g + 3] = __ldg(reinterpret_cast<const float2 *>(col + (size_t)q.w * n));
+                }
+#pragma unroll
+            for (int g = 0; g < kGatherRows; ++g)
+                if (k0 + g < total) {
+                    sum.x = sum.x + x[g].x;
+                    sum.y = sum.y + x[g].y;
+                }
+        }
+    }
+    if constexpr (!kLif) {
+        if (has) *reinterpret_cast<float2 *>(cur + at) = sum;
+    } else {
+        bool s0 = false, s1 = false;
+        if (has) {
+            s0 = lif_apply(P, sum.x, vv.x, ls.x, t, (int)at);
+            s1 = lif_apply(P, sum.y, vv.y, ls.y, t, (int)at + 1);
+            *reinterpret_cast<float2 *>(v + at) = vv;
+            *reinterpret_cast<int2 *>(last + at) = ls;
+        }
+        const unsigned even = __ballot_sync(0xffffffffu, s0), odd = __ballot_sync(0xffffffffu, s1);
+        if (has && (lane & 15) == 0) // a word is sixteen lanes' pairs
+            bits_out[at >> 5] = spread16(even >> lane & 0xffffu) | spread16(odd >> lane & 0xffffu) << 1;
+        if (lane == 0 && (even | odd)) atomicAdd(counts, __popc(even) + __popc(odd));
+    }
+}
+
 __global__ void __launch_bounds__(256) k_dense_lif(LifParams P, const float *__restrict__ partial, int nparts,
                                                    float *__restrict__ v, int *__restrict__ last,
-                                                   __nv_bfloat16 *__restrict__ s_out, int s_blocked_layout,
-                                                   unsigned *__restrict__ bits_out, int *__restrict__ counts, int t,
-                                                   int n, int total) {
+                                                   __nv_bfloat16 *__restrict__ s_out, int *__restrict__ counts, int t,
+                                                   int total) {
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     bool spk = false;
     if (idx < total) {
@@ -282,17 +368,10 @@ __global__ void __launch_bounds__(256) k_dense_lif(LifParams P, const float *__r
         spk = lif_apply(P, a, vv, ls, t, idx);
         v[idx] = vv;
         last[idx] = ls;
-        if (s_out) {
-            const __nv_bfloat16 one = __float2bfloat16_rn(spk ? 1.0f : 0.0f);
-            if (s_blocked_layout) s_out[s_blocked(idx / n, idx % n)] = one;
-            else s_out[idx] = one;
-        }
+        s_out[idx] = __float2bfloat16_rn(spk ? 1.0f : 0.0f);
     }
     const unsigned bal = __ballot_sync(0xffffffffu, spk);
-    if ((threadIdx.x & 31) == 0) {
-        if (bits_out && idx < total) bits_out[idx >> 5] = bal; // n % 32 == 0: a warp is one word
-        if (bal) atomicAdd(&counts[0], __popc(bal));
-    }
+    if ((threadIdx.x & 31) == 0 && bal) atomicAdd(&counts[0], __popc(bal));
 }
 
 // The step's neuron update fused into the tcgen05 delivery: the same update
@@ -362,23 +441,21 @@ nbg_status dense_reset(nbg_dense *d) {
     return NBG_OK;
 }
 
-// delivery of S (buffer `par`) into d->partial (parts, instance-major)
-nbg_status launch_delivery(nbg_dense *d, int par) {
-    if (d->precision == NBG_DENSE_SPLIT_BF16) {
-        dim3 grid(d->N / umma::kM, kSplitK);
-        umma::k_dense_umma<umma::NoFinish><<<grid, umma::kThreads, umma::kSmemBytes, d->stream>>>(
-            d->whi.p, d->wlo.p, d->s[par].p, d->partial.p, d->N, kSplitK, 0, d->err.p, d->tile_cnt.p,
-            umma::NoFinish{});
-    } else if (d->precision == NBG_DENSE_SPLIT_BF16_SYNC) {
-        dim3 grid(d->N / kBM, kSplitK);
-        k_dense_gemm<<<grid, kGemmThreads, kGemmSmem, d->stream>>>(d->whi.p, d->wlo.p, d->s[par].p, d->partial.p,
-                                                                   d->N);
-    } else {
-        dim3 grid(d->N / 256, d->B);
-        k_dense_fp32<<<grid, 256, (d->N / 32) * sizeof(unsigned), d->stream>>>(d->w.p, d->bits[par].p,
-                                                                                d->partial.p, d->N);
-    }
-    return NBG_OK;
+dim3 gather_grid(const nbg_dense *d) { return dim3(d->B, (d->N + kGatherCols - 1) / kGatherCols); }
+
+// A step's launch configuration, overlapping the step before (programmatic
+// dependent launch).
+cudaLaunchConfig_t step_config(const nbg_dense *d, dim3 grid, int threads, size_t smem, cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = d->stream;
+    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr->val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
 }
 
 } // namespace
@@ -508,48 +585,47 @@ nbg_status nbg_dense_run(nbg_dense *d, int steps) {
     DevBuf<int> dcnt;
     NBG_CUDA(dcnt.alloc((size_t)count));
     NBG_CUDA(cudaMemsetAsync(dcnt.p, 0, count * sizeof(int), d->stream));
-    // event pairs bracketing every delivery launch (reused across calls)
+    // event pairs bracketing every delivery launch of the two-launch path (reused across calls)
+    const bool sync_path = d->precision == NBG_DENSE_SPLIT_BF16_SYNC;
     const int chunk = 256;
-    while ((int)d->dev_pool.size() < 2 * chunk) {
+    while (sync_path && (int)d->dev_pool.size() < 2 * chunk) {
         cudaEvent_t ev;
         NBG_CUDA(cudaEventCreate(&ev));
         d->dev_pool.push_back(ev);
     }
     double dms = 0.0;
     NBG_CUDA(cudaEventRecord(d->ev0, d->stream));
-    const bool tensor = d->precision != NBG_DENSE_FP32;
-    const int blocked = d->precision == NBG_DENSE_SPLIT_BF16;
+    cudaLaunchAttribute attr[1];
     for (int k0 = 0; k0 < count; k0 += chunk) {
         const int k1 = std::min(count, k0 + chunk);
         for (int k = k0; k < k1; ++k) {
             const int t = d->next_t + k;
             const int in = (t + 1) & 1, outp = t & 1; // S_{t-1} lives in buffer (t-1)&1
-            if (blocked) { // tcgen05: delivery and update in one launch, back to back (PDL)
+            if (d->precision == NBG_DENSE_SPLIT_BF16) { // tcgen05: delivery and update in one launch
                 const LifFinish fin{d->P, d->v.p, d->last.p, d->s[outp].p, dcnt.p + k, t};
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3(d->N / umma::kM, kSplitK);
-                cfg.blockDim = dim3(umma::kThreads);
-                cfg.dynamicSmemBytes = umma::kSmemBytes;
-                cfg.stream = d->stream;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                attr[0].val.programmaticStreamSerializationAllowed = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
+                const cudaLaunchConfig_t cfg =
+                    step_config(d, dim3(d->N / umma::kM, kSplitK), umma::kThreads, umma::kSmemBytes, attr);
                 NBG_CUDA(cudaLaunchKernelEx(&cfg, umma::k_dense_umma<LifFinish>, (const __nv_bfloat16 *)d->whi.p,
                                             (const __nv_bfloat16 *)d->wlo.p, (const __nv_bfloat16 *)d->s[in].p,
                                             d->partial.p, d->N, (int)kSplitK, t & 1, d->err.p, d->tile_cnt.p, fin));
                 continue;
             }
+            if (d->precision == NBG_DENSE_FP32) { // gather and update in one launch
+                const cudaLaunchConfig_t cfg = step_config(d, gather_grid(d), kGatherThreads, 0, attr);
+                NBG_CUDA(cudaLaunchKernelEx(&cfg, k_dense_gather<true>, (const float *)d->w.p,
+                                            (const unsigned *)d->bits[in].p, (float *)nullptr, d->P, d->v.p, d->last.p,
+                                            d->bits[outp].p, dcnt.p + k, t, d->N));
+                continue;
+            }
             NBG_CUDA(cudaEventRecord(d->dev_pool[2 * (k - k0)], d->stream));
-            launch_delivery(d, in);
+            k_dense_gemm<<<dim3(d->N / kBM, kSplitK), kGemmThreads, kGemmSmem, d->stream>>>(d->whi.p, d->wlo.p, d->s[in].p,
+                                                                                          d->partial.p, d->N);
             NBG_CUDA(cudaEventRecord(d->dev_pool[2 * (k - k0) + 1], d->stream));
-            k_dense_lif<<<(total + 255) / 256, 256, 0, d->stream>>>(
-                d->P, d->partial.p, tensor ? kSplitK : 1, d->v.p, d->last.p, tensor ? d->s[outp].p : nullptr, blocked,
-                tensor ? nullptr : d->bits[outp].p, dcnt.p + k, t, d->N, total);
+            k_dense_lif<<<(total + 255) / 256, 256, 0, d->stream>>>(d->P, d->partial.p, kSplitK, d->v.p, d->last.p,
+                                                                    d->s[outp].p, dcnt.p + k, t, total);
         }
         NBG_CUDA(cudaGetLastError());
-        if (blocked) continue; // one launch per step, no per-step events (they would break the overlap)
+        if (!sync_path) continue; // one launch per step, no per-step events (they would break the overlap)
         NBG_CUDA(cudaEventSynchronize(d->dev_pool[2 * (k1 - 1 - k0) + 1]));
         for (int k = k0; k < k1; ++k) {
             float x = 0.0f;
@@ -562,8 +638,8 @@ nbg_status nbg_dense_run(nbg_dense *d, int steps) {
     float ms = 0.0f;
     NBG_CUDA(cudaEventElapsedTime(&ms, d->ev0, d->ev1));
     d->last_ms = ms;
-    d->last_delivery_ms = blocked ? ms : dms; // tcgen05: the whole step is the delivery launch
-    d->last_launches = (blocked ? 1LL : 2LL) * count;
+    d->last_delivery_ms = sync_path ? dms : ms; // else the whole step is the delivery launch
+    d->last_launches = (sync_path ? 2LL : 1LL) * count;
     NBG_CUDA(cudaMemcpy(cnt.data(), dcnt.p, count * sizeof(int), cudaMemcpyDeviceToHost));
     int errv = 0;
     NBG_CUDA(cudaMemcpy(&errv, d->err.p, sizeof(int), cudaMemcpyDeviceToHost));
@@ -653,8 +729,8 @@ nbg_status nbg_dense_deliver(nbg_dense *d, const uint8_t *s, float *out) {
         for (size_t i = 0; i < tot; ++i)
             if (s[i]) h[i >> 5] |= 1u << (i & 31);
         NBG_CUDA(bb.upload(h));
-        dim3 grid(d->N / 256, d->B);
-        k_dense_fp32<<<grid, 256, (d->N / 32) * sizeof(unsigned), d->stream>>>(d->w.p, bb.p, part.p, d->N);
+        k_dense_gather<false><<<gather_grid(d), kGatherThreads, 0, d->stream>>>(d->w.p, bb.p, part.p, d->P, nullptr,
+                                                                                nullptr, nullptr, nullptr, 0, d->N);
     }
     NBG_CUDA(cudaGetLastError());
     NBG_CUDA(cudaStreamSynchronize(d->stream));
