@@ -116,6 +116,18 @@ struct alignas(8) SynStatic {
     unsigned int meta;
 };
 
+// Static networks seldom have more than a few weights (one per projection).
+// With at most kPaletteSize different (weight, type) pairs, the palette, each
+// synapse has a two-bit code, kept as two bit planes per mask word: the codes
+// of the word's 32 synapses are one 8-byte value beside the arrival bits, and
+// an arrival takes its weight from registers instead of an 8-byte record at a
+// place of its own in memory (k_update_quad).
+constexpr int kPaletteSize = 4;
+struct Palette {
+    float w[kPaletteSize];
+    unsigned int types; // bit c: the synapse type of entry c
+};
+
 struct NetDev {
     int N, D, Wt, n_layers, semantics;
     float dt;
@@ -129,11 +141,15 @@ struct NetDev {
     // ones); exactly one of the two is set
     SynRec *rec;
     SynStatic *wst;
+    // palette networks: per mask word the code planes of its synapses
+    const uint2 *code;
+    const Palette *palette;
     const float2 *dtab; // [rule][dtab_len] {LTP factor, LTD factor} per step gap
     int dtab_len;
     int sdtab_len; // entries of rule 0's table copied into shared memory per CTA (0: none)
     unsigned int *mask;
-    unsigned int *wsum; // per slot: one bit per mask word, set while that word is non-zero
+    unsigned int *wsum; // per slot: one bit per mask word, set while that word is non-zero (null: k_update_quad
+                        // runs, which reads every word)
     int Ws;             // summary words per slot (ceil(Wt / 32) + 1 padding word)
     const int *out_ptr;
     // out lists (CSR by source): packed (mask bit << out_dbits | delay -
@@ -770,7 +786,24 @@ __device__ __forceinline__ void mark_out(const NetDev &n, int q, int q1, unsigne
         const unsigned int slot = (t + dl) % (unsigned int)n.D;
         const unsigned int wd = bit >> 5;
         atomicOr(&n.mask[(size_t)slot * n.Wt + wd], 1u << (bit & 31u));
-        atomicOr(&n.wsum[(size_t)slot * n.Ws + (wd >> 5)], 1u << (wd & 31u));
+        if (n.wsum) atomicOr(&n.wsum[(size_t)slot * n.Ws + (wd >> 5)], 1u << (wd & 31u));
+    }
+}
+
+// External spikes of the block's steps (InputSpike::ProcessEvent): one warp
+// per spike marks its out-synapses like a spike of the update (their arrivals
+// fall after this block, so marking first is safe); the raster entries are
+// added on the host, which holds the list.
+__device__ __forceinline__ void mark_external(const NetDev &n, int tid, int lane, int B, int T0, int toff) {
+    if (!n.ext_ptr) return;
+    const int e0 = n.ext_ptr[toff], e1 = n.ext_ptr[toff + B];
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    for (int g = tid >> 5; g < e1 - e0; g += nwarps) {
+        const int x = e0 + g;
+        int b = 0;
+        while (b + 1 < B && n.ext_ptr[toff + b + 1] <= x) ++b;
+        const int src = n.ext_ids[x];
+        mark_out(n, n.out_ptr[src] + lane, n.out_ptr[src + 1], (unsigned int)(T0 + b));
     }
 }
 
@@ -833,6 +866,94 @@ __device__ __forceinline__ void generator_steps(const NetDev &n, int g, int B, i
         }
 }
 
+// The block's spikes leave the warp after its last step: nothing in this
+// launch reads their marks (arrivals fall at or after T0 + B, and the ring
+// never aliases this block's slots), so the loads they need overlap with
+// other warps' steps instead of stalling every step.  Every lane of the warp
+// calls this; j is only used where spk_steps (bit b: neuron j spiked at step
+// T0 + b) is not zero.
+__device__ __forceinline__ void leave_warp(const NetDev &n, int j, int lane, bool record, unsigned int spk_steps, int T0,
+                                           unsigned int slot0, unsigned long long delivered) {
+    const unsigned int D = (unsigned int)n.D;
+    // Raster: output-layer spikes, one cursor reservation per warp; the
+    // reservation is requested here and its result used after the
+    // propagation, so that its round trip overlaps the marks.
+    const int nrec = record ? __popc(spk_steps) : 0;
+    int rincl = nrec;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, rincl, o);
+        if (lane >= o) rincl += y;
+    }
+    const int rtotal = __shfl_sync(0xffffffffu, rincl, 31);
+    unsigned int rpos = 0;
+    if (rtotal > 0 && lane == 31) rpos = atomicAdd(n.cursor, (unsigned int)rtotal);
+    // Propagation: the out-lists of all the warp's spiking lanes form one
+    // range that the 32 lanes stride over together (entry e belongs to the
+    // first lane whose inclusive prefix of list lengths exceeds e).  The
+    // list bounds of every spiking lane come in one round trip, and the
+    // entry loads of four rounds are issued before their marks.  Each
+    // synapse is loaded once and marked for every step its source spiked in.
+    {
+        int q0 = 0, cnt = 0;
+        if (spk_steps) {
+            q0 = n.out_ptr[j];
+            cnt = n.out_ptr[j + 1] - q0;
+        }
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        constexpr int kRounds = 4;
+        for (int e0 = 0; e0 < total; e0 += 32 * kRounds) {
+            unsigned int bit[kRounds], dl[kRounds], steps[kRounds];
+#pragma unroll
+            for (int k = 0; k < kRounds; ++k) {
+                const int e = e0 + 32 * k + lane;
+                int owner = 0; // first lane with incl > e (binary search over the warp's prefix)
+#pragma unroll
+                for (int w = 16; w > 0; w >>= 1) {
+                    const int c = __shfl_sync(0xffffffffu, incl, owner + w - 1);
+                    if (c <= e) owner += w;
+                }
+                const int oq = __shfl_sync(0xffffffffu, q0, owner & 31);
+                const int oe = __shfl_sync(0xffffffffu, incl - cnt, owner & 31);
+                steps[k] = __shfl_sync(0xffffffffu, spk_steps, owner & 31);
+                bit[k] = dl[k] = 0u;
+                if (e < total) out_entry(n, oq + (e - oe), bit[k], dl[k]);
+                else steps[k] = 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < kRounds; ++k) {
+                const unsigned int wd = bit[k] >> 5;
+                for (unsigned int m = steps[k]; m; m &= m - 1u) {
+                    const unsigned int slot = wrap_slot(slot0 + (unsigned int)(__ffs(m) - 1) + dl[k], D);
+                    atomicOr(&n.mask[(size_t)slot * n.Wt + wd], 1u << (bit[k] & 31u));
+                    if (n.wsum) atomicOr(&n.wsum[(size_t)slot * n.Ws + (wd >> 5)], 1u << (wd & 31u));
+                }
+            }
+        }
+    }
+    if (rtotal > 0) {
+        unsigned int pos = __shfl_sync(0xffffffffu, rpos, 31) + (unsigned int)(rincl - nrec);
+        if (nrec > 0) {
+            if (pos + (unsigned int)nrec <= (unsigned int)n.out_cap) {
+                for (unsigned int m = spk_steps; m; m &= m - 1u, ++pos) {
+                    n.out_ids[pos] = j;
+                    n.out_t[pos] = T0 + __ffs(m) - 1;
+                }
+            } else {
+                atomicOr(n.err, kErrOverflow);
+            }
+        }
+    }
+    // warp-aggregated delivered-event count
+    for (int o = 16; o > 0; o >>= 1) delivered += __shfl_down_sync(0xffffffffu, delivered, o);
+    if (lane == 0 && delivered) atomicAdd(n.n_events, delivered);
+}
+
 // One block of B steps starting toff steps after the run call's first step.
 template <class S>
 __global__ void __launch_bounds__(256, S::min_blocks) k_update(const __grid_constant__ NetDev n, int B, int toff) {
@@ -880,21 +1001,7 @@ __global__ void __launch_bounds__(256, S::min_blocks) k_update(const __grid_cons
     }
     // everything below reads or writes what the previous block's launch wrote
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    // external spikes of the block's steps (InputSpike::ProcessEvent): one
-    // warp per spike marks its out-synapses like a spike of the update (their
-    // arrivals fall after this block, so marking first is safe); the raster
-    // entries are added on the host, which holds the list
-    if (n.ext_ptr) {
-        const int e0 = n.ext_ptr[toff], e1 = n.ext_ptr[toff + B];
-        const int nwarps = (gridDim.x * blockDim.x) >> 5;
-        for (int g = tid >> 5; g < e1 - e0; g += nwarps) {
-            const int x = e0 + g;
-            int b = 0;
-            while (b + 1 < B && n.ext_ptr[toff + b + 1] <= x) ++b;
-            const int src = n.ext_ids[x];
-            mark_out(n, n.out_ptr[src] + lane, n.out_ptr[src + 1], (unsigned int)(T0 + b));
-        }
-    }
+    mark_external(n, tid, lane, B, T0, toff);
     if (gen_block) { // whole CTAs of generator threads
         generator_steps(n, tid - reg_blocks * (int)blockDim.x, B, T0, run_t0, lane);
         return;
@@ -1139,87 +1246,193 @@ __global__ void __launch_bounds__(256, S::min_blocks) k_update(const __grid_cons
         n.ginh[j] = r.ginh;
         n.last[j] = r.last;
     }
-    // The block's spikes leave the warp after its last step: nothing in this
-    // launch reads their marks (arrivals fall at or after T0 + B, and the
-    // ring never aliases this block's slots), so the loads they need overlap
-    // with other warps' steps instead of stalling every step.
-    // Raster: output-layer spikes, one cursor reservation per warp; the
-    // reservation is requested here and its result used after the
-    // propagation, so that its round trip overlaps the marks.
-    const int nrec = (active && L.record) ? __popc(spk_steps) : 0;
-    int rincl = nrec;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, rincl, o);
-        if (lane >= o) rincl += y;
-    }
-    const int rtotal = __shfl_sync(0xffffffffu, rincl, 31);
-    unsigned int rpos = 0;
-    if (rtotal > 0 && lane == 31) rpos = atomicAdd(n.cursor, (unsigned int)rtotal);
-    // Propagation: the out-lists of all the warp's spiking lanes form one
-    // range that the 32 lanes stride over together (entry e belongs to the
-    // first lane whose inclusive prefix of list lengths exceeds e).  The
-    // list bounds of every spiking lane come in one round trip, and the
-    // entry loads of four rounds are issued before their marks.  Each
-    // synapse is loaded once and marked for every step its source spiked in.
-    {
-        int q0 = 0, cnt = 0;
-        if (spk_steps) {
-            q0 = n.out_ptr[j];
-            cnt = n.out_ptr[j + 1] - q0;
+    leave_warp(n, j, lane, active && L.record, spk_steps, T0, slot0, delivered);
+}
+
+// ------------------------------------------------------ palette networks
+//
+// k_update for static networks whose synapses have palette codes: the same
+// steps, neuron updates and propagation, with another drain.
+//
+// What bounds it: a warp's own chain of instructions.  At about 2.2 arrivals
+// per neuron and step some lane of a warp has an arrival in every mask word at
+// every step, and the record drain of k_update spent about 840 instructions a
+// warp and step (1,000 neurons; 39 us per launch of 15 steps at any CTA size)
+// on finding words, generator bits and records lane by lane.  Here:
+//   * a neuron's mask words come in groups of four (a quad, 16 bytes, padded
+//     with words no synapse has): one asynchronous copy two steps ahead brings
+//     the quad, one store clears it, and there is no word summary to read, to
+//     clear or to set, which also halves the marks of a spike;
+//   * the codes of the first quad and the palette stay in registers, so a set
+//     bit costs its isolation, two tests, selects and one addition;
+//   * the four words are run through by the whole warp one after another, each
+//     until its fullest lane is done, in ascending order as before.
+// Measured per launch of 15 steps: 1,000 neurons 48.8 -> 25.6 us; 16 networks of
+// 500 to 50,000 neurons (172,000 in all) 113 (record drain with codes) -> 74.5
+// us.
+template <class S>
+__device__ __forceinline__ void apply_quad_word(unsigned int word, uint2 code, const float (&sw)[kPaletteSize],
+                                                unsigned int types, bool split, float &a, float &b) {
+    if (!split) { // a += the weight with its type's sign
+        while (word) {
+            const unsigned int m = word & (0u - word);
+            word ^= m;
+            const bool c0 = code.x & m, c1 = code.y & m;
+            a = a + (c1 ? (c0 ? sw[3] : sw[2]) : (c0 ? sw[1] : sw[0]));
         }
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const int total = __shfl_sync(0xffffffffu, incl, 31);
-        constexpr int kRounds = 4;
-        for (int e0 = 0; e0 < total; e0 += 32 * kRounds) {
-            unsigned int bit[kRounds], dl[kRounds], steps[kRounds];
-#pragma unroll
-            for (int k = 0; k < kRounds; ++k) {
-                const int e = e0 + 32 * k + lane;
-                int owner = 0; // first lane with incl > e (binary search over the warp's prefix)
-#pragma unroll
-                for (int w = 16; w > 0; w >>= 1) {
-                    const int c = __shfl_sync(0xffffffffu, incl, owner + w - 1);
-                    if (c <= e) owner += w;
-                }
-                const int oq = __shfl_sync(0xffffffffu, q0, owner & 31);
-                const int oe = __shfl_sync(0xffffffffu, incl - cnt, owner & 31);
-                steps[k] = __shfl_sync(0xffffffffu, spk_steps, owner & 31);
-                bit[k] = dl[k] = 0u;
-                if (e < total) out_entry(n, oq + (e - oe), bit[k], dl[k]);
-                else steps[k] = 0u;
-            }
-#pragma unroll
-            for (int k = 0; k < kRounds; ++k) {
-                const unsigned int wd = bit[k] >> 5;
-                for (unsigned int m = steps[k]; m; m &= m - 1u) {
-                    const unsigned int slot = wrap_slot(slot0 + (unsigned int)(__ffs(m) - 1) + dl[k], D);
-                    atomicOr(&n.mask[(size_t)slot * n.Wt + wd], 1u << (bit[k] & 31u));
-                    atomicOr(&n.wsum[(size_t)slot * n.Ws + (wd >> 5)], 1u << (wd & 31u));
-                }
-            }
+    } else { // dense-runtime LIF: one sum per type
+        while (word) {
+            const unsigned int m = word & (0u - word);
+            word ^= m;
+            const unsigned int c = (code.x & m ? 1u : 0u) | (code.y & m ? 2u : 0u);
+            const float w = c & 2u ? (c & 1u ? sw[3] : sw[2]) : (c & 1u ? sw[1] : sw[0]);
+            if (types >> c & 1u) b = b + -w;
+            else a = a + w;
         }
     }
-    if (rtotal > 0) {
-        unsigned int pos = __shfl_sync(0xffffffffu, rpos, 31) + (unsigned int)(rincl - nrec);
-        if (nrec > 0) {
-            if (pos + (unsigned int)nrec <= (unsigned int)n.out_cap) {
-                for (unsigned int m = spk_steps; m; m &= m - 1u, ++pos) {
-                    n.out_ids[pos] = j;
-                    n.out_t[pos] = T0 + __ffs(m) - 1;
-                }
-            } else {
-                atomicOr(n.err, kErrOverflow);
-            }
+}
+
+template <class S>
+__global__ void __launch_bounds__(256, 4) k_update_quad(const __grid_constant__ NetDev n, int B, int toff) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int reg_blocks = (n.N_upd + (int)blockDim.x - 1) / (int)blockDim.x;
+    const bool gen_block = (int)blockIdx.x >= reg_blocks;
+    const bool active = !gen_block && tid < n.N_upd;
+    const int j = active && n.upd_ids ? n.upd_ids[tid] : tid;
+    const int lane = threadIdx.x & 31;
+    const int run_t0 = *n.run_t0;
+    const int T0 = run_t0 + toff;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // as in k_update
+
+    Model L;
+    NeuronRegs r;
+    int woff = 0, nq = 0, tslot = -1, g0 = 0, g1 = 0;
+    uint2 code[4] = {};
+    if (active) {
+        L = load_model(n.layers[n.pop[j]]);
+        woff = n.woff[j];
+        nq = (n.woff[j + 1] - woff) >> 2;
+        if (n.trace_slot) tslot = n.trace_slot[j];
+        g0 = n.gen_ptr[j];
+        g1 = n.gen_ptr[j + 1];
+        if (nq > 0) {
+            const uint4 a = reinterpret_cast<const uint4 *>(n.code + woff)[0];
+            const uint4 b = reinterpret_cast<const uint4 *>(n.code + woff)[1];
+            code[0] = make_uint2(a.x, a.y);
+            code[1] = make_uint2(a.z, a.w);
+            code[2] = make_uint2(b.x, b.y);
+            code[3] = make_uint2(b.z, b.w);
         }
     }
-    // warp-aggregated delivered-event count
-    for (int o = 16; o > 0; o >>= 1) delivered += __shfl_down_sync(0xffffffffu, delivered, o);
-    if (lane == 0 && delivered) atomicAdd(n.n_events, delivered);
+    const Palette pal = *n.palette;
+    float sw[kPaletteSize]; // weights with the sign of their type
+#pragma unroll
+    for (int c = 0; c < kPaletteSize; ++c) sw[c] = (pal.types >> c) & 1u ? -pal.w[c] : pal.w[c];
+    // the first generator input: local hash index, delay, rank and probability
+    int gen_local = 0, gen_delay = 0, gen_pos = 0;
+    float gen_prob = -1.0f; // never fires
+    if (active && g0 < g1) {
+        gen_prob = generator_prob(n, n.gen_src[g0], &gen_local);
+        gen_delay = n.gen_delay[g0];
+        gen_pos = n.gen_pos[g0];
+    }
+    // everything below reads or writes what the previous block's launch wrote
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    mark_external(n, tid, lane, B, T0, toff);
+    if (gen_block) { // whole CTAs of generator threads
+        generator_steps(n, tid - reg_blocks * (int)blockDim.x, B, T0, run_t0, lane);
+        return;
+    }
+    if (active) {
+        r.v = n.v[j];
+        r.u = r.gexc = r.ginh = 0.0f; // no LIF or Poisson neuron has them
+        r.iext = n.iext[j];
+        r.last = n.last[j];
+        r.lif_cur = 0.0f;
+        if (L.model == NBG_MODEL_LIF_VJ) // current_dV += R * I / tau (two roundings)
+            r.lif_cur = r.lif_cur + L.p[3] * r.iext / L.p[1];
+    }
+    const unsigned int D = (unsigned int)n.D;
+    const unsigned int slot0 = (unsigned int)T0 % D; // the block's first slot; later ones by wrap_slot
+    // quads in flight: [step % 4][thread], read by the thread that asked for them
+    __shared__ uint4 s_quad[4][256];
+    const bool staged = active && nq > 0;
+    auto row = [&](int b) { return n.mask + (size_t)wrap_slot(slot0 + (unsigned int)b, D) * n.Wt + woff; };
+    auto stage = [&](int b) {
+        if (staged && b < B)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                             (unsigned int)__cvta_generic_to_shared(&s_quad[b & 3][threadIdx.x])),
+                         "l"(__cvta_generic_to_global(row(b)))
+                         : "memory");
+        stage_commit();
+    };
+    stage(0);
+    stage(1);
+    const bool lif = S::model(L.model) == NBG_MODEL_LIF_VJ;
+    const bool split = lif && n.semantics == NBG_SEM_DENSE; // one sum per synapse type
+    const bool jump = lif && !split;                        // arrivals move v unless the neuron is refractory
+    unsigned int delivered = 0, spk_steps = 0u;             // bit b: this neuron spiked at step T0 + b
+    for (int b = 0; b < B; ++b) {
+        const int t = T0 + b;
+        asm volatile("cp.async.wait_group 1;" ::: "memory"); // this step's quad
+        if (active) {
+            uint4 q = make_uint4(0u, 0u, 0u, 0u);
+            if (staged) {
+                q = s_quad[b & 3][threadIdx.x];
+                if (q.x | q.y | q.z | q.w) *reinterpret_cast<uint4 *>(row(b)) = make_uint4(0u, 0u, 0u, 0u);
+            }
+            unsigned int w[4] = {q.x, q.y, q.z, q.w};
+            // generator arrivals (pure functions of source and time)
+            const bool fired = t >= gen_delay && hash_uniform01(gen_local, t - gen_delay) < gen_prob;
+            const unsigned int gbit = fired ? 1u << (gen_pos & 31) : 0u;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) w[k] |= (gen_pos >> 5) == k ? gbit : 0u;
+            for (int g = g0 + 1; g < g1; ++g) // further generator inputs
+                if (n.gen_pos[g] < 128 && generator_fired(n, n.gen_src[g], t - (int)n.gen_delay[g])) {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) w[k] |= (n.gen_pos[g] >> 5) == k ? 1u << (n.gen_pos[g] & 31) : 0u;
+                }
+            const bool take = !jump || r.last > L.ip;
+            float a = jump ? r.v : 0.0f, c = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                delivered += __popc(w[k]);
+                apply_quad_word<S>(take ? w[k] : 0u, code[k], sw, pal.types, split, a, c);
+            }
+            for (int x = 1; x < nq; ++x) { // in-degrees above 128
+                unsigned int *const mrow = row(b) + 4 * x;
+                const uint4 e = *reinterpret_cast<const uint4 *>(mrow);
+                if (e.x | e.y | e.z | e.w) *reinterpret_cast<uint4 *>(mrow) = make_uint4(0u, 0u, 0u, 0u);
+                unsigned int we[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    we[k] |= (gen_pos >> 5) == 4 * x + k ? gbit : 0u;
+                    for (int g = g0 + 1; g < g1; ++g)
+                        if ((n.gen_pos[g] >> 5) == 4 * x + k &&
+                            generator_fired(n, n.gen_src[g], t - (int)n.gen_delay[g]))
+                            we[k] |= 1u << (n.gen_pos[g] & 31);
+                    delivered += __popc(we[k]);
+                    if (take && we[k])
+                        apply_quad_word<S>(we[k], n.code[woff + 4 * x + k], sw, pal.types, split, a, c);
+                }
+            }
+            if (jump) r.v = a;
+            const bool spk = update_neuron<S>(n, L, r, a, c, 0.0f, j, t);
+            if (tslot >= 0) n.trace[(size_t)(t - run_t0) * n.ntrace + tslot] = r.v;
+            if (spk) {
+                if (!spk_steps) // the out-list bounds the propagation reads after the last step
+                    asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(n.out_ptr + j)));
+                spk_steps |= 1u << b;
+            }
+        }
+        stage(b + 2);
+    }
+    if (active) {
+        n.v[j] = r.v;
+        n.last[j] = r.last;
+    }
+    __syncwarp();
+    leave_warp(n, j, lane, active && L.record, spk_steps, T0, slot0, delivered);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1292,6 +1505,16 @@ struct nbg_engine {
     DevBuf<LayerDev> d_layers;
     DevBuf<SynRec> rec;    // plastic network: synapse records
     DevBuf<SynStatic> wst; // static network: weight + meta
+    // palette: code planes per mask word; the update kernel is plain_kernel or,
+    // while the palette holds every weight, palette_kernel (null: the profile
+    // has none, or the network none)
+    DevBuf<uint2> code;
+    DevBuf<Palette> palette;
+    Palette palette_host{};
+    int palette_n = 0;                    // entries in use (0: plain_kernel runs)
+    std::vector<unsigned char> type_bits; // palette networks: synapse types, CSC order, one bit each
+    void (*plain_kernel)(NetDev, int, int) = nullptr;
+    void (*palette_kernel)(NetDev, int, int) = nullptr;
     DevBuf<float> init_w_d; // weights reset returns to, CSC order
     DevBuf<float> v, u, gexc, ginh, iext, trace, ev_w;
     DevBuf<float2> dtab;
@@ -1346,6 +1569,7 @@ struct nbg_engine {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t graph = nullptr;
     int graph_blocks = 0, graph_tail = 0, graph_B = 0, graph_threads = 0;
+    void (*graph_kernel)(NetDev, int, int) = nullptr;
     NetDev graph_nd{}; // kernel arguments baked into the graph
     double last_ms = 0.0, last_upd_ms = 0.0, last_prop_ms = 0.0;
     int64_t last_launches = 0;
@@ -1374,11 +1598,13 @@ struct nbg_engine {
         n.woff = woff.p;
         n.rec = rec.p;
         n.wst = wst.p;
+        n.code = code.p;
+        n.palette = palette.p;
         n.dtab = dtab.p;
         n.dtab_len = dtab_len;
         n.sdtab_len = plastic && n_rules > 0 ? std::min(dtab_len, kSharedDecayEntries) : 0;
         n.mask = mask.p;
-        n.wsum = wsum.p;
+        n.wsum = palette_n > 0 ? nullptr : wsum.p;
         n.Ws = Ws;
         n.out_ptr = out_ptr.p;
         n.out_pk = out_pk.p;
@@ -1519,6 +1745,128 @@ cudaError_t reset_synapses(nbg_engine *e, bool traces) {
                                                                        traces ? 1 : 0);
     const cudaError_t ce = cudaGetLastError();
     return ce != cudaSuccess ? ce : cudaStreamSynchronize(e->stream);
+}
+
+// The different (weight, type) pairs of S synapses into pal (free entries
+// repeat the first) and *used; false when there are more than kPaletteSize.
+template <class Type>
+bool collect_palette(const float *w, int64_t S, Type type, Palette &pal, int &used) {
+    pal = Palette{};
+    used = 0;
+    for (int64_t s = 0; s < S; ++s) {
+        const unsigned int ty = type(s);
+        int c = 0;
+        while (c < used && !(std::memcmp(&pal.w[c], &w[s], sizeof(float)) == 0 && ((pal.types >> c) & 1u) == ty)) ++c;
+        if (c < used) continue;
+        if (used == kPaletteSize) {
+            used = 0;
+            return false;
+        }
+        pal.w[used] = w[s];
+        pal.types |= ty << used;
+        ++used;
+    }
+    for (int c = used; c < kPaletteSize; ++c) { // no synapse gets their code
+        pal.w[c] = pal.w[0];
+        pal.types |= (pal.types & 1u) << c;
+    }
+    return true;
+}
+
+// The code planes of every mask word: one warp per neuron, one lane per synapse.
+__global__ void k_palette_codes(const SynStatic *__restrict__ wst, const int *__restrict__ csc_ptr,
+                                const int *__restrict__ woff, int N, const Palette *__restrict__ palette,
+                                uint2 *__restrict__ code) {
+    const int lane = threadIdx.x & 31;
+    const Palette pal = *palette;
+    for (int j = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < N; j += (int)((gridDim.x * blockDim.x) >> 5)) {
+        const int end = csc_ptr[j + 1];
+        int p = csc_ptr[j] + lane;
+        for (int x = woff[j]; x < woff[j + 1]; ++x, p += 32) { // padding words get code 0
+            unsigned int c = 0u;
+            if (p < end) {
+                const SynStatic y = wst[p];
+#pragma unroll
+                for (unsigned int k = kPaletteSize - 1; k > 0; --k)
+                    if (__float_as_uint(y.w) == __float_as_uint(pal.w[k]) && (y.meta & 1u) == ((pal.types >> k) & 1u)) c = k;
+                if (__float_as_uint(y.w) == __float_as_uint(pal.w[0]) && (y.meta & 1u) == (pal.types & 1u)) c = 0u;
+            }
+            const unsigned int lo = __ballot_sync(0xffffffffu, c & 1u), hi = __ballot_sync(0xffffffffu, c & 2u);
+            if (lane == 0) code[x] = make_uint2(lo, hi);
+        }
+    }
+}
+
+// Set the summary bit of every non-zero mask word (k_update_quad neither sets
+// nor reads them): one warp per 32 words.
+__global__ void k_summary_rebuild(const unsigned int *__restrict__ mask, unsigned int *__restrict__ wsum, int D, int Wt,
+                                  int Ws) {
+    const int lane = threadIdx.x & 31;
+    const long long rows = (long long)D * Ws;
+    for (long long x = (long long)(blockIdx.x * blockDim.x + threadIdx.x) >> 5; x < rows;
+         x += (gridDim.x * blockDim.x) >> 5) {
+        const int slot = (int)(x / Ws), w = (int)(x % Ws) * 32 + lane;
+        const unsigned int bits = __ballot_sync(0xffffffffu, w < Wt && mask[(size_t)slot * Wt + w] != 0u);
+        if (lane == 0) wsum[x] = bits;
+    }
+}
+
+// Run k_update_quad on palette_host (palette_n entries): codes from the
+// weights now in wst.  Synchronous.
+nbg_status use_palette(nbg_engine *e) {
+    if (!e->palette_kernel || e->palette_n == 0) return NBG_OK;
+    if (!e->palette.p) NBG_CUDA(e->palette.alloc(1));
+    if (e->code.n != (size_t)e->Wt) NBG_CUDA(e->code.alloc((size_t)e->Wt));
+    NBG_CUDA(cudaMemcpyAsync(e->palette.p, &e->palette_host, sizeof(Palette), cudaMemcpyHostToDevice, e->stream));
+    k_palette_codes<<<(unsigned)(4 * e->sm_count), 256, 0, e->stream>>>(e->wst.p, e->csc_ptr_d.p, e->woff.p, e->N,
+                                                                       e->palette.p, e->code.p);
+    NBG_CUDA(cudaGetLastError());
+    NBG_CUDA(cudaStreamSynchronize(e->stream));
+    e->update_kernel = e->palette_kernel;
+    return NBG_OK;
+}
+
+// Back to k_update, which reads the records: the arrivals pending in the ring
+// get their summary bits.
+nbg_status leave_palette(nbg_engine *e) {
+    if (e->palette_n == 0) return NBG_OK;
+    k_summary_rebuild<<<(unsigned)(8 * e->sm_count), 256, 0, e->stream>>>(e->mask.p, e->wsum.p, e->D, e->Wt, e->Ws);
+    NBG_CUDA(cudaGetLastError());
+    e->palette_n = 0;
+    e->update_kernel = e->plain_kernel;
+    return NBG_OK;
+}
+
+// The code of one synapse: bit `bit` of both planes of word `word`.
+__global__ void k_palette_patch(uint2 *code, unsigned int word, unsigned int bit, unsigned int c) {
+    uint2 q = code[word];
+    q.x = (q.x & ~(1u << bit)) | (c & 1u) << bit;
+    q.y = (q.y & ~(1u << bit)) | (c >> 1 & 1u) << bit;
+    code[word] = q;
+}
+
+// One weight was set (CSC position p): its code follows, in a free entry if
+// the weight is new; a weight that the full palette does not hold ends its use
+// until all weights are set again.
+nbg_status patch_palette(nbg_engine *e, int64_t p, float w) {
+    if (e->palette_n == 0) return NBG_OK;
+    const unsigned int type = (e->type_bits[(size_t)(p >> 3)] >> (p & 7)) & 1u;
+    Palette &pal = e->palette_host;
+    int c = 0;
+    while (c < e->palette_n && !(std::memcmp(&pal.w[c], &w, sizeof(float)) == 0 && ((pal.types >> c) & 1u) == type)) ++c;
+    if (c == kPaletteSize) return leave_palette(e);
+    if (c == e->palette_n) {
+        pal.w[c] = w;
+        pal.types = (pal.types & ~(1u << c)) | type << c;
+        NBG_CUDA(cudaMemcpy(e->palette.p, &pal, sizeof(pal), cudaMemcpyHostToDevice));
+        e->palette_n = c + 1;
+    }
+    const int j = (int)(std::upper_bound(e->csc_ptr.begin(), e->csc_ptr.end(), (int)p) - e->csc_ptr.begin()) - 1;
+    const int k = (int)p - e->csc_ptr[(size_t)j];
+    k_palette_patch<<<1, 1, 0, e->stream>>>(e->code.p, (unsigned)(e->woff_host[(size_t)j] + (k >> 5)), (unsigned)(k & 31),
+                                            (unsigned)c);
+    NBG_CUDA(cudaGetLastError());
+    return NBG_OK;
 }
 
 nbg_status upload_layers(nbg_engine *e) {
@@ -2100,10 +2448,51 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
     e->orig_pos.assign((size_t)S, 0);
     for (int64_t p = 0; p < S; ++p) e->orig_pos[e->csc_orig[p]] = p;
 
-    // ---- mask word offsets and per-synapse arrays
+    e->plastic = false;
+    for (int64_t s = 0; s < S && !e->plastic; ++s) e->plastic = d->rule[s] >= 0;
+    {   // update-kernel instance: the models the update threads meet (generator
+        // layers have their own threads) and whether anything learns
+        unsigned models = 0u;
+        for (const LayerDev &L : e->layers)
+            if (!L.generator) models |= 1u << L.model;
+        const unsigned lif_poisson = (1u << NBG_MODEL_LIF_VJ) | (1u << NBG_MODEL_POISSON);
+        if (models == (1u << NBG_MODEL_IZH_RK4) && e->plastic) {
+            e->plain_kernel = k_update<Spec<1u << NBG_MODEL_IZH_RK4, 1>>;
+        } else if (models == (1u << NBG_MODEL_LIF_VJ) && !e->plastic) {
+            e->plain_kernel = k_update<Spec<1u << NBG_MODEL_LIF_VJ, 0>>;
+            e->palette_kernel = k_update_quad<Spec<1u << NBG_MODEL_LIF_VJ, 0>>;
+        } else if ((models & ~lif_poisson) == 0u && !e->plastic) {
+            e->plain_kernel = k_update<Spec<lif_poisson, 0>>;
+            e->palette_kernel = k_update_quad<Spec<lif_poisson, 0>>;
+        } else {
+            e->plain_kernel = k_update<GenericSpec>;
+        }
+        e->update_kernel = e->plain_kernel;
+        // Palette networks: at most kPaletteSize pairs, no log of delivered
+        // events (its entries name the synapse), and at least 2 of the 4
+        // words of a quad used on average, so that the padded ring is at most
+        // twice the words that synapses have.
+        if (e->palette_kernel) {
+            int64_t words = 0, padded = 0;
+            for (int j = 0; j < e->N; ++j) {
+                const int nw = (indeg[j + 1] + 31) / 32;
+                words += nw;
+                padded += (nw + 3) / 4 * 4;
+            }
+            if (e->ev_cap > 0 || S == 0 || padded > 2 * words || padded > (1 << 27) ||
+                !collect_palette(d->weight, S, [&](int64_t s) { return (unsigned int)(d->type[s] & 1); }, e->palette_host,
+                                 e->palette_n))
+                e->palette_kernel = nullptr;
+        }
+    }
+    // ---- mask word offsets (whole quads for palette networks) and per-synapse arrays
+    const int word_group = e->palette_kernel ? 4 : 1;
     std::vector<int> woff((size_t)e->N + 1, 0);
-    for (int j = 0; j < e->N; ++j) woff[j + 1] = woff[j] + (cptr[j + 1] - cptr[j] + 31) / 32;
-    e->Wt = std::max(woff[e->N], 1);
+    for (int j = 0; j < e->N; ++j) {
+        const int nw = (cptr[j + 1] - cptr[j] + 31) / 32;
+        woff[j + 1] = woff[j] + (nw + word_group - 1) / word_group * word_group;
+    }
+    e->Wt = std::max(woff[e->N], word_group);
     e->woff_host = woff;
     // ring slots: every delay plus the longest block, so that no mark made
     // inside a block aliases a slot the block drains
@@ -2117,13 +2506,12 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
         src_of[p] = d->source[s];
     }
     e->init_w = w;
-    e->plastic = false;
-    for (int64_t s = 0; s < S && !e->plastic; ++s) e->plastic = d->rule[s] >= 0;
     // synapse records: 32 bytes with the STDP state when anything learns
     std::vector<SynRec> recs;
     std::vector<SynStatic> wsts;
     if (e->plastic) recs.resize((size_t)S);
     else wsts.resize((size_t)S);
+    if (e->palette_kernel) e->type_bits.assign((size_t)((S + 7) / 8), 0);
     for (int64_t p = 0; p < S; ++p) {
         const int64_t s = e->csc_orig[p];
         const unsigned int meta = (unsigned int)((d->type[s] & 1) | ((d->rule[s] + 1) << 1));
@@ -2139,6 +2527,7 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
             }
         } else {
             wsts[(size_t)p] = SynStatic{w[p], meta};
+            if (e->palette_kernel) e->type_bits[(size_t)(p >> 3)] |= (unsigned char)((meta & 1u) << (p & 7));
         }
     }
 
@@ -2234,21 +2623,6 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
         }
     }
 
-    {   // update-kernel instance: the models the update threads meet (generator
-        // layers have their own threads) and whether anything learns
-        unsigned models = 0u;
-        for (const LayerDev &L : e->layers)
-            if (!L.generator) models |= 1u << L.model;
-        const unsigned lif_poisson = (1u << NBG_MODEL_LIF_VJ) | (1u << NBG_MODEL_POISSON);
-        if (models == (1u << NBG_MODEL_IZH_RK4) && e->plastic)
-            e->update_kernel = k_update<Spec<1u << NBG_MODEL_IZH_RK4, 1>>;
-        else if (models == (1u << NBG_MODEL_LIF_VJ) && !e->plastic)
-            e->update_kernel = k_update<Spec<1u << NBG_MODEL_LIF_VJ, 0>>;
-        else if ((models & ~lif_poisson) == 0u && !e->plastic)
-            e->update_kernel = k_update<Spec<lif_poisson, 0>>;
-        else
-            e->update_kernel = k_update<GenericSpec>;
-    }
     int B = opt.block_steps > 0 ? std::min(opt.block_steps, e->dmin) : e->dmin;
     e->B = std::max(1, std::min(B, kMaxBlockSteps));
 
@@ -2331,6 +2705,7 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
     st = upload_layers(e);
     if (st == NBG_OK) st = ensure_decay_table(e, 4096);
     if (st == NBG_OK) st = reset_state(e);
+    if (st == NBG_OK) st = use_palette(e);
     if (st != NBG_OK) return bail(st);
     e->spike_capacity = opt.spike_capacity;
     *out = e;
@@ -2495,7 +2870,7 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
         nbg_status ps = ensure_timing_events(e, nblocks);
         if (ps != NBG_OK) return ps;
         if (!e->graph || e->graph_blocks != nfull || e->graph_tail != tail || e->graph_B != B ||
-            e->graph_threads != e->threads || std::memcmp(&e->graph_nd, &nd, sizeof(NetDev)) != 0) {
+            e->graph_threads != e->threads || e->graph_kernel != e->update_kernel || std::memcmp(&e->graph_nd, &nd, sizeof(NetDev)) != 0) {
             if (e->graph) {
                 cudaGraphExecDestroy(e->graph);
                 e->graph = nullptr;
@@ -2512,6 +2887,7 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
             e->graph_tail = tail;
             e->graph_B = B;
             e->graph_threads = e->threads;
+            e->graph_kernel = e->update_kernel;
             e->graph_nd = nd;
         }
         NBG_CUDA(cudaGraphLaunch(e->graph, e->stream));
@@ -2836,7 +3212,7 @@ nbg_status nbg_set_weight(nbg_engine *e, int64_t conn, float w) {
     NBG_CUDA(cudaMemcpy(dst, &w, sizeof(float), cudaMemcpyHostToDevice));
     NBG_CUDA(cudaMemcpy(e->init_w_d.p + p, &w, sizeof(float), cudaMemcpyHostToDevice));
     e->init_w[p] = w;
-    return NBG_OK;
+    return patch_palette(e, p, w);
 }
 
 nbg_status nbg_set_weights(nbg_engine *e, const float *w) {
@@ -2849,6 +3225,17 @@ nbg_status nbg_set_weights(nbg_engine *e, const float *w) {
     if (e->S > 0) {
         NBG_CUDA(cudaMemcpy(e->init_w_d.p, e->init_w.data(), e->S * sizeof(float), cudaMemcpyHostToDevice));
         NBG_CUDA(reset_synapses(e, false)); // weights only: the STDP traces stay
+    }
+    if (e->palette_kernel) {
+        Palette pal;
+        int used = 0;
+        if (!collect_palette(
+                e->init_w.data(), e->S,
+                [&](int64_t p) { return (unsigned int)((e->type_bits[(size_t)(p >> 3)] >> (p & 7)) & 1u); }, pal, used))
+            return leave_palette(e);
+        e->palette_host = pal;
+        e->palette_n = used;
+        return use_palette(e);
     }
     return NBG_OK;
 }
