@@ -242,8 +242,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // (cluster rank = split index) and run the same three split products into
 // TMEM.  Rank r owns batch rows [16 r, 16 r + 16) of the tile: every CTA
 // stores its partial of those rows straight into rank r's receive buffer
-// ([source rank][row][i], 64 KiB) through distributed shared memory, which
-// waits for nothing.  After one cluster barrier rank r adds the partials of
+// through distributed shared memory, which waits for nothing.  After one cluster barrier rank r adds the partials of
 // ranks 0..7 in order from its own shared memory -- the sum k_lif_adj_split
 // forms from g_parts, so the result is the same bit for bit -- and runs the
 // adjoint step on those elements, writing dI_t as the split
@@ -259,6 +258,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 // room for the receive buffer.
 constexpr int kAdjCluster = 8;
 constexpr int kAdjFusedStages = 2;
+// receive buffer [source rank][row / 4][i][row % 4]: a thread's sixteen
+// partials of one i are four 16-byte stores, and a warp's 32 of one of them are
+// contiguous (stores of the same size 80 bytes apart, free of bank conflicts
+// but scattered over packets, cost 2.6 us a step)
 constexpr int kAdjRecvBytes = kAdjN * kAdjM * 4;
 constexpr int kAdjFusedSmemBytes = kAdjFusedStages * kAdjStageBytes + kAdjRecvBytes + 1024 + 256;
 
@@ -273,7 +276,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
     long long k_off, long long k_cols, int *__restrict__ err) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *stages = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    float *recv = reinterpret_cast<float *>(stages + kAdjFusedStages * kAdjStageBytes); // [rank][row][i]
+    float *recv = reinterpret_cast<float *>(stages + kAdjFusedStages * kAdjStageBytes); // kAdjRecvBytes
     uint64_t *full = (uint64_t *)((uint8_t *)recv + kAdjRecvBytes);
     uint64_t *empty = full + kAdjFusedStages;
     uint64_t *done = empty + kAdjFusedStages;
@@ -403,7 +406,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
         const int q = warp & 3, h = warp >> 2;
         const int il = 32 * q + lane;
         if (!*abort) {
-            const uint32_t mine = smem_addr(recv) + (uint32_t)((ks * 16 * kAdjM + il) * 4);
+            const uint32_t mine = smem_addr(recv) + (uint32_t)((ks * 4 * kAdjM + il) * 16);
 #pragma unroll
             for (int c16 = 0; c16 < 4; ++c16) {
                 float acc[16];
@@ -411,8 +414,9 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
                 uint32_t ra;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(mine), "r"(4 * h + c16));
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra + (uint32_t)(c * kAdjM * 4)), "f"(acc[c])
+                for (int c = 0; c < 16; c += 4)
+                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * kAdjM * 16)),
+                                 "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3])
                                  : "memory");
             }
         }
@@ -424,18 +428,20 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
     {
         // every partial of the thread's rows, loaded back to back, then added
         // in rank order
-        float x[kRows][kAdjCluster];
+        float x[kAdjCluster][kRows];
 #pragma unroll
-        for (int k = 0; k < kRows; ++k)
+        for (int r = 0; r < kAdjCluster; ++r)
 #pragma unroll
-            for (int r = 0; r < kAdjCluster; ++r) x[k][r] = recv[(r * 16 + 8 * bsub + k) * kAdjM + il];
+            for (int k = 0; k < kRows; k += 4)
+                *reinterpret_cast<float4 *>(&x[r][k]) =
+                    *reinterpret_cast<const float4 *>(recv + ((r * 4 + 2 * bsub + k / 4) * kAdjM + il) * 4);
         uint32_t t_hi[kRows / 2], t_lo[kRows / 2]; // dI^T of the eight rows, split, packed in pairs
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
             const int b = 16 * ks + 8 * bsub + k;
-            float ge = x[k][0];
+            float ge = x[0][k];
 #pragma unroll
-            for (int r = 1; r < kAdjCluster; ++r) ge = ge + x[k][r];
+            for (int r = 1; r < kAdjCluster; ++r) ge = ge + x[r][k];
             const size_t idx = (size_t)b * n + i;
             const float uu = op_u[k], ss = op_s[k], lv = op_lv[k];
             const float dsdu = p.smooth ? p.slope * ss * (1.0f - ss) : surrogate(uu - th, p.slope);

@@ -91,6 +91,74 @@ __device__ __host__ __forceinline__ size_t s_blocked(int b, int k) {
     return ((size_t)(k / umma::kKChunk) * umma::kBlockB + umma::block_offset(b, k % umma::kKChunk)) / 2;
 }
 
+// ------------------------------------------------------- spikes in and out
+//
+// The caller's spikes are bytes [instance][neuron]; the delivery paths hold
+// them as BF16 in the blocked layout, BF16 rows or bit words.  One thread
+// converts eight neighbouring neurons: a 16-byte core-matrix row, 16 bytes of a
+// row or one byte of a word.  Done on the host, element by element, this took
+// 1.5 ms of a read-out of 64 x 8,192 and most of a small delivery; the copies
+// of the bytes (512 KiB) and this kernel (memory-bound, 1.6 MB) about 40 us.
+enum { kLayoutBlocked = 0, kLayoutRows = 1, kLayoutBits = 2 };
+
+template <int kLayout> __device__ __forceinline__ size_t spikes8_at(int b, int k, int n) { // element of the group's first neuron
+    return kLayout == kLayoutBlocked ? s_blocked(b, k) : (size_t)b * n + k;
+}
+
+template <int kLayout>
+__global__ void k_spikes_out(const void *__restrict__ s, uint8_t *__restrict__ out, int n, int groups) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= groups) return;
+    const int b = g / (n / 8), k = (g - b * (n / 8)) * 8;
+    unsigned bits = 0u;
+    if constexpr (kLayout == kLayoutBits) {
+        bits = reinterpret_cast<const uint8_t *>(s)[g];
+    } else {
+        const uint4 q = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __nv_bfloat16 *>(s) + spikes8_at<kLayout>(b, k, n));
+        const unsigned w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) bits |= ((w[i >> 1] >> (16 * (i & 1)) & 0x7fffu) ? 1u : 0u) << i;
+    }
+    uint2 o = make_uint2(0u, 0u);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        o.x |= (bits >> i & 1u) << (8 * i);
+        o.y |= (bits >> (i + 4) & 1u) << (8 * i);
+    }
+    reinterpret_cast<uint2 *>(out)[g] = o;
+}
+
+template <int kLayout>
+__global__ void k_spikes_in(const uint8_t *__restrict__ in, void *__restrict__ s, int n, int groups) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= groups) return;
+    const int b = g / (n / 8), k = (g - b * (n / 8)) * 8;
+    const uint2 q = reinterpret_cast<const uint2 *>(in)[g];
+    unsigned bits = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        bits |= (q.x >> (8 * i) & 0xffu ? 1u : 0u) << i;
+        bits |= (q.y >> (8 * i) & 0xffu ? 1u : 0u) << (i + 4);
+    }
+    if constexpr (kLayout == kLayoutBits) {
+        reinterpret_cast<uint8_t *>(s)[g] = (uint8_t)bits;
+    } else {
+        const unsigned one = 0x3f80u; // 1.0 in BF16
+        unsigned w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            w[i] = (bits >> (2 * i) & 1u ? one : 0u) | (bits >> (2 * i + 1) & 1u ? one << 16 : 0u);
+        *reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(s) + spikes8_at<kLayout>(b, k, n)) =
+            make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// out = partial[0] + partial[1]: the same fixed order as the update kernels
+__global__ void k_sum_split_partials(const float *__restrict__ part, float *__restrict__ out, int total) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx < total) out[idx] = part[idx] + part[(size_t)total + idx];
+}
+
 // ------------------------------------------------------------- GEMM (mma.sync)
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
@@ -411,6 +479,14 @@ struct nbg_dense {
     DevBuf<__nv_bfloat16> whi, wlo, s[2];
     DevBuf<unsigned> bits[2];
     DevBuf<int> last, err;
+    // conversions and deliveries outside the step loop: the caller's bytes, the
+    // spikes in the path's layout, the partial sums and the result.  Made at
+    // first use, one call at a time (io_mu), apart from the simulation's state
+    std::mutex io_mu;
+    DevBuf<uint8_t> io_bytes;
+    DevBuf<__nv_bfloat16> io_s;
+    DevBuf<float> io_part, io_out;
+    DevBuf<int> cnt; // spikes per step of a run call
     DevBuf<unsigned int> tile_cnt; // fused-update arrivals per tile (zero between launches)
     std::vector<cudaEvent_t> dev_pool; // delivery start/stop events, 2 per step
     int next_t = 0;
@@ -439,6 +515,12 @@ nbg_status dense_reset(nbg_dense *d) {
     d->ran = false;
     d->counts_host.clear();
     return NBG_OK;
+}
+
+int layout_of(const nbg_dense *d) {
+    return d->precision == NBG_DENSE_SPLIT_BF16 ? kLayoutBlocked
+           : d->precision == NBG_DENSE_FP32     ? kLayoutBits
+                                                : kLayoutRows;
 }
 
 dim3 gather_grid(const nbg_dense *d) { return dim3(d->B, (d->N + kGatherCols - 1) / kGatherCols); }
@@ -582,8 +664,8 @@ nbg_status nbg_dense_run(nbg_dense *d, int steps) {
     const int count = d->ran ? steps : steps + 1;
     const int total = d->B * d->N;
     std::vector<int> cnt((size_t)count, 0);
-    DevBuf<int> dcnt;
-    NBG_CUDA(dcnt.alloc((size_t)count));
+    if (d->cnt.n < (size_t)count) NBG_CUDA(d->cnt.alloc((size_t)count));
+    DevBuf<int> &dcnt = d->cnt;
     NBG_CUDA(cudaMemsetAsync(dcnt.p, 0, count * sizeof(int), d->stream));
     // event pairs bracketing every delivery launch of the two-launch path (reused across calls)
     const bool sync_path = d->precision == NBG_DENSE_SPLIT_BF16_SYNC;
@@ -683,68 +765,54 @@ nbg_status nbg_dense_get_spikes(nbg_dense *d, uint8_t *s) {
         std::memset(s, 0, tot);
         return NBG_OK;
     }
-    if (d->precision != NBG_DENSE_FP32) {
-        std::vector<__nv_bfloat16> h(tot);
-        NBG_CUDA(cudaMemcpy(h.data(), d->s[par].p, tot * sizeof(__nv_bfloat16), cudaMemcpyDeviceToHost));
-        const bool blocked = d->precision == NBG_DENSE_SPLIT_BF16;
-        for (size_t i = 0; i < tot; ++i) {
-            const size_t src = blocked ? s_blocked((int)(i / d->N), (int)(i % d->N)) : i;
-            s[i] = __bfloat162float(h[src]) != 0.0f;
-        }
-    } else {
-        std::vector<unsigned> h(tot / 32);
-        NBG_CUDA(cudaMemcpy(h.data(), d->bits[par].p, (tot / 32) * sizeof(unsigned), cudaMemcpyDeviceToHost));
-        for (size_t i = 0; i < tot; ++i) s[i] = (h[i >> 5] >> (i & 31)) & 1u;
+    std::lock_guard<std::mutex> lock(d->io_mu);
+    if (d->io_bytes.n < tot) NBG_CUDA(d->io_bytes.alloc(tot));
+    const int groups = (int)(tot / 8), grid = (groups + 255) / 256;
+    switch (layout_of(d)) {
+    case kLayoutBlocked: k_spikes_out<kLayoutBlocked><<<grid, 256, 0, d->stream>>>(d->s[par].p, d->io_bytes.p, d->N, groups); break;
+    case kLayoutRows: k_spikes_out<kLayoutRows><<<grid, 256, 0, d->stream>>>(d->s[par].p, d->io_bytes.p, d->N, groups); break;
+    default: k_spikes_out<kLayoutBits><<<grid, 256, 0, d->stream>>>(d->bits[par].p, d->io_bytes.p, d->N, groups); break;
     }
+    NBG_CUDA(cudaGetLastError());
+    NBG_CUDA(cudaMemcpyAsync(s, d->io_bytes.p, tot, cudaMemcpyDeviceToHost, d->stream));
+    NBG_CUDA(cudaStreamSynchronize(d->stream));
     return NBG_OK;
 }
 
 nbg_status nbg_dense_deliver(nbg_dense *d, const uint8_t *s, float *out) {
     if (!d || !s || !out) return nbg_fail(NBG_ERR_INVALID, "null argument");
     NBG_CUDA(cudaSetDevice(d->device));
-    NBG_CUDA(cudaStreamSynchronize(d->stream));
     const size_t tot = (size_t)d->B * d->N;
-    // stage S into the buffer of the next step's input, deliver, restore nothing:
-    // use a scratch parity-independent copy so the simulation state is untouched
-    DevBuf<__nv_bfloat16> sb;
-    DevBuf<unsigned> bb;
-    DevBuf<float> part;
-    NBG_CUDA(part.alloc((size_t)kSplitK * tot));
-    if (d->precision == NBG_DENSE_SPLIT_BF16) {
-        std::vector<__nv_bfloat16> h(tot);
-        for (size_t i = 0; i < tot; ++i)
-            h[s_blocked((int)(i / d->N), (int)(i % d->N))] = __float2bfloat16_rn(s[i] ? 1.0f : 0.0f);
-        NBG_CUDA(sb.upload(h));
-        dim3 grid(d->N / umma::kM, kSplitK);
-        umma::k_dense_umma<umma::NoFinish><<<grid, umma::kThreads, umma::kSmemBytes, d->stream>>>(
-            d->whi.p, d->wlo.p, sb.p, part.p, d->N, kSplitK, 0, d->err.p, d->tile_cnt.p, umma::NoFinish{});
-    } else if (d->precision == NBG_DENSE_SPLIT_BF16_SYNC) {
-        std::vector<__nv_bfloat16> h(tot);
-        for (size_t i = 0; i < tot; ++i) h[i] = __float2bfloat16_rn(s[i] ? 1.0f : 0.0f);
-        NBG_CUDA(sb.upload(h));
-        dim3 grid(d->N / kBM, kSplitK);
-        k_dense_gemm<<<grid, kGemmThreads, kGemmSmem, d->stream>>>(d->whi.p, d->wlo.p, sb.p, part.p, d->N);
-    } else {
-        std::vector<unsigned> h(tot / 32, 0u);
-        for (size_t i = 0; i < tot; ++i)
-            if (s[i]) h[i >> 5] |= 1u << (i & 31);
-        NBG_CUDA(bb.upload(h));
-        k_dense_gather<false><<<gather_grid(d), kGatherThreads, 0, d->stream>>>(d->w.p, bb.p, part.p, d->P, nullptr,
-                                                                                nullptr, nullptr, nullptr, 0, d->N);
-    }
-    NBG_CUDA(cudaGetLastError());
-    NBG_CUDA(cudaStreamSynchronize(d->stream));
+    std::lock_guard<std::mutex> lock(d->io_mu);
+    if (d->io_bytes.n < tot) NBG_CUDA(d->io_bytes.alloc(tot));
+    if (d->io_s.n < tot) NBG_CUDA(d->io_s.alloc(tot));
+    if (d->io_out.n < tot) NBG_CUDA(d->io_out.alloc(tot));
     const bool split = d->precision != NBG_DENSE_FP32;
-    std::vector<float> h((size_t)(split ? kSplitK : 1) * tot);
-    NBG_CUDA(cudaMemcpy(h.data(), part.p, h.size() * sizeof(float), cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < tot; ++i) {
-        float a = h[i];
-        if (split)
-            for (int k = 1; k < kSplitK; ++k) a = a + h[(size_t)k * tot + i];
-        out[i] = a;
+    if (split && d->io_part.n < (size_t)kSplitK * tot) NBG_CUDA(d->io_part.alloc((size_t)kSplitK * tot));
+    const int groups = (int)(tot / 8), grid8 = (groups + 255) / 256;
+    cudaStream_t st = d->stream;
+    NBG_CUDA(cudaMemcpyAsync(d->io_bytes.p, s, tot, cudaMemcpyHostToDevice, st));
+    if (d->precision == NBG_DENSE_SPLIT_BF16) {
+        k_spikes_in<kLayoutBlocked><<<grid8, 256, 0, st>>>(d->io_bytes.p, d->io_s.p, d->N, groups);
+        umma::k_dense_umma<umma::NoFinish><<<dim3(d->N / umma::kM, kSplitK), umma::kThreads, umma::kSmemBytes, st>>>(
+            d->whi.p, d->wlo.p, d->io_s.p, d->io_part.p, d->N, kSplitK, 0, d->err.p, d->tile_cnt.p, umma::NoFinish{});
+    } else if (d->precision == NBG_DENSE_SPLIT_BF16_SYNC) {
+        k_spikes_in<kLayoutRows><<<grid8, 256, 0, st>>>(d->io_bytes.p, d->io_s.p, d->N, groups);
+        k_dense_gemm<<<dim3(d->N / kBM, kSplitK), kGemmThreads, kGemmSmem, st>>>(d->whi.p, d->wlo.p, d->io_s.p,
+                                                                               d->io_part.p, d->N);
+    } else {
+        unsigned *const bits = reinterpret_cast<unsigned *>(d->io_s.p);
+        k_spikes_in<kLayoutBits><<<grid8, 256, 0, st>>>(d->io_bytes.p, bits, d->N, groups);
+        k_dense_gather<false><<<gather_grid(d), kGatherThreads, 0, st>>>(d->w.p, bits, d->io_out.p, d->P, nullptr, nullptr,
+                                                                         nullptr, nullptr, 0, d->N);
     }
+    if (split) k_sum_split_partials<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(d->io_part.p, d->io_out.p, (int)tot);
+    NBG_CUDA(cudaGetLastError());
+    NBG_CUDA(cudaMemcpyAsync(out, d->io_out.p, tot * sizeof(float), cudaMemcpyDeviceToHost, st));
     int errv = 0;
-    NBG_CUDA(cudaMemcpy(&errv, d->err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    if (d->precision == NBG_DENSE_SPLIT_BF16) // the only path that waits
+        NBG_CUDA(cudaMemcpyAsync(&errv, d->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    NBG_CUDA(cudaStreamSynchronize(st));
     if (errv) return nbg_fail(NBG_ERR_TIMEOUT, "tensor-core delivery gave up waiting on a pipeline barrier");
     return NBG_OK;
 }
@@ -773,12 +841,6 @@ namespace {
 constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noalloc_mu;
 float *g_noalloc_scratch[kNoAllocMaxDevices] = {};
-
-// out = partial[0] + partial[1]: the same fixed order as the update kernel
-__global__ void k_sum_split_partials(const float *__restrict__ part, float *__restrict__ out, int total) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < total) out[idx] = part[idx] + part[(size_t)total + idx];
-}
 
 } // namespace
 

@@ -87,9 +87,11 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
                  : "memory");
 }
 
-__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+// True when the phase with `parity` has completed; waits for it in hardware,
+// up to a limit of the implementation's.
+__device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
                  : "=r"(ok)
                  : "r"(smem_addr(bar)), "r"(parity)
                  : "memory");
@@ -100,13 +102,12 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
 // or when another role of the CTA already gave up.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort) {
     const long long t0 = clock64();
-    while (!mbar_test(bar, parity)) {
+    while (!mbar_try(bar, parity)) {
         if (*abort) return false;
         if (clock64() - t0 > kWaitCycles) {
             *abort = 1;
             return false;
         }
-        __nanosleep(64);
     }
     return true;
 }

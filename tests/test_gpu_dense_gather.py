@@ -54,3 +54,26 @@ def test_steps_equal_the_oracle(oracle_lib, n):
     assert np.array_equal(eng.spike_counts(), ref.counts()) and eng.spike_counts().sum() > 0
     assert np.array_equal(v.ravel(), rv.astype(np.float32)) and np.array_equal(last.ravel(), rlast)
     assert np.array_equal(eng.spikes().ravel(), rs)
+
+
+@pytest.mark.parametrize("precision", ["split_bf16", "split_bf16_sync", "fp32"])
+@pytest.mark.parametrize("n", [128, 384])
+def test_spikes_in_and_out_of_each_layout(precision, n):
+    """Out: a neuron spiked at the last step exactly where its LastSpike counter is 0.  In: any non-zero byte is a
+    spike, and a delivery leaves the simulation as it was."""
+    w = _weights(n)
+    eng = DensePopulations(w, _layer(), precision=precision)
+    assert not eng.spikes().any()
+    total = 0
+    for _ in range(30):
+        eng.run(5)
+        assert np.array_equal(eng.spikes(), (eng.state()[1] == 0).astype(np.uint8))
+        total += int(eng.spikes().sum())
+    assert total > 0
+    s = (np.random.default_rng(n).random((64, n)) < 0.1).astype(np.uint8)
+    before = eng.spikes()
+    out = eng.deliver(s)
+    assert np.array_equal(out, eng.deliver(s * 7)) and np.array_equal(eng.spikes(), before)
+    # |error| of a split product: 2^-16 of each weight that is added, and the FP32 sums
+    bound = 2.0 ** -15 * (s.astype(np.float64) @ np.abs(w).astype(np.float64)) + 1e-30
+    assert (np.abs(out - s.astype(np.float64) @ w.astype(np.float64)) <= bound).all()
