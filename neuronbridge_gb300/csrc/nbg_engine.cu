@@ -275,7 +275,7 @@ __device__ __forceinline__ Model load_model(const LayerDev &L) {
 // (1 yes, 0 no, -1 decided per launch from the STDP arrays).  With one model
 // the per-neuron dispatch folds away; without learning the STDP loads and
 // the post-synaptic pass are not compiled.
-template <unsigned kModels, int kPlastic>
+template <unsigned kModels, int kPlastic, bool kDeep = (kPlastic > 0)>
 struct Spec {
     static constexpr bool has(int m) { return (kModels >> m) & 1u; }
     // resident 256-thread CTAs per SM the register budget is sized for: the
@@ -292,7 +292,7 @@ struct Spec {
     // steps (the current-based Izhikevich + STDP profile).  Wide: every
     // flagged word one step ahead and arrivals loaded several at a time, for
     // networks with arrivals at most steps (Poisson-driven static LIF).
-    static constexpr bool deep = kPlastic > 0;
+    static constexpr bool deep = kDeep;
 };
 constexpr unsigned kAllModels = 0x3fu;
 using GenericSpec = Spec<kAllModels, -1>;
@@ -2456,6 +2456,8 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
         for (const LayerDev &L : e->layers)
             if (!L.generator) models |= 1u << L.model;
         const unsigned lif_poisson = (1u << NBG_MODEL_LIF_VJ) | (1u << NBG_MODEL_POISSON);
+        const unsigned lif_inputs =
+            (1u << NBG_MODEL_LIF_VJ) | (1u << NBG_MODEL_INPUT_SPIKE) | (1u << NBG_MODEL_INPUT_CURRENT);
         if (models == (1u << NBG_MODEL_IZH_RK4) && e->plastic) {
             e->plain_kernel = k_update<Spec<1u << NBG_MODEL_IZH_RK4, 1>>;
         } else if (models == (1u << NBG_MODEL_LIF_VJ) && !e->plastic) {
@@ -2464,6 +2466,12 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
         } else if ((models & ~lif_poisson) == 0u && !e->plastic) {
             e->plain_kernel = k_update<Spec<lif_poisson, 0>>;
             e->palette_kernel = k_update_quad<Spec<lif_poisson, 0>>;
+        } else if ((models & ~lif_inputs) == 0u && e->plastic) {
+            // wide drain: 97 us a launch against 110 deep and 119 by the generic
+            // instance (20,000 Poisson-driven neurons, plastic recurrent synapses),
+            // and no slower where arrivals are few (the 500-neuron control loop: 58,
+            // 61 and 65 us a call)
+            e->plain_kernel = k_update<Spec<lif_inputs, 1, false>>;
         } else {
             e->plain_kernel = k_update<GenericSpec>;
         }
