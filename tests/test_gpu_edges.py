@@ -92,3 +92,20 @@ def test_raster_capacity_overflow_is_an_error():
     sim = nb.Simulation(net, SimulationConfig(steps=3000, timestep=0.1), spike_capacity=10)
     with pytest.raises(nb.NbgError, match="capacity"):
         sim.run(3000)
+
+
+def test_weights_of_more_synapses_than_a_gather_chunk():
+    """Weights come back in original connection order in chunks of 2^24 synapses; traces of a static network are 0."""
+    from neuronbridge_gb300 import NetworkDescription, NeuronLayer
+    from neuronbridge_gb300.workloads import LIF_PARAMS
+
+    n, s = 5000, (1 << 24) + 70_001
+    rng = np.random.default_rng(2)
+    w = rng.random(s, dtype=np.float32)
+    d = NetworkDescription.from_arrays([NeuronLayer("TimeDrivenLIF_Voltage_jump", n, parameters=dict(LIF_PARAMS))],
+                                       rng.integers(0, n, s, dtype=np.int32), rng.integers(0, n, s, dtype=np.int32),
+                                       np.zeros(s, np.int32), w, delay=np.full(s, 3, np.int32))
+    sim = nb.Simulation(d, nb.SimulationConfig(steps=1, timestep=0.1))
+    got = sim.weights()
+    assert np.array_equal(got["weight"], w)
+    assert not got["apre"].any() and not got["apost"].any() and not got["last_update"].any()
