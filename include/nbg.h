@@ -287,9 +287,9 @@ nbg_status nbg_profile(nbg_engine *e, double *total_ms, double *update_ms, doubl
                        int64_t *launches);
 
 /* Raster phases of the last nbg_run call: the device ordering of its spike
- * raster into (step, id) order (CUDA events; order_launches kernels), the
- * download to the host and the append to the recorded raster (host wall
- * time).  The reference records output spikes from its host event loop
+ * raster into (step, id) order (order_launches kernels) and the download to
+ * the host (CUDA events; the download reads 0 when the host orders the
+ * entries), and the append to the recorded raster (host wall time).  The reference records output spikes from its host event loop
  * (communication/src/ArrayOutputSpikeDriver.cpp); here they are this
  * separate phase after the step loop.  If the device ordering fails (its
  * buffers cannot be allocated), nbg_run downloads the unordered entries and

@@ -1483,7 +1483,8 @@ struct nbg_engine {
     std::vector<int64_t> csc_orig; // CSC position -> original connection index
     std::vector<int64_t> orig_pos; // original connection index -> CSC position
     std::vector<nbg_stdp_desc> rules;
-    std::vector<float> init_v, init_u, init_iext;
+    std::vector<float> init_v, init_u, init_iext; // until they are on the device
+    DevBuf<float> init_v_d, init_u_d, init_iext_d;
     std::vector<int> woff_host; // first mask word of each neuron (N + 1 entries)
     int *pin_ids = nullptr, *pin_t = nullptr; // pinned staging of the raster download
     size_t pin_cap = 0;
@@ -1495,9 +1496,10 @@ struct nbg_engine {
     bool raster_order_fail = false;
     // raster ordering: per-step spike bitmap, tile sums / positions, running
     // base, ordered entries; timings of the last run call's raster phases
-    DevBuf<unsigned int> rbm, rtile, rbase;
+    DevBuf<unsigned int> rbm, rtile;
     DevBuf<int> ord_ids, ord_t;
-    cudaEvent_t evr0 = nullptr, evr1 = nullptr;
+    cudaEvent_t evr0 = nullptr, evr1 = nullptr, evr2 = nullptr; // raster: before, ordered, downloaded
+    bool raster_timed = false; // the three were recorded by the last run call
     double last_order_ms = 0.0, last_download_ms = 0.0, last_append_ms = 0.0;
     int64_t last_order_launches = 0;
     std::vector<float> init_w;
@@ -1524,12 +1526,19 @@ struct nbg_engine {
     DevBuf<float2> dtab;
     DevBuf<int> gen_ptr, gen_pos, gen_src;
     DevBuf<unsigned short> gen_delay;
-    DevBuf<int> last, csc_ptr_d, woff, out_ptr, out_ids, out_t, err, run_t0, trace_slot, ev_t, ev_pos;
+    DevBuf<int> last, csc_ptr_d, woff, out_ptr, out_ids, out_t, trace_slot, ev_t, ev_pos;
     DevBuf<unsigned int> mask, wsum, out_bit, out_pk;
     int out_dbits = 0, out_dmin = 0;
     int Ws = 1;
     DevBuf<unsigned short> out_delay;
-    DevBuf<unsigned int> cursor;
+    // a run call's words: raster cursor, error bits, entries ordered, first step
+    // (k_run_begin); one 16-byte copy reads them back
+    enum { kCursor, kErrWord, kOrdered, kRunT0, kWords };
+    DevBuf<unsigned int> words;
+    unsigned int *pin_words = nullptr; // pinned copy
+    static constexpr size_t kPinState = 64 << 10;
+    char *pin_state = nullptr; // pinned staging of nbg_get_state's small reads
+    std::mutex state_mu;       // one of them at a time
     DevBuf<unsigned long long> ev_cursor, n_events;
     int dtab_len = 0;
     bool dtab_complete = false; // table reached exact zero: longer gaps decay to 0
@@ -1549,8 +1558,9 @@ struct nbg_engine {
     // the current call
     std::vector<std::pair<int, int>> ext_pending;
     std::unordered_set<uint64_t> ext_keys;
-    std::vector<int> ext_ptr_h, ext_ids_h;
     DevBuf<int> ext_ptr_d, ext_ids_d;
+    int *pin_ext = nullptr; // pinned staging of both
+    size_t pin_ext_cap = 0;
     DevBuf<int> upd_ids_d, gen_ids_d; // thread map (NetDev::upd_ids, gen_ids)
     int N_upd = 0, N_gen = 0;
     // current synapses (type 3): per source the out-going ones (target,
@@ -1622,10 +1632,10 @@ struct nbg_engine {
         n.gen_delay = gen_delay.p;
         n.out_ids = out_ids.p;
         n.out_t = out_t.p;
-        n.cursor = cursor.p;
+        n.cursor = words.p + kCursor;
         n.out_cap = (long long)out_ids.n;
-        n.err = err.p;
-        n.run_t0 = run_t0.p;
+        n.err = reinterpret_cast<int *>(words.p + kErrWord);
+        n.run_t0 = reinterpret_cast<int *>(words.p + kRunT0);
         n.trace_slot = trace_ids.empty() ? nullptr : trace_slot.p;
         n.trace = trace.p;
         n.ntrace = (int)trace_ids.size();
@@ -1767,12 +1777,16 @@ __global__ void k_gather_weights(const SynRec *__restrict__ rec, const SynStatic
 constexpr size_t kWeightChunk = (size_t)1 << 24; // synapses of a chunk: 256 MiB of staging
 
 // Every synapse's weight back to init_w_d (and, with `traces`, its STDP state
-// to zero), on the engine's stream, synchronously.
-cudaError_t reset_synapses(nbg_engine *e, bool traces) {
+// to zero), on the engine's stream.
+cudaError_t set_synapses(nbg_engine *e, bool traces) {
     const long long S = e->S;
     k_set_synapses<<<(unsigned)((S + 255) / 256), 256, 0, e->stream>>>(e->rec.p, e->wst.p, e->init_w_d.p, S,
                                                                        traces ? 1 : 0);
-    const cudaError_t ce = cudaGetLastError();
+    return cudaGetLastError();
+}
+
+cudaError_t reset_synapses(nbg_engine *e, bool traces) { // synchronously
+    const cudaError_t ce = set_synapses(e, traces);
     return ce != cudaSuccess ? ce : cudaStreamSynchronize(e->stream);
 }
 
@@ -1905,21 +1919,42 @@ nbg_status upload_layers(nbg_engine *e) {
     return NBG_OK;
 }
 
+// Initial state of neurons [first, first + count).
+__global__ void k_reset_neurons(float *v, float *u, float *gexc, float *ginh, float *iext, int *last,
+                                const float *__restrict__ v0, const float *__restrict__ u0,
+                                const float *__restrict__ iext0, int first, int count) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= count) return;
+    const int j = first + k;
+    v[j] = v0[j];
+    u[j] = u0[j];
+    iext[j] = iext0[j];
+    gexc[j] = ginh[j] = 0.0f;
+    last[j] = 10000;
+}
+
+void reset_neurons(nbg_engine *e, int first, int count) {
+    k_reset_neurons<<<(unsigned)((count + 255) / 256), 256, 0, e->stream>>>(
+        e->v.p, e->u.p, e->gexc.p, e->ginh.p, e->iext.p, e->last.p, e->init_v_d.p, e->init_u_d.p, e->init_iext_d.p, first,
+        count);
+}
+
+// The words of a run call that starts at step t0.
+__global__ void k_run_begin(unsigned int *words, int t0) {
+    *reinterpret_cast<uint4 *>(words) = make_uint4(0u, 0u, 0u, (unsigned int)t0);
+}
+
 nbg_status reset_state(nbg_engine *e) {
-    NBG_CUDA(cudaMemcpy(e->v.p, e->init_v.data(), e->N * sizeof(float), cudaMemcpyHostToDevice));
-    NBG_CUDA(cudaMemcpy(e->u.p, e->init_u.data(), e->N * sizeof(float), cudaMemcpyHostToDevice));
-    NBG_CUDA(cudaMemcpy(e->iext.p, e->init_iext.data(), e->N * sizeof(float), cudaMemcpyHostToDevice));
-    NBG_CUDA(e->gexc.zero());
-    NBG_CUDA(e->ginh.zero());
-    std::vector<int> last0((size_t)e->N, 10000);
-    NBG_CUDA(cudaMemcpy(e->last.p, last0.data(), e->N * sizeof(int), cudaMemcpyHostToDevice));
-    if (e->S > 0) NBG_CUDA(reset_synapses(e, true));
-    NBG_CUDA(e->mask.zero());
-    NBG_CUDA(e->wsum.zero());
-    NBG_CUDA(e->err.zero());
-    NBG_CUDA(e->cursor.zero());
-    NBG_CUDA(e->ev_cursor.zero());
-    NBG_CUDA(e->n_events.zero());
+    cudaStream_t st = e->stream; // everything in its order, one wait at the end
+    reset_neurons(e, 0, e->N);
+    NBG_CUDA(cudaGetLastError());
+    if (e->S > 0) NBG_CUDA(set_synapses(e, true));
+    NBG_CUDA(cudaMemsetAsync(e->mask.p, 0, e->mask.n * sizeof(unsigned int), st));
+    NBG_CUDA(cudaMemsetAsync(e->wsum.p, 0, e->wsum.n * sizeof(unsigned int), st));
+    NBG_CUDA(cudaMemsetAsync(e->words.p, 0, e->words.n * sizeof(unsigned int), st));
+    NBG_CUDA(cudaMemsetAsync(e->ev_cursor.p, 0, sizeof(unsigned long long), st));
+    NBG_CUDA(cudaMemsetAsync(e->n_events.p, 0, sizeof(unsigned long long), st));
+    NBG_CUDA(cudaStreamSynchronize(st));
     e->next_t = 0;
     e->ran = false;
     e->spk_t.clear();
@@ -1952,9 +1987,13 @@ nbg_status ensure_timing_events(nbg_engine *e, int blocks) {
 
 // Launch one block of B steps.  With kernel timing, `slot` selects the event
 // pair bracketing the launch.
+// `chained`: the launch before it on the stream is an update launch, which it
+// may overlap (the first of a call follows k_run_begin, whose step it reads
+// ahead of the dependency wait).
 // Inside stream capture an event record must be "external" to become an
 // event-record node of the graph (a plain record is only a dependency).
-void launch_block(nbg_engine *e, const NetDev &nd, int B, int toff, int slot, bool capturing = false) {
+void launch_block(nbg_engine *e, const NetDev &nd, int B, int toff, int slot, bool capturing = false,
+                  bool chained = true) {
     const int gen_threads = (e->N_gen + kGenPerThread - 1) / kGenPerThread;
     const int grid = std::max(1, (e->N_upd + e->threads - 1) / e->threads + (gen_threads + e->threads - 1) / e->threads);
     const unsigned int flags = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
@@ -1968,7 +2007,7 @@ void launch_block(nbg_engine *e, const NetDev &nd, int B, int toff, int slot, bo
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chained ? 1 : 0;
     cudaLaunchKernelEx(&cfg, e->update_kernel, nd, B, toff); // errors surface at the call's cudaGetLastError
     if (e->kernel_timing) cudaEventRecordWithFlags(e->tev[2 * slot + 1], e->stream, flags);
 }
@@ -2121,13 +2160,23 @@ __global__ void __launch_bounds__(kRasterThreads) k_raster_emit(const uint4 *__r
     }
 }
 
-// Order this call's n device raster entries by (step, id) into ord_ids /
-// ord_t; returns the number of ordered entries in *n_out.
-nbg_status order_raster(nbg_engine *e, unsigned n, int t0, int count, unsigned *n_out) {
-    *n_out = 0;
-    e->last_order_ms = 0.0;
-    e->last_order_launches = 0;
-    if (n == 0) return NBG_OK;
+// Pinned staging for n raster entries, grown by half again when short.
+nbg_status pin_raster(nbg_engine *e, size_t n) {
+    if (n <= e->pin_cap) return NBG_OK;
+    if (e->pin_ids) cudaFreeHost(e->pin_ids);
+    if (e->pin_t) cudaFreeHost(e->pin_t);
+    e->pin_ids = e->pin_t = nullptr;
+    e->pin_cap = 0;
+    const size_t cap = n + n / 2;
+    NBG_CUDA(cudaMallocHost(&e->pin_ids, cap * sizeof(int)));
+    NBG_CUDA(cudaMallocHost(&e->pin_t, cap * sizeof(int)));
+    e->pin_cap = cap;
+    return NBG_OK;
+}
+
+// Order this call's n > 0 device raster entries by (step, id) and bring them to
+// pin_ids / pin_t: the four kernels of each chunk, the copies, one wait.
+nbg_status order_raster(nbg_engine *e, unsigned n, int t0, int count) {
     const int wp = (((e->N + 31) >> 5) + 3) & ~3;
     const int chunk =
         (int)std::max<int64_t>(1, std::min<int64_t>(count, (int64_t)(e->raster_bitmap_words / (size_t)wp)));
@@ -2139,13 +2188,12 @@ nbg_status order_raster(nbg_engine *e, unsigned n, int t0, int count, unsigned *
         return fail(NBG_ERR_CUDA, "raster bitmap: %s (injected)", cudaGetErrorString(cudaErrorMemoryAllocation));
     if (e->rbm.n < (size_t)max_tiles * kRasterTileWords) NBG_CUDA(e->rbm.alloc((size_t)max_tiles * kRasterTileWords));
     if (e->rtile.n < max_tiles) NBG_CUDA(e->rtile.alloc(max_tiles));
-    if (e->rbase.n < 1) NBG_CUDA(e->rbase.alloc(1));
     if (e->ord_ids.n < n) {
         NBG_CUDA(e->ord_ids.alloc(n));
         NBG_CUDA(e->ord_t.alloc(n));
     }
+    unsigned int *const base = e->words.p + nbg_engine::kOrdered; // 0 since k_run_begin
     NBG_CUDA(cudaEventRecord(e->evr0, e->stream));
-    NBG_CUDA(cudaMemsetAsync(e->rbase.p, 0, sizeof(unsigned), e->stream));
     const unsigned mark_grid =
         (unsigned)std::min<size_t>(((size_t)n + kRasterThreads - 1) / kRasterThreads, (size_t)e->sm_count * 8);
     int64_t launches = 0;
@@ -2157,20 +2205,22 @@ nbg_status order_raster(nbg_engine *e, unsigned n, int t0, int count, unsigned *
                                                                    (int)e->N, e->rbm.p);
         k_raster_count<<<tiles, kRasterThreads, 0, e->stream>>>(reinterpret_cast<const uint4 *>(e->rbm.p),
                                                                 e->rtile.p);
-        k_raster_scan<<<1, kRasterScanThreads, 0, e->stream>>>(e->rtile.p, tiles, e->rbase.p);
+        k_raster_scan<<<1, kRasterScanThreads, 0, e->stream>>>(e->rtile.p, tiles, base);
         k_raster_emit<<<tiles, kRasterThreads, 0, e->stream>>>(reinterpret_cast<const uint4 *>(e->rbm.p),
                                                                e->rtile.p, wp, t0 + c0, e->ord_ids.p, e->ord_t.p);
         launches += 4;
     }
     NBG_CUDA(cudaGetLastError());
     NBG_CUDA(cudaEventRecord(e->evr1, e->stream));
-    NBG_CUDA(cudaMemcpyAsync(n_out, e->rbase.p, sizeof(unsigned), cudaMemcpyDeviceToHost, e->stream));
+    NBG_CUDA(cudaMemcpyAsync(e->pin_words, e->words.p, e->kWords * sizeof(unsigned int), cudaMemcpyDeviceToHost, e->stream));
+    NBG_CUDA(cudaMemcpyAsync(e->pin_ids, e->ord_ids.p, n * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    NBG_CUDA(cudaMemcpyAsync(e->pin_t, e->ord_t.p, n * sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    NBG_CUDA(cudaEventRecord(e->evr2, e->stream));
     NBG_CUDA(cudaStreamSynchronize(e->stream));
-    float ms = 0.0f;
-    NBG_CUDA(cudaEventElapsedTime(&ms, e->evr0, e->evr1));
-    e->last_order_ms = ms;
+    const unsigned ordered = e->pin_words[nbg_engine::kOrdered];
+    if (ordered != n) return fail(NBG_ERR_STATE, "raster holds %u entries but %u distinct (step, neuron) pairs", n, ordered);
+    e->raster_timed = true;
     e->last_order_launches = launches;
-    if (*n_out != n) return fail(NBG_ERR_STATE, "raster holds %u entries but %u distinct (step, neuron) pairs", n, *n_out);
     return NBG_OK;
 }
 
@@ -2677,6 +2727,7 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
     chk(cudaEventCreate(&e->ev1), "event");
     chk(cudaEventCreate(&e->evr0), "event");
     chk(cudaEventCreate(&e->evr1), "event");
+    chk(cudaEventCreate(&e->evr2), "event");
     chk(cudaDeviceGetAttribute(&e->sm_count, cudaDevAttrMultiProcessorCount, e->device), "SM count");
     // the decay-table head in dynamic shared memory comes on top of the
     // kernel's static staging arrays: above the 48 KiB a launch gets by default
@@ -2727,9 +2778,13 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
         if (!prefix) chk(e->upd_ids_d.upload(upd), "thread map");
         if (!gen.empty()) chk(e->gen_ids_d.upload(gen), "generator ids");
     }
-    chk(e->err.alloc(1), "err");
-    chk(e->run_t0.alloc(1), "run_t0");
-    chk(e->cursor.alloc(1), "cursor");
+    chk(e->words.alloc(nbg_engine::kWords), "run words");
+    chk(cudaMallocHost(&e->pin_words, nbg_engine::kWords * sizeof(unsigned int)), "run words");
+    chk(cudaMallocHost(&e->pin_state, nbg_engine::kPinState), "state staging");
+    chk(e->init_v_d.upload(e->init_v), "initial v");
+    chk(e->init_u_d.upload(e->init_u), "initial u");
+    chk(e->init_iext_d.upload(e->init_iext), "initial current");
+    for (auto *h : {&e->init_v, &e->init_u, &e->init_iext}) std::vector<float>().swap(*h);
     chk(e->ev_cursor.alloc(1), "ev_cursor");
     chk(e->n_events.alloc(1), "n_events");
     if (e->ev_cap > 0) {
@@ -2757,12 +2812,16 @@ nbg_status nbg_destroy(nbg_engine *e) {
     if (e->ev0) cudaEventDestroy(e->ev0);
     if (e->evr0) cudaEventDestroy(e->evr0);
     if (e->evr1) cudaEventDestroy(e->evr1);
+    if (e->evr2) cudaEventDestroy(e->evr2);
     if (e->ev1) cudaEventDestroy(e->ev1);
     for (auto ev : e->tev)
         if (ev) cudaEventDestroy(ev);
     if (e->stream) cudaStreamDestroy(e->stream);
     if (e->pin_ids) cudaFreeHost(e->pin_ids);
     if (e->pin_t) cudaFreeHost(e->pin_t);
+    if (e->pin_words) cudaFreeHost(e->pin_words);
+    if (e->pin_state) cudaFreeHost(e->pin_state);
+    if (e->pin_ext) cudaFreeHost(e->pin_ext);
     delete e;
     return NBG_OK;
 }
@@ -2782,19 +2841,15 @@ nbg_status nbg_reset_neurons(nbg_engine *e, int first, int count) {
     NBG_CUDA(cudaSetDevice(e->device));
     NBG_CUDA(cudaStreamSynchronize(e->stream));
     const size_t f = (size_t)first, c = (size_t)count;
-    NBG_CUDA(cudaMemcpy(e->v.p + f, e->init_v.data() + f, c * sizeof(float), cudaMemcpyHostToDevice));
-    NBG_CUDA(cudaMemcpy(e->u.p + f, e->init_u.data() + f, c * sizeof(float), cudaMemcpyHostToDevice));
-    NBG_CUDA(cudaMemcpy(e->iext.p + f, e->init_iext.data() + f, c * sizeof(float), cudaMemcpyHostToDevice));
-    NBG_CUDA(cudaMemset(e->gexc.p + f, 0, c * sizeof(float)));
-    NBG_CUDA(cudaMemset(e->ginh.p + f, 0, c * sizeof(float)));
-    const std::vector<int> last0(c, 10000);
-    NBG_CUDA(cudaMemcpy(e->last.p + f, last0.data(), c * sizeof(int), cudaMemcpyHostToDevice));
+    reset_neurons(e, first, count);
+    NBG_CUDA(cudaGetLastError());
     // pending arrivals: the range's mask words in every ring slot (summary
     // bits left set only make the next drain read a zero word)
     const int w0 = e->woff_host[f], w1 = e->woff_host[f + c];
     if (w1 > w0)
-        NBG_CUDA(cudaMemset2D(e->mask.p + w0, (size_t)e->Wt * sizeof(unsigned int), 0,
-                              (size_t)(w1 - w0) * sizeof(unsigned int), (size_t)e->D));
+        NBG_CUDA(cudaMemset2DAsync(e->mask.p + w0, (size_t)e->Wt * sizeof(unsigned int), 0,
+                                   (size_t)(w1 - w0) * sizeof(unsigned int), (size_t)e->D, e->stream));
+    NBG_CUDA(cudaStreamSynchronize(e->stream));
     return NBG_OK;
 }
 
@@ -2833,25 +2888,27 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
         std::sort(ext_due.begin(), ext_due.end());
     }
     if (!ext_due.empty() || e->ext_ptr_d.p) {
-        if ((int64_t)e->ext_ptr_d.n < count + 1) NBG_CUDA(e->ext_ptr_d.alloc((size_t)count + 1));
-        if (e->ext_ids_d.n < std::max<size_t>(ext_due.size(), 1))
-            NBG_CUDA(e->ext_ids_d.alloc(std::max<size_t>(ext_due.size(), 1)));
-        e->ext_ptr_h.assign((size_t)count + 1, 0);
-        e->ext_ids_h.resize(ext_due.size());
-        for (size_t k = 0; k < ext_due.size(); ++k) {
-            e->ext_ptr_h[(size_t)(ext_due[k].first - t0) + 1]++;
-            e->ext_ids_h[k] = ext_due[k].second;
+        const size_t np = (size_t)count + 1, ni = ext_due.size();
+        if (e->ext_ptr_d.n < np) NBG_CUDA(e->ext_ptr_d.alloc(np));
+        if (e->ext_ids_d.n < std::max<size_t>(ni, 1)) NBG_CUDA(e->ext_ids_d.alloc(std::max<size_t>(ni + ni / 2, 1)));
+        if (e->pin_ext_cap < np + ni) {
+            if (e->pin_ext) cudaFreeHost(e->pin_ext);
+            e->pin_ext = nullptr;
+            e->pin_ext_cap = 0;
+            NBG_CUDA(cudaMallocHost(&e->pin_ext, (np + ni + ni / 2) * sizeof(int)));
+            e->pin_ext_cap = np + ni + ni / 2;
         }
-        for (int k = 0; k < count; ++k) e->ext_ptr_h[(size_t)k + 1] += e->ext_ptr_h[(size_t)k];
-        NBG_CUDA(cudaMemcpyAsync(e->ext_ptr_d.p, e->ext_ptr_h.data(), ((size_t)count + 1) * sizeof(int),
-                                 cudaMemcpyHostToDevice, e->stream));
-        if (!ext_due.empty())
-            NBG_CUDA(cudaMemcpyAsync(e->ext_ids_d.p, e->ext_ids_h.data(), ext_due.size() * sizeof(int),
-                                     cudaMemcpyHostToDevice, e->stream));
+        int *const ptr = e->pin_ext, *const ids = e->pin_ext + np;
+        std::fill(ptr, ptr + np, 0);
+        for (size_t k = 0; k < ni; ++k) {
+            ptr[(size_t)(ext_due[k].first - t0) + 1]++;
+            ids[k] = ext_due[k].second;
+        }
+        for (int k = 0; k < count; ++k) ptr[(size_t)k + 1] += ptr[(size_t)k];
+        NBG_CUDA(cudaMemcpyAsync(e->ext_ptr_d.p, ptr, np * sizeof(int), cudaMemcpyHostToDevice, e->stream));
+        if (ni > 0) NBG_CUDA(cudaMemcpyAsync(e->ext_ids_d.p, ids, ni * sizeof(int), cudaMemcpyHostToDevice, e->stream));
     }
-    NBG_CUDA(cudaMemcpyAsync(e->run_t0.p, &t0, sizeof(int), cudaMemcpyHostToDevice, e->stream));
-    NBG_CUDA(cudaMemsetAsync(e->cursor.p, 0, sizeof(unsigned int), e->stream));
-    NBG_CUDA(cudaMemsetAsync(e->err.p, 0, sizeof(int), e->stream));
+    k_run_begin<<<1, 1, 0, e->stream>>>(e->words.p, t0);
     const NetDev nd = e->dev();
 
     e->last_upd_ms = 0.0;
@@ -2900,7 +2957,9 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
                                                     const nbg_engine::CurrentEvent &b) { return a.t < b.t; });
     }
     const int t_end = t0 + count;
-    if (e->use_graph && due.empty()) {
+    // a few blocks cost less launched one by one than as a graph (about 3 us
+    // each against 10 for the graph's launch, and no instantiation)
+    if (e->use_graph && due.empty() && count > 3 * B) {
         // the whole call as one graph: nfull blocks of B steps and a tail block
         const int nfull = count / B, tail = count % B;
         const int nblocks = nfull + (tail ? 1 : 0);
@@ -2914,8 +2973,8 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
             }
             cudaGraph_t g;
             NBG_CUDA(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-            for (int k = 0; k < nfull; ++k) launch_block(e, nd, B, k * B, k, true);
-            if (tail) launch_block(e, nd, tail, nfull * B, nfull, true);
+            for (int k = 0; k < nfull; ++k) launch_block(e, nd, B, k * B, k, true, k > 0);
+            if (tail) launch_block(e, nd, tail, nfull * B, nfull, true, nfull > 0);
             NBG_CUDA(cudaStreamEndCapture(e->stream, &g));
             cudaError_t ie = cudaGraphInstantiate(&e->graph, g, 0);
             cudaGraphDestroy(g);
@@ -2950,7 +3009,7 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
             int slot = 0;
             for (int k = 0; k < nblocks; ++k) {
                 const int bk = std::min(B, seg - k * B);
-                launch_block(e, nd, bk, t + k * B - t0, slot++);
+                launch_block(e, nd, bk, t + k * B - t0, slot++, false, launches > 0);
                 ++launches;
                 if (slot == kLaunchChunk) {
                     nbg_status hs = harvest_timing(e, slot);
@@ -2965,14 +3024,14 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
     }
     NBG_CUDA(cudaGetLastError());
     NBG_CUDA(cudaEventRecord(e->ev1, e->stream));
+    NBG_CUDA(cudaMemcpyAsync(e->pin_words, e->words.p, e->kWords * sizeof(unsigned int), cudaMemcpyDeviceToHost, e->stream));
     NBG_CUDA(cudaStreamSynchronize(e->stream));
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, e->ev0, e->ev1);
     e->last_ms = ms;
     e->last_launches = launches;
 
-    int errv = 0;
-    NBG_CUDA(cudaMemcpy(&errv, e->err.p, sizeof(int), cudaMemcpyDeviceToHost));
+    const int errv = (int)e->pin_words[nbg_engine::kErrWord];
     e->next_t += count;
     e->ran = true;
     if (errv & kErrEventLog) return fail(NBG_ERR_OVERFLOW, "delivered-event log capacity exceeded");
@@ -2981,41 +3040,25 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
     // raster: the device's unordered (step, id) entries, ordered on the
     // device, downloaded through pinned staging buffers and merged with the
     // external spikes of output neurons
-    unsigned ndev = 0;
-    NBG_CUDA(cudaMemcpy(&ndev, e->cursor.p, sizeof(ndev), cudaMemcpyDeviceToHost));
+    const unsigned ndev = e->pin_words[nbg_engine::kCursor];
+    e->raster_timed = false;
+    e->last_order_ms = e->last_download_ms = 0.0;
+    e->last_order_launches = 0;
     // The step loop has run and the engine's time has moved on, so a failed
     // device ordering must not drop the call's spikes: the unordered entries
     // are then downloaded and ordered on the host instead.
-    const int *ord_ids = nullptr, *ord_t = nullptr;
     bool host_order = false;
-    {
-        unsigned nord = 0;
-        if (order_raster(e, ndev, t0, count, &nord) == NBG_OK) { // ordering may have grown ord_ids / ord_t
-            ord_ids = e->ord_ids.p;
-            ord_t = e->ord_t.p;
-        } else {
+    if (ndev > 0) {
+        nbg_status rs = pin_raster(e, ndev);
+        if (rs != NBG_OK) return rs;
+        if (order_raster(e, ndev, t0, count) != NBG_OK) {
             cudaGetLastError(); // an allocation failure is not sticky: clear it
             NBG_CUDA(cudaStreamSynchronize(e->stream));
-            ord_ids = e->out_ids.p;
-            ord_t = e->out_t.p;
+            NBG_CUDA(cudaMemcpy(e->pin_ids, e->out_ids.p, ndev * sizeof(int), cudaMemcpyDeviceToHost));
+            NBG_CUDA(cudaMemcpy(e->pin_t, e->out_t.p, ndev * sizeof(int), cudaMemcpyDeviceToHost));
             host_order = true;
             e->last_order_launches = -1;
         }
-    }
-    const auto h0 = std::chrono::steady_clock::now();
-    if ((size_t)ndev > e->pin_cap) { // grown by half again when short
-        if (e->pin_ids) cudaFreeHost(e->pin_ids);
-        if (e->pin_t) cudaFreeHost(e->pin_t);
-        e->pin_ids = e->pin_t = nullptr;
-        e->pin_cap = 0;
-        const size_t cap = (size_t)ndev + (size_t)ndev / 2;
-        NBG_CUDA(cudaMallocHost(&e->pin_ids, cap * sizeof(int)));
-        NBG_CUDA(cudaMallocHost(&e->pin_t, cap * sizeof(int)));
-        e->pin_cap = cap;
-    }
-    if (ndev > 0) {
-        NBG_CUDA(cudaMemcpy(e->pin_ids, ord_ids, ndev * sizeof(int), cudaMemcpyDeviceToHost));
-        NBG_CUDA(cudaMemcpy(e->pin_t, ord_t, ndev * sizeof(int), cudaMemcpyDeviceToHost));
     }
     if (host_order && ndev > 1) { // (step, id) order on the host
         std::vector<uint64_t> key((size_t)ndev);
@@ -3035,7 +3078,6 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
         append_raster(e, e->pin_t, e->pin_ids, (size_t)ndev, ext_rec);
     }
     const auto h2 = std::chrono::steady_clock::now();
-    e->last_download_ms = std::chrono::duration<double, std::milli>(h1 - h0).count();
     e->last_append_ms = std::chrono::duration<double, std::milli>(h2 - h1).count();
     if (ntr > 0) {
         const size_t rb = e->trace_rows.size();
@@ -3105,20 +3147,30 @@ nbg_status nbg_get_state(nbg_engine *e, int field, float *out) {
     NBG_CUDA(cudaSetDevice(e->device));
     NBG_CUDA(cudaStreamSynchronize(e->stream));
     const size_t bytes = (size_t)e->N * sizeof(float);
+    const void *src = nullptr;
     switch (field) {
-    case NBG_FIELD_V: NBG_CUDA(cudaMemcpy(out, e->v.p, bytes, cudaMemcpyDeviceToHost)); break;
-    case NBG_FIELD_U: NBG_CUDA(cudaMemcpy(out, e->u.p, bytes, cudaMemcpyDeviceToHost)); break;
-    case NBG_FIELD_G_EXC: NBG_CUDA(cudaMemcpy(out, e->gexc.p, bytes, cudaMemcpyDeviceToHost)); break;
-    case NBG_FIELD_G_INH: NBG_CUDA(cudaMemcpy(out, e->ginh.p, bytes, cudaMemcpyDeviceToHost)); break;
-    case NBG_FIELD_I_EXT: NBG_CUDA(cudaMemcpy(out, e->iext.p, bytes, cudaMemcpyDeviceToHost)); break;
-    case NBG_FIELD_LAST_SPIKE: {
-        std::vector<int> tmp((size_t)e->N);
-        NBG_CUDA(cudaMemcpy(tmp.data(), e->last.p, (size_t)e->N * sizeof(int), cudaMemcpyDeviceToHost));
-        for (int i = 0; i < e->N; ++i) out[i] = (float)tmp[i];
-        break;
-    }
+    case NBG_FIELD_V: src = e->v.p; break;
+    case NBG_FIELD_U: src = e->u.p; break;
+    case NBG_FIELD_G_EXC: src = e->gexc.p; break;
+    case NBG_FIELD_G_INH: src = e->ginh.p; break;
+    case NBG_FIELD_I_EXT: src = e->iext.p; break;
+    case NBG_FIELD_LAST_SPIKE: src = e->last.p; break;
     default: return fail(NBG_ERR_INVALID, "unknown state field %d", field);
     }
+    if (bytes <= nbg_engine::kPinState) { // through pinned memory: without the driver's own staging
+        std::lock_guard<std::mutex> lock(e->state_mu);
+        NBG_CUDA(cudaMemcpyAsync(e->pin_state, src, bytes, cudaMemcpyDeviceToHost, e->stream));
+        NBG_CUDA(cudaStreamSynchronize(e->stream));
+        std::memcpy(out, e->pin_state, bytes);
+    } else {
+        NBG_CUDA(cudaMemcpy(out, src, bytes, cudaMemcpyDeviceToHost));
+    }
+    if (field == NBG_FIELD_LAST_SPIKE) // int32 on the device
+        for (int i = 0; i < e->N; ++i) {
+            int k;
+            std::memcpy(&k, out + i, sizeof(k));
+            out[i] = (float)k;
+        }
     return NBG_OK;
 }
 
@@ -3411,6 +3463,14 @@ nbg_status nbg_profile(nbg_engine *e, double *total_ms, double *update_ms, doubl
 nbg_status nbg_raster_profile(nbg_engine *e, double *order_ms, double *download_ms, double *append_ms,
                               int64_t *order_launches) {
     if (!e) return fail(NBG_ERR_INVALID, "null engine");
+    if (e->raster_timed) { // the events of the last run call, read when asked for
+        float order = 0.0f, download = 0.0f;
+        NBG_CUDA(cudaEventElapsedTime(&order, e->evr0, e->evr1));
+        NBG_CUDA(cudaEventElapsedTime(&download, e->evr1, e->evr2));
+        e->last_order_ms = order;
+        e->last_download_ms = download;
+        e->raster_timed = false;
+    }
     if (order_ms) *order_ms = e->last_order_ms;
     if (download_ms) *download_ms = e->last_download_ms;
     if (append_ms) *append_ms = e->last_append_ms;
