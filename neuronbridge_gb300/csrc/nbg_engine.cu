@@ -424,6 +424,20 @@ __device__ __forceinline__ void post_stdp_lane(const NetDev &n, int s, int s1, i
     }
 }
 
+// Post-synaptic STDP (STDP::ApplyPostSynaticSpike) of every spiking lane at
+// step t, the warp striding over that neuron's in-synapses [base, end).
+template <class S>
+__device__ __forceinline__ void post_passes(const NetDev &n, int base, int end, int lane, bool spk, int t) {
+    unsigned int sbal = S::plastic(n) ? __ballot_sync(0xffffffffu, spk && end > base) : 0u;
+    while (sbal) {
+        const int l = __ffs(sbal) - 1;
+        sbal &= sbal - 1u;
+        const int s0 = __shfl_sync(0xffffffffu, base, l), s1 = __shfl_sync(0xffffffffu, end, l);
+        post_stdp_lane<S>(n, s0 + lane, s1, t);
+    }
+    __syncwarp(); // the owners read these synapses at their next arrivals
+}
+
 // Apply one arrival on synapse s of a target, its record y already loaded:
 // its ProcessSpike with the weight as it is before this step's pre hook,
 // then the pre hook if the synapse is plastic (the decay factors of its gap,
@@ -730,6 +744,11 @@ __device__ __forceinline__ void stage_u32(unsigned int *dst, const unsigned int 
 }
 __device__ __forceinline__ void stage_16(void *dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned int)__cvta_generic_to_shared(dst)),
+                 "l"(__cvta_generic_to_global(src))
+                 : "memory");
+}
+__device__ __forceinline__ void stage_quad(uint4 *dst, const unsigned int *src) { // past L1: read once
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned int)__cvta_generic_to_shared(dst)),
                  "l"(__cvta_generic_to_global(src))
                  : "memory");
 }
@@ -1229,16 +1248,7 @@ __global__ void __launch_bounds__(256, S::min_blocks) k_update(const __grid_cons
                 asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(n.out_ptr + j)));
             spk_steps |= 1u << b;
         }
-        // post-synaptic STDP (STDP::ApplyPostSynaticSpike) of every spiking
-        // lane, the warp striding over that neuron's in-synapses
-        unsigned int sbal = S::plastic(n) ? __ballot_sync(0xffffffffu, spk && end > base) : 0u;
-        while (sbal) {
-            const int l = __ffs(sbal) - 1;
-            sbal &= sbal - 1u;
-            const int s0 = __shfl_sync(0xffffffffu, base, l), s1 = __shfl_sync(0xffffffffu, end, l);
-            post_stdp_lane<S>(n, s0 + lane, s1, t);
-        }
-        __syncwarp(); // the owners read these synapses at their next arrivals
+        post_passes<S>(n, base, end, lane, spk, t);
     }
     if (active) {
         n.v[j] = r.v;
@@ -1268,9 +1278,9 @@ __global__ void __launch_bounds__(256, S::min_blocks) k_update(const __grid_cons
 //     bit costs its isolation, two tests, selects and one addition;
 //   * the four words are run through by the whole warp one after another, each
 //     until its fullest lane is done, in ascending order as before.
-// Measured per launch of 15 steps: 1,000 neurons 48.8 -> 25.6 us; 16 networks of
-// 500 to 50,000 neurons (172,000 in all) 113 (record drain with codes) -> 74.5
-// us.
+// Measured per launch of 15 steps: 1,000 neurons 48.8 -> 23.2 us (25.6 without
+// the staged second quad); 16 networks of 500 to 50,000 neurons (172,000 in all)
+// 113 (record drain with codes) -> 74.5 us.
 template <class S>
 __device__ __forceinline__ void apply_quad_word(unsigned int word, uint2 code, const float (&sw)[kPaletteSize],
                                                 unsigned int types, bool split, float &a, float &b) {
@@ -1355,16 +1365,17 @@ __global__ void __launch_bounds__(256, 4) k_update_quad(const __grid_constant__ 
     }
     const unsigned int D = (unsigned int)n.D;
     const unsigned int slot0 = (unsigned int)T0 % D; // the block's first slot; later ones by wrap_slot
-    // quads in flight: [step % 4][thread], read by the thread that asked for them
-    __shared__ uint4 s_quad[4][256];
+    // quads in flight: [step % 4][thread], read by the thread that asked for
+    // them; the second one of the few neurons that have one (in-degrees around
+    // 100 reach past 128 now and then), which a warp would wait for otherwise
+    __shared__ uint4 s_quad[4][256], s_quad1[4][256];
     const bool staged = active && nq > 0;
     auto row = [&](int b) { return n.mask + (size_t)wrap_slot(slot0 + (unsigned int)b, D) * n.Wt + woff; };
     auto stage = [&](int b) {
-        if (staged && b < B)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                             (unsigned int)__cvta_generic_to_shared(&s_quad[b & 3][threadIdx.x])),
-                         "l"(__cvta_generic_to_global(row(b)))
-                         : "memory");
+        if (staged && b < B) {
+            stage_quad(&s_quad[b & 3][threadIdx.x], row(b));
+            if (nq > 1) stage_quad(&s_quad1[b & 3][threadIdx.x], row(b) + 4);
+        }
         stage_commit();
     };
     stage(0);
@@ -1402,7 +1413,7 @@ __global__ void __launch_bounds__(256, 4) k_update_quad(const __grid_constant__ 
             }
             for (int x = 1; x < nq; ++x) { // in-degrees above 128
                 unsigned int *const mrow = row(b) + 4 * x;
-                const uint4 e = *reinterpret_cast<const uint4 *>(mrow);
+                const uint4 e = x == 1 ? s_quad1[b & 3][threadIdx.x] : *reinterpret_cast<const uint4 *>(mrow);
                 if (e.x | e.y | e.z | e.w) *reinterpret_cast<uint4 *>(mrow) = make_uint4(0u, 0u, 0u, 0u);
                 unsigned int we[4] = {e.x, e.y, e.z, e.w};
 #pragma unroll
@@ -1433,6 +1444,164 @@ __global__ void __launch_bounds__(256, 4) k_update_quad(const __grid_constant__ 
         n.last[j] = r.last;
     }
     __syncwarp();
+    leave_warp(n, j, lane, active && L.record, spk_steps, T0, slot0, delivered);
+}
+
+// ------------------------------------------------- plastic networks in quads
+//
+// k_update for plastic networks whose neurons have one quad of mask words each
+// (in-degree at most 128): the same steps, arrivals, learning and propagation,
+// with the quad in place of the word summary and the words it points at.
+//
+// What bounds it: as k_update, the chain of a warp's steps, of which finding
+// the arrivals (the summary's two words asked for three steps ahead, decoded
+// and cleared with atomics, the flagged word two steps ahead) was the largest
+// part after the arrivals themselves.  A quad is one 16-byte copy two steps
+// ahead and one store; the deep form still stages the record of the next
+// step's first arrival, found in the quad that has come.  The ring row of a
+// step is read whole (16 bytes a neuron: 16 MB per 10 steps of 100,000, where
+// the launch has bandwidth to spare), and a spike marks one word per synapse
+// instead of two.  Measured per launch of 10 steps: 100,000 Izhikevich neurons
+// with 10 million synapses 28.0 -> 24.6 us, 5,000 with 500,000 16.1 -> 15.0 us;
+// the control loop of 500 plastic LIF neurons 62 -> 54 us of device time a call.
+template <class S>
+__global__ void __launch_bounds__(256, S::min_blocks) k_update_quad_rec(const __grid_constant__ NetDev n, int B, int toff) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    const int reg_blocks = (n.N_upd + (int)blockDim.x - 1) / (int)blockDim.x;
+    const bool gen_block = (int)blockIdx.x >= reg_blocks;
+    const bool active = !gen_block && tid < n.N_upd;
+    const int j = active && n.upd_ids ? n.upd_ids[tid] : tid;
+    const int lane = threadIdx.x & 31;
+    const int run_t0 = *n.run_t0;
+    const int T0 = run_t0 + toff;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // as in k_update
+    for (int k = threadIdx.x; k < n.sdtab_len; k += blockDim.x) s_dtab[k] = n.dtab[k];
+    if (n.sdtab_len) __syncthreads();
+
+    Model L;
+    NeuronRegs r;
+    int base = 0, end = 0, woff = 0, tslot = -1, g0 = 0, g1 = 0;
+    if (active) {
+        L = load_model(n.layers[n.pop[j]]);
+        base = n.csc_ptr[j];
+        end = n.csc_ptr[j + 1];
+        woff = n.woff[j];
+        if (n.trace_slot) tslot = n.trace_slot[j];
+        g0 = n.gen_ptr[j];
+        g1 = n.gen_ptr[j + 1];
+    }
+    int gen_local = 0, gen_delay = 0, gen_pos = 0; // the first generator input
+    float gen_prob = -1.0f;                        // never fires
+    if (active && g0 < g1) {
+        gen_prob = generator_prob(n, n.gen_src[g0], &gen_local);
+        gen_delay = n.gen_delay[g0];
+        gen_pos = n.gen_pos[g0];
+    }
+    // everything below reads or writes what the previous block's launch wrote
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    mark_external(n, tid, lane, B, T0, toff);
+    if (gen_block) { // whole CTAs of generator threads
+        generator_steps(n, tid - reg_blocks * (int)blockDim.x, B, T0, run_t0, lane);
+        return;
+    }
+    if (active) {
+        r.v = n.v[j];
+        r.u = n.u[j];
+        r.gexc = r.ginh = 0.0f; // no model of these profiles has conductances
+        r.iext = n.iext[j];
+        r.last = n.last[j];
+        r.lif_cur = 0.0f;
+        if (S::has(NBG_MODEL_LIF_VJ) && L.model == NBG_MODEL_LIF_VJ) // current_dV += R * I / tau (two roundings)
+            r.lif_cur = r.lif_cur + L.p[3] * r.iext / L.p[1];
+    }
+    const bool noisy = S::has(NBG_MODEL_IZH_RK4) && active && L.model == NBG_MODEL_IZH_RK4 && L.p[5] != 0.0f;
+    const unsigned int nkey = noisy ? noise_key(n.seed, j) : 0u;
+    const unsigned int D = (unsigned int)n.D;
+    const unsigned int slot0 = (unsigned int)T0 % D; // the block's first slot; later ones by wrap_slot
+    // in flight: the quad of the step after next, and (deep) the record of the
+    // next step's first arrival, [step parity][thread]; pos_nxt is its CSC
+    // position (-1: none, or stale)
+    __shared__ uint4 s_quad[2][256];
+    __shared__ uint4 s_rec[S::deep ? 2 * 256 * 2 : 1];
+    int pos_nxt = -1;
+    const bool staged = active && end > base;
+    auto row = [&](int b) { return n.mask + (size_t)wrap_slot(slot0 + (unsigned int)b, D) * n.Wt + woff; };
+    uint4 q_cur = make_uint4(0u, 0u, 0u, 0u);
+    if (staged) {
+        q_cur = *reinterpret_cast<const uint4 *>(row(0));
+        if (B > 1) stage_quad(&s_quad[1][threadIdx.x], row(1));
+        stage_commit();
+    }
+    unsigned long long delivered = 0;
+    unsigned int spk_steps = 0u; // bit b: this neuron spiked at step T0 + b
+    for (int b = 0; b < B; ++b) {
+        const int t = T0 + b;
+        bool spk = false;
+        const int pos_cur = pos_nxt; // deep: the staged record of this step, if any
+        pos_nxt = -1;
+        if (active) {
+            float acc_a = 0.0f, acc_b = 0.0f;
+            const bool gate = r.last > L.ip;
+            const uint4 q = q_cur;
+            if (staged) stage_wait(); // the quad of step b + 1, the record of pos_cur
+            if (staged && b + 1 < B) {
+                q_cur = s_quad[(b + 1) & 1][threadIdx.x];
+                if (b + 2 < B) stage_quad(&s_quad[b & 1][threadIdx.x], row(b + 2));
+                if constexpr (S::deep) {
+                    if (q_cur.x | q_cur.y | q_cur.z | q_cur.w) { // the record of step b + 1's first arrival
+                        const int wi = q_cur.x ? 0 : q_cur.y ? 1 : q_cur.z ? 2 : 3;
+                        const unsigned int fw = q_cur.x ? q_cur.x : q_cur.y ? q_cur.y : q_cur.z ? q_cur.z : q_cur.w;
+                        pos_nxt = base + wi * 32 + __ffs(fw) - 1;
+                        uint4 *const d = s_rec + (((b + 1) & 1) * 256 + threadIdx.x) * 2;
+                        stage_16(d, n.rec + pos_nxt);
+                        stage_16(d + 1, reinterpret_cast<const uint4 *>(n.rec + pos_nxt) + 1);
+                        const unsigned int rest = fw & (fw - 1u); // the record of its second arrival into L2
+                        if (rest) prefetch_syn<S>(n, base + wi * 32 + __ffs(rest) - 1);
+                    }
+                }
+                stage_commit();
+            }
+            unsigned int w[4] = {q.x, q.y, q.z, q.w};
+            if (q.x | q.y | q.z | q.w) *reinterpret_cast<uint4 *>(row(b)) = make_uint4(0u, 0u, 0u, 0u);
+            // generator arrivals (pure functions of source and time)
+            if (g0 < g1) {
+                const bool fired = t >= gen_delay && hash_uniform01(gen_local, t - gen_delay) < gen_prob;
+                const unsigned int gbit = fired ? 1u << (gen_pos & 31) : 0u;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) w[k] |= (gen_pos >> 5) == k ? gbit : 0u;
+                for (int g = g0 + 1; g < g1; ++g) // further generator inputs
+                    if (generator_fired(n, n.gen_src[g], t - (int)n.gen_delay[g])) {
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) w[k] |= (n.gen_pos[g] >> 5) == k ? 1u << (n.gen_pos[g] & 31) : 0u;
+                    }
+            }
+            if (w[0] | w[1] | w[2] | w[3]) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    delivered += __popc(w[k]);
+                    if constexpr (S::deep)
+                        apply_word_staged<S>(n, L, r, acc_a, acc_b, gate, w[k], base + k * 32, t, pos_cur,
+                                             s_rec + ((b & 1) * 256 + threadIdx.x) * 2, pos_nxt);
+                    else
+                        apply_word_batched<S>(n, L, r, acc_a, acc_b, gate, w[k], base + k * 32, t);
+                }
+            }
+            spk = update_neuron<S>(n, L, r, acc_a, acc_b, noisy ? L.p[5] * gauss12(nkey, t) : 0.0f, j, t);
+            if (tslot >= 0) n.trace[(size_t)(t - run_t0) * n.ntrace + tslot] = r.v;
+        }
+        if (spk) {
+            pos_nxt = -1; // the post-synaptic pass below rewrites every record of this neuron
+            if (!spk_steps) // the out-list bounds the propagation reads after the last step
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(__cvta_generic_to_global(n.out_ptr + j)));
+            spk_steps |= 1u << b;
+        }
+        post_passes<S>(n, base, end, lane, spk, t);
+    }
+    if (active) {
+        n.v[j] = r.v;
+        n.u[j] = r.u;
+        n.last[j] = r.last;
+    }
     leave_warp(n, j, lane, active && L.record, spk_steps, T0, slot0, delivered);
 }
 
@@ -1518,6 +1687,7 @@ struct nbg_engine {
     std::vector<unsigned char> type_bits; // palette networks: synapse types, CSC order, one bit each
     void (*plain_kernel)(NetDev, int, int) = nullptr;
     void (*palette_kernel)(NetDev, int, int) = nullptr;
+    bool rec_quads = false; // plain_kernel is k_update_quad_rec
     DevBuf<float> init_w_d; // weights reset returns to, CSC order
     DevBuf<unsigned int> orig_pos_d; // orig_pos, from the first nbg_get_weights on
     DevBuf<float> wout;              // its staging
@@ -1618,7 +1788,7 @@ struct nbg_engine {
         n.dtab_len = dtab_len;
         n.sdtab_len = plastic && n_rules > 0 ? std::min(dtab_len, kSharedDecayEntries) : 0;
         n.mask = mask.p;
-        n.wsum = palette_n > 0 ? nullptr : wsum.p;
+        n.wsum = palette_n > 0 || rec_quads ? nullptr : wsum.p;
         n.Ws = Ws;
         n.out_ptr = out_ptr.p;
         n.out_pk = out_pk.p;
@@ -2546,6 +2716,7 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
             e->plain_kernel = k_update<Spec<lif_poisson, 0>>;
             e->palette_kernel = k_update_quad<Spec<lif_poisson, 0>>;
         } else if ((models & ~lif_inputs) == 0u && e->plastic) {
+            // (in quads where it may, below; of k_update:)
             // wide drain: 97 us a launch against 110 deep and 119 by the generic
             // instance (20,000 Poisson-driven neurons, plastic recurrent synapses),
             // and no slower where arrivals are few (the 500-neuron control loop: 58,
@@ -2554,26 +2725,36 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
         } else {
             e->plain_kernel = k_update<GenericSpec>;
         }
-        e->update_kernel = e->plain_kernel;
-        // Palette networks: at most kPaletteSize pairs, no log of delivered
-        // events (its entries name the synapse), and at least 2 of the 4
-        // words of a quad used on average, so that the padded ring is at most
-        // twice the words that synapses have.
-        if (e->palette_kernel) {
-            int64_t words = 0, padded = 0;
-            for (int j = 0; j < e->N; ++j) {
-                const int nw = (indeg[j + 1] + 31) / 32;
-                words += nw;
-                padded += (nw + 3) / 4 * 4;
-            }
-            if (e->ev_cap > 0 || S == 0 || padded > 2 * words || padded > (1 << 27) ||
-                !collect_palette(d->weight, S, [&](int64_t s) { return (unsigned int)(d->type[s] & 1); }, e->palette_host,
-                                 e->palette_n))
-                e->palette_kernel = nullptr;
+        // Quads: on average at least 2 of the 4 words of a quad hold synapses,
+        // so that the padded ring is at most twice the words that synapses have.
+        int64_t words = 0, padded = 0;
+        int most = 0;
+        for (int j = 0; j < e->N; ++j) {
+            const int nw = (indeg[j + 1] + 31) / 32;
+            words += nw;
+            padded += (nw + 3) / 4 * 4;
+            most = std::max(most, nw);
         }
+        const bool quads = S > 0 && padded <= 2 * words && padded <= (1 << 27);
+        // plastic: one quad per neuron (a second one would be waited for at
+        // every step)
+        if (quads && most <= 4 && e->plain_kernel == k_update<Spec<1u << NBG_MODEL_IZH_RK4, 1>>) {
+            e->plain_kernel = k_update_quad_rec<Spec<1u << NBG_MODEL_IZH_RK4, 1>>;
+            e->rec_quads = true;
+        } else if (quads && most <= 4 && e->plain_kernel == k_update<Spec<lif_inputs, 1, false>>) {
+            e->plain_kernel = k_update_quad_rec<Spec<lif_inputs, 1, false>>;
+            e->rec_quads = true;
+        }
+        e->update_kernel = e->plain_kernel;
+        // Palette networks: at most kPaletteSize pairs, and no log of delivered
+        // events (its entries name the synapse).
+        if (e->palette_kernel && (!quads || e->ev_cap > 0 ||
+                                  !collect_palette(d->weight, S, [&](int64_t s) { return (unsigned int)(d->type[s] & 1); },
+                                                   e->palette_host, e->palette_n)))
+            e->palette_kernel = nullptr;
     }
-    // ---- mask word offsets (whole quads for palette networks) and per-synapse arrays
-    const int word_group = e->palette_kernel ? 4 : 1;
+    // ---- mask word offsets (whole quads where a kernel reads quads) and per-synapse arrays
+    const int word_group = e->palette_kernel || e->rec_quads ? 4 : 1;
     std::vector<int> woff((size_t)e->N + 1, 0);
     for (int j = 0; j < e->N; ++j) {
         const int nw = (cptr[j + 1] - cptr[j] + 31) / 32;
