@@ -330,10 +330,10 @@ __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_segment(
 // can be asked for, so a step is one chain -- spike list, row loads, sums,
 // threshold, list -- and a warp's own instructions on it weigh as much as the
 // loads' latency.  So:
-//   * a thread owns two neighbouring columns (four above 1,024 neurons, single
-//     ones where N or a pointer is not aligned), adds them packed, and has up
-//     to 24 rows in flight; the list holds byte offsets of rows, read four at
-//     a time, padded to whole groups of four;
+//   * a thread owns four neighbouring columns (two, or single ones, where N or
+//     a pointer is not aligned), adds them packed, and has up to 24 rows in
+//     flight; the list holds byte offsets of rows, read four at a time, padded
+//     to whole groups of four;
 //   * the input rows of step t + 1 do not depend on the spikes of step t: they
 //     are requested behind the recurrent rows of step t and summed into the
 //     next step's start value;
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_segment(
 // eight warps of four columns each, unpacked, 2.45 ms: 1,506 instructions a
 // warp and step, few of them waiting for memory).  A training step of 128 rows
 // x 1,024 neurons x 1,000 steps: 14.96 -> 11.50 ms.
-constexpr int kRing = 8;
+constexpr int kRing = 8, kHalfRing = kRing / 2;
 constexpr int kRowsMaxInputs = 4096;
 constexpr int kRowsMaxNeurons = 2048;
 
@@ -420,7 +420,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
     const float *__restrict__ c, const float *__restrict__ alpha, const float *__restrict__ theta,
     nbg_lif_grad_params p, int L, int B, int N) {
     static_assert(V == 1 || NC == V, "a group is the thread's neighbouring columns");
-    constexpr int kGroups = NC == 4 ? 3 : NC == 2 ? 6 : 8; // groups of four rows in flight: 48 registers at most
+    // groups of four rows in flight: 96 registers at most, 48 where 512 threads share them
+    constexpr int kGroups = kMaxThreads <= 256 ? 24 / NC : NC == 4 ? 3 : NC == 2 ? 6 : 8;
     constexpr int kSegs = V == 1 ? NC : 1;                 // segments of the ascending order: (column group, warp)
     __shared__ __align__(16) unsigned list[kRowsMaxNeurons + 4]; // ascending spikes of the step before: row offsets
     __shared__ int seg_cnt[64];                                  // spikes per (column group, warp)
@@ -494,13 +495,12 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
         for (int r = 0; r < 4; ++r)
             if (left > r) acc.add_scaled(xv[r], d[r]);
     };
-    auto ring_load = [&](int step, int slot) {
-        if (step < L) {
-            const float *xr = x + ((size_t)step * B + b) * C;
-            float *d = ring + slot * C;
-            for (int ch = tid; ch < C; ch += T) ring_copy(d + ch, xr + ch);
+    auto ring_load = [&](int step, int rows) { // rows step .. step + rows - 1 of the inputs
+        for (int ch = tid; ch < C; ch += T) {
+            const float *xr = x + ((size_t)step * B + b) * C + ch;
+            float *d = ring + (step % kRing) * C + ch;
+            for (int k = 0; k < rows && step + k < L; ++k) ring_copy(d + k * C, xr + (size_t)k * B * C);
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto list_inputs = [&](int step) { // one warp: the nonzero channels of `step`, ascending
         const float *xr = ring + (step % kRing) * C;
@@ -520,8 +520,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
     int n_spk = cnt[b];
     for (int k = tid; k < n_spk + 4; k += T) list[k] = k < n_spk ? (unsigned)spk[row + k] * row_bytes : 0u;
     if constexpr (kGather) {
-        for (int k = 0; k < kRing; ++k) ring_load(k, k);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        ring_load(0, kRing);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
         if (wid == 0) {
             list_inputs(0);
@@ -543,6 +543,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
         start.load(xi + row, 0u, at);
     }
     int lister = 0; // the warp that lists next
+    size_t o = row; // this step's row of the record
     for (int step = 0; step < L; ++step) {
         Row acc = start;
         const float ct = z ? c[step] : 0.0f;
@@ -564,9 +565,10 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
             }
             if (wid == lister && step + 2 < L) list_inputs(step + 2);
             lister = lister + 1 == nw ? 0 : lister + 1;
-            if (step > 0) ring_load(step + kRing - 1, (step - 1) % kRing); // over the row listed three steps ago
+            // half the ring at a time, over rows listed two steps ago and before
+            if (step > 0 && step % kHalfRing == 0) ring_load(step + kHalfRing, kHalfRing);
         } else {
-            if (more) start.load(xi + (size_t)(step + 1) * plane + row, 0u, at);
+            if (more) start.load(xi + o + plane, 0u, at);
         }
         for (int k = 0;;) {
 #pragma unroll
@@ -606,7 +608,8 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
                 seg_cnt[wid] = k;
             }
         }
-        if constexpr (kGather) asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 5) : "memory"); // the row listed next step
+        if constexpr (kGather) // rows asked for a step ago, the first of them listed next step
+            if (step % kHalfRing == 1) asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads(); // counts; everyone has read the list
         const unsigned lt = (1u << lane) - 1u;
         int total = 0;
@@ -637,7 +640,6 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
         if (tid < 4) list[total + tid] = 0u; // the last group's padding: row 0, not added
         // the record, and the next step's input term, off the spikes' chain
         {
-            const size_t o = (size_t)step * plane + row;
             float sv[NC];
 #pragma unroll
             for (int i = 0; i < NC; ++i) sv[i] = sp[i] ? 1.0f : 0.0f;
@@ -684,6 +686,7 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
                 add_in(start, di[0], xv[0], n_in - k);
             }
         }
+        o += plane;
         __syncthreads(); // the list; the input list of step + 2
     }
 #pragma unroll
@@ -697,10 +700,11 @@ __global__ void __launch_bounds__(kMaxThreads) k_lif_fwd_rows(
     if (tid == 0) cnt[b] = n_spk;
 }
 
-// Launch k_lif_fwd_rows: neighbouring columns where N is a multiple of their
-// number and every matrix aligned to them, else single columns.  Two a thread
-// up to 1,024 neurons: sixteen warps issue a step's row loads and sums in half
-// the instructions a warp that eight warps of four columns take.
+// Launch k_lif_fwd_rows: four (two) neighbouring columns a thread where N is a
+// multiple of them and every matrix aligned, else single columns.  Eight warps
+// of four columns, 24 rows in flight, were faster than sixteen of two (1,000
+// neurons: 2.3 against 2.5 us a step): few more instructions a warp, half the
+// warps in each other's way.
 template <bool kGather>
 nbg_status launch_rows(const float *xi, const float *x, const float *w_in, int C, const float *w, int *spk, int *cnt,
                        float *v, int *ref, float *s_out, float *s_last, float *u_rec, unsigned char *m_rec,
@@ -713,12 +717,12 @@ nbg_status launch_rows(const float *xi, const float *x, const float *w_in, int C
                            (uintptr_t)u_rec | (uintptr_t)vprev_rec | (uintptr_t)m_rec * 4u;
     Kernel k;
     int threads;
-    if (N % 2 == 0 && N <= 1024 && (bits & 7u) == 0) {
+    if (N % 4 == 0 && (bits & 15u) == 0) {
+        threads = (N / 4 + 31) & ~31;
+        k = threads <= 256 ? k_lif_fwd_rows<kGather, 4, 4, 256> : k_lif_fwd_rows<kGather, 4, 4, 512>;
+    } else if (N % 2 == 0 && N <= 1024 && (bits & 7u) == 0) {
         threads = (N / 2 + 31) & ~31;
         k = k_lif_fwd_rows<kGather, 2, 2, 512>;
-    } else if (N % 4 == 0 && N > 1024 && (bits & 15u) == 0) {
-        threads = (N / 4 + 31) & ~31;
-        k = k_lif_fwd_rows<kGather, 4, 4, 512>;
     } else {
         threads = std::min(512, (N + 31) & ~31);
         const int nc = (N + threads - 1) / threads;
