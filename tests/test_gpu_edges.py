@@ -109,3 +109,20 @@ def test_weights_of_more_synapses_than_a_gather_chunk():
     got = sim.weights()
     assert np.array_equal(got["weight"], w)
     assert not got["apre"].any() and not got["apost"].any() and not got["last_update"].any()
+
+
+def test_a_reset_is_complete_when_the_next_call_starts():
+    """Trials of a network whose ring takes longer to clear than a run call takes to start: every trial after a reset
+    records the same spikes."""
+    from neuronbridge_gb300 import workloads
+
+    net, cfg = workloads.izhikevich_stdp(n=60_000, in_degree=100, steps=120, seed=6)
+    sim = nb.Simulation(net, cfg, seed=6)
+    first = None
+    for _ in range(12):
+        sim.reset()
+        sim.run(120)
+        t, i = sim.spike_raster()
+        if first is None:
+            first = t.copy(), i.copy()
+        assert len(t) > 0 and np.array_equal(t, first[0]) and np.array_equal(i, first[1])

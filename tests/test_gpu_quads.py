@@ -1,4 +1,4 @@
-"""Plastic networks in quads of mask words (in-degree up to 128) and beside them (more, or mostly one word a neuron),
+"""Plastic networks in quads of mask words (in-degree up to 128) and beside them (more, or mostly one word),
 bit for bit the CPU oracle: raster, state, weights and traces; noisy Izhikevich neurons with few arrivals, and LIF
 neurons with many, from recurrent synapses, Poisson generators and external spikes."""
 import numpy as np
@@ -48,7 +48,7 @@ def _lif(in_degree, n=90, n_in=20):
 
 
 @pytest.mark.parametrize("model", ["izhikevich", "lif"])
-@pytest.mark.parametrize("in_degree", [5, 32, 33, 64, 96, 97, 127, 128, 129])
+@pytest.mark.parametrize("in_degree", [5, 32, 33, 64, 96, 97, 127, 128, 129, 160])
 @pytest.mark.parametrize("threads,block_steps", [(256, 0), (32, 2)])
 def test_plastic_networks_equal_the_oracle(oracle_lib, model, in_degree, threads, block_steps):
     import oracle
