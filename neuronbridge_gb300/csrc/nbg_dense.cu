@@ -443,8 +443,8 @@ __global__ void __launch_bounds__(256) k_dense_lif(LifParams P, const float *__r
 }
 
 // The step's neuron update fused into the tcgen05 delivery: the same update
-// as k_dense_lif for the elements of the tile a CTA completes, with their
-// state loads batched ahead of the updates; S_t is written in the blocked
+// as k_dense_lif for the elements a CTA completes, with their state loaded
+// while the products run; S_t is written in the blocked
 // layout the next delivery reads.
 struct LifFinish {
     static constexpr bool kActive = true;
@@ -458,7 +458,7 @@ struct LifFinish {
         vv = v[idx];
         ls = last[idx];
     }
-    __device__ bool update(int b, int j, int idx, float a, float vv, int ls) const {
+    __device__ bool update(int b, int j, int idx, float a, float &vv, int &ls) const {
         const bool spk = lif_apply(P, a, vv, ls, t, idx);
         v[idx] = vv;
         last[idx] = ls;
@@ -487,7 +487,6 @@ struct nbg_dense {
     DevBuf<__nv_bfloat16> io_s;
     DevBuf<float> io_part, io_out;
     DevBuf<int> cnt; // spikes per step of a run call
-    DevBuf<unsigned int> tile_cnt; // fused-update arrivals per tile (zero between launches)
     std::vector<cudaEvent_t> dev_pool; // delivery start/stop events, 2 per step
     int next_t = 0;
     bool ran = false;
@@ -510,7 +509,6 @@ nbg_status dense_reset(nbg_dense *d) {
         NBG_CUDA(d->s[k].zero());
         NBG_CUDA(d->bits[k].zero());
     }
-    if (d->tile_cnt.p) NBG_CUDA(d->tile_cnt.zero());
     d->next_t = 0;
     d->ran = false;
     d->counts_host.clear();
@@ -527,16 +525,20 @@ dim3 gather_grid(const nbg_dense *d) { return dim3(d->B, (d->N + kGatherCols - 1
 
 // A step's launch configuration, overlapping the step before (programmatic
 // dependent launch).
-cudaLaunchConfig_t step_config(const nbg_dense *d, dim3 grid, int threads, size_t smem, cudaLaunchAttribute *attr) {
+cudaLaunchConfig_t step_config(const nbg_dense *d, dim3 grid, int threads, size_t smem, cudaLaunchAttribute (&attr)[2],
+                               int cluster_y = 1) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = d->stream;
-    attr->id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr->val.programmaticStreamSerializationAllowed = 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.z = 1;
+    attr[1].val.clusterDim.y = (unsigned)cluster_y;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster_y > 1 ? 2 : 1;
     return cfg;
 }
 
@@ -594,7 +596,7 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
     chk(d->last.alloc(tot));
     chk(d->err.alloc(1));
     chk(d->err.zero());
-    chk(d->partial.alloc((size_t)kSplitK * tot));
+    if (precision == NBG_DENSE_SPLIT_BF16_SYNC) chk(d->partial.alloc((size_t)kSplitK * tot));
     for (int k = 0; k < 2; ++k) {
         chk(d->s[k].alloc(tot));
         chk(d->bits[k].alloc(tot / 32));
@@ -617,9 +619,7 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes));
             if (ce == cudaSuccess)
                 chk(cudaFuncSetAttribute(umma::k_dense_umma<LifFinish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         umma::kSmemBytes));
-            if (ce == cudaSuccess) chk(d->tile_cnt.alloc((size_t)neurons / umma::kM));
-            if (ce == cudaSuccess) chk(d->tile_cnt.zero());
+                                         umma::kFusedSmemBytes));
         } else if (ce == cudaSuccess) {
             dim3 grid(neurons / 32, neurons / 32), block(32, 8);
             k_split_transpose<<<grid, block>>>(tmp.p, d->whi.p, d->wlo.p, neurons);
@@ -677,7 +677,8 @@ nbg_status nbg_dense_run(nbg_dense *d, int steps) {
     }
     double dms = 0.0;
     NBG_CUDA(cudaEventRecord(d->ev0, d->stream));
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    const int kept = umma::kept_iters(d->N, kSplitK);
     for (int k0 = 0; k0 < count; k0 += chunk) {
         const int k1 = std::min(count, k0 + chunk);
         for (int k = k0; k < k1; ++k) {
@@ -686,10 +687,10 @@ nbg_status nbg_dense_run(nbg_dense *d, int steps) {
             if (d->precision == NBG_DENSE_SPLIT_BF16) { // tcgen05: delivery and update in one launch
                 const LifFinish fin{d->P, d->v.p, d->last.p, d->s[outp].p, dcnt.p + k, t};
                 const cudaLaunchConfig_t cfg =
-                    step_config(d, dim3(d->N / umma::kM, kSplitK), umma::kThreads, umma::kSmemBytes, attr);
+                    step_config(d, dim3(d->N / umma::kM, kSplitK), umma::kThreads, umma::kFusedSmemBytes, attr, kSplitK);
                 NBG_CUDA(cudaLaunchKernelEx(&cfg, umma::k_dense_umma<LifFinish>, (const __nv_bfloat16 *)d->whi.p,
                                             (const __nv_bfloat16 *)d->wlo.p, (const __nv_bfloat16 *)d->s[in].p,
-                                            d->partial.p, d->N, (int)kSplitK, t & 1, d->err.p, d->tile_cnt.p, fin));
+                                            (float *)nullptr, d->N, (int)kSplitK, t & 1, kept, d->err.p, fin));
                 continue;
             }
             if (d->precision == NBG_DENSE_FP32) { // gather and update in one launch
@@ -795,7 +796,7 @@ nbg_status nbg_dense_deliver(nbg_dense *d, const uint8_t *s, float *out) {
     if (d->precision == NBG_DENSE_SPLIT_BF16) {
         k_spikes_in<kLayoutBlocked><<<grid8, 256, 0, st>>>(d->io_bytes.p, d->io_s.p, d->N, groups);
         umma::k_dense_umma<umma::NoFinish><<<dim3(d->N / umma::kM, kSplitK), umma::kThreads, umma::kSmemBytes, st>>>(
-            d->whi.p, d->wlo.p, d->io_s.p, d->io_part.p, d->N, kSplitK, 0, d->err.p, d->tile_cnt.p, umma::NoFinish{});
+            d->whi.p, d->wlo.p, d->io_s.p, d->io_part.p, d->N, kSplitK, 0, 0, d->err.p, umma::NoFinish{});
     } else if (d->precision == NBG_DENSE_SPLIT_BF16_SYNC) {
         k_spikes_in<kLayoutRows><<<grid8, 256, 0, st>>>(d->io_bytes.p, d->io_s.p, d->N, groups);
         k_dense_gemm<<<dim3(d->N / kBM, kSplitK), kGemmThreads, kGemmSmem, st>>>(d->whi.p, d->wlo.p, d->io_s.p,

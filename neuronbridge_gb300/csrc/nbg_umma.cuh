@@ -26,14 +26,27 @@
 // records kUmmaTimeout in the error word, stops issuing, waits (bounded) for
 // the MMAs it already issued, frees its TMEM and returns.
 //
-// Fused step (split = 2): with an active `Finish` functor, the CTA that
-// completes a tile (the second of its two split-K contributors to arrive,
-// found with one atomic per CTA on a per-tile counter after every thread's
-// release fence; nothing waits) adds the other CTA's partial to the
-// accumulator it still holds in registers (two-term float addition is
-// commutative, so the sum equals partial 0 + partial 1 whichever CTA
-// finishes) and runs the functor on each of its elements -- the neuron
-// update of the step -- then rearms the counter for the next launch.
+// Fused step (split = 2): with an active `Finish` functor the two split-K CTAs
+// of a tile form a cluster.  CTA r finishes instances [32 r, 32 r + 32): each
+// sends the other its partial of the other's instances through distributed
+// shared memory (16 KiB), and after one cluster barrier adds what it received
+// to the accumulator it holds (two-term float addition is commutative, so the
+// sum equals partial 0 + partial 1 in both) and runs the functor on each of its
+// elements -- the neuron update of the step -- whose state it loaded while the
+// products ran.
+//
+// What bounds a step: the stream of W above about 5,000 neurons, and the way
+// from the last product to the next step's first operand at every size.  With
+// the partials in global memory, the second CTA to arrive (found by an atomic)
+// reading the other's and updating the whole tile alone, a step took 46.9 us at
+// 8,192 neurons, 23.1 at 4,096 and 13.3 at 1,024; now 39.5, 18.9 and 9.4.
+//
+// W larger than the L2: the chunks of a step's last iterations (about 34 MB in
+// all) are the next step's first ones and are kept (evict_last), the others
+// pass through (evict_first): 46.9 -> 43.5 us at 8,192 neurons and 32.7 -> 30.5
+// at 6,144 without the change above.  Kept shares of 17 to 50 MB are within 0.5
+// us of it, 100 MB gives 45.6; below 100 MB of W nothing is marked (no
+// difference at 4,096 neurons, 67 MB).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -48,6 +61,16 @@ constexpr int kBlockB = kN * kKChunk * 2;  // 8 KiB
 constexpr int kStageBytes = 2 * kBlockA + kBlockB;
 // stages (aligned up to 1024 B inside the allocation) + barrier block
 constexpr int kSmemBytes = kUStages * kStageBytes + 1024 + 256;
+constexpr int kRecvBytes = kM * (kN / 2) * 4; // fused step: the other CTA's partial of this one's instances
+constexpr int kFusedSmemBytes = kSmemBytes + kRecvBytes;
+constexpr long long kKeepBytes = 34000000, kKeepAbove = 100000000; // of W, see above
+
+// Iterations at a step's end whose chunks of W are kept in L2 (0: nothing is
+// marked) for n neurons in `split` K ranges.
+inline int kept_iters(int n, int split) {
+    const long long w = 4ll * n * n, iters = n / kKChunk / split;
+    return w > kKeepAbove ? (int)((iters * kKeepBytes + w / 2) / w) : 0;
+}
 constexpr int kThreads = 256;
 constexpr int kTmemCols = 64;
 constexpr int kUmmaTimeout = 4;
@@ -120,6 +143,15 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t b
         : "memory");
 }
 
+// bulk_copy with an L2 eviction policy (createpolicy).
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t bytes, uint64_t *bar, uint64_t policy) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(
+            smem_addr(dst)),
+        "l"(src), "r"(bytes), "r"(smem_addr(bar)), "l"(policy)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -155,7 +187,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 struct NoFinish {
     static constexpr bool kActive = false;
     __device__ void load(int, float &, int &) const {}
-    __device__ bool update(int, int, int, float, float, int) const { return false; }
+    __device__ bool update(int, int, int, float, float &, int &) const { return false; }
     __device__ void count(int) const {}
 };
 
@@ -163,7 +195,7 @@ template <class Finish>
 __global__ void __launch_bounds__(kThreads, 1)
     k_dense_umma(const __nv_bfloat16 *__restrict__ wt_hi, const __nv_bfloat16 *__restrict__ wt_lo,
                  const __nv_bfloat16 *__restrict__ s_blk, float *__restrict__ partial, int n, int split,
-                 int reverse, int *__restrict__ err, unsigned int *__restrict__ tile_cnt, const Finish fin) {
+                 int reverse, int kept, int *__restrict__ err, const Finish fin) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *stages = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = (uint64_t *)(stages + kUStages * kStageBytes);
@@ -171,6 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t *done = empty + kUStages;
     uint32_t *tmem_slot = (uint32_t *)(done + 1);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
+    float4 *recv = reinterpret_cast<float4 *>(stages + kUStages * kStageBytes + 256); // Finish: [16 columns / 4][j][4]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int mt = blockIdx.x, ks = blockIdx.y;
@@ -205,18 +238,30 @@ __global__ void __launch_bounds__(kThreads, 1)
     // dependency wait (a no-op without a programmatic launch), and S and all
     // state after it.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (Finish::kActive) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     // K chunks in ascending order, or descending when `reverse`: the chunks a
     // step streams last are still in L2 when the next step, run in the other
     // direction, streams them first
     auto chunk = [&](int it) { return reverse ? kc0 + iters - 1 - it : kc0 + it; };
     if (warp == 0 && lane == 0) { // producer: bulk copies into free stages
+        uint64_t keep, pass;
+        asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
+        asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pass));
+        auto copy_w = [&](int it, uint8_t *st, uint64_t *bar) {
+            const size_t at = ((size_t)mt * kchunks + chunk(it)) * kBlockA;
+            if (kept == 0) {
+                bulk_copy(st, (const uint8_t *)wt_hi + at, kBlockA, bar);
+                bulk_copy(st + kBlockA, (const uint8_t *)wt_lo + at, kBlockA, bar);
+            } else {
+                const uint64_t p = it >= iters - kept ? keep : pass;
+                bulk_copy(st, (const uint8_t *)wt_hi + at, kBlockA, bar, p);
+                bulk_copy(st + kBlockA, (const uint8_t *)wt_lo + at, kBlockA, bar, p);
+            }
+        };
         const int pre = iters < kUStages ? iters : kUStages;
         for (int it = 0; it < pre; ++it) {
-            uint8_t *st = stages + it * kStageBytes;
-            const size_t blk = (size_t)mt * kchunks + chunk(it);
             mbar_expect_tx(&full[it], kStageBytes);
-            bulk_copy(st, (const uint8_t *)wt_hi + blk * kBlockA, kBlockA, &full[it]);
-            bulk_copy(st + kBlockA, (const uint8_t *)wt_lo + blk * kBlockA, kBlockA, &full[it]);
+            copy_w(it, stages + it * kStageBytes, &full[it]);
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
         for (int it = 0; it < pre; ++it)
@@ -226,12 +271,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int s = it % kUStages;
             if (!mbar_wait(&empty[s], ((it / kUStages) & 1) ^ 1, abort)) break;
             uint8_t *st = stages + s * kStageBytes;
-            const int kc = chunk(it);
-            const size_t blk = (size_t)mt * kchunks + kc;
             mbar_expect_tx(&full[s], kStageBytes);
-            bulk_copy(st, (const uint8_t *)wt_hi + blk * kBlockA, kBlockA, &full[s]);
-            bulk_copy(st + kBlockA, (const uint8_t *)wt_lo + blk * kBlockA, kBlockA, &full[s]);
-            bulk_copy(st + 2 * kBlockA, (const uint8_t *)s_blk + (size_t)kc * kBlockB, kBlockB, &full[s]);
+            copy_w(it, st, &full[s]);
+            bulk_copy(st + 2 * kBlockA, (const uint8_t *)s_blk + (size_t)chunk(it) * kBlockB, kBlockB, &full[s]);
         }
     } else if (warp == 1 && lane == 0) { // MMA issuer
         constexpr uint32_t idesc = make_idesc();
@@ -256,59 +298,74 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     __syncwarp();
     asm volatile("griddepcontrol.wait;" ::: "memory"); // before touching anything the previous step wrote
-    // epilogue: warp w reads TMEM lanes 32*(w%4).. (post neurons) and
-    // columns 32*(w/4).. (instances).  The abort decision is made uniform
-    // across the block before the warp-collective tcgen05.ld.
-    mbar_wait(done, 0, abort);
-    __syncthreads();
-    fence_after();
     const int q = warp & 3, h = warp >> 2;
-    const int j = mt * kM + 32 * q + lane;
-    float acc[2][16];
-    if (!*abort) {
-        float *out = partial + (size_t)ks * kN * n;
-        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * h), acc[0]);
-        tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * h + 16), acc[1]);
+    const int jl = 32 * q + lane, j = mt * kM + jl;
+    if constexpr (Finish::kActive) {
+        // warp w finishes post neurons 32*(w%4).. and instances 32*ks + 16*(w/4)..
+        const int b0 = 32 * ks + 16 * h, sent = 32 * (ks ^ 1) + 16 * h;
+        float vv[16];
+        int ls[16];
 #pragma unroll
-        for (int c = 0; c < 32; ++c) out[(size_t)(32 * h + c) * n + j] = acc[c >> 4][c & 15];
+        for (int c = 0; c < 16; ++c) fin.load((b0 + c) * n + j, vv[c], ls[c]); // while the products run
+        mbar_wait(done, 0, abort);
+        // uniform across the block before the warp-collective tcgen05.ld
+        __syncthreads();
+        fence_after();
+        const bool ok = !*abort;
+        float own[16], oth[16];
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); // the other CTA has started
+        if (ok) {
+            const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16);
+            tmem_ld16(lanes + (uint32_t)sent, oth);
+            uint32_t ra;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(ra)
+                         : "r"(smem_addr(recv + 4 * h * kM + jl)), "r"(ks ^ 1));
+#pragma unroll
+            for (int c = 0; c < 16; c += 4)
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * kM * 16)),
+                             "f"(oth[c]), "f"(oth[c + 1]), "f"(oth[c + 2]), "f"(oth[c + 3])
+                             : "memory");
+            tmem_ld16(lanes + (uint32_t)b0, own);
+        }
+        fence_before();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (ok) {
+#pragma unroll
+            for (int c = 0; c < 16; c += 4) {
+                const float4 x = recv[(4 * h + c / 4) * kM + jl];
+                oth[c] = x.x;
+                oth[c + 1] = x.y;
+                oth[c + 2] = x.z;
+                oth[c + 3] = x.w;
+            }
+            int spikes = 0;
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+                spikes += fin.update(b0 + c, j, (b0 + c) * n + j, own[c] + oth[c], vv[c], ls[c]) ? 1 : 0;
+            for (int o = 16; o > 0; o >>= 1) spikes += __shfl_down_sync(0xffffffffu, spikes, o);
+            if (lane == 0) fin.count(spikes);
+        }
+    } else {
+        // warp w reads TMEM lanes 32*(w%4).. (post neurons) and columns 32*(w/4).. (instances)
+        mbar_wait(done, 0, abort);
+        __syncthreads();
+        fence_after();
+        if (!*abort) {
+            float acc[2][16];
+            float *out = partial + (size_t)ks * kN * n;
+            tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * h), acc[0]);
+            tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * h + 16), acc[1]);
+#pragma unroll
+            for (int c = 0; c < 32; ++c) out[(size_t)(32 * h + c) * n + j] = acc[c >> 4][c & 15];
+        }
+        fence_before();
     }
-    fence_before();
-    if constexpr (Finish::kActive) __threadfence(); // this thread's partial before the CTA's arrival
     __syncthreads();
     if (threadIdx.x == 0 && *abort) atomicOr(err, kUmmaTimeout);
     if (warp == 2) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
-    }
-    if constexpr (Finish::kActive) {
-        __shared__ int finisher;
-        if (threadIdx.x == 0)
-            finisher = !*abort && atomicAdd(&tile_cnt[mt], 1u) == (unsigned int)(split - 1);
-        __syncthreads();
-        if (finisher) {
-            __threadfence(); // the other contributor's partial is visible after its arrival
-            const float *other = partial + (size_t)(ks ^ 1) * kN * n;
-            int spikes = 0;
-#pragma unroll
-            for (int half = 0; half < 2; ++half) { // loads of 16 elements in flight, then their updates
-                float oth[16], vv[16];
-                int ls[16];
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    const int idx = (32 * h + 16 * half + c) * n + j;
-                    oth[c] = __ldcg(other + idx);
-                    fin.load(idx, vv[c], ls[c]);
-                }
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    const int b = 32 * h + 16 * half + c;
-                    spikes += fin.update(b, j, b * n + j, acc[half][c] + oth[c], vv[c], ls[c]) ? 1 : 0;
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) spikes += __shfl_down_sync(0xffffffffu, spikes, o);
-            if (lane == 0) fin.count(spikes);
-            if (threadIdx.x == 0) tile_cnt[mt] = 0u;
-        }
     }
 }
 
