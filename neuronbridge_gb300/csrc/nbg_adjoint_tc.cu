@@ -45,6 +45,7 @@ constexpr int kAdjBlockB = kAdjN * kKChunk * 2;
 constexpr int kAdjStageBytes = 2 * kAdjBlockA + 2 * kAdjBlockB; // A_hi A_lo B_hi B_lo
 constexpr int kAdjSmemBytes = kAdjStages * kAdjStageBytes + 1024 + 256;
 constexpr int kAdjTmemCols = 128;
+constexpr int kThreads = 256; // of a product whose result is stored
 
 // kind::f16 instruction descriptor: BF16 x BF16 -> F32, K-major, M = N = 128.
 constexpr uint32_t kAdjIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kAdjN >> 3) << 17) |

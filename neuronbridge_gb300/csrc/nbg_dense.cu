@@ -290,11 +290,16 @@ struct LifParams {
     int t_ref;
 };
 
-// One neuron's update: summed arrival, refractory-gated voltage jump,
-// forward-Euler voltage-jump LIF (TimeDrivenLIF_Voltage_jump.cpp:49-86),
-// state vv, ls in registers, `a` its summed arrival; idx = the element of the instance-major state (the drive's hash index).
-__device__ __forceinline__ bool lif_apply(const LifParams &P, float a, float &vv, int &ls, int t, int idx) {
-    if (t >= 1 && nbg_hash_uniform01(idx, t - 1) < P.drive_p) a = a + P.drive_w;
+// Whether the drive spikes at element idx of the instance-major state (its hash index).
+__device__ __forceinline__ bool lif_drive(const LifParams &P, int t, int idx) {
+    return t >= 1 && nbg_hash_uniform01(idx, t - 1) < P.drive_p;
+}
+
+// One neuron's update: summed arrival `a`, the drive's spike, refractory-gated
+// voltage jump, forward-Euler voltage-jump LIF
+// (TimeDrivenLIF_Voltage_jump.cpp:49-86), state vv, ls in registers.
+__device__ __forceinline__ bool lif_apply(const LifParams &P, float a, bool drive, float &vv, int &ls) {
+    if (drive) a = a + P.drive_w;
     if (ls > P.t_ref) vv = vv + a;
     float cur = 0.0f;
     cur = cur + P.r * P.i_ext / P.tau;
@@ -410,8 +415,8 @@ __global__ void __launch_bounds__(kGatherThreads) k_dense_gather(const float *__
     } else {
         bool s0 = false, s1 = false;
         if (has) {
-            s0 = lif_apply(P, sum.x, vv.x, ls.x, t, (int)at);
-            s1 = lif_apply(P, sum.y, vv.y, ls.y, t, (int)at + 1);
+            s0 = lif_apply(P, sum.x, lif_drive(P, t, (int)at), vv.x, ls.x);
+            s1 = lif_apply(P, sum.y, lif_drive(P, t, (int)at + 1), vv.y, ls.y);
             *reinterpret_cast<float2 *>(v + at) = vv;
             *reinterpret_cast<int2 *>(last + at) = ls;
         }
@@ -433,7 +438,7 @@ __global__ void __launch_bounds__(256) k_dense_lif(LifParams P, const float *__r
         for (int k = 1; k < nparts; ++k) a = a + partial[(size_t)k * total + idx];
         float vv = v[idx];
         int ls = last[idx];
-        spk = lif_apply(P, a, vv, ls, t, idx);
+        spk = lif_apply(P, a, lif_drive(P, t, idx), vv, ls);
         v[idx] = vv;
         last[idx] = ls;
         s_out[idx] = __float2bfloat16_rn(spk ? 1.0f : 0.0f);
@@ -458,8 +463,9 @@ struct LifFinish {
         vv = v[idx];
         ls = last[idx];
     }
-    __device__ bool update(int b, int j, int idx, float a, float &vv, int &ls) const {
-        const bool spk = lif_apply(P, a, vv, ls, t, idx);
+    __device__ bool drive(int idx) const { return lif_drive(P, t, idx); }
+    __device__ bool update(int b, int j, int idx, float a, bool drive, float &vv, int &ls) const {
+        const bool spk = lif_apply(P, a, drive, vv, ls);
         v[idx] = vv;
         last[idx] = ls;
         s_out[s_blocked(b, j)] = __float2bfloat16_rn(spk ? 1.0f : 0.0f);
@@ -474,6 +480,7 @@ struct LifFinish {
 
 struct nbg_dense {
     int device = 0, B = 64, N = 0, precision = 0;
+    bool half_tiles = false; // tcgen05 step: tiles of 64 post neurons instead of 128
     LifParams P{};
     DevBuf<float> w, partial, v;
     DevBuf<__nv_bfloat16> whi, wlo, s[2];
@@ -618,8 +625,14 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
                 chk(cudaFuncSetAttribute(umma::k_dense_umma<umma::NoFinish>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes));
             if (ce == cudaSuccess)
-                chk(cudaFuncSetAttribute(umma::k_dense_umma<LifFinish>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         umma::kFusedSmemBytes));
+                chk(cudaFuncSetAttribute(umma::k_dense_umma<LifFinish, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         umma::Tile<128>::fused_smem));
+            if (ce == cudaSuccess)
+                chk(cudaFuncSetAttribute(umma::k_dense_umma<LifFinish, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         umma::Tile<64>::fused_smem));
+            int sms = 0;
+            chk(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+            d->half_tiles = neurons / 64 * kSplitK <= sms;
         } else if (ce == cudaSuccess) {
             dim3 grid(neurons / 32, neurons / 32), block(32, 8);
             k_split_transpose<<<grid, block>>>(tmp.p, d->whi.p, d->wlo.p, neurons);
@@ -686,11 +699,14 @@ nbg_status nbg_dense_run(nbg_dense *d, int steps) {
             const int in = (t + 1) & 1, outp = t & 1; // S_{t-1} lives in buffer (t-1)&1
             if (d->precision == NBG_DENSE_SPLIT_BF16) { // tcgen05: delivery and update in one launch
                 const LifFinish fin{d->P, d->v.p, d->last.p, d->s[outp].p, dcnt.p + k, t};
+                const int m = d->half_tiles ? 64 : 128;
                 const cudaLaunchConfig_t cfg =
-                    step_config(d, dim3(d->N / umma::kM, kSplitK), umma::kThreads, umma::kFusedSmemBytes, attr, kSplitK);
-                NBG_CUDA(cudaLaunchKernelEx(&cfg, umma::k_dense_umma<LifFinish>, (const __nv_bfloat16 *)d->whi.p,
-                                            (const __nv_bfloat16 *)d->wlo.p, (const __nv_bfloat16 *)d->s[in].p,
-                                            (float *)nullptr, d->N, (int)kSplitK, t & 1, kept, d->err.p, fin));
+                    step_config(d, dim3(d->N / m, kSplitK), umma::threads<LifFinish>(),
+                                d->half_tiles ? umma::Tile<64>::fused_smem : umma::Tile<128>::fused_smem, attr, kSplitK);
+                NBG_CUDA(cudaLaunchKernelEx(
+                    &cfg, d->half_tiles ? umma::k_dense_umma<LifFinish, 64> : umma::k_dense_umma<LifFinish, 128>,
+                    (const __nv_bfloat16 *)d->whi.p, (const __nv_bfloat16 *)d->wlo.p, (const __nv_bfloat16 *)d->s[in].p,
+                    (float *)nullptr, d->N, (int)kSplitK, t & 1, kept, d->err.p, fin));
                 continue;
             }
             if (d->precision == NBG_DENSE_FP32) { // gather and update in one launch
@@ -795,7 +811,7 @@ nbg_status nbg_dense_deliver(nbg_dense *d, const uint8_t *s, float *out) {
     NBG_CUDA(cudaMemcpyAsync(d->io_bytes.p, s, tot, cudaMemcpyHostToDevice, st));
     if (d->precision == NBG_DENSE_SPLIT_BF16) {
         k_spikes_in<kLayoutBlocked><<<grid8, 256, 0, st>>>(d->io_bytes.p, d->io_s.p, d->N, groups);
-        umma::k_dense_umma<umma::NoFinish><<<dim3(d->N / umma::kM, kSplitK), umma::kThreads, umma::kSmemBytes, st>>>(
+        umma::k_dense_umma<umma::NoFinish><<<dim3(d->N / umma::kM, kSplitK), umma::threads<umma::NoFinish>(), umma::kSmemBytes, st>>>(
             d->whi.p, d->wlo.p, d->io_s.p, d->io_part.p, d->N, kSplitK, 0, 0, d->err.p, umma::NoFinish{});
     } else if (d->precision == NBG_DENSE_SPLIT_BF16_SYNC) {
         k_spikes_in<kLayoutRows><<<grid8, 256, 0, st>>>(d->io_bytes.p, d->io_s.p, d->N, groups);

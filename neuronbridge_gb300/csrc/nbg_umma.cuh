@@ -5,10 +5,10 @@
 //
 //   D[j][b] = sum_k W_hi^T[j][k] S[b][k] + W_lo^T[j][k] S[b][k]
 //
-// One CTA owns 128 post-synaptic neurons (UMMA M = 128) and all 64 instances
+// One CTA owns 128 post-synaptic neurons (UMMA M = 128, or 64: below) and all 64 instances
 // (UMMA N = 64) over one K range (split-K).  Per 64-wide K chunk it copies
 // three pre-tiled blocks (W_hi^T 16 KiB, W_lo^T 16 KiB, S 8 KiB) with
-// cp.async.bulk into one of kUStages stages; one elected thread issues
+// cp.async.bulk into one of the stages; one elected thread issues
 // 4 k-steps x 2 (hi, lo) tcgen05.mma of K = 16 into the same TMEM
 // accumulator and commits the stage back to the producer.  The epilogue
 // reads the 128 x 64 FP32 accumulator with tcgen05.ld.
@@ -26,6 +26,12 @@
 // records kUmmaTimeout in the error word, stops issuing, waits (bounded) for
 // the MMAs it already issued, frees its TMEM and returns.
 //
+// Tiles of 64 post neurons (M = 64, half of a W block: its first or last eight
+// row groups, which are contiguous) where all of them get an SM at once: up to
+// 4,864 neurons on 152 SMs.  A step's tail is then half as long: 4.12 us against
+// 5.02 with tiles of 128 at 128 neurons, 10.2 against 11.1 at 2,048, 19.5 against
+// 19.9 at 4,864.  Above, the last of them would wait for the first.
+//
 // Fused step (split = 2): with an active `Finish` functor the two split-K CTAs
 // of a tile form a cluster.  CTA r finishes instances [32 r, 32 r + 32): each
 // sends the other its partial of the other's instances through distributed
@@ -39,7 +45,12 @@
 // from the last product to the next step's first operand at every size.  With
 // the partials in global memory, the second CTA to arrive (found by an atomic)
 // reading the other's and updating the whole tile alone, a step took 46.9 us at
-// 8,192 neurons, 23.1 at 4,096 and 13.3 at 1,024; now 39.5, 18.9 and 9.4.
+// 8,192 neurons, 23.1 at 4,096 and 13.3 at 1,024; with the exchange and 16
+// instances a thread 39.5, 18.9 and 9.4.  Now sixteen warps finish, eight
+// instances a thread (four with M = 64), and draw the step's external spikes
+// before they wait for the step before, which they do not depend on; the
+// producer and the issuer have warps of their own, so that neither's work is
+// behind that: 37.9, 16.8 and 7.0.
 //
 // W larger than the L2: the chunks of a step's last iterations (about 34 MB in
 // all) are the next step's first ones and are kept (evict_last), the others
@@ -61,8 +72,15 @@ constexpr int kBlockB = kN * kKChunk * 2;  // 8 KiB
 constexpr int kStageBytes = 2 * kBlockA + kBlockB;
 // stages (aligned up to 1024 B inside the allocation) + barrier block
 constexpr int kSmemBytes = kUStages * kStageBytes + 1024 + 256;
-constexpr int kRecvBytes = kM * (kN / 2) * 4; // fused step: the other CTA's partial of this one's instances
-constexpr int kFusedSmemBytes = kSmemBytes + kRecvBytes;
+// a tile of M = 128 or 64 post neurons (half of a W block): its stages, and the
+// fused step's receive buffer (the other CTA's partial of this one's instances)
+template <int M> struct Tile {
+    static_assert(M == 128 || M == 64, "UMMA M");
+    static constexpr int block_a = M * kKChunk * 2, stage_bytes = 2 * block_a + kBlockB;
+    static constexpr int stages = M == 128 ? kUStages : 6;
+    static constexpr int recv_bytes = M * (kN / 2) * 4;
+    static constexpr int fused_smem = stages * stage_bytes + recv_bytes + 1024 + 256;
+};
 constexpr long long kKeepBytes = 34000000, kKeepAbove = 100000000; // of W, see above
 
 // Iterations at a step's end whose chunks of W are kept in L2 (0: nothing is
@@ -71,7 +89,9 @@ inline int kept_iters(int n, int split) {
     const long long w = 4ll * n * n, iters = n / kKChunk / split;
     return w > kKeepAbove ? (int)((iters * kKeepBytes + w / 2) / w) : 0;
 }
-constexpr int kThreads = 256;
+// the warps that finish (16 for the fused step, 8 for partials), the producer's and the issuer's
+constexpr int kFinishWarps = 16, kPartialWarps = 8;
+template <class Finish> constexpr int threads() { return 32 * ((Finish::kActive ? kFinishWarps : kPartialWarps) + 2); }
 constexpr int kTmemCols = 64;
 constexpr int kUmmaTimeout = 4;
 constexpr long long kWaitCycles = 2000000000ll; // ~1 s at 2 GHz
@@ -94,11 +114,11 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
 }
 
 // UMMA instruction descriptor, kind::f16: BF16 x BF16 -> F32, K-major A/B.
-__host__ __device__ constexpr uint32_t make_idesc() {
+template <int M> __host__ __device__ constexpr uint32_t make_idesc() {
     return (1u << 4)                 // D format F32
            | (1u << 7)               // A format BF16
            | (1u << 10)              // B format BF16
-           | ((uint32_t)(kN >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
+           | ((uint32_t)(kN >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
@@ -167,7 +187,17 @@ __device__ __forceinline__ void commit(uint64_t *bar) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// 16 consecutive FP32 columns of this warp's 32 TMEM lanes.
+// 8 / 16 consecutive FP32 columns of this warp's 32 TMEM lanes.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
     asm volatile(
@@ -186,25 +216,30 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // No fused update: the partial sums are the result.
 struct NoFinish {
     static constexpr bool kActive = false;
+    __device__ bool drive(int) const { return false; }
     __device__ void load(int, float &, int &) const {}
-    __device__ bool update(int, int, int, float, float &, int &) const { return false; }
+    __device__ bool update(int, int, int, float, bool, float &, int &) const { return false; }
     __device__ void count(int) const {}
 };
 
-template <class Finish>
-__global__ void __launch_bounds__(kThreads, 1)
+// M: post neurons of a tile (M = 64: the two halves of a 128-row block of W).
+template <class Finish, int M = kM>
+__global__ void __launch_bounds__(threads<Finish>(), 1)
     k_dense_umma(const __nv_bfloat16 *__restrict__ wt_hi, const __nv_bfloat16 *__restrict__ wt_lo,
                  const __nv_bfloat16 *__restrict__ s_blk, float *__restrict__ partial, int n, int split,
                  int reverse, int kept, int *__restrict__ err, const Finish fin) {
+    using T = Tile<M>;
+    constexpr int kStages = T::stages;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *stages = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t *full = (uint64_t *)(stages + kUStages * kStageBytes);
-    uint64_t *empty = full + kUStages;
-    uint64_t *done = empty + kUStages;
+    uint64_t *full = (uint64_t *)(stages + kStages * T::stage_bytes);
+    uint64_t *empty = full + kStages;
+    uint64_t *done = empty + kStages;
     uint32_t *tmem_slot = (uint32_t *)(done + 1);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
-    float4 *recv = reinterpret_cast<float4 *>(stages + kUStages * kStageBytes + 256); // Finish: [16 columns / 4][j][4]
+    float4 *recv = reinterpret_cast<float4 *>(stages + kStages * T::stage_bytes + 256); // Finish: [16 columns / 4][j][4]
 
+    constexpr int kProducer = threads<Finish>() / 32 - 2, kIssuer = kProducer + 1; // warps
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int mt = blockIdx.x, ks = blockIdx.y;
     const int kchunks = n / kKChunk;
@@ -213,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int iters = (ks == split - 1) ? kchunks - kc0 : per;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kUStages; ++s) {
+        for (int s = 0; s < kStages; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
@@ -243,48 +278,49 @@ __global__ void __launch_bounds__(kThreads, 1)
     // step streams last are still in L2 when the next step, run in the other
     // direction, streams them first
     auto chunk = [&](int it) { return reverse ? kc0 + iters - 1 - it : kc0 + it; };
-    if (warp == 0 && lane == 0) { // producer: bulk copies into free stages
+    if (warp == kProducer && lane == 0) { // producer: bulk copies into free stages
         uint64_t keep, pass;
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(keep));
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pass));
         auto copy_w = [&](int it, uint8_t *st, uint64_t *bar) {
-            const size_t at = ((size_t)mt * kchunks + chunk(it)) * kBlockA;
+            const size_t at = M == kM ? ((size_t)mt * kchunks + chunk(it)) * kBlockA
+                                      : ((size_t)(mt >> 1) * kchunks + chunk(it)) * kBlockA + (size_t)(mt & 1) * T::block_a;
             if (kept == 0) {
-                bulk_copy(st, (const uint8_t *)wt_hi + at, kBlockA, bar);
-                bulk_copy(st + kBlockA, (const uint8_t *)wt_lo + at, kBlockA, bar);
+                bulk_copy(st, (const uint8_t *)wt_hi + at, T::block_a, bar);
+                bulk_copy(st + T::block_a, (const uint8_t *)wt_lo + at, T::block_a, bar);
             } else {
                 const uint64_t p = it >= iters - kept ? keep : pass;
-                bulk_copy(st, (const uint8_t *)wt_hi + at, kBlockA, bar, p);
-                bulk_copy(st + kBlockA, (const uint8_t *)wt_lo + at, kBlockA, bar, p);
+                bulk_copy(st, (const uint8_t *)wt_hi + at, T::block_a, bar, p);
+                bulk_copy(st + T::block_a, (const uint8_t *)wt_lo + at, T::block_a, bar, p);
             }
         };
-        const int pre = iters < kUStages ? iters : kUStages;
+        const int pre = iters < kStages ? iters : kStages;
         for (int it = 0; it < pre; ++it) {
-            mbar_expect_tx(&full[it], kStageBytes);
-            copy_w(it, stages + it * kStageBytes, &full[it]);
+            mbar_expect_tx(&full[it], T::stage_bytes);
+            copy_w(it, stages + it * T::stage_bytes, &full[it]);
         }
         asm volatile("griddepcontrol.wait;" ::: "memory");
         for (int it = 0; it < pre; ++it)
-            bulk_copy(stages + it * kStageBytes + 2 * kBlockA, (const uint8_t *)s_blk + (size_t)chunk(it) * kBlockB,
+            bulk_copy(stages + it * T::stage_bytes + 2 * T::block_a, (const uint8_t *)s_blk + (size_t)chunk(it) * kBlockB,
                       kBlockB, &full[it]);
         for (int it = pre; it < iters; ++it) {
-            const int s = it % kUStages;
-            if (!mbar_wait(&empty[s], ((it / kUStages) & 1) ^ 1, abort)) break;
-            uint8_t *st = stages + s * kStageBytes;
-            mbar_expect_tx(&full[s], kStageBytes);
+            const int s = it % kStages;
+            if (!mbar_wait(&empty[s], ((it / kStages) & 1) ^ 1, abort)) break;
+            uint8_t *st = stages + s * T::stage_bytes;
+            mbar_expect_tx(&full[s], T::stage_bytes);
             copy_w(it, st, &full[s]);
-            bulk_copy(st + 2 * kBlockA, (const uint8_t *)s_blk + (size_t)chunk(it) * kBlockB, kBlockB, &full[s]);
+            bulk_copy(st + 2 * T::block_a, (const uint8_t *)s_blk + (size_t)chunk(it) * kBlockB, kBlockB, &full[s]);
         }
-    } else if (warp == 1 && lane == 0) { // MMA issuer
-        constexpr uint32_t idesc = make_idesc();
+    } else if (warp == kIssuer && lane == 0) { // MMA issuer
+        constexpr uint32_t idesc = make_idesc<M>();
         int issued = 0;
         for (int it = 0; it < iters; ++it) {
-            const int s = it % kUStages;
-            if (!mbar_wait(&full[s], (it / kUStages) & 1, abort)) break;
+            const int s = it % kStages;
+            if (!mbar_wait(&full[s], (it / kStages) & 1, abort)) break;
             fence_after();
-            const uint32_t a_hi = smem_addr(stages + s * kStageBytes);
-            const uint32_t a_lo = a_hi + kBlockA;
-            const uint32_t b = a_hi + 2 * kBlockA;
+            const uint32_t a_hi = smem_addr(stages + s * T::stage_bytes);
+            const uint32_t a_lo = a_hi + T::block_a;
+            const uint32_t b = a_hi + 2 * T::block_a;
 #pragma unroll
             for (int k = 0; k < kKChunk / 16; ++k) {
                 mma(tmem, make_desc(a_hi + 256 * k), make_desc(b + 256 * k), idesc, (it | k) != 0);
@@ -297,43 +333,64 @@ __global__ void __launch_bounds__(kThreads, 1)
         (void)issued;
     }
     __syncwarp();
-    asm volatile("griddepcontrol.wait;" ::: "memory"); // before touching anything the previous step wrote
-    const int q = warp & 3, h = warp >> 2;
-    const int jl = 32 * q + lane, j = mt * kM + jl;
     if constexpr (Finish::kActive) {
-        // warp w finishes post neurons 32*(w%4).. and instances 32*ks + 16*(w/4)..
-        const int b0 = 32 * ks + 16 * h, sent = 32 * (ks ^ 1) + 16 * h;
-        float vv[16];
-        int ls[16];
+        // warp w finishes the post neurons of TMEM lanes 32*(w%4).. and instances
+        // 32*ks + 8*(w/4)..; with M = 64 a quarter of the lanes holds sixteen rows in
+        // its first half, and the two halves of the warp share the eight instances
+        constexpr int kOwn = M == kM ? 8 : 4;
+        const bool finishes = warp < kFinishWarps;
+        const int q = warp & 3, g = warp >> 2;
+        const int jl = M == kM ? 32 * q + lane : 16 * q + (lane & 15), j = mt * M + jl;
+        const int c0 = M == kM ? 0 : lane >> 4 << 2;
+        const int b0 = 32 * ks + 8 * g, sent = 32 * (ks ^ 1) + 8 * g;
+        float vv[kOwn];
+        int ls[kOwn];
+        unsigned drive = 0u; // this step's external spikes do not depend on the step before
+        if (finishes) {
 #pragma unroll
-        for (int c = 0; c < 16; ++c) fin.load((b0 + c) * n + j, vv[c], ls[c]); // while the products run
+            for (int c = 0; c < kOwn; ++c) drive |= fin.drive((b0 + c0 + c) * n + j) ? 1u << c : 0u;
+        }
+        asm volatile("griddepcontrol.wait;" ::: "memory"); // before touching anything the previous step wrote
+        if (finishes) {
+#pragma unroll
+            for (int c = 0; c < kOwn; ++c) fin.load((b0 + c0 + c) * n + j, vv[c], ls[c]); // while the products run
+        }
         mbar_wait(done, 0, abort);
         // uniform across the block before the warp-collective tcgen05.ld
         __syncthreads();
         fence_after();
-        const bool ok = !*abort;
-        float own[16], oth[16];
+        const bool ok = finishes && !*abort;
+        float own[8], oth[8];
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); // the other CTA has started
         if (ok) {
             const uint32_t lanes = tmem + ((uint32_t)(32 * q) << 16);
-            tmem_ld16(lanes + (uint32_t)sent, oth);
+            tmem_ld8(lanes + (uint32_t)sent, oth);
             uint32_t ra;
             asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
                          : "=r"(ra)
-                         : "r"(smem_addr(recv + 4 * h * kM + jl)), "r"(ks ^ 1));
+                         : "r"(smem_addr(recv + 2 * g * M + jl)), "r"(ks ^ 1));
+            if (M == kM || lane < 16) {
 #pragma unroll
-            for (int c = 0; c < 16; c += 4)
-                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * kM * 16)),
-                             "f"(oth[c]), "f"(oth[c + 1]), "f"(oth[c + 2]), "f"(oth[c + 3])
-                             : "memory");
-            tmem_ld16(lanes + (uint32_t)b0, own);
+                for (int c = 0; c < 8; c += 4)
+                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * M * 16)),
+                                 "f"(oth[c]), "f"(oth[c + 1]), "f"(oth[c + 2]), "f"(oth[c + 3])
+                                 : "memory");
+            }
+            tmem_ld8(lanes + (uint32_t)b0, own);
+            if constexpr (M != kM) {
+#pragma unroll
+                for (int c = 0; c < kOwn; ++c) {
+                    const float x = __shfl_sync(0xffffffffu, own[c + 4], lane & 15);
+                    own[c] = lane < 16 ? own[c] : x;
+                }
+            }
         }
         fence_before();
         asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (ok) {
 #pragma unroll
-            for (int c = 0; c < 16; c += 4) {
-                const float4 x = recv[(4 * h + c / 4) * kM + jl];
+            for (int c = 0; c < kOwn; c += 4) {
+                const float4 x = recv[(2 * g + (c0 + c) / 4) * M + jl];
                 oth[c] = x.x;
                 oth[c + 1] = x.y;
                 oth[c + 2] = x.z;
@@ -341,17 +398,22 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
             int spikes = 0;
 #pragma unroll
-            for (int c = 0; c < 16; ++c)
-                spikes += fin.update(b0 + c, j, (b0 + c) * n + j, own[c] + oth[c], vv[c], ls[c]) ? 1 : 0;
+            for (int c = 0; c < kOwn; ++c)
+                spikes += fin.update(b0 + c0 + c, j, (b0 + c0 + c) * n + j, own[c] + oth[c], drive >> c & 1u, vv[c], ls[c])
+                              ? 1
+                              : 0;
             for (int o = 16; o > 0; o >>= 1) spikes += __shfl_down_sync(0xffffffffu, spikes, o);
             if (lane == 0) fin.count(spikes);
         }
     } else {
+        static_assert(M == kM, "partials are written for whole blocks");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const int q = warp & 3, h = warp >> 2, j = mt * M + 32 * q + lane;
         // warp w reads TMEM lanes 32*(w%4).. (post neurons) and columns 32*(w/4).. (instances)
         mbar_wait(done, 0, abort);
         __syncthreads();
         fence_after();
-        if (!*abort) {
+        if (warp < kPartialWarps && !*abort) {
             float acc[2][16];
             float *out = partial + (size_t)ks * kN * n;
             tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * h), acc[0]);
