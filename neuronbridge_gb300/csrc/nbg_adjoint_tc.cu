@@ -251,14 +251,24 @@ __global__ void __launch_bounds__(kThreads, 1)
 // (the next launch reads this one while writing its own), in FP32 (when dI
 // is given) and as the split BF16 operand of the weight gradients (when dT_hi
 // is given: dI^T, row i, column k_off + b of a k_cols-column blocked matrix,
-// eight consecutive b of one i per 16-byte store).  No CTA reads another's
+// four consecutive b of one i per 8-byte store).  No CTA reads another's
 // shared memory, so none waits for its peers before it exits.  Waits on
 // mbarriers are bounded as in k_adj_umma; a CTA that gives up still takes
 // part in the cluster barrier, and the error word marks the step's results
 // invalid.  Two pipeline stages (a CTA has two K chunks at N = 1024) leave
 // room for the receive buffer.
+//
+// What bounds it: the chain from the operands to the next step's (1,000 dependent
+// steps in a sweep of 1,000): at N = 1024 hand-over 1.2 us, copies and products
+// 1.7, exchange 3.3 (64 KiB a CTA through distributed shared memory), the tail.
+// With eight warps, eight rows a thread, and all of the step's arithmetic behind
+// the products, the tail was 1.4 us and a forward and backward of 1,000 steps of
+// 128 x 1,024 took 11.24 ms; as below 10.74.
 constexpr int kAdjCluster = 8;
 constexpr int kAdjFusedStages = 2;
+// sixteen warps run the step's tail, four batch rows a thread; the producer and
+// the issuer are warps of their own
+constexpr int kAdjTailWarps = 16, kAdjStepThreads = 32 * (kAdjTailWarps + 2);
 // receive buffer [source rank][row / 4][i][row % 4]: a thread's sixteen
 // partials of one i are four 16-byte stores, and a warp's 32 of one of them are
 // contiguous (stores of the same size 80 bytes apart, free of bank conflicts
@@ -266,7 +276,7 @@ constexpr int kAdjFusedStages = 2;
 constexpr int kAdjRecvBytes = kAdjN * kAdjM * 4;
 constexpr int kAdjFusedSmemBytes = kAdjFusedStages * kAdjStageBytes + kAdjRecvBytes + 1024 + 256;
 
-__global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 1) k_adj_step_umma(
+__global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepThreads, 1) k_adj_step_umma(
     const __nv_bfloat16 *__restrict__ w_hi, const __nv_bfloat16 *__restrict__ w_lo,
     const __nv_bfloat16 *__restrict__ d_hi_in, const __nv_bfloat16 *__restrict__ d_lo_in,
     __nv_bfloat16 *__restrict__ d_hi_out, __nv_bfloat16 *__restrict__ d_lo_out, const float *__restrict__ g_read,
@@ -317,7 +327,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
     // the first stages' W tiles are requested before the wait for the
     // previous step (which writes dI_{t+1}, lam_v and the gradients).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (warp == 0 && lane == 0) { // producer
+    if (warp == kAdjTailWarps && lane == 0) { // producer
         const int pre = iters < kAdjFusedStages ? iters : kAdjFusedStages;
         for (int it = 0; it < pre; ++it) {
             uint8_t *st = stages + it * kAdjStageBytes;
@@ -347,7 +357,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
             bulk_copy(st + 2 * kAdjBlockA + kAdjBlockB, (const uint8_t *)d_lo_in + (size_t)kc * kAdjBlockB,
                       kAdjBlockB, &full[st_i]);
         }
-    } else if (warp == 1 && lane == 0) { // MMA issuer
+    } else if (warp == kAdjTailWarps + 1 && lane == 0) { // MMA issuer
         for (int it = 0; it < iters; ++it) {
             const int st_i = it % kAdjFusedStages;
             if (!mbar_wait(&full[st_i], (it / kAdjFusedStages) & 1, abort)) break;
@@ -367,88 +377,100 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
         commit(done);
     }
     __syncwarp();
-    // this thread's share of the adjoint step: batch rows 16 ks + 8 bsub + k
-    // of column i (eight consecutive rows: one 16-byte store of dI^T).  Its
-    // operands are loaded while the products run: first those no adjoint
-    // step writes (the forward's record, g_read and the parameters, all
-    // complete before the first step of the sweep), before the wait for the
-    // previous step, then the accumulators that step updated.
+    // this thread's share of the adjoint step: batch rows 16 ks + 4 bsub + k
+    // of column i (four consecutive rows: one 8-byte store of dI^T).  What needs
+    // no product is done while the products run: first what no adjoint step
+    // writes (the forward's record, g_read and the parameters, all complete
+    // before the first step of the sweep), before the wait for the previous
+    // step, then the accumulators that step updated.
+    const bool tail = warp < kAdjTailWarps;
     const int il = threadIdx.x & 127, bsub = threadIdx.x >> 7;
     const int i = mt * kAdjM + il;
-    constexpr int kRows = 8;
-    float op_u[kRows], op_s[kRows], op_lv[kRows], op_gr[kRows], op_gt[kRows], op_ga[kRows], op_vp[kRows];
+    constexpr int kRows = 4;
+    float op_u[kRows], op_ds[kRows], op_ns[kRows], op_lv[kRows], op_gr[kRows], op_gt[kRows], op_ga[kRows], op_vp[kRows];
     unsigned char op_m[kRows];
+    float th = 0.0f, al = 0.0f;
+    if (tail) {
+        th = theta[i];
+        al = alpha[i];
 #pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-        const size_t idx = (size_t)(16 * ks + 8 * bsub + k) * n + i;
-        op_u[k] = u[idx];
-        op_s[k] = s[idx];
-        op_gr[k] = g_read[idx];
-        op_vp[k] = vprev[idx];
-        op_m[k] = m[idx];
+        for (int k = 0; k < kRows; ++k) {
+            const size_t idx = (size_t)(16 * ks + 4 * bsub + k) * n + i;
+            op_u[k] = u[idx];
+            op_ns[k] = s[idx];
+            op_gr[k] = g_read[idx];
+            op_vp[k] = vprev[idx];
+            op_m[k] = m[idx];
+        }
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            const float ss = op_ns[k];
+            op_ds[k] = p.smooth ? p.slope * ss * (1.0f - ss) : surrogate(op_u[k] - th, p.slope);
+            op_ns[k] = 1.0f - ss;
+            op_gr[k] = c_t * op_gr[k];
+            op_u[k] = op_u[k] - p.v_reset;
+            op_vp[k] = p.v_rest - op_vp[k];
+        }
     }
-    const float th = theta[i], al = alpha[i];
     asm volatile("griddepcontrol.wait;" ::: "memory"); // the previous step's writes are visible
+    if (tail) {
 #pragma unroll
-    for (int k = 0; k < kRows; ++k) {
-        const size_t idx = (size_t)(16 * ks + 8 * bsub + k) * n + i;
-        op_lv[k] = lam_v[idx];
-        op_gt[k] = g_theta[idx];
-        op_ga[k] = g_alpha[idx];
+        for (int k = 0; k < kRows; ++k) {
+            const size_t idx = (size_t)(16 * ks + 4 * bsub + k) * n + i;
+            op_lv[k] = lam_v[idx];
+            op_gt[k] = g_theta[idx];
+            op_ga[k] = g_alpha[idx];
+        }
+#pragma unroll
+        for (int k = 0; k < kRows; ++k) {
+            op_gr[k] = op_gr[k] - op_lv[k] * op_u[k];
+            op_ns[k] = op_lv[k] * op_ns[k];
+        }
     }
     mbar_wait(done, 0, abort);
     __syncthreads();
     fence_after();
     // the partial accumulator to the rows' owners: warp w holds rows
-    // i = 32 (w % 4) + lane and batch columns b = 64 (w / 4) + 16 c16 + c,
-    // which rank 4 (w / 4) + c16 owns; they land in its receive buffer at
+    // i = 32 (w % 4) + lane and batch columns b = 32 (w / 4) + 16 c16 + c,
+    // which rank 2 (w / 4) + c16 owns; they land in its receive buffer at
     // [this rank][c][i]
-    {
-        const int q = warp & 3, h = warp >> 2;
-        const int il = 32 * q + lane;
-        if (!*abort) {
-            const uint32_t mine = smem_addr(recv) + (uint32_t)((ks * 4 * kAdjM + il) * 16);
+    if (tail && !*abort) {
+        const int q = warp & 3, g = warp >> 2;
+        const uint32_t mine = smem_addr(recv) + (uint32_t)((ks * 4 * kAdjM + il) * 16);
 #pragma unroll
-            for (int c16 = 0; c16 < 4; ++c16) {
-                float acc[16];
-                tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(64 * h + 16 * c16), acc);
-                uint32_t ra;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(mine), "r"(4 * h + c16));
+        for (int c16 = 0; c16 < 2; ++c16) {
+            float acc[16];
+            tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * g + 16 * c16), acc);
+            uint32_t ra;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(mine), "r"(2 * g + c16));
 #pragma unroll
-                for (int c = 0; c < 16; c += 4)
-                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * kAdjM * 16)),
-                                 "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3])
-                                 : "memory");
-            }
+            for (int c = 0; c < 16; c += 4)
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * kAdjM * 16)),
+                             "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3])
+                             : "memory");
         }
     }
     fence_before();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     // reduce this rank's batch rows over the cluster's partials, in rank
     // order, and run the adjoint step on them
-    {
+    if (tail) {
         // every partial of the thread's rows, loaded back to back, then added
         // in rank order
         float x[kAdjCluster][kRows];
 #pragma unroll
         for (int r = 0; r < kAdjCluster; ++r)
-#pragma unroll
-            for (int k = 0; k < kRows; k += 4)
-                *reinterpret_cast<float4 *>(&x[r][k]) =
-                    *reinterpret_cast<const float4 *>(recv + ((r * 4 + 2 * bsub + k / 4) * kAdjM + il) * 4);
-        uint32_t t_hi[kRows / 2], t_lo[kRows / 2]; // dI^T of the eight rows, split, packed in pairs
+            *reinterpret_cast<float4 *>(x[r]) = *reinterpret_cast<const float4 *>(recv + ((r * 4 + bsub) * kAdjM + il) * 4);
+        uint32_t t_hi[kRows / 2], t_lo[kRows / 2]; // dI^T of the rows, split, packed in pairs
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
-            const int b = 16 * ks + 8 * bsub + k;
+            const int b = 16 * ks + 4 * bsub + k;
             float ge = x[0][k];
 #pragma unroll
             for (int r = 1; r < kAdjCluster; ++r) ge = ge + x[r][k];
             const size_t idx = (size_t)b * n + i;
-            const float uu = op_u[k], ss = op_s[k], lv = op_lv[k];
-            const float dsdu = p.smooth ? p.slope * ss * (1.0f - ss) : surrogate(uu - th, p.slope);
-            float gs = c_t * op_gr[k] - lv * (uu - p.v_reset);
-            gs = gs + ge;
-            const float gu = gs * dsdu + lv * (1.0f - ss);
+            const float gs = op_gr[k] + ge;
+            const float gu = gs * op_ds[k] + op_ns[k];
             const float gm = op_m[k] ? gu : 0.0f;
             if (dI) dI[idx] = gm;
             const size_t o = blocked_index(b, i, n);
@@ -465,13 +487,13 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kThreads, 
                 t_lo[k >> 1] = lb;
             }
             lam_v[idx] = gm * (1.0f - al);
-            g_theta[idx] = op_gt[k] - gs * dsdu;
-            g_alpha[idx] = op_ga[k] + gm * (p.v_rest - op_vp[k]);
+            g_theta[idx] = op_gt[k] - gs * op_ds[k];
+            g_alpha[idx] = op_ga[k] + gm * op_vp[k];
         }
         if (dT_hi) {
-            const size_t o = blocked_index(i, (int)(k_off + 16 * ks + 8 * bsub), (int)k_cols);
-            reinterpret_cast<uint4 *>(dT_hi + o)[0] = make_uint4(t_hi[0], t_hi[1], t_hi[2], t_hi[3]);
-            reinterpret_cast<uint4 *>(dT_lo + o)[0] = make_uint4(t_lo[0], t_lo[1], t_lo[2], t_lo[3]);
+            const size_t o = blocked_index(i, (int)(k_off + 16 * ks + 4 * bsub), (int)k_cols);
+            reinterpret_cast<uint2 *>(dT_hi + o)[0] = make_uint2(t_hi[0], t_hi[1]);
+            reinterpret_cast<uint2 *>(dT_lo + o)[0] = make_uint2(t_lo[0], t_lo[1]);
         }
     }
     if (threadIdx.x == 0 && *abort) atomicOr(err, kUmmaTimeout);
@@ -749,7 +771,7 @@ nbg_status nbg_lif_adjoint_step_fused(const void *w_hi, const void *w_lo, const 
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(N / kAdjM, kAdjCluster);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kAdjStepThreads);
     cfg.dynamicSmemBytes = kAdjFusedSmemBytes;
     cfg.stream = (cudaStream_t)stream;
     cudaLaunchAttribute attr[1];
