@@ -66,9 +66,9 @@ _SIG = {
     "nbg_lif_adjoint_step_split": (ctypes.c_int, [_vp, ctypes.c_int, _vp, ctypes.c_float] + [_vp] * 12 +
                                    [ctypes.POINTER(GradParams), ctypes.c_int, ctypes.c_int, _vp]),
     "nbg_adjoint_rec_grad": (ctypes.c_int, [_vp] * 5 + [ctypes.c_int] * 3 + [_vp, _vp]),
-    "nbg_lif_adjoint_step_fused": (ctypes.c_int, [_vp] * 7 + [ctypes.c_float] + [_vp] * 10 +
+    "nbg_lif_adjoint_step_parts": (ctypes.c_int, [_vp] * 7 + [ctypes.c_float] + [_vp] * 10 +
                                    [ctypes.POINTER(GradParams), ctypes.c_int, ctypes.c_int, _vp, _vp,
-                                    ctypes.c_int64, ctypes.c_int64, _vp, _vp]),
+                                    ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp]),
     "nbg_adjoint_blocked_t": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, _vp,
                                              _vp]),
     "nbg_small_gemm": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, ctypes.c_int, _vp,
@@ -196,9 +196,9 @@ def _tc_ok(p, B: int, N: int) -> bool:
 
 
 # With N >= 512 the product and the adjoint step that consumes it are one
-# launch per step (nbg_lif_adjoint_step_fused: an 8-CTA cluster per 128-row
-# tile reduces its split-K partials through distributed shared memory); the
-# same sums in the same order as the two-launch form.
+# launch per step (nbg_lif_adjoint_step_parts: an 8-CTA cluster per 128-row
+# tile exchanges its split-K partials); the same sums in the same order as the
+# two-launch form.
 FUSED_STEP = True
 
 
@@ -377,7 +377,7 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
         d_hi = [torch.zeros(B * N, device=dev, dtype=torch.bfloat16) for _ in range(2 if fused else 1)]
         d_lo = [torch.zeros(B * N, device=dev, dtype=torch.bfloat16) for _ in range(2 if fused else 1)]
         split = min(TC_SPLIT, N // 64)
-        g_parts = None if fused else torch.empty((split, B, N), device=dev, dtype=torch.float32)
+        g_parts = torch.empty((8 if fused else split, B, N), device=dev, dtype=torch.float32)
         tc_err = torch.zeros(1, device=dev, dtype=torch.int32)
         _lib.check(lib.nbg_adjoint_rec_prepare(_ptr(w_rec), _ptr(w_hi), _ptr(w_lo), N, st))
     # weight gradients on the tensor cores: the product's column operand (S^T,
@@ -453,11 +453,11 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
             if fused:  # dI_{t+1} W_rec^T (zero at the run's last step) and step t, one launch
                 cur, nxt = t & 1, (t + 1) & 1
                 k_off, k_cols = (t * B, T * B) if whole else (k * B, L * B)
-                _lib.check(lib.nbg_lif_adjoint_step_fused(
+                _lib.check(lib.nbg_lif_adjoint_step_parts(
                     _ptr(w_hi), _ptr(w_lo), _ptr(d_hi[nxt]), _ptr(d_lo[nxt]), _ptr(d_hi[cur]), _ptr(d_lo[cur]),
                     _ptr(g_read), float(coef[t]), _ptr(U[k]), _ptr(S[k + 1]), _ptr(M[k]), _ptr(VP[k]),
                     _ptr(lam_v), None, _ptr(g_theta), _ptr(g_alpha), _ptr(alpha), _ptr(theta), ctypes.byref(p), B,
-                    N, _ptr(dT_hi), _ptr(dT_lo), k_off, k_cols, _ptr(tc_err), st))
+                    N, _ptr(dT_hi), _ptr(dT_lo), k_off, k_cols, _ptr(g_parts), _ptr(tc_err), st))
                 continue
             if tc:  # g_parts holds dI_{t+1} W_rec^T from the previous iteration
                 _lib.check(lib.nbg_lif_adjoint_step_split(

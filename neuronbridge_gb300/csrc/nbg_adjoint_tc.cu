@@ -242,10 +242,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 // range of one 128-row tile of W exactly as k_adj_umma's split-K does
 // (cluster rank = split index) and run the same three split products into
 // TMEM.  Rank r owns batch rows [16 r, 16 r + 16) of the tile: every CTA
-// stores its partial of those rows straight into rank r's receive buffer
-// through distributed shared memory, which waits for nothing.  After one cluster barrier rank r adds the partials of
-// ranks 0..7 in order from its own shared memory -- the sum k_lif_adj_split
-// forms from g_parts, so the result is the same bit for bit -- and runs the
+// stores its partial of those rows into rank r's part of the workspace (kParts)
+// or straight into its receive buffer through distributed shared memory, which
+// waits for nothing.  After one cluster barrier rank r adds the partials of ranks
+// 0..7 in order -- the sum k_lif_adj_split forms from g_parts, so the result is
+// the same bit for bit -- and runs the
 // adjoint step on those elements, writing dI_t as the split
 // BF16 operand of the next step's product into the other of two buffers
 // (the next launch reads this one while writing its own), in FP32 (when dI
@@ -255,17 +256,21 @@ __global__ void __launch_bounds__(kThreads, 1)
 // shared memory, so none waits for its peers before it exits.  Waits on
 // mbarriers are bounded as in k_adj_umma; a CTA that gives up still takes
 // part in the cluster barrier, and the error word marks the step's results
-// invalid.  Two pipeline stages (a CTA has two K chunks at N = 1024) leave
-// room for the receive buffer.
+// invalid.  Without kParts, two pipeline stages (a CTA has two K chunks at
+// N = 1024) leave room for the receive buffer.
 //
 // What bounds it: the chain from the operands to the next step's (1,000 dependent
 // steps in a sweep of 1,000): at N = 1024 hand-over 1.2 us, copies and products
-// 1.7, exchange 3.3 (64 KiB a CTA through distributed shared memory), the tail.
-// With eight warps, eight rows a thread, and all of the step's arithmetic behind
-// the products, the tail was 1.4 us and a forward and backward of 1,000 steps of
-// 128 x 1,024 took 11.24 ms; as below 10.74.
+// 1.7, the exchange, the tail.  With eight warps, eight rows a thread, and all of
+// the step's arithmetic behind the products, the tail was 1.4 us and a forward and
+// backward of 1,000 steps of 128 x 1,024 took 11.24 ms; as below 10.85.  An SM
+// moves about 12 bytes a clock through distributed shared memory, so the exchange
+// of 64 KiB a CTA took 3.3 us; through the L2 (4 MiB of partials, which stay
+// there) 9.95 ms; half of it either way 10.05.
 constexpr int kAdjCluster = 8;
-constexpr int kAdjFusedStages = 2;
+// pipeline stages, and the shared memory: with the partials in global memory
+// (kParts) there is no receive buffer
+template <bool kParts> constexpr int adj_stages() { return kParts ? 3 : 2; }
 // sixteen warps run the step's tail, four batch rows a thread; the producer and
 // the issuer are warps of their own
 constexpr int kAdjTailWarps = 16, kAdjStepThreads = 32 * (kAdjTailWarps + 2);
@@ -274,8 +279,11 @@ constexpr int kAdjTailWarps = 16, kAdjStepThreads = 32 * (kAdjTailWarps + 2);
 // contiguous (stores of the same size 80 bytes apart, free of bank conflicts
 // but scattered over packets, cost 2.6 us a step)
 constexpr int kAdjRecvBytes = kAdjN * kAdjM * 4;
-constexpr int kAdjFusedSmemBytes = kAdjFusedStages * kAdjStageBytes + kAdjRecvBytes + 1024 + 256;
+template <bool kParts> constexpr int adj_smem() {
+    return adj_stages<kParts>() * kAdjStageBytes + (kParts ? 0 : kAdjRecvBytes) + 1024 + 256;
+}
 
+template <bool kParts>
 __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepThreads, 1) k_adj_step_umma(
     const __nv_bfloat16 *__restrict__ w_hi, const __nv_bfloat16 *__restrict__ w_lo,
     const __nv_bfloat16 *__restrict__ d_hi_in, const __nv_bfloat16 *__restrict__ d_lo_in,
@@ -284,13 +292,14 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     const float *__restrict__ vprev, float *__restrict__ lam_v, float *__restrict__ dI, float *__restrict__ g_theta,
     float *__restrict__ g_alpha, const float *__restrict__ alpha, const float *__restrict__ theta,
     nbg_lif_grad_params p, int n, __nv_bfloat16 *__restrict__ dT_hi, __nv_bfloat16 *__restrict__ dT_lo,
-    long long k_off, long long k_cols, int *__restrict__ err) {
+    long long k_off, long long k_cols, float4 *parts, int *__restrict__ err) {
+    constexpr int kStages = adj_stages<kParts>();
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *stages = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    float *recv = reinterpret_cast<float *>(stages + kAdjFusedStages * kAdjStageBytes); // kAdjRecvBytes
-    uint64_t *full = (uint64_t *)((uint8_t *)recv + kAdjRecvBytes);
-    uint64_t *empty = full + kAdjFusedStages;
-    uint64_t *done = empty + kAdjFusedStages;
+    float4 *recv = reinterpret_cast<float4 *>(stages + kStages * kAdjStageBytes); // kAdjRecvBytes, or parts
+    uint64_t *full = (uint64_t *)((uint8_t *)recv + (kParts ? 0 : kAdjRecvBytes));
+    uint64_t *empty = full + kStages;
+    uint64_t *done = empty + kStages;
     uint32_t *tmem_slot = (uint32_t *)(done + 1);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
 
@@ -304,7 +313,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     const int iters = (ks == kAdjCluster - 1) ? kchunks - kc0 : per;
 
     if (threadIdx.x == 0) {
-        for (int st = 0; st < kAdjFusedStages; ++st) {
+        for (int st = 0; st < kStages; ++st) {
             mbar_init(&full[st], 1);
             mbar_init(&empty[st], 1);
         }
@@ -328,7 +337,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     // previous step (which writes dI_{t+1}, lam_v and the gradients).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == kAdjTailWarps && lane == 0) { // producer
-        const int pre = iters < kAdjFusedStages ? iters : kAdjFusedStages;
+        const int pre = iters < kStages ? iters : kStages;
         for (int it = 0; it < pre; ++it) {
             uint8_t *st = stages + it * kAdjStageBytes;
             const size_t a_blk = (size_t)mt * kchunks + kc0 + it;
@@ -345,8 +354,8 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
                       kAdjBlockB, &full[it]);
         }
         for (int it = pre; it < iters; ++it) {
-            const int st_i = it % kAdjFusedStages;
-            if (!mbar_wait(&empty[st_i], ((it / kAdjFusedStages) & 1) ^ 1, abort)) break;
+            const int st_i = it % kStages;
+            if (!mbar_wait(&empty[st_i], ((it / kStages) & 1) ^ 1, abort)) break;
             uint8_t *st = stages + st_i * kAdjStageBytes;
             const int kc = kc0 + it;
             const size_t a_blk = (size_t)mt * kchunks + kc;
@@ -359,8 +368,8 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
         }
     } else if (warp == kAdjTailWarps + 1 && lane == 0) { // MMA issuer
         for (int it = 0; it < iters; ++it) {
-            const int st_i = it % kAdjFusedStages;
-            if (!mbar_wait(&full[st_i], (it / kAdjFusedStages) & 1, abort)) break;
+            const int st_i = it % kStages;
+            if (!mbar_wait(&full[st_i], (it / kStages) & 1, abort)) break;
             fence_after();
             const uint32_t a_hi = smem_addr(stages + st_i * kAdjStageBytes);
             const uint32_t a_lo = a_hi + kAdjBlockA;
@@ -434,20 +443,29 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     // i = 32 (w % 4) + lane and batch columns b = 32 (w / 4) + 16 c16 + c,
     // which rank 2 (w / 4) + c16 owns; they land in its receive buffer at
     // [this rank][c][i]
+    constexpr int kRecv = kAdjCluster * 4 * kAdjM; // 16-byte pieces a rank receives
     if (tail && !*abort) {
         const int q = warp & 3, g = warp >> 2;
-        const uint32_t mine = smem_addr(recv) + (uint32_t)((ks * 4 * kAdjM + il) * 16);
+        const int mine = ks * 4 * kAdjM + il;
 #pragma unroll
         for (int c16 = 0; c16 < 2; ++c16) {
             float acc[16];
             tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * g + 16 * c16), acc);
-            uint32_t ra;
-            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(mine), "r"(2 * g + c16));
+            const int to = 2 * g + c16;
+            if constexpr (kParts) {
+                float4 *out = parts + ((size_t)mt * kAdjCluster + to) * kRecv + mine;
 #pragma unroll
-            for (int c = 0; c < 16; c += 4)
-                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * kAdjM * 16)),
-                             "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3])
-                             : "memory");
+                for (int c = 0; c < 16; c += 4)
+                    __stcg(out + c / 4 * kAdjM, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]));
+            } else {
+                uint32_t ra;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_addr(recv + mine)), "r"(to));
+#pragma unroll
+                for (int c = 0; c < 16; c += 4)
+                    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)(c / 4 * kAdjM * 16)),
+                                 "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3])
+                                 : "memory");
+            }
         }
     }
     fence_before();
@@ -459,8 +477,11 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
         // in rank order
         float x[kAdjCluster][kRows];
 #pragma unroll
-        for (int r = 0; r < kAdjCluster; ++r)
-            *reinterpret_cast<float4 *>(x[r]) = *reinterpret_cast<const float4 *>(recv + ((r * 4 + bsub) * kAdjM + il) * 4);
+        for (int r = 0; r < kAdjCluster; ++r) {
+            const int at = (r * 4 + bsub) * kAdjM + il;
+            *reinterpret_cast<float4 *>(x[r]) =
+                kParts ? __ldcg(parts + ((size_t)mt * kAdjCluster + ks) * kRecv + at) : recv[at];
+        }
         uint32_t t_hi[kRows / 2], t_lo[kRows / 2]; // dI^T of the rows, split, packed in pairs
 #pragma unroll
         for (int k = 0; k < kRows; ++k) {
@@ -682,6 +703,48 @@ bool adj_shape_ok(int B, int N) { return B == kAdjN && N > 0 && N % kAdjM == 0; 
 
 } // namespace
 
+template <bool kParts>
+static nbg_status adj_step(const char *name, float *parts, const void *w_hi, const void *w_lo, const void *dI_hi_in, const void *dI_lo_in,
+                                      void *dI_hi_out, void *dI_lo_out, const float *g_read, float c_t,
+                                      const float *u, const float *s, const uint8_t *m, const float *vprev,
+                                      float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
+                                      const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
+                                      void *dT_lo, int64_t k_off, int64_t k_cols, int *err, void *stream) {
+    if (!w_hi || !w_lo || !dI_hi_in || !dI_lo_in || !dI_hi_out || !dI_lo_out || !g_read || !u || !s || !m ||
+        !vprev || !lam_v || !g_theta || !g_alpha || !alpha || !theta || !p || !err || !adj_shape_ok(B, N) ||
+        N / kKChunk < kAdjCluster || dI_hi_in == dI_hi_out || dI_lo_in == dI_lo_out)
+        return nbg_fail(NBG_ERR_INVALID, "%s: bad arguments (B must be %d, N a multiple of %d "
+                        "and at least %d, distinct in and out operand buffers)", name, kAdjN, kAdjM,
+                        kAdjCluster * kKChunk);
+    if (dT_hi && (!dT_lo || k_off < 0 || k_off % kAdjN || k_cols % kKChunk || k_off + kAdjN > k_cols ||
+                  k_cols > 0x7fffffff))
+        return nbg_fail(NBG_ERR_INVALID, "%s: dT needs dT_lo, k_off a multiple of %d with "
+                        "k_off + %d <= k_cols, k_cols a multiple of %d below 2^31", name, kAdjN, kAdjN, kKChunk);
+    static bool attr_set = false;
+    if (!attr_set) {
+        NBG_CUDA(cudaFuncSetAttribute(k_adj_step_umma<kParts>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      adj_smem<kParts>()));
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(N / kAdjM, kAdjCluster);
+    cfg.blockDim = dim3(kAdjStepThreads);
+    cfg.dynamicSmemBytes = adj_smem<kParts>();
+    cfg.stream = (cudaStream_t)stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    NBG_CUDA(cudaLaunchKernelEx(&cfg, k_adj_step_umma<kParts>, (const __nv_bfloat16 *)w_hi, (const __nv_bfloat16 *)w_lo,
+                                (const __nv_bfloat16 *)dI_hi_in, (const __nv_bfloat16 *)dI_lo_in,
+                                (__nv_bfloat16 *)dI_hi_out, (__nv_bfloat16 *)dI_lo_out, g_read, c_t, u, s, m, vprev,
+                                lam_v, dI, g_theta, g_alpha, alpha, theta, *p, N, (__nv_bfloat16 *)dT_hi,
+                                (__nv_bfloat16 *)dT_lo, (long long)k_off, (long long)k_cols, (float4 *)parts, err));
+    NBG_CUDA(cudaGetLastError());
+    return NBG_OK;
+}
+
 extern "C" {
 
 nbg_status nbg_adjoint_rec_prepare(const float *w_rec, void *w_hi, void *w_lo, int N, void *stream) {
@@ -753,39 +816,19 @@ nbg_status nbg_lif_adjoint_step_fused(const void *w_hi, const void *w_lo, const 
                                       float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
                                       const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
                                       void *dT_lo, int64_t k_off, int64_t k_cols, int *err, void *stream) {
-    if (!w_hi || !w_lo || !dI_hi_in || !dI_lo_in || !dI_hi_out || !dI_lo_out || !g_read || !u || !s || !m ||
-        !vprev || !lam_v || !g_theta || !g_alpha || !alpha || !theta || !p || !err || !adj_shape_ok(B, N) ||
-        N / kKChunk < kAdjCluster || dI_hi_in == dI_hi_out || dI_lo_in == dI_lo_out)
-        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_step_fused: bad arguments (B must be %d, N a multiple of %d "
-                        "and at least %d, distinct in and out operand buffers)", kAdjN, kAdjM,
-                        kAdjCluster * kKChunk);
-    if (dT_hi && (!dT_lo || k_off < 0 || k_off % kAdjN || k_cols % kKChunk || k_off + kAdjN > k_cols ||
-                  k_cols > 0x7fffffff))
-        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_step_fused: dT needs dT_lo, k_off a multiple of %d with "
-                        "k_off + %d <= k_cols, k_cols a multiple of %d below 2^31", kAdjN, kAdjN, kKChunk);
-    static bool attr_set = false;
-    if (!attr_set) {
-        NBG_CUDA(cudaFuncSetAttribute(k_adj_step_umma, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      kAdjFusedSmemBytes));
-        attr_set = true;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(N / kAdjM, kAdjCluster);
-    cfg.blockDim = dim3(kAdjStepThreads);
-    cfg.dynamicSmemBytes = kAdjFusedSmemBytes;
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    NBG_CUDA(cudaLaunchKernelEx(&cfg, k_adj_step_umma, (const __nv_bfloat16 *)w_hi, (const __nv_bfloat16 *)w_lo,
-                                (const __nv_bfloat16 *)dI_hi_in, (const __nv_bfloat16 *)dI_lo_in,
-                                (__nv_bfloat16 *)dI_hi_out, (__nv_bfloat16 *)dI_lo_out, g_read, c_t, u, s, m, vprev,
-                                lam_v, dI, g_theta, g_alpha, alpha, theta, *p, N, (__nv_bfloat16 *)dT_hi,
-                                (__nv_bfloat16 *)dT_lo, (long long)k_off, (long long)k_cols, err));
-    NBG_CUDA(cudaGetLastError());
-    return NBG_OK;
+    return adj_step<false>("nbg_lif_adjoint_step_fused", nullptr, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
+                           dI, g_theta, g_alpha, alpha, theta, p, B, N, dT_hi, dT_lo, k_off, k_cols, err, stream);
+}
+
+nbg_status nbg_lif_adjoint_step_parts(const void *w_hi, const void *w_lo, const void *dI_hi_in, const void *dI_lo_in,
+                                      void *dI_hi_out, void *dI_lo_out, const float *g_read, float c_t,
+                                      const float *u, const float *s, const uint8_t *m, const float *vprev,
+                                      float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
+                                      const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
+                                      void *dT_lo, int64_t k_off, int64_t k_cols, float *parts, int *err, void *stream) {
+    if (!parts) return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_step_parts: parts is NULL");
+    return adj_step<true>("nbg_lif_adjoint_step_parts", parts, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
+                           dI, g_theta, g_alpha, alpha, theta, p, B, N, dT_hi, dT_lo, k_off, k_cols, err, stream);
 }
 
 nbg_status nbg_adjoint_blocked_t(const float *src, int L, int B, int R, int R_pad, void *hi, void *lo,

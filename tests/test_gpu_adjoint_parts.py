@@ -1,0 +1,53 @@
+"""The fused adjoint step's two ways to exchange its split-K partials (distributed shared memory, a workspace in global
+memory) give the same bits in every output, at the smallest N, an odd multiple of 128 (ragged K split) and above one pipeline."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [512, 640, 1152, 1664])
+def test_exchange_through_global_memory_equals_distributed_shared_memory(n):
+    from neuronbridge_gb300 import adjoint
+    from neuronbridge_gb300.adjoint import _bind, _ptr
+
+    lib = _bind()
+    fused = lib.nbg_lif_adjoint_step_fused
+    fused.restype, fused.argtypes = ctypes.c_int, lib.nbg_lif_adjoint_step_parts.argtypes[:-3] + [ctypes.c_void_p] * 2
+    b, k_cols = 128, 256
+    g = torch.Generator(device="cuda").manual_seed(n)
+    r = lambda *shape: torch.randn(*shape, generator=g, device="cuda")
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    w = r(n, n) / n ** 0.5
+    w_hi, w_lo, d_hi, d_lo = (torch.empty(k, device="cuda", dtype=torch.bfloat16) for k in (n * n, n * n, b * n, b * n))
+    assert lib.nbg_adjoint_rec_prepare(_ptr(w), _ptr(w_hi), _ptr(w_lo), n, st) == 0
+    d_hi.copy_(r(b * n))
+    d_lo.copy_(r(b * n) * 2.0 ** -9)
+    g_read, u, vprev = r(b, n), r(b, n), r(b, n)
+    s, m = (u > 0.5).float(), (r(b, n) > -1.0).to(torch.uint8)
+    alpha, theta = torch.full((n,), 0.9, device="cuda"), torch.full((n,), 0.5, device="cuda")
+    acc = [r(b, n) for _ in range(3)]
+    p = adjoint.GradParams()
+    p.v_rest, p.v_reset, p.slope, p.smooth = 0.0, -0.1, 10.0, 0
+    out = []
+    for parts in (None, torch.empty(8 * b * n, device="cuda")):
+        lam_v, g_theta, g_alpha = (x.clone() for x in acc)
+        dI = torch.empty(b, n, device="cuda")
+        o = [torch.empty(b * n, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+        t = [torch.zeros(n * k_cols, device="cuda", dtype=torch.bfloat16) for _ in range(2)]
+        err = torch.zeros(1, device="cuda", dtype=torch.int32)
+        args = [_ptr(w_hi), _ptr(w_lo), _ptr(d_hi), _ptr(d_lo), _ptr(o[0]), _ptr(o[1]), _ptr(g_read), 0.25, _ptr(u), _ptr(s),
+                _ptr(m), _ptr(vprev), _ptr(lam_v), _ptr(dI), _ptr(g_theta), _ptr(g_alpha), _ptr(alpha), _ptr(theta),
+                ctypes.byref(p), b, n, _ptr(t[0]), _ptr(t[1]), 128, k_cols]
+        if parts is None:
+            assert fused(*args, _ptr(err), st) == 0
+        else:
+            assert lib.nbg_lif_adjoint_step_parts(*args, _ptr(parts), _ptr(err), st) == 0
+            assert lib.nbg_lif_adjoint_step_parts(*args, None, _ptr(err), st) != 0  # refused, nothing launched
+        assert int(err.item()) == 0
+        out.append((dI, lam_v, g_theta, g_alpha, *o, *t))
+    assert torch.isfinite(out[0][0]).all() and out[0][0].abs().sum() > 0
+    for x, y in zip(*out):
+        assert torch.equal(x, y)
