@@ -147,6 +147,22 @@ nbg_status nbg_lif_adjoint_step_parts(const void *w_hi, const void *w_lo, const 
                                       const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
                                       void *dT_lo, int64_t k_off, int64_t k_cols, float *parts, int *err, void *stream);
 
+/* The steps t0 + steps - 1 .. t0 in one launch, with the results of as many
+ * calls of nbg_lif_adjoint_step_parts: u, s, m and vprev are the record of step
+ * t0 and the following ones, B x N each; coef the steps' readout coefficients on
+ * the device; step t reads dI_{t+1} from d_hi/lo[(t + 1) % 2] and writes
+ * d_hi/lo[t % 2]; its columns of dT start at k_off + (t - t0) * B.  `work` is
+ * nbg_lif_adjoint_sweep_work floats, 16-byte aligned and not shared with another
+ * stream; that call returns 0 where the device cannot hold all CTAs at once (or
+ * the shape is not the step's), and the sweep is refused. */
+int64_t nbg_lif_adjoint_sweep_work(int B, int N);
+nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0, void *d_lo0, void *d_hi1, void *d_lo1,
+                                 const float *g_read, const float *coef, const float *u, const float *s,
+                                 const uint8_t *m, const float *vprev, float *lam_v, float *g_theta, float *g_alpha,
+                                 const float *alpha, const float *theta, const nbg_lif_grad_params *p, int steps, int t0,
+                                 int B, int N, void *dT_hi, void *dT_lo, int64_t k_off, int64_t k_cols, float *work,
+                                 int *err, void *stream);
+
 /* The recurrent weight gradient of a checkpoint segment on the tensor cores,
  * dW_rec += sum over its L steps of S_{t-1}^T dI_t, in three calls:
  *   nbg_adjoint_blocked_t   src [L][B][R] FP32 -> the R_pad x (L*B) matrix,

@@ -525,6 +525,363 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     }
 }
 
+// The adjoint steps of a whole segment in one cooperative launch: the products,
+// partial sums and step of k_adj_step_umma, so the same results bit for bit, with
+// the loop over the steps inside.  Between two launches a step waited for the last
+// CTA of the one before, for its writes and for its own set-up; here the CTAs
+// stay: lam_v and the gradients are registers, W stays in shared memory where a
+// CTA's chunks have a stage each, the next step's operands are on their way during
+// this one, and a CTA's product waits only for the dI that its K range reads.
+//
+// Split: 32 batch rows of a 128-row tile of W are a chain of their own, run by a
+// cluster of four CTAs with two of the eight K ranges each (two accumulators): at
+// N = 1024 32 clusters, of which 36 fit on 152 SMs (15 of eight CTAs).  A CTA sends
+// its peers 24 KiB of partials a step through distributed shared memory and reads
+// 32 KiB of dI, half of what the step launch moves.
+//
+// What bounds it: the latency of two exchanges a step, that of the partials in the
+// cluster and that of dI through the L2 (publish, poll, copy: about 2 us).  Forward
+// and backward of 1,000 steps of 128 x 1,024: 9.97 ms with a launch a step, 9.45
+// in one launch with clusters of eight (64 CTAs, partials through the L2), 9.53 as
+// here but through the L2, 9.31 as here.
+//
+// Order.  The product of step j overwrites the accumulators after `exchanged` of
+// step j - 1, which comes after their last read.  The receive buffers alternate,
+// since a CTA may be a step ahead of a peer that still reads; it cannot be two
+// ahead (`exchanged` between).  dI alternates likewise: a CTA writes step j's into
+// the buffer of step j - 2 after `exchanged` of step j, so after dI of step j - 1 of
+// every tile (a cluster's K ranges cover all of them), which their CTAs wrote after
+// their products had read it.
+//
+// The launch is cooperative, so all CTAs run at once; every wait is bounded all the
+// same.  A CTA that gives up goes through the remaining steps without waiting,
+// reading or publishing anything, its peers' waits run out once, and the error
+// word marks the results.
+constexpr int kSweepN = 32, kSweepCluster = 4, kSweepStages = 4; // batch rows of a CTA; CTAs of a cluster; pipeline stages
+constexpr int kSweepParts = kAdjN / kSweepN;
+constexpr int kSweepBlockB = kSweepN * kKChunk * 2; // 4 KiB
+constexpr int kSweepStageBytes = 2 * kAdjBlockA + 2 * kSweepBlockB;
+constexpr int kSweepTailWarps = 8, kSweepThreads = 32 * (kSweepTailWarps + 2);
+constexpr uint32_t kSweepIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kSweepN >> 3) << 17) |
+                                 ((uint32_t)(kAdjM >> 4) << 24);
+constexpr int kReadyStride = 32; // a count has a line of its own
+constexpr int kSweepRecv = kAdjCluster * 2 * kAdjM; // 16-byte pieces that a rank receives in a step
+constexpr int kSweepSmemBytes = kSweepStages * kSweepStageBytes + 2 * kSweepRecv * 16 + 1024 + 256;
+static_assert(kSweepSmemBytes <= 232448, "shared memory of a CTA");
+
+__device__ __forceinline__ bool sweep_ready(const int *flag, int want, volatile int *abort) {
+    const long long t0 = clock64();
+    for (;;) {
+        int x;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(x) : "l"(flag) : "memory");
+        if (x >= want) return true;
+        if (*abort) return false;
+        if (clock64() - t0 > kWaitCycles) {
+            *abort = 1;
+            return false;
+        }
+    }
+}
+
+// mbar_wait for what the cluster's other CTAs wrote before they arrived.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity, volatile int *abort) {
+    const long long t0 = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}"
+                     : "=r"(ok)
+                     : "r"(smem_addr(bar)), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+        if (*abort) return false;
+        if (clock64() - t0 > kWaitCycles) {
+            *abort = 1;
+            return false;
+        }
+    }
+}
+
+// Waits (bounded) for a phase although the CTA has given up.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try(bar, parity) && clock64() - t0 < kWaitCycles) {
+    }
+}
+
+__global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
+    const __nv_bfloat16 *__restrict__ w_hi, const __nv_bfloat16 *__restrict__ w_lo, __nv_bfloat16 *d_hi0,
+    __nv_bfloat16 *d_lo0, __nv_bfloat16 *d_hi1, __nv_bfloat16 *d_lo1, const float *__restrict__ g_read,
+    const float *__restrict__ coef, const float *__restrict__ u, const float *__restrict__ s,
+    const unsigned char *__restrict__ m, const float *__restrict__ vprev, float *__restrict__ lam_v,
+    float *__restrict__ g_theta, float *__restrict__ g_alpha, const float *__restrict__ alpha,
+    const float *__restrict__ theta, nbg_lif_grad_params p, int n, int steps, int t0, __nv_bfloat16 *__restrict__ dT_hi,
+    __nv_bfloat16 *__restrict__ dT_lo, long long k_off, long long k_cols, int *ready,
+    int *__restrict__ err) {
+    constexpr int kStages = kSweepStages, kRows = 4;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *stages = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    float4 *recv = reinterpret_cast<float4 *>(stages + kStages * kSweepStageBytes); // of the even and the odd steps
+    uint64_t *full_w = (uint64_t *)(recv + 2 * kSweepRecv);
+    uint64_t *full_d = full_w + kStages;
+    uint64_t *empty = full_d + kStages;
+    uint64_t *done = empty + kStages, *exchanged = done + 1;
+    uint32_t *tmem_slot = (uint32_t *)(exchanged + 1);
+    volatile int *abort = (volatile int *)(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int mt = blockIdx.x / kSweepParts, bq = blockIdx.x % kSweepParts, ks = (int)rank;
+    const int kchunks = n / kKChunk;
+    const int per = kchunks / kAdjCluster;
+    const int kc0 = 2 * ks * per; // two of the eight K ranges; the last takes the rest
+    const int iters = (ks == kSweepCluster - 1) ? kchunks - kc0 : 2 * per;
+    const int pre = iters < kStages ? iters : kStages;
+
+    if (threadIdx.x == 0) {
+        for (int st = 0; st < kStages; ++st) {
+            mbar_init(&full_w[st], 1);
+            mbar_init(&full_d[st], 1);
+            mbar_init(&empty[st], 1);
+        }
+        mbar_init(done, 1);
+        mbar_init(exchanged, kSweepCluster);
+        *abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *tmem_slot;
+    // the cluster's barriers are initialised
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+
+    // Chunk c of step j is piece g = j * iters + c.  Where a CTA's chunks have a
+    // stage each, W stays there; else piece g passes through stage g % kStages.
+    const bool stay = iters <= kStages;
+    auto stage = [&](int j, int c) { return stay ? c : (int)(((long long)j * iters + c) % kStages); };
+    auto phase = [&](int j, int c) { return stay ? (uint32_t)j & 1u : (uint32_t)(((long long)j * iters + c) / kStages) & 1u; };
+    long long sent_w = 0, sent_d = 0; // producer: pieces requested
+    auto send_w = [&](int j, int c) { // once the products on the stage's last piece are done
+        const long long g = (long long)j * iters + c;
+        const int st_i = stage(j, c);
+        if ((stay ? j > 0 : g >= kStages) && !mbar_wait(&empty[st_i], phase(j, c) ^ 1u, abort)) return false;
+        sent_w = g + 1;
+        if (stay && j > 0) return true;
+        uint8_t *st = stages + st_i * kSweepStageBytes;
+        const size_t a_blk = ((size_t)mt * kchunks + kc0 + c) * kAdjBlockA;
+        mbar_expect_tx(&full_w[st_i], 2 * kAdjBlockA);
+        bulk_copy(st, (const uint8_t *)w_hi + a_blk, kAdjBlockA, &full_w[st_i]);
+        bulk_copy(st + kAdjBlockA, (const uint8_t *)w_lo + a_blk, kAdjBlockA, &full_w[st_i]);
+        return true;
+    };
+    const bool tail = warp < kSweepTailWarps;
+    const int il = threadIdx.x & 127, bsub = threadIdx.x >> 7;
+    const int i = mt * kAdjM + il, b0 = bq * kSweepN + 8 * ks + 4 * bsub;
+    float gr[kRows], lv[kRows], gt[kRows], ga[kRows], op_u[kRows], op_s[kRows], op_vp[kRows];
+    unsigned char op_m[kRows];
+    float th = 0.0f, al = 0.0f;
+    const size_t at0 = (size_t)b0 * n + i, per_step = (size_t)kAdjN * n;
+    auto operands = [&](int k) { // of step t0 + k
+        const size_t at = (size_t)k * per_step + at0;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            op_u[r] = u[at + (size_t)r * n];
+            op_s[r] = s[at + (size_t)r * n];
+            op_vp[r] = vprev[at + (size_t)r * n];
+            op_m[r] = m[at + (size_t)r * n];
+        }
+    };
+    if (tail) {
+        th = theta[i];
+        al = alpha[i];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            gr[r] = g_read[at0 + (size_t)r * n];
+            lv[r] = lam_v[at0 + (size_t)r * n];
+            gt[r] = g_theta[at0 + (size_t)r * n];
+            ga[r] = g_alpha[at0 + (size_t)r * n];
+        }
+        operands(steps - 1);
+    } else if (warp == kSweepTailWarps && lane == 0) {
+        for (int c = 0; c < pre; ++c) send_w(0, c);
+    }
+    for (int j = 0; j < steps; ++j) {
+        const int k = steps - 1 - j, t = t0 + k;
+        __nv_bfloat16 *const out_hi = t & 1 ? d_hi1 : d_hi0, *const out_lo = t & 1 ? d_lo1 : d_lo0;
+        float4 *const got = recv + (j & 1) * kSweepRecv;
+        if (warp == kSweepTailWarps) {
+            if (lane == 0) { // producer
+                const uint8_t *in_hi = (const uint8_t *)(t & 1 ? d_hi0 : d_hi1);
+                const uint8_t *in_lo = (const uint8_t *)(t & 1 ? d_lo0 : d_lo1);
+                const long long g0 = (long long)j * iters;
+                for (int c = 0; c < iters && !*abort; ++c) {
+                    if (g0 + c >= sent_w && !send_w(j, c)) break;
+                    const int kc = kc0 + c, st_i = stage(j, c);
+                    if (j > 0 && (c == 0 || kc % 2 == 0)) { // the tile's CTAs of these rows have written step j - 1's dI
+                        if (!sweep_ready(ready + (kc / 2 * kSweepParts + bq) * kReadyStride, kSweepCluster * j, abort)) break;
+                        asm volatile("fence.proxy.async.global;" ::: "memory");
+                    }
+                    uint8_t *st = stages + st_i * kSweepStageBytes;
+                    const size_t d_at = (size_t)kc * kAdjBlockB + (size_t)bq * kSweepBlockB;
+                    mbar_expect_tx(&full_d[st_i], 2 * kSweepBlockB);
+                    bulk_copy(st + 2 * kAdjBlockA, in_hi + d_at, kSweepBlockB, &full_d[st_i]);
+                    bulk_copy(st + 2 * kAdjBlockA + kSweepBlockB, in_lo + d_at, kSweepBlockB, &full_d[st_i]);
+                    sent_d = g0 + c + 1;
+                }
+                if (j + 1 < steps) // the next step's W, as its stages get free
+                    for (int c = 0; c < pre && !*abort; ++c)
+                        if (!send_w(j + 1, c)) break;
+            }
+            __syncwarp();
+        } else if (warp == kSweepTailWarps + 1) {
+            if (lane == 0 && j > 0 && mbar_wait_cluster(exchanged, (j - 1) & 1, abort)) // the accumulator has been read
+                fence_after();
+            if (lane == 0 && !*abort) { // MMA issuer
+                for (int c = 0; c < iters; ++c) {
+                    const int st_i = stage(j, c);
+                    const uint32_t ph = phase(j, c);
+                    if (!mbar_wait(&full_w[st_i], stay ? 0u : ph, abort) || !mbar_wait(&full_d[st_i], ph, abort)) break;
+                    fence_after();
+                    const uint32_t a_hi = smem_addr(stages + st_i * kSweepStageBytes);
+                    const uint32_t a_lo = a_hi + kAdjBlockA;
+                    const uint32_t b_hi = a_hi + 2 * kAdjBlockA;
+                    const uint32_t b_lo = b_hi + kSweepBlockB;
+                    const bool second = c >= per; // of the CTA's two K ranges
+                    const uint32_t acc = tmem + (second ? kSweepN : 0u);
+                    const bool first = c == (second ? per : 0);
+#pragma unroll
+                    for (int q = 0; q < kKChunk / 16; ++q) {
+                        mma(acc, make_desc(a_hi + 256 * q), make_desc(b_hi + 256 * q), kSweepIdesc, !first || q != 0);
+                        mma(acc, make_desc(a_lo + 256 * q), make_desc(b_hi + 256 * q), kSweepIdesc, 1u);
+                        mma(acc, make_desc(a_hi + 256 * q), make_desc(b_lo + 256 * q), kSweepIdesc, 1u);
+                    }
+                    commit(&empty[st_i]);
+                }
+                commit(done);
+                if (*abort) mbar_drain(done, j & 1);
+            }
+            __syncwarp();
+        }
+        float ds[kRows], gs0[kRows], gu0[kRows], dv[kRows];
+        bool keep[kRows];
+        if (tail) {
+            const float c_t = coef[k];
+#pragma unroll
+            for (int r = 0; r < kRows; ++r) {
+                const float ss = op_s[r];
+                ds[r] = p.smooth ? p.slope * ss * (1.0f - ss) : surrogate(op_u[r] - th, p.slope);
+                gs0[r] = c_t * gr[r] - lv[r] * (op_u[r] - p.v_reset);
+                gu0[r] = lv[r] * (1.0f - ss);
+                dv[r] = p.v_rest - op_vp[r];
+                keep[r] = op_m[r];
+            }
+            mbar_wait(done, j & 1, abort);
+            __syncwarp();
+            fence_after();
+            if (__all_sync(0xffffffffu, !*abort)) {
+                const int q = warp & 3, g = warp >> 2;
+                // K range 2 ks + g, rows i = 32 q + lane, batch columns 8 o + c of rank o
+                const uint32_t mine = smem_addr(got + (2 * ks + g) * 2 * kAdjM + il);
+#pragma unroll
+                for (int c16 = 0; c16 < 2; ++c16) {
+                    float acc[16];
+                    tmem_ld16(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * g + 16 * c16), acc);
+#pragma unroll
+                    for (int c = 0; c < 16; c += 4) {
+                        uint32_t ra;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(mine), "r"(2 * c16 + c / 8));
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra + (uint32_t)((c / 4 & 1) * kAdjM * 16)),
+                                     "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3])
+                                     : "memory");
+                    }
+                }
+            }
+            fence_before();
+            // the partials are in place and the accumulator read: one arrival at each of the cluster's CTAs
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kSweepTailWarps) : "memory");
+            if (threadIdx.x < kSweepCluster && !*abort) {
+                uint32_t ra;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_addr(exchanged)), "r"(threadIdx.x));
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(ra) : "memory");
+            }
+            __syncwarp();
+            mbar_wait_cluster(exchanged, j & 1, abort);
+            float x[kAdjCluster][kRows];
+#pragma unroll
+            for (int r = 0; r < kAdjCluster; ++r)
+                *reinterpret_cast<float4 *>(x[r]) = got[(r * 2 + bsub) * kAdjM + il];
+            uint32_t t_hi[kRows / 2], t_lo[kRows / 2]; // dI^T of the rows, split, packed in pairs
+#pragma unroll
+            for (int r = 0; r < kRows; ++r) {
+                float ge = x[0][r];
+#pragma unroll
+                for (int c = 1; c < kAdjCluster; ++c) ge = ge + x[c][r];
+                const float gs = gs0[r] + ge;
+                const float gu = gs * ds[r] + gu0[r];
+                const float gm = keep[r] ? gu : 0.0f;
+                const size_t o = blocked_index(b0 + r, i, n);
+                __nv_bfloat16 h, l;
+                split_bf16(gm, h, l);
+                out_hi[o] = h;
+                out_lo[o] = l;
+                const uint32_t hb = __bfloat16_as_ushort(h), lb = __bfloat16_as_ushort(l);
+                if (r & 1) {
+                    t_hi[r >> 1] |= hb << 16;
+                    t_lo[r >> 1] |= lb << 16;
+                } else {
+                    t_hi[r >> 1] = hb;
+                    t_lo[r >> 1] = lb;
+                }
+                lv[r] = gm * (1.0f - al);
+                gt[r] = gt[r] - gs * ds[r];
+                ga[r] = ga[r] + gm * dv[r];
+            }
+            // publish: all of this CTA's dI, then one count
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kSweepTailWarps) : "memory");
+            if (threadIdx.x == 0 && !*abort)
+                asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(ready + blockIdx.x * kReadyStride) : "memory");
+            if (k > 0) operands(k - 1);
+            const size_t o = blocked_index(i, (int)(k_off + (long long)k * kAdjN + b0), (int)k_cols);
+            reinterpret_cast<uint2 *>(dT_hi + o)[0] = make_uint2(t_hi[0], t_hi[1]);
+            reinterpret_cast<uint2 *>(dT_lo + o)[0] = make_uint2(t_lo[0], t_lo[1]);
+        }
+    }
+    if (tail) {
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            lam_v[at0 + (size_t)r * n] = lv[r];
+            g_theta[at0 + (size_t)r * n] = gt[r];
+            g_alpha[at0 + (size_t)r * n] = ga[r];
+        }
+    } else if (warp == kSweepTailWarps && lane == 0 && *abort) { // its own copies in flight
+        for (int c = 0; c < kStages; ++c) {
+            const long long gw = sent_w - 1 - c, gd = sent_d - 1 - c;
+            if (gw >= 0)
+                mbar_drain(&full_w[stage((int)(gw / iters), (int)(gw % iters))],
+                           stay ? 0u : phase((int)(gw / iters), (int)(gw % iters)));
+            if (gd >= 0)
+                mbar_drain(&full_d[stage((int)(gd / iters), (int)(gd % iters))], phase((int)(gd / iters), (int)(gd % iters)));
+        }
+    }
+    __syncthreads();
+    // no CTA leaves before its peers have arrived at its barrier
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (threadIdx.x == 0 && *abort) atomicOr(err, kUmmaTimeout);
+    if (warp == 2) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols)
+                     : "memory");
+    }
+}
+
 // [L][B][R] FP32 -> the R x (L*B) matrix (row r, K = l*B + b) in the blocked
 // layout, split into hi and lo (lo may be null: the values are exact in BF16).
 // [L][B][R] FP32 -> the R_pad x (L*B) matrix (row r, K = l*B + b) in the
@@ -745,6 +1102,22 @@ static nbg_status adj_step(const char *name, float *parts, const void *w_hi, con
     return NBG_OK;
 }
 
+static void sweep_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute (&attr)[2], int N, void *stream) {
+    cfg = {};
+    cfg.gridDim = dim3(N / kAdjM * kSweepParts, kSweepCluster);
+    cfg.blockDim = dim3(kSweepThreads);
+    cfg.dynamicSmemBytes = kSweepSmemBytes;
+    cfg.stream = (cudaStream_t)stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = kSweepCluster;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeCooperative;
+    attr[1].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+}
+
 extern "C" {
 
 nbg_status nbg_adjoint_rec_prepare(const float *w_rec, void *w_hi, void *w_lo, int N, void *stream) {
@@ -829,6 +1202,54 @@ nbg_status nbg_lif_adjoint_step_parts(const void *w_hi, const void *w_lo, const 
     if (!parts) return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_step_parts: parts is NULL");
     return adj_step<true>("nbg_lif_adjoint_step_parts", parts, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
                            dI, g_theta, g_alpha, alpha, theta, p, B, N, dT_hi, dT_lo, k_off, k_cols, err, stream);
+}
+
+int64_t nbg_lif_adjoint_sweep_work(int B, int N) {
+    if (!adj_shape_ok(B, N) || N / kKChunk < kAdjCluster) return 0;
+    if (cudaFuncSetAttribute(k_adj_sweep_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmemBytes) !=
+        cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    sweep_config(cfg, attr, N, nullptr);
+    cfg.numAttrs = 1; // the cluster's
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_adj_sweep_umma, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return 0;
+    }
+    const int tiles = N / kAdjM * kSweepParts;
+    return clusters >= tiles ? tiles * kReadyStride : 0;
+}
+
+nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0, void *d_lo0, void *d_hi1, void *d_lo1,
+                                 const float *g_read, const float *coef, const float *u, const float *s,
+                                 const uint8_t *m, const float *vprev, float *lam_v, float *g_theta, float *g_alpha,
+                                 const float *alpha, const float *theta, const nbg_lif_grad_params *p, int steps, int t0,
+                                 int B, int N, void *dT_hi, void *dT_lo, int64_t k_off, int64_t k_cols, float *work,
+                                 int *err, void *stream) {
+    if (!w_hi || !w_lo || !d_hi0 || !d_lo0 || !d_hi1 || !d_lo1 || !g_read || !coef || !u || !s || !m || !vprev || !lam_v ||
+        !g_theta || !g_alpha || !alpha || !theta || !p || !dT_hi || !dT_lo || !work || !err || steps <= 0 || t0 < 0 ||
+        d_hi0 == d_hi1 || d_lo0 == d_lo1 || k_off < 0 || k_off % kAdjN || k_cols % kKChunk ||
+        k_off + (int64_t)steps * B > k_cols || k_cols > 0x7fffffff || steps > 0x7fffffff / kAdjCluster)
+        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_sweep: bad arguments");
+    if (!nbg_lif_adjoint_sweep_work(B, N))
+        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_sweep: B must be %d, N a multiple of %d, at least %d and not "
+                        "more than the device holds at once", kAdjN, kAdjM, kAdjCluster * kKChunk);
+    int *ready = (int *)work;
+    NBG_CUDA(cudaMemsetAsync(ready, 0, (size_t)(N / kAdjM * kSweepParts) * kReadyStride * sizeof(int), (cudaStream_t)stream));
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    sweep_config(cfg, attr, N, stream);
+    NBG_CUDA(cudaLaunchKernelEx(&cfg, k_adj_sweep_umma, (const __nv_bfloat16 *)w_hi, (const __nv_bfloat16 *)w_lo,
+                                (__nv_bfloat16 *)d_hi0, (__nv_bfloat16 *)d_lo0, (__nv_bfloat16 *)d_hi1,
+                                (__nv_bfloat16 *)d_lo1, g_read, coef, u, s, (const unsigned char *)m, vprev, lam_v, g_theta,
+                                g_alpha, alpha, theta, *p, N, steps, t0, (__nv_bfloat16 *)dT_hi, (__nv_bfloat16 *)dT_lo,
+                                (long long)k_off, (long long)k_cols, ready, err));
+    NBG_CUDA(cudaGetLastError());
+    return NBG_OK;
 }
 
 nbg_status nbg_adjoint_blocked_t(const float *src, int L, int B, int R, int R_pad, void *hi, void *lo,

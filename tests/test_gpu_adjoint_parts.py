@@ -51,3 +51,67 @@ def test_exchange_through_global_memory_equals_distributed_shared_memory(n):
     assert torch.isfinite(out[0][0]).all() and out[0][0].abs().sum() > 0
     for x, y in zip(*out):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("n,record", [(512, True), (640, False), (768, False), (896, True), (1024, False), (1152, True)])
+def test_sweep_equals_the_steps(monkeypatch, n, record):
+    """A segment's steps in one launch against one launch each, bit for bit: N with two K chunks a CTA, with a last
+    CTA of more chunks than pipeline stages (768 and 1152: six, 896: eight), the largest that 152 SMs hold; the whole run or segments of 20 of 47 steps."""
+    from neuronbridge_gb300 import adjoint
+    from neuronbridge_gb300.adjoint import RecurrentLIF, _bind, poisson_inputs
+
+    torch.manual_seed(0)
+    model = RecurrentLIF(n_in=40, n_rec=n, n_out=5, checkpoint=20, seed=11, smooth=False, device="cuda", use_graphs=False,
+                         record=record)
+    x = poisson_inputs(torch.linspace(50.0, 400.0, 40), 47, 128, dt=1.0, seed=3)
+    labels = torch.arange(128, device="cuda") % 5
+    assert _bind().nbg_lif_adjoint_sweep_work(128, n) > 0 and _bind().nbg_lif_adjoint_sweep_work(128, 384) == 0
+    out = []
+    for sweep in (True, False):
+        monkeypatch.setattr(adjoint, "SWEEP", sweep)
+        model.zero_grad(set_to_none=True)
+        torch.nn.functional.cross_entropy(model(x), labels).backward()
+        out.append([q.grad.clone() for q in model.parameters()])
+    assert any(g.abs().sum() > 0 for g in out[0])
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
+def test_sweeps_on_two_streams_of_two_threads():
+    """Cooperative launches that do not fit beside one another, on streams of different priority: each gives what it gives
+    alone, and none of its bounded waits runs out."""
+    import threading
+
+    from neuronbridge_gb300.adjoint import RecurrentLIF, poisson_inputs
+
+    x = poisson_inputs(torch.linspace(50.0, 400.0, 40), 100, 128, dt=1.0, seed=3)
+    labels = torch.arange(128, device="cuda") % 5
+    models = []
+    for _ in range(2):
+        torch.manual_seed(0)
+        models.append(RecurrentLIF(n_in=40, n_rec=1024, n_out=5, seed=11, smooth=False, device="cuda", use_graphs=False))
+
+    def grads(model):
+        model.zero_grad(set_to_none=True)
+        torch.nn.functional.cross_entropy(model(x), labels).backward()
+        return [q.grad.clone() for q in model.parameters()]
+
+    want = grads(models[0])
+    torch.cuda.synchronize()
+    out = [None, None]
+
+    def work(k):
+        stream = torch.cuda.Stream(priority=-k)
+        with torch.cuda.stream(stream):
+            out[k] = [grads(models[k]) for _ in range(10)]
+            stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for runs in out:
+        for got in runs:
+            for a, b in zip(got, want):
+                assert torch.equal(a, b)
