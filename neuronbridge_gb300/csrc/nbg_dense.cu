@@ -332,6 +332,12 @@ __device__ __forceinline__ bool lif_apply(const LifParams &P, float a, bool driv
 // several of them need is read from memory once.  Measured, update included:
 // 154 -> 32.9 us a step at 8,192 neurons (8.2 TB/s of row reads), 100 steps
 // and their read-out at 2,048 neurons 2.61 -> 0.78 ms.
+//
+// The external spikes are drawn before the wait for the step before.  Registers
+// (kCtas, the CTAs an SM is to hold): where the grid has at most three CTAs an SM
+// the 73 that the loads in flight want, else 62 for four: 5.79 -> 4.95 us a step at
+// 2,048 neurons (5.65 with 62), 7.35 -> 5.97 (7.17) at 3,072, 8.81 -> 8.63 (9.57
+// with 73) at 4,096, 29.1 -> 29.0 (33.7) at 8,192.
 constexpr int kGatherThreads = 256;
 constexpr int kGatherCols = 2 * kGatherThreads; // columns of a CTA
 constexpr int kGatherWords = 256;               // spike words listed at a time (8,192 neurons)
@@ -345,8 +351,8 @@ __device__ __forceinline__ unsigned spread16(unsigned x) {
     return (x | x << 1) & 0x55555555u;
 }
 
-template <bool kLif>
-__global__ void __launch_bounds__(kGatherThreads) k_dense_gather(const float *__restrict__ w,
+template <bool kLif, int kCtas>
+__global__ void __launch_bounds__(kGatherThreads, kCtas) k_dense_gather(const float *__restrict__ w,
                                                                  const unsigned *__restrict__ sbits,
                                                                  float *__restrict__ cur, LifParams P, float *v,
                                                                  int *last, unsigned *__restrict__ bits_out,
@@ -359,8 +365,10 @@ __global__ void __launch_bounds__(kGatherThreads) k_dense_gather(const float *__
     const float *const col = w + (has ? j : 0);
     const int nw = n / 32;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory"); // the previous step's spikes, v and last
     const size_t at = (size_t)b * n + j;
+    // this step's external spikes do not depend on the step before
+    const bool d0 = kLif && has && lif_drive(P, t, (int)at), d1 = kLif && has && lif_drive(P, t, (int)at + 1);
+    asm volatile("griddepcontrol.wait;" ::: "memory"); // the previous step's spikes, v and last
     float2 vv = make_float2(0.0f, 0.0f);
     int2 ls = make_int2(0, 0);
     if (kLif && has) {
@@ -415,8 +423,8 @@ __global__ void __launch_bounds__(kGatherThreads) k_dense_gather(const float *__
     } else {
         bool s0 = false, s1 = false;
         if (has) {
-            s0 = lif_apply(P, sum.x, lif_drive(P, t, (int)at), vv.x, ls.x);
-            s1 = lif_apply(P, sum.y, lif_drive(P, t, (int)at + 1), vv.y, ls.y);
+            s0 = lif_apply(P, sum.x, d0, vv.x, ls.x);
+            s1 = lif_apply(P, sum.y, d1, vv.y, ls.y);
             *reinterpret_cast<float2 *>(v + at) = vv;
             *reinterpret_cast<int2 *>(last + at) = ls;
         }
@@ -481,6 +489,7 @@ struct LifFinish {
 struct nbg_dense {
     int device = 0, B = 64, N = 0, precision = 0;
     bool half_tiles = false; // tcgen05 step: tiles of 64 post neurons instead of 128
+    bool few_ctas = false;   // FP32 step: at most three CTAs an SM
     LifParams P{};
     DevBuf<float> w, partial, v;
     DevBuf<__nv_bfloat16> whi, wlo, s[2];
@@ -594,6 +603,11 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
     auto chk = [&](cudaError_t x) {
         if (ce == cudaSuccess) ce = x;
     };
+    int sms = 0;
+    chk(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const dim3 gg = gather_grid(d);
+    d->few_ctas = (int)(gg.x * gg.y) <= 3 * sms;
+    d->half_tiles = neurons / 64 * kSplitK <= sms;
     chk(cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking));
     chk(cudaEventCreate(&d->ev0));
     chk(cudaEventCreate(&d->ev1));
@@ -630,9 +644,6 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
             if (ce == cudaSuccess)
                 chk(cudaFuncSetAttribute(umma::k_dense_umma<LifFinish, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          umma::Tile<64>::fused_smem));
-            int sms = 0;
-            chk(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-            d->half_tiles = neurons / 64 * kSplitK <= sms;
         } else if (ce == cudaSuccess) {
             dim3 grid(neurons / 32, neurons / 32), block(32, 8);
             k_split_transpose<<<grid, block>>>(tmp.p, d->whi.p, d->wlo.p, neurons);
@@ -711,9 +722,9 @@ nbg_status nbg_dense_run(nbg_dense *d, int steps) {
             }
             if (d->precision == NBG_DENSE_FP32) { // gather and update in one launch
                 const cudaLaunchConfig_t cfg = step_config(d, gather_grid(d), kGatherThreads, 0, attr);
-                NBG_CUDA(cudaLaunchKernelEx(&cfg, k_dense_gather<true>, (const float *)d->w.p,
-                                            (const unsigned *)d->bits[in].p, (float *)nullptr, d->P, d->v.p, d->last.p,
-                                            d->bits[outp].p, dcnt.p + k, t, d->N));
+                NBG_CUDA(cudaLaunchKernelEx(&cfg, d->few_ctas ? k_dense_gather<true, 1> : k_dense_gather<true, 4>,
+                                            (const float *)d->w.p, (const unsigned *)d->bits[in].p, (float *)nullptr,
+                                            d->P, d->v.p, d->last.p, d->bits[outp].p, dcnt.p + k, t, d->N));
                 continue;
             }
             NBG_CUDA(cudaEventRecord(d->dev_pool[2 * (k - k0)], d->stream));
@@ -820,7 +831,7 @@ nbg_status nbg_dense_deliver(nbg_dense *d, const uint8_t *s, float *out) {
     } else {
         unsigned *const bits = reinterpret_cast<unsigned *>(d->io_s.p);
         k_spikes_in<kLayoutBits><<<grid8, 256, 0, st>>>(d->io_bytes.p, bits, d->N, groups);
-        k_dense_gather<false><<<gather_grid(d), kGatherThreads, 0, st>>>(d->w.p, bits, d->io_out.p, d->P, nullptr, nullptr,
+        k_dense_gather<false, 1><<<gather_grid(d), kGatherThreads, 0, st>>>(d->w.p, bits, d->io_out.p, d->P, nullptr, nullptr,
                                                                          nullptr, nullptr, 0, d->N);
     }
     if (split) k_sum_split_partials<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(d->io_part.p, d->io_out.p, (int)tot);
