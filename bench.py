@@ -57,16 +57,13 @@ BYTES_PER_LIF_NEURON_STEP = 24  # V r/w 8, refractory counter r/w 8, ring word r
 BYTES_PER_PLASTIC_EVENT = 40
 BYTES_PER_STATIC_EVENT = 12
 BYTES_PER_POST_UPDATE = 36
-# DRAM bytes (read + write) of one k_update launch of this workload (10 steps x
-# 100k neurons) from an ncu capture of that launch with a cold L2
-# (30.24 MB read + 0.16 MB written)
-KUPDATE_TRAFFIC_BYTES = 30.39e6
-# DRAM bytes (read + write) of one k_update launch of the 256-instance batched
-# workload (15 steps), scaled from an ncu capture on its first 32 instances
-BATCHED_TRAFFIC_BYTES = 2.478e9  # 267.7 MB on 282,235 LIF neurons x 2,612,540 / 282,235 (256 x 15 launches)
+# DRAM bytes (read + write) of one k_update_quad_rec launch of this workload (10
+# steps x 100k neurons) from an ncu capture with a cold L2 (the middle of three:
+# 34.01 MB read + 0.01 MB written)
+KUPDATE_TRAFFIC_BYTES = 34.02e6
 # DRAM bytes (read + write) of one dense step launch (64 x 8192, delivery and
 # update) from an ncu capture with a cold L2
-DENSE_TRAFFIC_BYTES = 277.5e6
+DENSE_TRAFFIC_BYTES = 273.8e6
 # device -> host bytes of a run call besides its raster entries (8 B each: step
 # and id) and traces: error word, raster cursor, ordered-entry count (4 B each)
 # and the delivered-event counter read by num_events (8 B)
@@ -225,7 +222,7 @@ def sigma5_sample(args, local: int, choice: dict | None) -> dict:
 
 def phase_split(neuron_bytes: float, delivery_bytes: float, dev_s: float, launches: int, silent: dict,
                 peak: float) -> dict:
-    """Roofline fractions of the two phases of k_update.  The neuron update
+    """Roofline fractions of the two phases of the update kernel.  The neuron update
     (with the drain of an empty arrival ring) is timed on the silent sigma-5
     network, the same launches with no spike and no arrival; delivery + STDP
     is the rest of the headline launch.  Each phase's algorithmic bytes over
@@ -356,7 +353,7 @@ def bench_lif(args) -> dict:
 
     net, cfg = workloads.plain_lif()
     # no per-launch events: they would sit between the launches of the graph
-    # and stretch it; the only kernel of the call is k_update, so the call's
+    # and stretch it; the update kernel is the only one of the call, so the call's
     # device time over its launches is the launch duration
     sim = nb.Simulation(net, cfg)
     tune = _launch_shape(sim, args, 1000)  # launch shape only; resets the simulation
@@ -393,7 +390,7 @@ def bench_lif(args) -> dict:
                     "block_steps": sim.block_steps, "tuned": tune["choice"],
                     "recorded": "raster of the LIF layer and V of neurons 0, 100, ..., 900 every step"},
                    neuron_steps_per_s=n * cfg.steps * args.steps / dev,
-                   roofline={"bound": "hbm", "kernel": "k_update", "achieved": upd_bytes / upd / 1e9, "peak": peak,
+                   roofline={"bound": "hbm", "kernel": "k_update_quad", "achieved": upd_bytes / upd / 1e9, "peak": peak,
                              "unit": "GB/s", "frac": upd_bytes / upd / 1e9 / peak, "peak_kind": kind,
                              "traffic": None},
                    e2e={"value": ev / wall, "unit": "synaptic events/s", "h2d_bytes_per_step": 16,
@@ -508,14 +505,13 @@ def bench_batched(args) -> dict | None:
         config["shard_lif_neurons"] = [int(x) for x in loads]
     line = _common(args, "synaptic events/s", value, "synaptic events/s", 1e3 * dev_all / args.steps, config,
                    neuron_steps_per_s=int(sizes.sum()) * cfg.steps * args.steps / dev_all,
-                   roofline={"bound": "hbm", "kernel": "k_update<Spec<1, 0>> (LIF, static; Poisson generators "
+                   roofline={"bound": "hbm", "kernel": "k_update_quad (LIF, static, palette codes; Poisson generators "
                                                        "packed eight per thread)",
                              "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "peak_kind": kind,
                              "scope": "per GPU" if world == 1 else
                              f"per GPU: all {world} ranks' bytes / slowest rank's time / {world}",
-                             "traffic": (BATCHED_TRAFFIC_BYTES if args.instances == 256 and world == 1 else None),
-                             "traffic_unit": "bytes per launch (ncu on 32 instances, scaled by units)",
+                             "traffic": None,
                              "algorithmic_bytes_per_launch": upd_bytes / (per_launch * args.steps),
                              "avg_update_launch_us": 1e6 * dev / launches if launches else None},
                    plain={"value": plain, "unit": "synaptic events/s", "device_s_per_1000_steps": p_dev_all,
@@ -679,7 +675,7 @@ def main() -> None:
     net, cfg = workloads.izhikevich_stdp()
     desc = net.to_native()
     # no per-launch events (they would sit between the graph's launches and
-    # stretch it): k_update is the only kernel of a run call, so the call's
+    # stretch it): the update kernel is the only one of a run call, so the call's
     # device time (CUDA events on the engine stream) over its launch count is
     # the average launch duration
     sim = nb.Simulation(desc, cfg, device=local, seed=2)
@@ -752,7 +748,7 @@ def main() -> None:
         "launch_shape": {"block_steps": sim.block_steps, "tuned": tune["choice"]},
         "neuron_steps_per_s": n * sim_steps * world / tot_dev,
         "spikes_per_s_simulated": tot_spk / (sim_steps * 1e-4) / n,
-        "roofline": {"bound": "hbm", "kernel": "k_update (drain + RK4 + STDP + spike propagation)",
+        "roofline": {"bound": "hbm", "kernel": "k_update_quad_rec (drain + RK4 + STDP + spike propagation)",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "peak_kind": peak_kind,
                      "traffic": KUPDATE_TRAFFIC_BYTES if args.sim_steps % 10 == 0 else None,
