@@ -147,8 +147,9 @@ nbg_status nbg_lif_adjoint_step_parts(const void *w_hi, const void *w_lo, const 
                                       const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
                                       void *dT_lo, int64_t k_off, int64_t k_cols, float *parts, int *err, void *stream);
 
-/* The steps t0 + steps - 1 .. t0 in one launch, with the results of as many
- * calls of nbg_lif_adjoint_step_parts: u, s, m and vprev are the record of step
+/* The steps t0 + steps - 1 .. t0 in one launch, for every N that is a multiple of
+ * 128, with the results of as many calls of nbg_lif_adjoint_step_parts (N < 512: of
+ * nbg_lif_adjoint_step_split and nbg_adjoint_rec_grad): u, s, m and vprev are the record of step
  * t0 and the following ones, B x N each; coef the steps' readout coefficients on
  * the device; step t reads dI_{t+1} from d_hi/lo[(t + 1) % 2] and writes
  * d_hi/lo[t % 2]; its columns of dT start at k_off + (t - t0) * B.  `work` is

@@ -205,8 +205,9 @@ def _tc_ok(p, B: int, N: int) -> bool:
 FUSED_STEP = True
 # ... and one launch per segment where the device holds all of its CTAs at once
 # (nbg_lif_adjoint_sweep; up to 1,152 neurons on 152 SMs): faster at every such size,
-# 2.95 ms against 3.39 for a forward and backward of 400 steps at 512 neurons, 4.47
-# against 4.69 at 896, 4.19 against 4.48 at 1,152.
+# 2.99 ms against 3.69 (two launches a step) for a forward and backward of 400 steps at
+# 128 neurons, 3.02 against 3.94 at 384, 2.95 against 3.39 (one) at 512, 4.47 against
+# 4.69 at 896, 4.19 against 4.48 at 1,152.
 SWEEP = True
 
 
@@ -366,6 +367,8 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
     # with the state recorded, the weight gradients run once, over every
     # (step, row) pair of the run
     whole = rec is not None and (fused or not tc)
+    sweep = lib.nbg_lif_adjoint_sweep_work(B, N) if tc and FUSED_STEP and SWEEP else 0
+    fused = fused or sweep > 0
     smooth = _Smooth(lib, w_in, w_rec, B, st) if p.smooth and rec is None else None
     I = None if sparse or smooth else torch.empty((B, N), device=dev, dtype=torch.float32)
     # the fused step writes dI^T for the weight gradients itself (no FP32 dI,
@@ -385,7 +388,6 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
         d_hi = [torch.zeros(B * N, device=dev, dtype=torch.bfloat16) for _ in range(2 if fused else 1)]
         d_lo = [torch.zeros(B * N, device=dev, dtype=torch.bfloat16) for _ in range(2 if fused else 1)]
         split = min(TC_SPLIT, N // 64)
-        sweep = lib.nbg_lif_adjoint_sweep_work(B, N) if fused and SWEEP else 0
         g_parts = torch.empty(sweep or (8 if fused else split) * B * N, device=dev, dtype=torch.float32)
         coef_dev = _coef_device(coef, dev) if sweep else None
         tc_err = torch.zeros(1, device=dev, dtype=torch.int32)

@@ -535,7 +535,8 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
 //
 // Split: 32 batch rows of a 128-row tile of W are a chain of their own, run by a
 // cluster of four CTAs with two of the eight K ranges each (two accumulators): at
-// N = 1024 32 clusters, of which 36 fit on 152 SMs (15 of eight CTAs).  A CTA sends
+// N = 1024 32 clusters, of which 36 fit on 152 SMs (15 of eight CTAs).  Below 512
+// neurons there are as many ranges as chunks, as in the two-launch form.  A CTA sends
 // its peers 24 KiB of partials a step through distributed shared memory and reads
 // 32 KiB of dI, half of what the step launch moves.
 //
@@ -543,7 +544,8 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
 // cluster and that of dI through the L2 (publish, poll, copy: about 2 us).  Forward
 // and backward of 1,000 steps of 128 x 1,024: 9.97 ms with a launch a step, 9.45
 // in one launch with clusters of eight (64 CTAs, partials through the L2), 9.53 as
-// here but through the L2, 9.31 as here.
+// here but through the L2, 9.31 as here.  400 steps at 384 neurons: 3.94 ms with two
+// launches a step, 3.02 as here.
 //
 // Order.  The product of step j overwrites the accumulators after `exchanged` of
 // step j - 1, which comes after their last read.  The receive buffers alternate,
@@ -634,9 +636,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int mt = blockIdx.x / kSweepParts, bq = blockIdx.x % kSweepParts, ks = (int)rank;
     const int kchunks = n / kKChunk;
-    const int per = kchunks / kAdjCluster;
-    const int kc0 = 2 * ks * per; // two of the eight K ranges; the last takes the rest
-    const int iters = (ks == kSweepCluster - 1) ? kchunks - kc0 : 2 * per;
+    // two of the K ranges, eight or as many as there are chunks; the last CTA that
+    // has any takes the rest, one without runs its rows of the step alone
+    const int ranges = kchunks < kAdjCluster ? kchunks : kAdjCluster;
+    const int per = kchunks / ranges;
+    const int kc0 = 2 * ks * per;
+    const int iters = 2 * ks >= ranges ? 0 : 2 * ks + 2 == ranges ? kchunks - kc0 : 2 * per;
     const int pre = iters < kStages ? iters : kStages;
 
     if (threadIdx.x == 0) {
@@ -786,7 +791,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
             mbar_wait(done, j & 1, abort);
             __syncwarp();
             fence_after();
-            if (__all_sync(0xffffffffu, !*abort)) {
+            if (__all_sync(0xffffffffu, !*abort) && iters > 0) {
                 const int q = warp & 3, g = warp >> 2;
                 // K range 2 ks + g, rows i = 32 q + lane, batch columns 8 o + c of rank o
                 const uint32_t mine = smem_addr(got + (2 * ks + g) * 2 * kAdjM + il);
@@ -817,13 +822,15 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
             float x[kAdjCluster][kRows];
 #pragma unroll
             for (int r = 0; r < kAdjCluster; ++r)
-                *reinterpret_cast<float4 *>(x[r]) = got[(r * 2 + bsub) * kAdjM + il];
+                if (r < ranges)
+                    *reinterpret_cast<float4 *>(x[r]) = got[(r * 2 + bsub) * kAdjM + il];
             uint32_t t_hi[kRows / 2], t_lo[kRows / 2]; // dI^T of the rows, split, packed in pairs
 #pragma unroll
             for (int r = 0; r < kRows; ++r) {
                 float ge = x[0][r];
 #pragma unroll
-                for (int c = 1; c < kAdjCluster; ++c) ge = ge + x[c][r];
+                for (int c = 1; c < kAdjCluster; ++c)
+                    if (c < ranges) ge = ge + x[c][r];
                 const float gs = gs0[r] + ge;
                 const float gu = gs * ds[r] + gu0[r];
                 const float gm = keep[r] ? gu : 0.0f;
@@ -1205,7 +1212,7 @@ nbg_status nbg_lif_adjoint_step_parts(const void *w_hi, const void *w_lo, const 
 }
 
 int64_t nbg_lif_adjoint_sweep_work(int B, int N) {
-    if (!adj_shape_ok(B, N) || N / kKChunk < kAdjCluster) return 0;
+    if (!adj_shape_ok(B, N)) return 0;
     if (cudaFuncSetAttribute(k_adj_sweep_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, kSweepSmemBytes) !=
         cudaSuccess) {
         (void)cudaGetLastError();
@@ -1236,8 +1243,8 @@ nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0
         k_off + (int64_t)steps * B > k_cols || k_cols > 0x7fffffff || steps > 0x7fffffff / kAdjCluster)
         return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_sweep: bad arguments");
     if (!nbg_lif_adjoint_sweep_work(B, N))
-        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_sweep: B must be %d, N a multiple of %d, at least %d and not "
-                        "more than the device holds at once", kAdjN, kAdjM, kAdjCluster * kKChunk);
+        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_sweep: B must be %d, N a multiple of %d and not more than the "
+                        "device holds at once", kAdjN, kAdjM);
     int *ready = (int *)work;
     NBG_CUDA(cudaMemsetAsync(ready, 0, (size_t)(N / kAdjM * kSweepParts) * kReadyStride * sizeof(int), (cudaStream_t)stream));
     cudaLaunchConfig_t cfg;

@@ -53,9 +53,9 @@ def test_exchange_through_global_memory_equals_distributed_shared_memory(n):
         assert torch.equal(x, y)
 
 
-@pytest.mark.parametrize("n,record", [(512, True), (640, False), (768, False), (896, True), (1024, False), (1152, True)])
+@pytest.mark.parametrize("n,record", [(128, False), (256, True), (384, True), (512, True), (640, False), (768, False), (896, True), (1024, False), (1152, True)])
 def test_sweep_equals_the_steps(monkeypatch, n, record):
-    """A segment's steps in one launch against one launch each, bit for bit: N with two K chunks a CTA, with a last
+    """A segment's steps in one launch against one or two launches each, bit for bit: N below eight K ranges, with two K chunks a CTA, with a last
     CTA of more chunks than pipeline stages (768 and 1152: six, 896: eight), the largest that 152 SMs hold; the whole run or segments of 20 of 47 steps."""
     from neuronbridge_gb300 import adjoint
     from neuronbridge_gb300.adjoint import RecurrentLIF, _bind, poisson_inputs
@@ -65,7 +65,7 @@ def test_sweep_equals_the_steps(monkeypatch, n, record):
                          record=record)
     x = poisson_inputs(torch.linspace(50.0, 400.0, 40), 47, 128, dt=1.0, seed=3)
     labels = torch.arange(128, device="cuda") % 5
-    assert _bind().nbg_lif_adjoint_sweep_work(128, n) > 0 and _bind().nbg_lif_adjoint_sweep_work(128, 384) == 0
+    assert _bind().nbg_lif_adjoint_sweep_work(128, n) > 0 and _bind().nbg_lif_adjoint_sweep_work(64, n) == 0
     out = []
     for sweep in (True, False):
         monkeypatch.setattr(adjoint, "SWEEP", sweep)
