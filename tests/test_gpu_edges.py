@@ -126,3 +126,23 @@ def test_a_reset_is_complete_when_the_next_call_starts():
         if first is None:
             first = t.copy(), i.copy()
         assert len(t) > 0 and np.array_equal(t, first[0]) and np.array_equal(i, first[1])
+
+
+def test_trials_after_a_reset_equal_the_oracle(oracle_lib):
+    """The same at the headline size against the oracle's raster, so that a loss that every trial has would show."""
+    import oracle
+    from neuronbridge_gb300 import workloads
+
+    net, cfg = workloads.izhikevich_stdp(n=100_000, in_degree=100, steps=500, seed=6)
+    ref = oracle.OracleNet(net.to_native().flat(cfg.timestep, seed=6)).set_threads(8)
+    ref.run(500)
+    ot, oi = ref.spikes()  # every layer of this network is an output layer
+    order = np.lexsort((oi, ot))
+    v, u = (ref.state(f).astype(np.float32) for f in (0, 1))
+    sim = nb.Simulation(net, cfg, seed=6)
+    for _ in range(3):
+        sim.reset()
+        sim.run(500)
+        t, i = sim.spike_raster()
+        assert len(t) > 0 and np.array_equal(t, ot[order]) and np.array_equal(i, oi[order])
+        assert np.array_equal(sim.state_field(0), v) and np.array_equal(sim.state_field(1), u)
