@@ -15,12 +15,16 @@
 // Record `fmt` as the calling thread's last error and return `code`.
 NBG_HIDDEN nbg_status nbg_fail(nbg_status code, const char *fmt, ...);
 
+// The error is reported once: the runtime's own last error, which the next
+// launch check would find again, is cleared.
 #define NBG_CUDA(call)                                                                                   \
     do {                                                                                                 \
         cudaError_t e_ = (call);                                                                         \
-        if (e_ != cudaSuccess)                                                                           \
+        if (e_ != cudaSuccess) {                                                                         \
+            (void)cudaGetLastError();                                                                    \
             return nbg_fail(e_ == cudaErrorMemoryAllocation ? NBG_ERR_OOM : NBG_ERR_CUDA,                \
                             "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+        }                                                                                                \
     } while (0)
 
 template <typename T>
@@ -36,11 +40,19 @@ struct DevBuf {
         p = nullptr;
         n = 0;
     }
+    // n is the size only once the memory is there: callers keep a buffer whose n
+    // is large enough, also after a failed call has been repeated
     cudaError_t alloc(size_t count) {
         release();
-        n = count;
         if (count == 0) return cudaSuccess;
-        return cudaMalloc(&p, count * sizeof(T));
+        const cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+        if (e == cudaSuccess) {
+            n = count;
+        } else {
+            p = nullptr;
+            (void)cudaGetLastError(); // returned here: not also by the next launch check
+        }
+        return e;
     }
     cudaError_t upload(const std::vector<T> &h) {
         cudaError_t e = alloc(h.size());

@@ -1846,6 +1846,7 @@ nbg_status dense_decay_table(nbg_engine *e) {
         }
     }
     if (len > ((int64_t)1 << 24)) return fail(NBG_ERR_UNSUPPORTED, "STDP decay table would exceed 2^24 entries");
+    e->dtab_len = 0; // until the new table is there
     NBG_CUDA(e->dtab.alloc((size_t)e->n_rules * len));
     NBG_CUDA(nbg_device_decay_table(reinterpret_cast<float *>(e->dtab.p), inv.data(), e->n_rules * 2, (int)len,
                                     e->dt));
@@ -1899,6 +1900,7 @@ nbg_status ensure_decay_table(nbg_engine *e, int64_t needed) {
         complete = complete && zp && zm;
     }
     if (!complete && needed > len) return fail(NBG_ERR_UNSUPPORTED, "STDP decay table would exceed 2^24 entries");
+    e->dtab_len = 0; // until the new table is there
     NBG_CUDA(e->dtab.upload(tab));
     e->dtab_len = (int)len;
     e->dtab_complete = complete;
@@ -2358,10 +2360,8 @@ nbg_status order_raster(nbg_engine *e, unsigned n, int t0, int count) {
         return fail(NBG_ERR_CUDA, "raster bitmap: %s (injected)", cudaGetErrorString(cudaErrorMemoryAllocation));
     if (e->rbm.n < (size_t)max_tiles * kRasterTileWords) NBG_CUDA(e->rbm.alloc((size_t)max_tiles * kRasterTileWords));
     if (e->rtile.n < max_tiles) NBG_CUDA(e->rtile.alloc(max_tiles));
-    if (e->ord_ids.n < n) {
-        NBG_CUDA(e->ord_ids.alloc(n));
-        NBG_CUDA(e->ord_t.alloc(n));
-    }
+    if (e->ord_ids.n < n) NBG_CUDA(e->ord_ids.alloc(n));
+    if (e->ord_t.n < n) NBG_CUDA(e->ord_t.alloc(n));
     unsigned int *const base = e->words.p + nbg_engine::kOrdered; // 0 since k_run_begin
     NBG_CUDA(cudaEventRecord(e->evr0, e->stream));
     const unsigned mark_grid =
@@ -3047,10 +3047,9 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
     int64_t cap = e->spike_capacity > 0 ? e->spike_capacity
                                         : std::min<int64_t>((int64_t)e->N * count, (int64_t)1 << 26);
     cap = std::min<int64_t>(std::max<int64_t>(cap, 1), 0x7FFFFFFF); // 32-bit device cursor
-    if ((int64_t)e->out_ids.n < cap) {
-        NBG_CUDA(e->out_ids.alloc((size_t)cap));
-        NBG_CUDA(e->out_t.alloc((size_t)cap));
-    }
+    // each by its own size: the second allocation of a call may have failed
+    if ((int64_t)e->out_ids.n < cap) NBG_CUDA(e->out_ids.alloc((size_t)cap));
+    if ((int64_t)e->out_t.n < cap) NBG_CUDA(e->out_t.alloc((size_t)cap));
     const int ntr = (int)e->trace_ids.size();
     if (ntr > 0 && (int64_t)e->trace.n < (int64_t)count * ntr) NBG_CUDA(e->trace.alloc((size_t)count * ntr));
     const int t0 = e->next_t;
