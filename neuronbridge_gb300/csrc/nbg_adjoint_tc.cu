@@ -550,7 +550,13 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
 // Order.  The product of step j overwrites the accumulators after `exchanged` of
 // step j - 1, which comes after their last read.  The receive buffers alternate,
 // since a CTA may be a step ahead of a peer that still reads; it cannot be two
-// ahead (`exchanged` between).  dI alternates likewise: a CTA writes step j's into
+// ahead (`exchanged` between).  `exchanged` alternates too: its arrivals are
+// counted, not named, and a CTA that has all of step j may arrive for step j + 1
+// at a peer that still lacks a third one's of step j (at once where it has no K
+// range to wait for), so with one barrier it could stand in for that one.  With
+// two, its next arrival at the same barrier is that of step j + 2, after the wait
+// for step j + 1, so after the peer's arrival for step j + 1, which the peer makes
+// when it has all of step j.  dI alternates likewise: a CTA writes step j's into
 // the buffer of step j - 2 after `exchanged` of step j, so after dI of step j - 1 of
 // every tile (a cluster's K ranges cover all of them), which their CTAs wrote after
 // their products had read it.
@@ -567,6 +573,7 @@ constexpr int kSweepTailWarps = 8, kSweepThreads = 32 * (kSweepTailWarps + 2);
 constexpr uint32_t kSweepIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kSweepN >> 3) << 17) |
                                  ((uint32_t)(kAdjM >> 4) << 24);
 constexpr int kReadyStride = 32; // a count has a line of its own
+constexpr int kExchangeBarriers = 2; // step j's: j % 2
 constexpr int kSweepRecv = kAdjCluster * 2 * kAdjM; // 16-byte pieces that a rank receives in a step
 constexpr int kSweepSmemBytes = kSweepStages * kSweepStageBytes + 2 * kSweepRecv * 16 + 1024 + 256;
 static_assert(kSweepSmemBytes <= 232448, "shared memory of a CTA");
@@ -628,7 +635,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
     uint64_t *full_d = full_w + kStages;
     uint64_t *empty = full_d + kStages;
     uint64_t *done = empty + kStages, *exchanged = done + 1;
-    uint32_t *tmem_slot = (uint32_t *)(exchanged + 1);
+    uint32_t *tmem_slot = (uint32_t *)(exchanged + kExchangeBarriers);
     volatile int *abort = (volatile int *)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -651,7 +658,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
             mbar_init(&empty[st], 1);
         }
         mbar_init(done, 1);
-        mbar_init(exchanged, kSweepCluster);
+        for (int k = 0; k < kExchangeBarriers; ++k) mbar_init(&exchanged[k], kSweepCluster);
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -673,6 +680,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
     const bool stay = iters <= kStages;
     auto stage = [&](int j, int c) { return stay ? c : (int)(((long long)j * iters + c) % kStages); };
     auto phase = [&](int j, int c) { return stay ? (uint32_t)j & 1u : (uint32_t)(((long long)j * iters + c) / kStages) & 1u; };
+    auto exchange_phase = [](int j) { return (uint32_t)(j / kExchangeBarriers) & 1u; };
     long long sent_w = 0, sent_d = 0; // producer: pieces requested
     auto send_w = [&](int j, int c) { // once the products on the stage's last piece are done
         const long long g = (long long)j * iters + c;
@@ -747,7 +755,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
             }
             __syncwarp();
         } else if (warp == kSweepTailWarps + 1) {
-            if (lane == 0 && j > 0 && mbar_wait_cluster(exchanged, (j - 1) & 1, abort)) // the accumulator has been read
+            if (lane == 0 && j > 0 && // the accumulator has been read
+                mbar_wait_cluster(&exchanged[(j - 1) % kExchangeBarriers], exchange_phase(j - 1), abort))
                 fence_after();
             if (lane == 0 && !*abort) { // MMA issuer
                 for (int c = 0; c < iters; ++c) {
@@ -814,11 +823,11 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
             asm volatile("bar.sync 1, %0;" ::"n"(32 * kSweepTailWarps) : "memory");
             if (threadIdx.x < kSweepCluster && !*abort) {
                 uint32_t ra;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_addr(exchanged)), "r"(threadIdx.x));
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(smem_addr(&exchanged[j % kExchangeBarriers])), "r"(threadIdx.x));
                 asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(ra) : "memory");
             }
             __syncwarp();
-            mbar_wait_cluster(exchanged, j & 1, abort);
+            mbar_wait_cluster(&exchanged[j % kExchangeBarriers], exchange_phase(j), abort);
             float x[kAdjCluster][kRows];
 #pragma unroll
             for (int r = 0; r < kAdjCluster; ++r)
