@@ -147,6 +147,18 @@ nbg_status nbg_lif_adjoint_step_parts(const void *w_hi, const void *w_lo, const 
                                       const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
                                       void *dT_lo, int64_t k_off, int64_t k_cols, float *parts, int *err, void *stream);
 
+/* nbg_lif_adjoint_step_parts for a step whose launch directly follows that of
+ * another step of the same sweep on the stream (by either call): it overlaps that
+ * step and reads W and its record before that one has ended, so nothing may be
+ * launched between the two.  The first step after W was prepared or a record
+ * written is nbg_lif_adjoint_step_parts. */
+nbg_status nbg_lif_adjoint_step_chained(const void *w_hi, const void *w_lo, const void *dI_hi_in, const void *dI_lo_in,
+                                        void *dI_hi_out, void *dI_lo_out, const float *g_read, float c_t,
+                                        const float *u, const float *s, const uint8_t *m, const float *vprev,
+                                        float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
+                                        const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
+                                        void *dT_lo, int64_t k_off, int64_t k_cols, float *parts, int *err, void *stream);
+
 /* The steps t0 + steps - 1 .. t0 in one launch, for every N that is a multiple of
  * 128, with the results of as many calls of nbg_lif_adjoint_step_parts (N < 512: of
  * nbg_lif_adjoint_step_split and nbg_adjoint_rec_grad): u, s, m and vprev are the record of step

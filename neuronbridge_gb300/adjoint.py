@@ -69,6 +69,9 @@ _SIG = {
     "nbg_lif_adjoint_step_parts": (ctypes.c_int, [_vp] * 7 + [ctypes.c_float] + [_vp] * 10 +
                                    [ctypes.POINTER(GradParams), ctypes.c_int, ctypes.c_int, _vp, _vp,
                                     ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp]),
+    "nbg_lif_adjoint_step_chained": (ctypes.c_int, [_vp] * 7 + [ctypes.c_float] + [_vp] * 10 +
+                                     [ctypes.POINTER(GradParams), ctypes.c_int, ctypes.c_int, _vp, _vp,
+                                      ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp]),
     "nbg_lif_adjoint_sweep_work": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int]),
     "nbg_lif_adjoint_sweep": (ctypes.c_int, [_vp] * 17 + [ctypes.POINTER(GradParams)] + [ctypes.c_int] * 4 + [_vp, _vp] +
                               [ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp]),
@@ -474,7 +477,10 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
             if fused:  # dI_{t+1} W_rec^T (zero at the run's last step) and step t, one launch
                 cur, nxt = t & 1, (t + 1) & 1
                 k_off, k_cols = (t * B, T * B) if whole else (k * B, L * B)
-                _lib.check(lib.nbg_lif_adjoint_step_parts(
+                # chained to the launch before it, where that is the step t + 1: not after W was prepared or a segment replayed
+                chained = t < T - 1 and (whole or k < L - 1)
+                step = lib.nbg_lif_adjoint_step_chained if chained else lib.nbg_lif_adjoint_step_parts
+                _lib.check(step(
                     _ptr(w_hi), _ptr(w_lo), _ptr(d_hi[nxt]), _ptr(d_lo[nxt]), _ptr(d_hi[cur]), _ptr(d_lo[cur]),
                     _ptr(g_read), float(coef[t]), _ptr(U[k]), _ptr(S[k + 1]), _ptr(M[k]), _ptr(VP[k]),
                     _ptr(lam_v), None, _ptr(g_theta), _ptr(g_alpha), _ptr(alpha), _ptr(theta), ctypes.byref(p), B,

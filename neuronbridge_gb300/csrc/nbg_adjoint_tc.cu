@@ -154,30 +154,15 @@ __global__ void __launch_bounds__(kThreads, 1)
     fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // Programmatic dependent launch: W does not change during the backward,
-    // so the first stages' W tiles are requested before the wait for the
-    // adjoint step that writes dI (a no-op without a programmatic launch).
+    // Programmatic dependent launch: the set-up above overlaps the launch
+    // before, whatever that is (the adjoint step that writes dI, or the kernel
+    // that writes W); only the wait makes what it wrote visible.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp == 0 && lane == 0) { // producer
-        const int pre = iters < kAdjStages ? iters : kAdjStages;
-        for (int it = 0; it < pre; ++it) {
-            uint8_t *st = stages + it * kAdjStageBytes;
-            const size_t a_blk = (size_t)mt * kchunks + kc0 + it;
-            mbar_expect_tx(&full[it], kAdjStageBytes);
-            bulk_copy(st, (const uint8_t *)w_hi + a_blk * kAdjBlockA, kAdjBlockA, &full[it]);
-            bulk_copy(st + kAdjBlockA, (const uint8_t *)w_lo + a_blk * kAdjBlockA, kAdjBlockA, &full[it]);
-        }
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        for (int it = 0; it < pre; ++it) {
-            uint8_t *st = stages + it * kAdjStageBytes;
-            const int kc = kc0 + it;
-            bulk_copy(st + 2 * kAdjBlockA, (const uint8_t *)d_hi + (size_t)kc * kAdjBlockB, kAdjBlockB, &full[it]);
-            bulk_copy(st + 2 * kAdjBlockA + kAdjBlockB, (const uint8_t *)d_lo + (size_t)kc * kAdjBlockB, kAdjBlockB,
-                      &full[it]);
-        }
-        for (int it = pre; it < iters; ++it) {
+        for (int it = 0; it < iters; ++it) {
             const int s = it % kAdjStages;
-            if (!mbar_wait(&empty[s], ((it / kAdjStages) & 1) ^ 1, abort)) break;
+            if (it >= kAdjStages && !mbar_wait(&empty[s], ((it / kAdjStages) & 1) ^ 1, abort)) break;
             uint8_t *st = stages + s * kAdjStageBytes;
             const int kc = kc0 + it;
             const size_t a_blk = (size_t)mt * kchunks + kc;
@@ -208,7 +193,6 @@ __global__ void __launch_bounds__(kThreads, 1)
         commit(done);
     }
     __syncwarp();
-    asm volatile("griddepcontrol.wait;" ::: "memory"); // the previous adjoint step has read g_parts
     // epilogue: warp w reads TMEM lanes 32*(w%4).. (rows i) and columns
     // 64*(w/4).. (batch rows b)
     mbar_wait(done, 0, abort);
@@ -332,9 +316,12 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // Programmatic dependent launch: W is constant during the backward, so
-    // the first stages' W tiles are requested before the wait for the
-    // previous step (which writes dI_{t+1}, lam_v and the gradients).
+    // Programmatic dependent launch of a step that follows another of its sweep
+    // (`chained` on the host): W is constant during the sweep, so the first
+    // stages' W tiles are requested before the wait for the previous step (which
+    // writes dI_{t+1}, lam_v and the gradients).  The kernels that write W and
+    // the record have ended before a sweep's or a replayed segment's first step
+    // starts, since that one is launched without the attribute.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == kAdjTailWarps && lane == 0) { // producer
         const int pre = iters < kStages ? iters : kStages;
@@ -1077,7 +1064,7 @@ bool adj_shape_ok(int B, int N) { return B == kAdjN && N > 0 && N % kAdjM == 0; 
 } // namespace
 
 template <bool kParts>
-static nbg_status adj_step(const char *name, float *parts, const void *w_hi, const void *w_lo, const void *dI_hi_in, const void *dI_lo_in,
+static nbg_status adj_step(const char *name, bool chained, float *parts, const void *w_hi, const void *w_lo, const void *dI_hi_in, const void *dI_lo_in,
                                       void *dI_hi_out, void *dI_lo_out, const float *g_read, float c_t,
                                       const float *u, const float *s, const uint8_t *m, const float *vprev,
                                       float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
@@ -1108,7 +1095,7 @@ static nbg_status adj_step(const char *name, float *parts, const void *w_hi, con
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chained ? 1 : 0;
     NBG_CUDA(cudaLaunchKernelEx(&cfg, k_adj_step_umma<kParts>, (const __nv_bfloat16 *)w_hi, (const __nv_bfloat16 *)w_lo,
                                 (const __nv_bfloat16 *)dI_hi_in, (const __nv_bfloat16 *)dI_lo_in,
                                 (__nv_bfloat16 *)dI_hi_out, (__nv_bfloat16 *)dI_lo_out, g_read, c_t, u, s, m, vprev,
@@ -1205,7 +1192,7 @@ nbg_status nbg_lif_adjoint_step_fused(const void *w_hi, const void *w_lo, const 
                                       float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
                                       const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
                                       void *dT_lo, int64_t k_off, int64_t k_cols, int *err, void *stream) {
-    return adj_step<false>("nbg_lif_adjoint_step_fused", nullptr, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
+    return adj_step<false>("nbg_lif_adjoint_step_fused", false, nullptr, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
                            dI, g_theta, g_alpha, alpha, theta, p, B, N, dT_hi, dT_lo, k_off, k_cols, err, stream);
 }
 
@@ -1216,7 +1203,18 @@ nbg_status nbg_lif_adjoint_step_parts(const void *w_hi, const void *w_lo, const 
                                       const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
                                       void *dT_lo, int64_t k_off, int64_t k_cols, float *parts, int *err, void *stream) {
     if (!parts) return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_step_parts: parts is NULL");
-    return adj_step<true>("nbg_lif_adjoint_step_parts", parts, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
+    return adj_step<true>("nbg_lif_adjoint_step_parts", false, parts, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
+                           dI, g_theta, g_alpha, alpha, theta, p, B, N, dT_hi, dT_lo, k_off, k_cols, err, stream);
+}
+
+nbg_status nbg_lif_adjoint_step_chained(const void *w_hi, const void *w_lo, const void *dI_hi_in, const void *dI_lo_in,
+                                        void *dI_hi_out, void *dI_lo_out, const float *g_read, float c_t,
+                                        const float *u, const float *s, const uint8_t *m, const float *vprev,
+                                        float *lam_v, float *dI, float *g_theta, float *g_alpha, const float *alpha,
+                                        const float *theta, const nbg_lif_grad_params *p, int B, int N, void *dT_hi,
+                                        void *dT_lo, int64_t k_off, int64_t k_cols, float *parts, int *err, void *stream) {
+    if (!parts) return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_step_chained: parts is NULL");
+    return adj_step<true>("nbg_lif_adjoint_step_chained", true, parts, w_hi, w_lo, dI_hi_in, dI_lo_in, dI_hi_out, dI_lo_out, g_read, c_t, u, s, m, vprev, lam_v,
                            dI, g_theta, g_alpha, alpha, theta, p, B, N, dT_hi, dT_lo, k_off, k_cols, err, stream);
 }
 
