@@ -323,6 +323,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     // the record have ended before a sweep's or a replayed segment's first step
     // starts, since that one is launched without the attribute.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (!kParts) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     if (warp == kAdjTailWarps && lane == 0) { // producer
         const int pre = iters < kStages ? iters : kStages;
         for (int it = 0; it < pre; ++it) {
@@ -426,6 +427,7 @@ __global__ void __cluster_dims__(1, kAdjCluster, 1) __launch_bounds__(kAdjStepTh
     mbar_wait(done, 0, abort);
     __syncthreads();
     fence_after();
+    if constexpr (!kParts) asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); // the receiving CTAs have started
     // the partial accumulator to the rows' owners: warp w holds rows
     // i = 32 (w % 4) + lane and batch columns b = 32 (w / 4) + 16 c16 + c,
     // which rank 2 (w / 4) + c16 owns; they land in its receive buffer at
