@@ -515,16 +515,25 @@ struct nbg_dense {
 
 namespace {
 
+__global__ void k_dense_reset(float *__restrict__ v, int *__restrict__ last, float v0, int total) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= total) return;
+    v[idx] = v0;
+    last[idx] = 10000;
+}
+
+// On the engine's stream, which nothing on the default stream is ordered with,
+// and done on return.
 nbg_status dense_reset(nbg_dense *d) {
-    const size_t tot = (size_t)d->B * d->N;
-    std::vector<float> v0(tot, d->P.v_reset); // V_reset + random_mu (legacy init)
-    NBG_CUDA(cudaMemcpy(d->v.p, v0.data(), tot * sizeof(float), cudaMemcpyHostToDevice));
-    std::vector<int> l0(tot, 10000);
-    NBG_CUDA(cudaMemcpy(d->last.p, l0.data(), tot * sizeof(int), cudaMemcpyHostToDevice));
+    const int total = d->B * d->N;
+    cudaStream_t st = d->stream;
+    k_dense_reset<<<(total + 255) / 256, 256, 0, st>>>(d->v.p, d->last.p, d->P.v_reset, total); // V_reset + random_mu (legacy init)
+    NBG_CUDA(cudaGetLastError());
     for (int k = 0; k < 2; ++k) {
-        NBG_CUDA(d->s[k].zero());
-        NBG_CUDA(d->bits[k].zero());
+        NBG_CUDA(cudaMemsetAsync(d->s[k].p, 0, d->s[k].n * sizeof(__nv_bfloat16), st));
+        NBG_CUDA(cudaMemsetAsync(d->bits[k].p, 0, d->bits[k].n * sizeof(unsigned), st));
     }
+    NBG_CUDA(cudaStreamSynchronize(st));
     d->next_t = 0;
     d->ran = false;
     d->counts_host.clear();
@@ -616,7 +625,7 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
     chk(d->v.alloc(tot));
     chk(d->last.alloc(tot));
     chk(d->err.alloc(1));
-    chk(d->err.zero());
+    if (ce == cudaSuccess) chk(cudaMemsetAsync(d->err.p, 0, sizeof(int), d->stream));
     if (precision == NBG_DENSE_SPLIT_BF16_SYNC) chk(d->partial.alloc((size_t)kSplitK * tot));
     for (int k = 0; k < 2; ++k) {
         chk(d->s[k].alloc(tot));
@@ -624,7 +633,7 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
     }
     if (precision == NBG_DENSE_FP32) {
         chk(d->w.alloc(nn));
-        if (ce == cudaSuccess) chk(cudaMemcpy(d->w.p, w, nn * sizeof(float), cudaMemcpyHostToDevice));
+        if (ce == cudaSuccess) chk(cudaMemcpyAsync(d->w.p, w, nn * sizeof(float), cudaMemcpyHostToDevice, d->stream));
     } else {
         DevBuf<float> tmp;
         chk(tmp.alloc(nn));

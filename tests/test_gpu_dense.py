@@ -96,3 +96,19 @@ def test_split_bf16_simulation_tracks_fp32(precision):
     # identical before any threshold decision flips, close in aggregate after
     assert np.array_equal(ca[:20], cb[:20])
     assert abs(int(ca.sum()) - int(cb.sum())) <= 0.05 * cb.sum()
+
+
+@pytest.mark.parametrize("n,precision", [(8192, "split_bf16"), (8192, "fp32"), (1024, "split_bf16_sync")])
+def test_a_reset_is_complete_when_the_next_run_starts(n, precision):
+    """A run after a reset gives what a new engine gives: nothing of the reset is still under way when its first step starts."""
+    w = dense_weights(n, seed=4)
+    eng = DensePopulations(w, _layer(), precision=precision)
+    eng.run(20)
+    want = (eng.spike_counts(), *eng.state(), eng.spikes())
+    for _ in range(6):
+        eng.run(100)
+        assert eng.spikes().any()  # left behind if the reset is not complete
+        eng.reset()
+        eng.run(20)
+        for a, b in zip(want, (eng.spike_counts(), *eng.state(), eng.spikes())):
+            assert np.array_equal(a, b)
