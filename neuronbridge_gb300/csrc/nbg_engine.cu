@@ -2060,6 +2060,12 @@ __global__ void k_palette_patch(uint2 *code, unsigned int word, unsigned int bit
     code[word] = q;
 }
 
+// Host data to the device in the order of the engine's stream, which the
+// default stream is not ordered with; src may go when the stream has been waited for.
+cudaError_t write_device(nbg_engine *e, void *dst, const void *src, size_t bytes) {
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->stream);
+}
+
 // One weight was set (CSC position p): its code follows, in a free entry if
 // the weight is new; a weight that the full palette does not hold ends its use
 // until all weights are set again.
@@ -2073,7 +2079,7 @@ nbg_status patch_palette(nbg_engine *e, int64_t p, float w) {
     if (c == e->palette_n) {
         pal.w[c] = w;
         pal.types = (pal.types & ~(1u << c)) | type << c;
-        NBG_CUDA(cudaMemcpy(e->palette.p, &pal, sizeof(pal), cudaMemcpyHostToDevice));
+        NBG_CUDA(write_device(e, e->palette.p, &pal, sizeof(pal)));
         e->palette_n = c + 1;
     }
     const int j = (int)(std::upper_bound(e->csc_ptr.begin(), e->csc_ptr.end(), (int)p) - e->csc_ptr.begin()) - 1;
@@ -2086,8 +2092,8 @@ nbg_status patch_palette(nbg_engine *e, int64_t p, float w) {
 
 nbg_status upload_layers(nbg_engine *e) {
     NBG_CUDA(e->d_layers.alloc(e->layers.size()));
-    NBG_CUDA(cudaMemcpy(e->d_layers.p, e->layers.data(), e->layers.size() * sizeof(LayerDev),
-                        cudaMemcpyHostToDevice));
+    NBG_CUDA(write_device(e, e->d_layers.p, e->layers.data(), e->layers.size() * sizeof(LayerDev)));
+    NBG_CUDA(cudaStreamSynchronize(e->stream));
     return NBG_OK;
 }
 
@@ -3361,11 +3367,12 @@ nbg_status nbg_set_state(nbg_engine *e, int field, const float *in) {
     NBG_CUDA(cudaStreamSynchronize(e->stream));
     const size_t bytes = (size_t)e->N * sizeof(float);
     switch (field) {
-    case NBG_FIELD_V: NBG_CUDA(cudaMemcpy(e->v.p, in, bytes, cudaMemcpyHostToDevice)); break;
-    case NBG_FIELD_U: NBG_CUDA(cudaMemcpy(e->u.p, in, bytes, cudaMemcpyHostToDevice)); break;
-    case NBG_FIELD_I_EXT: NBG_CUDA(cudaMemcpy(e->iext.p, in, bytes, cudaMemcpyHostToDevice)); break;
+    case NBG_FIELD_V: NBG_CUDA(write_device(e, e->v.p, in, bytes)); break;
+    case NBG_FIELD_U: NBG_CUDA(write_device(e, e->u.p, in, bytes)); break;
+    case NBG_FIELD_I_EXT: NBG_CUDA(write_device(e, e->iext.p, in, bytes)); break;
     default: return fail(NBG_ERR_INVALID, "state field %d is not writable", field);
     }
+    NBG_CUDA(cudaStreamSynchronize(e->stream));
     return NBG_OK;
 }
 
@@ -3402,7 +3409,8 @@ nbg_status nbg_set_layer_record(nbg_engine *e, int layer, int record) {
     NBG_CUDA(cudaSetDevice(e->device));
     NBG_CUDA(cudaStreamSynchronize(e->stream));
     e->layers[layer].record = record != 0 ? 1 : 0;
-    NBG_CUDA(cudaMemcpy(e->d_layers.p + layer, &e->layers[layer], sizeof(LayerDev), cudaMemcpyHostToDevice));
+    NBG_CUDA(write_device(e, e->d_layers.p + layer, &e->layers[layer], sizeof(LayerDev)));
+    NBG_CUDA(cudaStreamSynchronize(e->stream));
     return NBG_OK;
 }
 
@@ -3484,10 +3492,12 @@ nbg_status nbg_set_weight(nbg_engine *e, int64_t conn, float w) {
     NBG_CUDA(cudaStreamSynchronize(e->stream));
     const int64_t p = e->orig_pos[conn];
     float *dst = e->plastic ? &e->rec.p[p].w : &e->wst.p[p].w;
-    NBG_CUDA(cudaMemcpy(dst, &w, sizeof(float), cudaMemcpyHostToDevice));
-    NBG_CUDA(cudaMemcpy(e->init_w_d.p + p, &w, sizeof(float), cudaMemcpyHostToDevice));
     e->init_w[p] = w;
-    return patch_palette(e, p, w);
+    NBG_CUDA(write_device(e, dst, &e->init_w[p], sizeof(float)));
+    NBG_CUDA(write_device(e, e->init_w_d.p + p, &e->init_w[p], sizeof(float)));
+    const nbg_status st = patch_palette(e, p, w);
+    NBG_CUDA(cudaStreamSynchronize(e->stream));
+    return st;
 }
 
 nbg_status nbg_set_weights(nbg_engine *e, const float *w) {
@@ -3498,7 +3508,7 @@ nbg_status nbg_set_weights(nbg_engine *e, const float *w) {
     NBG_CUDA(cudaStreamSynchronize(e->stream));
     for (int64_t s = 0; s < e->S; ++s) e->init_w[e->orig_pos[s]] = w[s];
     if (e->S > 0) {
-        NBG_CUDA(cudaMemcpy(e->init_w_d.p, e->init_w.data(), e->S * sizeof(float), cudaMemcpyHostToDevice));
+        NBG_CUDA(write_device(e, e->init_w_d.p, e->init_w.data(), e->S * sizeof(float)));
         NBG_CUDA(reset_synapses(e, false)); // weights only: the STDP traces stay
     }
     if (e->palette_kernel) {

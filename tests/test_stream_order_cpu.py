@@ -1,0 +1,19 @@
+"""The engines run on non-blocking streams, with which nothing on the default stream is ordered: what the host writes to the
+device goes through the engine's stream (a pageable copy may return before its data is there, a memset is asynchronous)."""
+import os
+import re
+
+import pytest
+
+from neuronbridge_gb300 import build
+
+
+@pytest.mark.parametrize("name", ["nbg_engine.cu", "nbg_dense.cu"])
+def test_no_copy_to_the_device_on_the_default_stream(name):
+    src = open(os.path.join(build.CSRC, name)).read()
+    copies = re.findall(r"cudaMemcpy\(.*?\);", src, re.S)
+    assert copies
+    # the dense engine waits for the device after its weights, which it converts on the default stream
+    made = "cudaMemcpy(tmp.p, w, nn * sizeof(float), cudaMemcpyHostToDevice));"
+    for c in copies:
+        assert "cudaMemcpyDeviceToHost" in c or c == made, c
