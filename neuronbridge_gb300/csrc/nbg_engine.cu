@@ -3288,7 +3288,8 @@ nbg_status nbg_run(nbg_engine *e, int steps) {
             e->log_conn.push_back(e->csc_orig[ep[k]]);
             e->log_w.push_back(ew[k]);
         }
-        NBG_CUDA(cudaMemset(e->ev_cursor.p, 0, sizeof(unsigned long long)));
+        // ordered ahead of the next call's first entry
+        NBG_CUDA(cudaMemsetAsync(e->ev_cursor.p, 0, sizeof(unsigned long long), e->stream));
     }
     return NBG_OK;
 }

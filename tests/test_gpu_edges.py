@@ -146,3 +146,22 @@ def test_trials_after_a_reset_equal_the_oracle(oracle_lib):
         t, i = sim.spike_raster()
         assert len(t) > 0 and np.array_equal(t, ot[order]) and np.array_equal(i, oi[order])
         assert np.array_equal(sim.state_field(0), v) and np.array_equal(sim.state_field(1), u)
+
+
+def test_event_log_of_many_short_calls(oracle_lib):
+    """Each call's log is emptied before the next call writes its first entry: every delivered event is in it once."""
+    import oracle
+    from neuronbridge_gb300 import workloads
+
+    net, cfg = workloads.plain_lif(steps=400)
+    sim = nb.Simulation(net, cfg, event_log_capacity=2_000_000)
+    for _ in range(100):
+        sim.run(4)
+    o = oracle.OracleNet(net.to_native().flat(cfg.timestep))
+    o.set_event_log(True)
+    o.run(400)
+    gt, gc, gw = sim.logged_events()
+    ot, oc, ow = o.events()
+    g, k = np.lexsort((gc, gt)), np.lexsort((oc, ot))
+    assert len(ot) > 0 and np.array_equal(gt[g], ot[k]) and np.array_equal(gc[g], oc[k])
+    assert np.array_equal(gw[g], ow[k].astype(np.float32))

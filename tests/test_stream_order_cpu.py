@@ -17,3 +17,9 @@ def test_no_copy_to_the_device_on_the_default_stream(name):
     made = "cudaMemcpy(tmp.p, w, nn * sizeof(float), cudaMemcpyHostToDevice));"
     for c in copies:
         assert "cudaMemcpyDeviceToHost" in c or c == made, c
+
+
+@pytest.mark.parametrize("name", ["nbg_engine.cu", "nbg_dense.cu"])
+def test_no_memset_on_the_default_stream(name):
+    src = open(os.path.join(build.CSRC, name)).read()
+    assert "cudaMemsetAsync(" in src and not re.findall(r"cudaMemset(?:2D)?\(|\.zero\(\)", src)
