@@ -54,12 +54,14 @@ struct DevBuf {
         }
         return e;
     }
+    // On the device when it returns, for streams that the default one is not
+    // ordered with (the copy alone may return with its last part staged).
     cudaError_t upload(const std::vector<T> &h) {
         cudaError_t e = alloc(h.size());
         if (e != cudaSuccess || h.empty()) return e;
-        return cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+        e = cudaMemcpy(p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+        return e == cudaSuccess ? cudaStreamSynchronize(nullptr) : e;
     }
-    cudaError_t zero() { return n ? cudaMemset(p, 0, n * sizeof(T)) : cudaSuccess; }
 };
 
 // PoissonRate hash (reference PoissonRate.cpp:12-22)

@@ -23,3 +23,9 @@ def test_no_copy_to_the_device_on_the_default_stream(name):
 def test_no_memset_on_the_default_stream(name):
     src = open(os.path.join(build.CSRC, name)).read()
     assert "cudaMemsetAsync(" in src and not re.findall(r"cudaMemset(?:2D)?\(|\.zero\(\)", src)
+
+
+def test_an_upload_waits_for_its_copy():
+    src = open(os.path.join(build.CSRC, "nbg_common.cuh")).read()
+    body = re.search(r"cudaError_t upload\(.*?\n    }\n", src, re.S).group(0)
+    assert body.index("cudaMemcpy(") < body.index("cudaStreamSynchronize(")
