@@ -351,6 +351,10 @@ __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_segment(
 constexpr int kRing = 8, kHalfRing = kRing / 2;
 constexpr int kRowsMaxInputs = 4096;
 constexpr int kRowsMaxNeurons = 2048;
+// the lists of two steps' nonzero inputs and the ring of C channels
+constexpr size_t rows_smem_bytes(int C) {
+    return 2 * ((size_t)(C + 5) & ~(size_t)1) * sizeof(uint2) + (size_t)kRing * C * sizeof(float);
+}
 
 __device__ __forceinline__ void ring_copy(float *dst, const float *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
@@ -730,9 +734,10 @@ nbg_status launch_rows(const float *xi, const float *x, const float *w_in, int C
             : nc == 2 ? k_lif_fwd_rows<kGather, 1, 2, 512>
                       : k_lif_fwd_rows<kGather, 1, 4, 512>;
     }
-    const size_t smem = kGather ? 2 * ((size_t)(C + 5) & ~(size_t)1) * sizeof(uint2) + (size_t)kRing * C * sizeof(float) : 0;
+    const size_t smem = kGather ? rows_smem_bytes(C) : 0;
+    // the limit is the kernel's, for every thread: always what its largest shape needs, never lowered to this one's
     if (smem > 32 * 1024)
-        NBG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NBG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem_bytes(kRowsMaxInputs)));
     k<<<B, threads, smem, stream>>>(xi, x, w_in, C, w, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec, z, c,
                                     alpha, theta, p, L, B, N);
     NBG_CUDA(cudaGetLastError());
@@ -927,9 +932,10 @@ nbg_status nbg_lif_forward_segment_gather(const float *x, const float *w_in, int
         return launch_rows<true>(nullptr, x, w_in, C, w_rec, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec,
                                  z, c, alpha, theta, *p, L, B, N, (cudaStream_t)stream);
     const size_t smem = (2 * (size_t)N + 2 * (size_t)C) * sizeof(int);
-    if (smem > 200 * 1024) return nbg_fail(NBG_ERR_UNSUPPORTED, "too many inputs for the gather form (C = %d)", C);
-    if (smem > 48 * 1024)
-        NBG_CUDA(cudaFuncSetAttribute(k_lif_fwd_segment, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t most = 200 * 1024;
+    if (smem > most) return nbg_fail(NBG_ERR_UNSUPPORTED, "too many inputs for the gather form (C = %d)", C);
+    if (smem > 32 * 1024) // as in launch_rows
+        NBG_CUDA(cudaFuncSetAttribute(k_lif_fwd_segment, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     k_lif_fwd_segment<<<B, kSparseThreads, smem, (cudaStream_t)stream>>>(
         x, w_in, C, w_rec, spk, cnt, v, ref, s_out, s_last, u_rec, m_rec, vprev_rec, z, c, alpha, theta,
         *p, L, B, N);

@@ -86,6 +86,10 @@ constexpr int kRedLd = 36;                 // partial tiles: 32 lanes of a store
 constexpr int kRecvFloats = kTile * kTile; // partials of this rank's rows from every rank
 
 __host__ __device__ constexpr int nt_ld(int kc) { return kc + 4; } // kc a multiple of 8: rows 16 bytes apart mod 128
+constexpr size_t nt_smem_bytes(int stages, int kc) {
+    const int ops = stages * 2 * kTile * nt_ld(kc), red = kNtWarps * kTile * kRedLd;
+    return (size_t)(kRecvFloats + (ops > red ? ops : red)) * sizeof(float);
+}
 
 struct NtShape {
     int M, N, K;
@@ -366,11 +370,10 @@ template <class Epi>
 nbg_status launch_nt(const float *A, const float *W, NtShape sh, const Epi &epi, bool chained, cudaStream_t stream) {
     void (*const kernel)(const float *, const float *, NtShape, Epi) =
         sh.ranks >= 4 ? k_product_nt<Epi, 1> : sh.ranks == 2 ? k_product_nt<Epi, 2> : k_product_nt<Epi, 4>;
-    const int red = kNtWarps * kTile * kRedLd;
-    const size_t smem =
-        (size_t)(kRecvFloats + std::max(sh.stages * 2 * kTile * nt_ld(sh.kc), red)) * sizeof(float);
+    const size_t smem = nt_smem_bytes(sh.stages, sh.kc);
+    // the limit is the kernel's, for every thread: always what its largest shape needs, never lowered to this one's
     if (smem > 48 * 1024)
-        NBG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NBG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nt_smem_bytes(2, kNtChunk)));
     const long long rows = (sh.M + kTile - 1) / kTile;
     if (rows > 65535) return nbg_fail(NBG_ERR_UNSUPPORTED, "product of %d rows", sh.M);
     cudaLaunchConfig_t cfg = {};
