@@ -124,7 +124,10 @@ __global__ void __launch_bounds__(kNtThreads, 2) k_product_nt(const float *__res
     float *const ops = nt_smem + kRecvFloats; // [stage][A tile, W tile], then the partial tiles
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rank = sh.ranks > 1 ? (int)(blockIdx.x % (unsigned)sh.ranks) : 0; // = %cluster_ctarank
-    const int j0 = (int)(blockIdx.x / (unsigned)sh.ranks) * kTile, r0 = (int)blockIdx.y * kTile;
+    const int j0 = (int)(blockIdx.x / (unsigned)sh.ranks) * kTile;
+    const long long row_tile = (long long)blockIdx.z * gridDim.y + blockIdx.y; // of a cluster's CTAs the same
+    if (row_tile * kTile >= sh.M) return;
+    const int r0 = (int)row_tile * kTile;
     const int k_beg = min(rank * sh.per, sh.K), k_end = min(k_beg + sh.per, sh.K);
     const int chunks = A ? (k_end - k_beg + kc - 1) / kc : 0;
     const int stage_floats = 2 * kTile * ld;
@@ -374,10 +377,9 @@ nbg_status launch_nt(const float *A, const float *W, NtShape sh, const Epi &epi,
     // the limit is the kernel's, for every thread: always what its largest shape needs, never lowered to this one's
     if (smem > 48 * 1024)
         NBG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)nt_smem_bytes(2, kNtChunk)));
-    const long long rows = (sh.M + kTile - 1) / kTile;
-    if (rows > 65535) return nbg_fail(NBG_ERR_UNSUPPORTED, "product of %d rows", sh.M);
+    const long long rows = ((long long)sh.M + kTile - 1) / kTile, y = std::min<long long>(rows, 65535);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((sh.N + kTile - 1) / kTile * sh.ranks), (unsigned)rows);
+    cfg.gridDim = dim3((unsigned)((sh.N + kTile - 1) / kTile * sh.ranks), (unsigned)y, (unsigned)((rows + y - 1) / y));
     cfg.blockDim = dim3(kNtThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -405,14 +407,17 @@ nbg_status launch_nt(const float *A, const float *W, NtShape sh, const Epi &epi,
 __global__ void __launch_bounds__(256) k_transpose(const float *__restrict__ in, float *__restrict__ out, int R,
                                                    int C) {
     __shared__ float tile[32][33];
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int c0 = blockIdx.x * 32, x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    for (long long r0 = (long long)blockIdx.y * 32; r0 < R; r0 += (long long)gridDim.y * 32) {
 #pragma unroll
-    for (int k = 0; k < 32; k += 8)
-        if (r0 + y + k < R && c0 + x < C) tile[y + k][x] = in[(size_t)(r0 + y + k) * C + c0 + x];
-    __syncthreads();
+        for (int k = 0; k < 32; k += 8)
+            if (r0 + y + k < R && c0 + x < C) tile[y + k][x] = in[(size_t)(r0 + y + k) * C + c0 + x];
+        __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 32; k += 8)
-        if (c0 + y + k < C && r0 + x < R) out[(size_t)(c0 + y + k) * R + r0 + x] = tile[x][y + k];
+        for (int k = 0; k < 32; k += 8)
+            if (c0 + y + k < C && r0 + x < R) out[(size_t)(c0 + y + k) * R + r0 + x] = tile[x][y + k];
+        __syncthreads();
+    }
 }
 
 // -------------------------------------------------------------- A^T times B
@@ -443,8 +448,9 @@ __global__ void __launch_bounds__(kTnThreads) k_product_tn(const float *__restri
                                                            float *__restrict__ part, int M, int N, int K, int per,
                                                            int vec_a, int vec_b) {
     __shared__ __align__(16) float st[kTnStages][2][kTnK * kTnTile];
-    const int n0 = blockIdx.x * kTnTile, m0 = blockIdx.y * kTnTile;
-    const int k_beg = min((int)blockIdx.z * per, K), k_end = min(k_beg + per, K);
+    const unsigned n_tiles = (unsigned)((N + kTnTile - 1) / kTnTile); // tiles of n first, then of m
+    const int n0 = (int)(blockIdx.x % n_tiles) * kTnTile, m0 = (int)(blockIdx.x / n_tiles) * kTnTile;
+    const int k_beg = (int)min((long long)blockIdx.z * per, (long long)K), k_end = k_beg + min(per, K - k_beg);
     const int chunks = (k_end - k_beg + kTnK - 1) / kTnK;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ml = (warp >> 1) * 32 + (lane >> 3) * 8, nl = (warp & 1) * 32 + (lane & 7) * 4;
@@ -518,25 +524,15 @@ extern "C" {
 
 nbg_status nbg_transpose(const float *in, float *out, int rows, int cols, void *stream) {
     if (!in || !out || in == out || rows <= 0 || cols <= 0) return nbg_fail(NBG_ERR_INVALID, "nbg_transpose: bad arguments");
-    if ((rows + 31) / 32 > 65535) return nbg_fail(NBG_ERR_UNSUPPORTED, "nbg_transpose: %d rows", rows);
-    k_transpose<<<dim3((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32)), 256, 0, (cudaStream_t)stream>>>(
-        in, out, rows, cols);
+    const unsigned y = (unsigned)std::min(((long long)rows + 31) / 32, 65535LL);
+    k_transpose<<<dim3((unsigned)(((long long)cols + 31) / 32), y), 256, 0, (cudaStream_t)stream>>>(in, out, rows, cols);
     NBG_CUDA(cudaGetLastError());
     return NBG_OK;
 }
 
 nbg_status nbg_product_nt(const float *A, const float *W, float *C, int M, int N, int K, void *stream) {
     if (!A || !W || !C || M <= 0 || N <= 0 || K <= 0) return nbg_fail(NBG_ERR_INVALID, "nbg_product_nt: bad arguments");
-    // row tiles beyond a grid's y extent go in further launches
-    const int most = 65535 * kTile;
-    for (long long r = 0; r < M; r += most) {
-        const float *a = A + (size_t)r * K;
-        const int m = (int)std::min<long long>(most, M - r);
-        const StoreEpi epi{C + (size_t)r * N, N};
-        const nbg_status st = launch_nt(a, W, nt_shape(a, W, m, N, K), epi, false, (cudaStream_t)stream);
-        if (st != NBG_OK) return st;
-    }
-    return NBG_OK;
+    return launch_nt(A, W, nt_shape(A, W, M, N, K), StoreEpi{C, N}, false, (cudaStream_t)stream);
 }
 
 nbg_status nbg_lif_forward_step_smooth(const float *s_prev, const float *w_rec_t, const float *xi, float *v,
@@ -576,9 +572,10 @@ nbg_status nbg_product_tn(const float *A, const float *B, float *part, int split
                           void *stream) {
     if (!A || !B || !part || split <= 0 || split > 65535 || M <= 0 || N <= 0 || K <= 0)
         return nbg_fail(NBG_ERR_INVALID, "nbg_product_tn: bad arguments");
-    if ((M + kTnTile - 1) / kTnTile > 65535) return nbg_fail(NBG_ERR_UNSUPPORTED, "nbg_product_tn: %d rows", M);
-    const int per = ((K + split - 1) / split + kTnK - 1) / kTnK * kTnK;
-    const dim3 grid((unsigned)((N + kTnTile - 1) / kTnTile), (unsigned)((M + kTnTile - 1) / kTnTile), (unsigned)split);
+    const long long tiles = (((long long)M + kTnTile - 1) / kTnTile) * (((long long)N + kTnTile - 1) / kTnTile);
+    if (tiles > 0x7fffffff) return nbg_fail(NBG_ERR_UNSUPPORTED, "nbg_product_tn: %d x %d outputs", M, N);
+    const int per = (int)std::min<long long>((((long long)K + split - 1) / split + kTnK - 1) / kTnK * kTnK, 0x7fffffe0);
+    const dim3 grid((unsigned)tiles, 1, (unsigned)split);
     const int vec_a = M % 4 == 0 && ((uintptr_t)A & 15u) == 0, vec_b = N % 4 == 0 && ((uintptr_t)B & 15u) == 0;
     k_product_tn<<<grid, kTnThreads, 0, (cudaStream_t)stream>>>(A, B, part, M, N, K, per, vec_a, vec_b);
     NBG_CUDA(cudaGetLastError());

@@ -122,3 +122,49 @@ def test_fused_smooth_forward_equals_product_then_step(B, N):
         out.append([v, z, S, U, M, VP])
     for x, y in zip(*out):
         assert torch.equal(x, y)
+
+
+def test_more_row_tiles_than_a_grid_has_rows():
+    """2^16 and more tiles of rows: batches and input widths beyond 65,535 tiles run as any other."""
+    from neuronbridge_gb300.adjoint import GradParams
+
+    lib, check, ptr, st = _lib()
+    r = 65535 * 32 + 40
+    x = _randn(r, 3, seed=1)
+    t = torch.empty(3, r, device="cuda")
+    check(lib.nbg_transpose(ptr(x), ptr(t), r, 3, st))
+    assert torch.equal(t, x.t())
+    w = torch.eye(3, device="cuda") * 0.5
+    c = torch.full((r, 3), float("nan"), device="cuda")
+    check(lib.nbg_product_nt(ptr(x), ptr(w), ptr(c), r, 3, 3, st))
+    assert torch.equal(c, 0.5 * x)
+    # a step of both directions against the product and the plain step
+    p = GradParams(-65.0, -65.0, 0.5, 2, 1)
+    al, th = torch.full((3,), 0.05, device="cuda"), torch.full((3,), -50.0, device="cuda")
+    full = lambda v: torch.full((r, 3), v, device="cuda")
+    s, m, u = torch.sigmoid(x), torch.ones(r, 3, device="cuda", dtype=torch.uint8), -60.0 + x
+    out = []
+    for fused in (False, True):
+        v, z, s1, u1, m1, vp1, lam, gt, ga, d = full(-60.0), full(0.0), full(0.0), full(0.0), m.clone(), full(0.0), full(0.1), \
+            full(0.0), full(0.0), full(0.0)
+        if fused:
+            check(lib.nbg_lif_forward_step_smooth(ptr(s), ptr(w), ptr(x), ptr(v), ptr(s1), ptr(u1), ptr(m1), ptr(vp1), ptr(z),
+                                                  0.3, ptr(al), ptr(th), ctypes.byref(p), 0, r, 3, st))
+            check(lib.nbg_lif_adjoint_step_product(ptr(x), ptr(w), ptr(x), 0.3, ptr(u), ptr(s), ptr(m), ptr(u1), ptr(lam), ptr(d),
+                                                   ptr(gt), ptr(ga), ptr(al), ptr(th), ctypes.byref(p), 0, r, 3, st))
+        else:
+            cur, ref = 0.5 * s + x, torch.zeros(r, 3, device="cuda", dtype=torch.int32)
+            check(lib.nbg_lif_forward_step(ptr(cur), ptr(v), ptr(ref), ptr(s1), ptr(u1), ptr(m1), ptr(vp1), ptr(z), 0.3, ptr(al),
+                                           ptr(th), ctypes.byref(p), r, 3, st))
+            ge = 0.5 * x
+            check(lib.nbg_lif_adjoint_step(ptr(ge), ptr(x), 0.3, ptr(u), ptr(s), ptr(m), ptr(u1), ptr(lam), ptr(d), ptr(gt),
+                                           ptr(ga), ptr(al), ptr(th), ctypes.byref(p), r, 3, st))
+        out.append((v, z, s1, u1, m1, vp1, lam, gt, ga, d))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+    rows = 65535 * 64 + 70
+    a, b = _randn(1, rows, seed=2), _randn(1, 3, seed=3)
+    part, g = torch.empty(rows, 3, device="cuda"), torch.zeros(rows, 3, device="cuda")
+    check(lib.nbg_product_tn(ptr(a), ptr(b), ptr(part), 1, rows, 3, 1, st))
+    check(lib.nbg_adjoint_reduce_add(ptr(g), ptr(part), 1, rows * 3, rows * 3, st))
+    assert torch.equal(g, a.t() * b)
