@@ -229,6 +229,13 @@ def record_bytes(T: int, B: int, N: int) -> int:
     return T * B * N * 9 + (T + 1) * B * N * 4
 
 
+def _whole_dI(T: int, B: int, N: int) -> bool:
+    """Whether a recorded FP32 backward keeps dI of the whole run instead of a segment's: its 4 bytes an element, twice
+    under graph capture (the warm-up's and the graph's), count against the record's budget, and the (step, row) pairs
+    are one 32-bit dimension of the products."""
+    return record_bytes(T, B, N) + 8 * T * B * N <= RECORD_BUDGET_BYTES and T * B < 2 ** 31
+
+
 def _record_buffers(T, B, N, dev):
     """(U, S, M, VP): U[t] = u_t, S[t + 1] = s_t (S[0] = 0), M[t] = m_t,
     VP[t] = v_{t-1}."""
@@ -368,8 +375,8 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
     tc = _tc_ok(p, B, N)
     fused = _fused_ok(p, B, N)
     # with the state recorded, the weight gradients run once, over every
-    # (step, row) pair of the run
-    whole = rec is not None and (fused or not tc)
+    # (step, row) pair of the run (in FP32 where the run's dI fits beside the record)
+    whole = rec is not None and (fused or (not tc and _whole_dI(T, B, N)))
     sweep = lib.nbg_lif_adjoint_sweep_work(B, N) if tc and FUSED_STEP and SWEEP else 0
     fused = fused or sweep > 0
     smooth = _Smooth(lib, w_in, w_rec, B, st) if p.smooth and rec is None else None

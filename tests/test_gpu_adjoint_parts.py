@@ -115,3 +115,23 @@ def test_sweeps_on_two_streams_of_two_threads():
         for got in runs:
             for a, b in zip(got, want):
                 assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("smooth", [False, True])
+def test_recorded_gradients_by_segment(monkeypatch, smooth):
+    """A record beside which dI of the whole run does not fit: the gradients of a replayed run, segment by segment, bit for bit."""
+    from neuronbridge_gb300 import adjoint
+    from neuronbridge_gb300.adjoint import RecurrentLIF, poisson_inputs
+
+    monkeypatch.setattr(adjoint, "RECORD_BUDGET_BYTES", 0)
+    x = poisson_inputs(torch.linspace(50.0, 400.0, 30), 47, 20, dt=1.0, seed=3)
+    labels = torch.arange(20, device="cuda") % 5
+    out = []
+    for record in (True, False):
+        model = RecurrentLIF(n_in=30, n_rec=150, n_out=5, checkpoint=20, seed=11, smooth=smooth, weight_scale=5.0,
+                             use_graphs=False, record=record)
+        torch.nn.functional.cross_entropy(model(x), labels).backward()
+        out.append([q.grad for q in model.parameters()])
+    assert all(g.abs().sum() > 0 for g in out[0][:3])
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
