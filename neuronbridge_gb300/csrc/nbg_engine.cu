@@ -1927,8 +1927,8 @@ __global__ void k_set_synapses(SynRec *rec, SynStatic *wst, const float *__restr
 // + k] = field f (w, Apre, Apost, LastUpdate) of the synapse at CSC position
 // pos[k].  Bound by the sector that each position costs (32 bytes for 16 of use,
 // a plastic record's first half); the copies that follow are a few times its
-// time.  The scatter on the host that it replaces took 1.0 ms for 500,000
-// synapses and 40 ms for ten million.
+// time.  The scatter on the host, which stays for a device without room for the
+// staging, took 1.0 ms for 500,000 synapses and 40 ms for ten million.
 __global__ void k_gather_weights(const SynRec *__restrict__ rec, const SynStatic *__restrict__ wst,
                                  const unsigned int *__restrict__ pos, unsigned int count, float *__restrict__ out,
                                  size_t stride) {
@@ -1946,7 +1946,25 @@ __global__ void k_gather_weights(const SynRec *__restrict__ rec, const SynStatic
     out[3 * stride + k] = __uint_as_float(a.w); // the bits of an int
 }
 
-constexpr size_t kWeightChunk = (size_t)1 << 24; // synapses of a chunk: 256 MiB of staging
+constexpr size_t kWeightChunk = (size_t)1 << 22; // synapses of a chunk: 64 MiB of staging, 16 for a static network
+
+// The same from a download of all records, scattered by the host.
+nbg_status scatter_weights(nbg_engine *e, float *w, float *apre, float *apost, int32_t *last) {
+    const size_t S = (size_t)e->S;
+    std::vector<SynRec> r(e->plastic ? S : 0);
+    std::vector<SynStatic> ws(e->plastic ? 0 : S);
+    if (e->plastic) NBG_CUDA(cudaMemcpy(r.data(), e->rec.p, S * sizeof(SynRec), cudaMemcpyDeviceToHost));
+    else NBG_CUDA(cudaMemcpy(ws.data(), e->wst.p, S * sizeof(SynStatic), cudaMemcpyDeviceToHost));
+    for (size_t p = 0; p < S; ++p) {
+        const SynRec y = e->plastic ? r[p] : SynRec{};
+        const int64_t o = e->csc_orig[p];
+        if (w) w[o] = e->plastic ? y.w : ws[p].w;
+        if (apre) apre[o] = y.apre;
+        if (apost) apost[o] = y.apost;
+        if (last) last[o] = y.last;
+    }
+    return NBG_OK;
+}
 
 // Every synapse's weight back to init_w_d (and, with `traces`, its STDP state
 // to zero), on the engine's stream.
@@ -3458,13 +3476,18 @@ nbg_status nbg_get_weights(nbg_engine *e, float *w, float *apre, float *apost, i
     if (S == 0) return NBG_OK;
     // gathered on the device a chunk at a time, then one copy per field
     std::lock_guard<std::mutex> lock(e->weights_mu);
-    const size_t chunk = std::min(S, kWeightChunk);
-    if (e->wout.n < 4 * chunk) NBG_CUDA(e->wout.alloc(4 * chunk));
-    if (e->orig_pos_d.n < S) {
+    const size_t chunk = std::min(S, kWeightChunk), staging = (e->plastic ? 4 : 1) * chunk;
+    cudaError_t room = e->wout.n < staging ? e->wout.alloc(staging) : cudaSuccess;
+    if (room == cudaSuccess && e->orig_pos_d.n < S) {
         std::vector<unsigned int> pos(S);
         for (size_t o = 0; o < S; ++o) pos[o] = (unsigned int)e->orig_pos[o];
-        NBG_CUDA(e->orig_pos_d.upload(pos));
+        room = e->orig_pos_d.upload(pos);
     }
+    if (room == cudaErrorMemoryAllocation) {
+        e->wout.release();
+        return scatter_weights(e, w, apre, apost, last);
+    }
+    NBG_CUDA(room);
     for (size_t o0 = 0; o0 < S; o0 += chunk) {
         const size_t m = std::min(chunk, S - o0);
         k_gather_weights<<<(unsigned)((m + 255) / 256), 256, 0, e->stream>>>(e->rec.p, e->wst.p, e->orig_pos_d.p + o0, (unsigned)m,
