@@ -2548,7 +2548,12 @@ nbg_status nbg_create_batch(const nbg_net_desc *const *descs, int n, const nbg_o
     return st;
 }
 
-nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engine **out) {
+// nbg_create; quads_allowed: the mask ring may be padded to whole quads for the
+// kernels that read them, and *padded says whether it was (more words than the
+// synapses have).
+static nbg_status create_engine(const nbg_net_desc *d, const nbg_options *opt_in, bool quads_allowed, bool *padded_ring,
+                                nbg_engine **out) {
+    *padded_ring = false;
     if (!d || !out) return fail(NBG_ERR_INVALID, "null argument");
     *out = nullptr;
     nbg_options opt;
@@ -2596,7 +2601,8 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
     e->n_rules = d->n_rules;
     e->rules.assign(d->rules, d->rules + d->n_rules);
     auto bail = [&](nbg_status s) {
-        delete e;
+        if (e->stream) nbg_destroy(e); // with its events and pinned memory
+        else delete e;
         return s;
     };
     // ---- layers
@@ -2759,7 +2765,7 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
             padded += (nw + 3) / 4 * 4;
             most = std::max(most, nw);
         }
-        const bool quads = S > 0 && padded <= 2 * words && padded <= (1 << 27);
+        const bool quads = quads_allowed && S > 0 && padded <= 2 * words && padded <= (1 << 27);
         // plastic: one quad per neuron (with a second one staged for those that
         // have it, the instance spills: 1,000 Poisson-driven neurons of in-degree
         // about 100 took 94 us a launch against 82 by the word drain)
@@ -2777,6 +2783,7 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
                                   !collect_palette(d->weight, S, [&](int64_t s) { return (unsigned int)(d->type[s] & 1); },
                                                    e->palette_host, e->palette_n)))
             e->palette_kernel = nullptr;
+        *padded_ring = (e->palette_kernel || e->rec_quads) && padded > words;
     }
     // ---- mask word offsets (whole quads where a kernel reads quads) and per-synapse arrays
     const int word_group = e->palette_kernel || e->rec_quads ? 4 : 1;
@@ -3008,6 +3015,13 @@ nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt_in, nbg_engi
     e->spike_capacity = opt.spike_capacity;
     *out = e;
     return NBG_OK;
+}
+
+nbg_status nbg_create(const nbg_net_desc *d, const nbg_options *opt, nbg_engine **out) {
+    bool padded = false;
+    const nbg_status st = create_engine(d, opt, true, &padded, out);
+    // a device that holds the ring but not its padding runs the kernels without it
+    return st == NBG_ERR_OOM && padded ? create_engine(d, opt, false, &padded, out) : st;
 }
 
 nbg_status nbg_destroy(nbg_engine *e) {

@@ -90,3 +90,21 @@ def test_a_delivery_again_after_one_without_room():
         with pytest.raises(_lib.NbgError):  # nor does it launch on what it did not get
             b.deliver(s)
     assert np.array_equal(b.deliver(s), want)
+
+
+def test_a_ring_that_fits_without_its_padding():
+    """In-degree 40 (two mask words a neuron, four with padding) over 4,000 steps of delay: 0.65 GB, 1.29 padded.  The network
+    is created where only the former fits, and runs as with the latter."""
+    cfg = nb.SimulationConfig(steps=4400, timestep=0.1)
+    net = _network(20_000, 40, True, delay=4000)
+    with _leaving(1 << 30):
+        tight = nb.Simulation(net, cfg, seed=3)
+    wide = nb.Simulation(net, cfg, seed=3)
+    for s in (tight, wide):
+        s.run(4400)
+    assert tight.num_events == wide.num_events > 0
+    for a, b in zip(tight.spike_raster(), wide.spike_raster()):
+        assert len(a) > 0 and np.array_equal(a, b)
+    a, b = tight.weights(), wide.weights()
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
