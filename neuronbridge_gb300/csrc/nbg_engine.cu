@@ -1399,11 +1399,17 @@ __global__ void __launch_bounds__(256, 4) k_update_quad(const __grid_constant__ 
             const unsigned int gbit = fired ? 1u << (gen_pos & 31) : 0u;
 #pragma unroll
             for (int k = 0; k < 4; ++k) w[k] |= (gen_pos >> 5) == k ? gbit : 0u;
-            for (int g = g0 + 1; g < g1; ++g) // further generator inputs
-                if (n.gen_pos[g] < 128 && generator_fired(n, n.gen_src[g], t - (int)n.gen_delay[g])) {
+            int g = g0 + 1; // further generator inputs, ascending in rank: each quad takes its own
+            auto more_generators = [&](unsigned int(&word)[4], int x) {
+                for (; g < g1; ++g) {
+                    const int pos = n.gen_pos[g];
+                    if (pos >> 7 != x) break;
+                    if (!generator_fired(n, n.gen_src[g], t - (int)n.gen_delay[g])) continue;
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) w[k] |= (n.gen_pos[g] >> 5) == k ? 1u << (n.gen_pos[g] & 31) : 0u;
+                    for (int k = 0; k < 4; ++k) word[k] |= (pos >> 5 & 3) == k ? 1u << (pos & 31) : 0u;
                 }
+            };
+            more_generators(w, 0);
             const bool take = !jump || r.last > L.ip;
             float a = jump ? r.v : 0.0f, c = 0.0f;
 #pragma unroll
@@ -1416,13 +1422,10 @@ __global__ void __launch_bounds__(256, 4) k_update_quad(const __grid_constant__ 
                 const uint4 e = x == 1 ? s_quad1[b & 3][threadIdx.x] : *reinterpret_cast<const uint4 *>(mrow);
                 if (e.x | e.y | e.z | e.w) *reinterpret_cast<uint4 *>(mrow) = make_uint4(0u, 0u, 0u, 0u);
                 unsigned int we[4] = {e.x, e.y, e.z, e.w};
+                more_generators(we, x);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     we[k] |= (gen_pos >> 5) == 4 * x + k ? gbit : 0u;
-                    for (int g = g0 + 1; g < g1; ++g)
-                        if ((n.gen_pos[g] >> 5) == 4 * x + k &&
-                            generator_fired(n, n.gen_src[g], t - (int)n.gen_delay[g]))
-                            we[k] |= 1u << (n.gen_pos[g] & 31);
                     delivered += __popc(we[k]);
                     if (take && we[k])
                         apply_quad_word<S>(we[k], n.code[woff + 4 * x + k], sw, pal.types, split, a, c);

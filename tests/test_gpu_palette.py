@@ -114,3 +114,28 @@ def _same_as_fresh(sim, d, w, cfg):
     for a, b in zip(sim.spike_raster(), fresh.spike_raster()):
         assert np.array_equal(a, b)
     assert np.array_equal(sim.state_field(0), fresh.state_field(0)) and np.array_equal(sim.weights()["weight"], w)
+
+
+@pytest.mark.parametrize("inputs,in_degree", [(2, 200), (40, 100), (70, 300), (300, 20), (784, 0)])
+def test_many_generator_inputs_equal_the_oracle(oracle_lib, inputs, in_degree):
+    """Several Poisson inputs a neuron in every quad of its mask words (their ranks are mixed with the recurrent ones')."""
+    import oracle
+
+    n = 70
+    rng = np.random.default_rng(inputs)
+    tgt = np.repeat(np.arange(n, dtype=np.int32), in_degree)
+    src = rng.integers(0, n, len(tgt)).astype(np.int32)
+    gsrc = (n + np.tile(np.arange(inputs), n)).astype(np.int32)
+    gtgt = np.repeat(np.arange(n, dtype=np.int32), inputs)
+    order = rng.permutation(len(tgt) + len(gtgt))
+    layers = [NeuronLayer("TimeDrivenLIF_Voltage_jump", n, output=True, parameters=dict(LIF_PARAMS)),
+              NeuronLayer.poisson_rate(inputs, rate_bias_hz=9000.0 / inputs, rate_gain_hz_per_current=0.0)]
+    w = np.concatenate([np.resize(np.asarray([0.3, 0.2], np.float32), len(tgt)), np.full(len(gtgt), 0.5, np.float32)])
+    delay = np.concatenate([rng.integers(4, 9, len(tgt)), rng.integers(1, 4, len(gtgt))]).astype(np.int32)
+    d = NetworkDescription.from_arrays(layers, np.concatenate([src, gsrc])[order], np.concatenate([tgt, gtgt])[order],
+                                       np.zeros(len(order), np.int32), w[order], delay=delay[order])
+    sim = nb.Simulation(d, nb.SimulationConfig(steps=300, timestep=0.1))
+    sim.run(300)
+    ref = oracle.OracleNet(sim.flat)
+    ref.run(300)
+    _check(sim, ref)
