@@ -84,6 +84,8 @@ inline nbg_status fail(nbg_status code, const char *fmt, A... a) {
 }
 
 constexpr int kMaxBlockSteps = 32;
+constexpr int kSummaryWords = 32; // mask words of a neuron up to which k_update uses their summary
+constexpr int kQuadWords = 8, kQuadInputs = 8; // mask words and generator inputs for which quads pay (nbg_create)
 constexpr int kErrOverflow = 1;
 constexpr int kErrEventLog = 2;
 
@@ -1061,7 +1063,7 @@ __global__ void __launch_bounds__(256, S::min_blocks) k_update(const __grid_cons
     //   memory round trip.  (Prefetching step b + 1's records at the end of
     //   step b, and keeping the generator synapse's record in registers, both
     //   made the static networks slower.)
-    const bool fast = nw <= 32 && (g1 - g0) <= 32;
+    const bool fast = nw <= kSummaryWords && (g1 - g0) <= 32;
     const unsigned int D = (unsigned int)n.D;
     const unsigned int slot0 = (unsigned int)T0 % D; // the block's first slot; later ones by wrap_slot
     constexpr int kWide = 4;
@@ -2760,15 +2762,36 @@ static nbg_status create_engine(const nbg_net_desc *d, const nbg_options *opt_in
         }
         // Quads: on average at least 2 of the 4 words of a quad hold synapses,
         // so that the padded ring is at most twice the words that synapses have.
+        // No neuron has 9 to 32 words: the quads from the third on are loaded one
+        // after the other whether or not they hold arrivals, where k_update's
+        // summary skips empty words (above 32 words it reads every word itself:
+        // in-degree 2,000, 34.4 us a step against 12.0 in quads).  us a step,
+        // k_update / quads, of 2,000 and of 50,000 neurons:
+        //   in-degree  no recurrent spikes       16 Hz                     150 Hz
+        //   120        1.05/0.67   1.49/1.06     1.67/0.93   2.55/1.55     4.37/1.60   7.33/2.89
+        //   250        1.05/1.05   1.49/1.59     2.19/1.52   7.12/2.66     8.70/3.01   32.8/5.94
+        //   400        1.04/1.69   1.49/2.62     2.76/2.70   15.1/4.80     13.7/5.34   78.1/10.8
+        //   1,000      1.05/3.00   1.49/4.86     4.57/5.44   54.4/11.4     31.8/13.6   259/30.3
+        // And no more than 8 generator inputs (in-degree 100, 16 Hz: 8 of them
+        // 3.33/2.84 and 4.48/4.01, 12 of them 4.12/3.76 and 7.82/11.6, 100 of them
+        // 44.4/55.4 and 143/160): k_update looks up the position of an input only
+        // when it has fired.
         int64_t words = 0, padded = 0;
         int most = 0;
+        bool few_quads = true, few_inputs = true;
         for (int j = 0; j < e->N; ++j) {
             const int nw = (indeg[j + 1] + 31) / 32;
             words += nw;
             padded += (nw + 3) / 4 * 4;
             most = std::max(most, nw);
+            few_quads = few_quads && (nw <= kQuadWords || nw > kSummaryWords);
         }
-        const bool quads = quads_allowed && S > 0 && padded <= 2 * words && padded <= (1 << 27);
+        {
+            std::vector<int> inputs((size_t)e->N, 0);
+            for (int64_t s = 0; s < S && few_inputs; ++s)
+                few_inputs = !e->layers[pop[d->source[s]]].generator || ++inputs[(size_t)d->target[s]] <= kQuadInputs;
+        }
+        const bool quads = quads_allowed && few_quads && few_inputs && S > 0 && padded <= 2 * words && padded <= (1 << 27);
         // plastic: one quad per neuron (with a second one staged for those that
         // have it, the instance spills: 1,000 Poisson-driven neurons of in-degree
         // about 100 took 94 us a launch against 82 by the word drain)

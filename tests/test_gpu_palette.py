@@ -116,9 +116,10 @@ def _same_as_fresh(sim, d, w, cfg):
     assert np.array_equal(sim.state_field(0), fresh.state_field(0)) and np.array_equal(sim.weights()["weight"], w)
 
 
-@pytest.mark.parametrize("inputs,in_degree", [(2, 200), (40, 100), (70, 300), (300, 20), (784, 0)])
+@pytest.mark.parametrize("inputs,in_degree", [(2, 200), (8, 248), (9, 100), (5, 300), (8, 1100), (40, 100), (300, 20), (784, 0)])
 def test_many_generator_inputs_equal_the_oracle(oracle_lib, inputs, in_degree):
-    """Several Poisson inputs a neuron in every quad of its mask words (their ranks are mixed with the recurrent ones')."""
+    """Several Poisson inputs a neuron in every quad of its mask words (their ranks are mixed with the recurrent ones'), on
+    both sides of the rules that choose quads: 8 words or more than 32, 8 inputs."""
     import oracle
 
     n = 70
