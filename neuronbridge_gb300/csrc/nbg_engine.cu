@@ -1580,15 +1580,25 @@ __global__ void __launch_bounds__(256, S::min_blocks) k_update_quad_rec(const __
                         for (int k = 0; k < 4; ++k) w[k] |= (n.gen_pos[g] >> 5) == k ? 1u << (n.gen_pos[g] & 31) : 0u;
                     }
             }
-            if (w[0] | w[1] | w[2] | w[3]) {
+            if constexpr (S::deep) {
+                if (w[0] | w[1] | w[2] | w[3]) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    delivered += __popc(w[k]);
-                    if constexpr (S::deep)
+                    for (int k = 0; k < 4; ++k) {
+                        delivered += __popc(w[k]);
                         apply_word_staged<S>(n, L, r, acc_a, acc_b, gate, w[k], base + k * 32, t, pos_cur,
                                              s_rec + ((b & 1) * 256 + threadIdx.x) * 2, pos_nxt);
-                    else
-                        apply_word_batched<S>(n, L, r, acc_a, acc_b, gate, w[k], base + k * 32, t);
+                    }
+                }
+            } else {
+                // each lane its own first word, so that a round of record loads serves
+                // lanes with arrivals in different words
+                while (w[0] | w[1] | w[2] | w[3]) {
+                    const int k = w[0] ? 0 : w[1] ? 1 : w[2] ? 2 : 3;
+                    const unsigned int word = w[0] ? w[0] : w[1] ? w[1] : w[2] ? w[2] : w[3];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) w[x] = x == k ? 0u : w[x];
+                    delivered += __popc(word);
+                    apply_word_batched<S>(n, L, r, acc_a, acc_b, gate, word, base + k * 32, t);
                 }
             }
             spk = update_neuron<S>(n, L, r, acc_a, acc_b, noisy ? L.p[5] * gauss12(nkey, t) : 0.0f, j, t);
