@@ -824,6 +824,13 @@ __global__ void k_small_gemm(const float *__restrict__ A, int a_rs, int a_cs, co
     Cm[o] = acc;
 }
 
+// kAhead: the loop unrolled eight times, for the loads of eight terms in flight.
+// Where few warps run (the readout z W_out) they wait for each other's latency:
+// 64 x 10 outputs of K = 1,000 8.2 -> 6.0 us.  From about 4,096 outputs on the
+// SMs have warps enough, and the longer loop only costs (40 x 2,500 of 1,000: 158
+// us, unrolled 172), as its remainder does below K = 256 (64 x 10 of 128: 2.3,
+// unrolled 2.4).
+template <bool kAhead>
 __global__ void k_small_gemm_warp(const float *__restrict__ A, int a_rs, int a_cs, const float *__restrict__ Bm,
                                   int b_rs, int b_cs, float *__restrict__ Cm, int M, int N, int K) {
     const long long o = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -831,9 +838,13 @@ __global__ void k_small_gemm_warp(const float *__restrict__ A, int a_rs, int a_c
     if (o >= (long long)M * N) return; // whole warps: o is the same for all 32 lanes
     const int i = (int)(o / N), j = (int)(o % N);
     float acc = 0.0f;
+    auto term = [&](int k) { acc = acc + A[(size_t)i * a_rs + (size_t)k * a_cs] * Bm[(size_t)k * b_rs + (size_t)j * b_cs]; };
+    if constexpr (kAhead) {
 #pragma unroll 8
-    for (int k = lane; k < K; k += 32) // unrolled: eight terms' loads in flight (z W_out of 64 x 1,000: 15 -> 12 us)
-        acc = acc + A[(size_t)i * a_rs + (size_t)k * a_cs] * Bm[(size_t)k * b_rs + (size_t)j * b_cs];
+        for (int k = lane; k < K; k += 32) term(k);
+    } else {
+        for (int k = lane; k < K; k += 32) term(k);
+    }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) acc = acc + __shfl_down_sync(0xffffffffu, acc, d);
     if (lane == 0) Cm[o] = acc;
@@ -846,8 +857,9 @@ nbg_status nbg_small_gemm(const float *A, int a_rs, int a_cs, const float *B, in
     if (!A || !B || !C || M <= 0 || N <= 0 || K <= 0) return nbg_fail(NBG_ERR_INVALID, "nbg_small_gemm: bad arguments");
     const long long total = (long long)M * N;
     if (K >= kSmallGemmWarpK)
-        k_small_gemm_warp<<<(unsigned)((total + 3) / 4), 128, 0, (cudaStream_t)stream>>>(A, a_rs, a_cs, B, b_rs, b_cs,
-                                                                                         C, M, N, K);
+        (K >= 256 && total < 4096 ? k_small_gemm_warp<true> : k_small_gemm_warp<false>)<<<(unsigned)((total + 3) / 4), 128, 0,
+                                                                                       (cudaStream_t)stream>>>(
+            A, a_rs, a_cs, B, b_rs, b_cs, C, M, N, K);
     else
         k_small_gemm<<<(unsigned)((total + 127) / 128), 128, 0, (cudaStream_t)stream>>>(A, a_rs, a_cs, B, b_rs, b_cs,
                                                                                        C, M, N, K);

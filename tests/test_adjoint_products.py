@@ -168,3 +168,16 @@ def test_more_row_tiles_than_a_grid_has_rows():
     check(lib.nbg_product_tn(ptr(a), ptr(b), ptr(part), 1, rows, 3, 1, st))
     check(lib.nbg_adjoint_reduce_add(ptr(g), ptr(part), 1, rows * 3, rows * 3, st))
     assert torch.equal(g, a.t() * b)
+
+
+@pytest.mark.parametrize("K", [64, 255, 256, 1000, 1031])
+def test_small_product_of_few_and_of_many_outputs(K):
+    """The readout's product with the loads of eight terms in flight (fewer than 4,096 outputs, K >= 256) and without: the same
+    bits, within the bound of its lanes' chains and their tree."""
+    lib, check, ptr, st = _lib()
+    a, b = _randn(512, K, seed=1), _randn(K, 10, seed=2)
+    out = [torch.full((m, 10), float("nan"), device="cuda") for m in (409, 512)]
+    for c in out:
+        check(lib.nbg_small_gemm(ptr(a), K, 1, ptr(b), 10, 1, ptr(c), len(c), 10, K, st))
+    assert torch.equal(out[0], out[1][:409])
+    _within_bound(out[1], a, b, K)
