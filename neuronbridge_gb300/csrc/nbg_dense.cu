@@ -647,12 +647,12 @@ nbg_status nbg_dense_create(int instances, int neurons, const float *w, const nb
             if (ce == cudaSuccess)
                 chk(cudaFuncSetAttribute(umma::k_dense_umma<umma::NoFinish>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, umma::kSmemBytes));
+            // of the fused step only the tile this engine runs: an attribute loads its kernel
             if (ce == cudaSuccess)
-                chk(cudaFuncSetAttribute(umma::k_dense_umma<LifFinish, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         umma::Tile<128>::fused_smem));
-            if (ce == cudaSuccess)
-                chk(cudaFuncSetAttribute(umma::k_dense_umma<LifFinish, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         umma::Tile<64>::fused_smem));
+                chk(d->half_tiles ? cudaFuncSetAttribute(umma::k_dense_umma<LifFinish, 64>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, umma::Tile<64>::fused_smem)
+                                  : cudaFuncSetAttribute(umma::k_dense_umma<LifFinish, 128>,
+                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, umma::Tile<128>::fused_smem));
         } else if (ce == cudaSuccess) {
             dim3 grid(neurons / 32, neurons / 32), block(32, 8);
             k_split_transpose<<<grid, block>>>(tmp.p, d->whi.p, d->wlo.p, neurons);
