@@ -352,7 +352,11 @@ int sm_count() {
 
 // The K split of an M x N x K product: CTAs are added while tiles times ranks
 // leave SMs without one and a rank keeps 32 k (four rounds of its eight
-// warps' granules; fewer and the exchange costs more than it shortens).
+// warps' granules; fewer and the exchange costs more than it shortens).  Above
+// K = 128 there are two at least: sixteen chains of K / 16 terms, as one CTA
+// keeps, leave a larger error than the 32 lane sums of nbg_small_gemm, which
+// these products replaced (1000 x 1024 outputs of K = 1,000: 1.53e-7 of the norm
+// against 1.23e-7, in two ranks 1.19e-7).
 NtShape nt_shape(const float *A, const float *W, int M, int N, int K) {
     NtShape sh{};
     sh.M = M;
@@ -361,7 +365,7 @@ NtShape nt_shape(const float *A, const float *W, int M, int N, int K) {
     const long long tiles = (long long)((M + kTile - 1) / kTile) * ((N + kTile - 1) / kTile);
     const int sms = sm_count();
     sh.ranks = 1;
-    while (sh.ranks < 8 && tiles * sh.ranks < sms && K >= 64 * sh.ranks) sh.ranks *= 2;
+    while (sh.ranks < 8 && (tiles * sh.ranks < sms || (sh.ranks == 1 && K > 128)) && K >= 64 * sh.ranks) sh.ranks *= 2;
     sh.per = ((K + sh.ranks - 1) / sh.ranks + 7) & ~7;
     sh.kc = std::min(sh.per, kNtChunk);
     sh.stages = sh.per > sh.kc ? 2 : 1;
@@ -426,12 +430,17 @@ __global__ void __launch_bounds__(256) k_transpose(const float *__restrict__ in,
 // B: K x N, both row major: S^T dI and X^T dI with K = the (step, row) pairs.
 // Compute-bound (2 M N K operations on (M + N) K values): 64 x 64 tiles, 128
 // threads of 8 x 4 outputs, pairs of m packed, three cp.async stages of 32 k,
-// split K to fill the SMs.  Sixteen terms are one chain, their sums another,
-// the splits a third (nbg_adjoint_reduce_add).
+// split K to fill the SMs.  Sixteen terms are one chain, their sums another, the
+// splits a third (nbg_adjoint_reduce_add).  In a split of at most 128 terms the
+// sixteen are four chains of four, added in pairs: one chain leaves a larger error
+// there than the lane sums of nbg_small_gemm, which this product replaced (512 x
+// 512 outputs of K = 100: 8.7e-8 of the norm against 7.5e-8, in pairs 7.3e-8).  In a
+// long split the chain of the sums decides (chains of eight, 512 x 512 x 8000:
+// 2.2e-7 against 1.7e-7), and the additions would cost.
 //
 // Measured, 512 x 512 x 8000 in 8 splits: 13.5 ms -> 113 us (37 TFLOP/s);
 // error against 64 bits 2.9e-7 -> 1.7e-7 of the norm.
-constexpr int kTnTile = 64, kTnThreads = 128, kTnK = 32, kTnStages = 3, kTnChain = 16;
+constexpr int kTnTile = 64, kTnThreads = 128, kTnK = 32, kTnStages = 3;
 
 template <int kBytes>
 __device__ __forceinline__ void tn_load(float *dst, const float *src, int c0, int cols, int k0, int k_end) {
@@ -444,6 +453,36 @@ __device__ __forceinline__ void tn_load(float *dst, const float *src, int c0, in
     }
 }
 
+// acc = the kN terms from k0 of a stage, in one chain
+template <int kN>
+__device__ __forceinline__ void tn_chain(unsigned long long (&acc)[4][4], const float *as, const float *bs, int k0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+#pragma unroll
+    for (int k = k0; k < k0 + kN; ++k) {
+        const ulonglong2 a01 = *reinterpret_cast<const ulonglong2 *>(as + k * kTnTile);
+        const ulonglong2 a23 = *reinterpret_cast<const ulonglong2 *>(as + k * kTnTile + 4);
+        const float4 b = *reinterpret_cast<const float4 *>(bs + k * kTnTile);
+        const unsigned long long bb[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            fma2(acc[0][j], a01.x, bb[j]);
+            fma2(acc[1][j], a01.y, bb[j]);
+            fma2(acc[2][j], a23.x, bb[j]);
+            fma2(acc[3][j], a23.y, bb[j]);
+        }
+    }
+}
+__device__ __forceinline__ void tn_add(unsigned long long (&d)[4][4], const unsigned long long (&a)[4][4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) add2(d[i][j], a[i][j]);
+}
+
+template <bool kPairs>
 __global__ void __launch_bounds__(kTnThreads) k_product_tn(const float *__restrict__ A, const float *__restrict__ B,
                                                            float *__restrict__ part, int M, int N, int K, int per,
                                                            int vec_a, int vec_b) {
@@ -478,30 +517,21 @@ __global__ void __launch_bounds__(kTnThreads) k_product_tn(const float *__restri
         copy_commit();
         const float *const as = st[c % kTnStages][0] + ml, *const bs = st[c % kTnStages][1] + nl;
 #pragma unroll 1
-        for (int h = 0; h < kTnK; h += kTnChain) {
+        for (int h = 0; h < kTnK; h += 16) {
             unsigned long long acc[4][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
-#pragma unroll
-            for (int k = h; k < h + kTnChain; ++k) {
-                const ulonglong2 a01 = *reinterpret_cast<const ulonglong2 *>(as + k * kTnTile);
-                const ulonglong2 a23 = *reinterpret_cast<const ulonglong2 *>(as + k * kTnTile + 4);
-                const float4 b = *reinterpret_cast<const float4 *>(bs + k * kTnTile);
-                const unsigned long long bb[4] = {pack2(b.x, b.x), pack2(b.y, b.y), pack2(b.z, b.z), pack2(b.w, b.w)};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    fma2(acc[0][j], a01.x, bb[j]);
-                    fma2(acc[1][j], a01.y, bb[j]);
-                    fma2(acc[2][j], a23.x, bb[j]);
-                    fma2(acc[3][j], a23.y, bb[j]);
-                }
+            if constexpr (kPairs) {
+                unsigned long long x[4][4], y[4][4];
+                tn_chain<4>(acc, as, bs, h);
+                tn_chain<4>(x, as, bs, h + 4);
+                tn_add(acc, x);
+                tn_chain<4>(x, as, bs, h + 8);
+                tn_chain<4>(y, as, bs, h + 12);
+                tn_add(x, y);
+                tn_add(acc, x);
+            } else {
+                tn_chain<16>(acc, as, bs, h);
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) add2(total[i][j], acc[i][j]);
+            tn_add(total, acc);
         }
     }
     float *const out = part + (size_t)blockIdx.z * M * N;
@@ -577,7 +607,8 @@ nbg_status nbg_product_tn(const float *A, const float *B, float *part, int split
     const int per = (int)std::min<long long>((((long long)K + split - 1) / split + kTnK - 1) / kTnK * kTnK, 0x7fffffe0);
     const dim3 grid((unsigned)tiles, 1, (unsigned)split);
     const int vec_a = M % 4 == 0 && ((uintptr_t)A & 15u) == 0, vec_b = N % 4 == 0 && ((uintptr_t)B & 15u) == 0;
-    k_product_tn<<<grid, kTnThreads, 0, (cudaStream_t)stream>>>(A, B, part, M, N, K, per, vec_a, vec_b);
+    (per <= 128 ? k_product_tn<true> : k_product_tn<false>)<<<grid, kTnThreads, 0, (cudaStream_t)stream>>>(A, B, part, M, N, K,
+                                                                                               per, vec_a, vec_b);
     NBG_CUDA(cudaGetLastError());
     return NBG_OK;
 }

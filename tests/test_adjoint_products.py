@@ -181,3 +181,32 @@ def test_small_product_of_few_and_of_many_outputs(K):
         check(lib.nbg_small_gemm(ptr(a), K, 1, ptr(b), 10, 1, ptr(c), len(c), 10, K, st))
     assert torch.equal(out[0], out[1][:409])
     _within_bound(out[1], a, b, K)
+
+
+@pytest.mark.parametrize("K", [24, 64, 100, 129, 240, 480, 1000, 2048])
+def test_products_are_no_further_from_64_bits_than_the_small_product(K):
+    """Error of the norm against 64 bits, of K split over CTAs (12 rows) and not (1,000), and of A^T B, against nbg_small_gemm on
+    the same operands: no larger, but for the 2 % that 10^4 to 10^6 outputs leave uncertain (their own spread is below 1 %)."""
+    lib, check, ptr, st = _lib()
+
+    def error(got, ref):
+        return ((got.double() - ref).norm() / ref.norm()).item()
+
+    def small(a, a_rs, a_cs, b, b_rs, b_cs, M, N):
+        c = torch.empty(M, N, device="cuda")
+        check(lib.nbg_small_gemm(ptr(a), a_rs, a_cs, ptr(b), b_rs, b_cs, ptr(c), M, N, K, st))
+        return c
+
+    for M in (12, 1000):
+        a, w = _randn(M, K, seed=1), _randn(1024, K, seed=2)
+        ref, c = a.double() @ w.double().t(), torch.empty(M, 1024, device="cuda")
+        check(lib.nbg_product_nt(ptr(a), ptr(w), ptr(c), M, 1024, K, st))
+        assert error(c, ref) <= 1.02 * error(small(a, K, 1, w, 1, K, M, 1024), ref)
+    for M in (50, 512):
+        a, b = _randn(K, M, seed=3), _randn(K, 512, seed=4)
+        ref, c = a.double().t() @ b.double(), torch.zeros(M, 512, device="cuda")
+        split = lib.nbg_product_tn_split(M, 512, K)
+        part = torch.empty((split, M, 512), device="cuda")
+        check(lib.nbg_product_tn(ptr(a), ptr(b), ptr(part), split, M, 512, K, st))
+        check(lib.nbg_adjoint_reduce_add(ptr(c), ptr(part), split, M * 512, M * 512, st))
+        assert error(c, ref) <= 1.02 * error(small(a, 1, M, b, 512, 1, M, 512), ref)
