@@ -628,8 +628,13 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
     volatile int *abort = (volatile int *)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t rank;
+    uint32_t rank, ranks;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    if (ranks != kSweepCluster) { // launched without its cluster (as a profiler may): no peer to send to
+        if (threadIdx.x == 0) atomicOr(err, kUmmaTimeout);
+        return;
+    }
     const int mt = blockIdx.x / kSweepParts, bq = blockIdx.x % kSweepParts, ks = (int)rank;
     const int kchunks = n / kKChunk;
     // two of the K ranges, eight or as many as there are chunks; the last CTA that
