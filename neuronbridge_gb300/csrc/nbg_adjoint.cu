@@ -344,10 +344,10 @@ __global__ void __launch_bounds__(kSparseThreads) k_lif_fwd_segment(
 //     counts: two block barriers a step.
 // The kernel before it listed, summed and ranked one after the other with
 // about twenty barriers a step.  Measured, 500 steps of 64 rows, 1,000
-// neurons, 200 inputs, 2.2 % firing: 3.17 -> 1.27 ms (6.3 -> 2.5 us a step;
-// eight warps of four columns each, unpacked, 2.45 ms: 1,506 instructions a
-// warp and step, few of them waiting for memory).  A training step of 128 rows
-// x 1,024 neurons x 1,000 steps: 14.96 -> 11.50 ms.
+// neurons, 200 inputs, 2.2 % firing: 6.2 -> 2.2 us a step, the call with its
+// inputs and readout 3.14 -> 1.13 ms.  (With eight warps of four unpacked columns
+// 4.9 us: 1,506 instructions a warp and step, few of them waiting for memory; with
+// sixteen warps of two packed columns 2.5.)
 constexpr int kRing = 8, kHalfRing = kRing / 2;
 constexpr int kRowsMaxInputs = 4096;
 constexpr int kRowsMaxNeurons = 2048;

@@ -76,8 +76,8 @@ template <int kLeft> __device__ __forceinline__ void copy_wait() {
 // (programmatic dependent launch).
 //
 // Measured: the steps of a training step of 32 rows, 512 neurons, 250 steps
-// (forward by gather) 21.3 -> 2.1 ms in all; smoothed, 12 rows, 300 neurons,
-// 60 steps each way, 1,238 -> 548 us.  Error against 64 bits at 64 x 1000 x
+// (forward by gather) 21.2 -> 1.66 ms in all; smoothed, 12 rows, 300 neurons,
+// 60 steps each way, 1,241 -> 545 us.  Error against 64 bits at 64 x 1000 x
 // 1000: 1.23e-7 -> 1.05e-7 of the norm.
 constexpr int kTile = 32;
 constexpr int kNtThreads = 256, kNtWarps = kNtThreads / 32;

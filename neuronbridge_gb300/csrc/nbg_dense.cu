@@ -330,8 +330,8 @@ __device__ __forceinline__ bool lif_apply(const LifParams &P, float a, bool driv
 // neighbouring columns and asks for kGatherRows rows before it adds the first.
 // The instances of one column slice are neighbours in the grid, so a row that
 // several of them need is read from memory once.  Measured, update included:
-// 154 -> 32.9 us a step at 8,192 neurons (8.2 TB/s of row reads), 100 steps
-// and their read-out at 2,048 neurons 2.61 -> 0.78 ms.
+// 154 -> 29.0 us a step at 8,192 neurons (9.3 TB/s of row reads), 100 steps
+// and their read-out at 2,048 neurons 2.59 -> 0.63 ms.
 //
 // The external spikes are drawn before the wait for the step before.  Registers
 // (kCtas, the CTAs an SM is to hold): where the grid has at most three CTAs an SM
