@@ -2796,7 +2796,7 @@ static nbg_status create_engine(const nbg_net_desc *d, const nbg_options *opt_in
             most = std::max(most, nw);
             few_quads = few_quads && (nw <= kQuadWords || nw > kSummaryWords);
         }
-        {
+        if (std::any_of(e->layers.begin(), e->layers.end(), [](const LayerDev &L) { return L.generator; })) {
             std::vector<int> inputs((size_t)e->N, 0);
             for (int64_t s = 0; s < S && few_inputs; ++s)
                 few_inputs = !e->layers[pop[d->source[s]]].generator || ++inputs[(size_t)d->target[s]] <= kQuadInputs;
