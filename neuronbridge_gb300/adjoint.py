@@ -232,8 +232,8 @@ def record_bytes(T: int, B: int, N: int) -> int:
 def _whole_dI(T: int, B: int, N: int) -> bool:
     """Whether a recorded FP32 backward keeps dI of the whole run instead of a segment's: its 4 bytes an element, twice
     under graph capture (the warm-up's and the graph's), count against the record's budget, and the (step, row) pairs
-    are one 32-bit dimension of the products."""
-    return record_bytes(T, B, N) + 8 * T * B * N <= RECORD_BUDGET_BYTES and T * B < 2 ** 31
+    are one 32-bit dimension of the products, of at least one."""
+    return T > 0 and record_bytes(T, B, N) + 8 * T * B * N <= RECORD_BUDGET_BYTES and T * B < 2 ** 31
 
 
 def _record_buffers(T, B, N, dev):

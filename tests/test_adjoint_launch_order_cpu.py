@@ -56,3 +56,8 @@ def test_dI_of_a_whole_run_counts_against_the_record_budget(monkeypatch):
     assert products() == 6  # per segment of three steps
     monkeypatch.setattr(adjoint, "RECORD_BUDGET_BYTES", 1 << 60)
     assert not adjoint._whole_dI(1 << 16, 1 << 15, 1) and adjoint._whole_dI((1 << 16) - 1, 1 << 15, 1)
+
+
+def test_a_run_without_steps_has_no_products(monkeypatch):
+    """No step, no term: the gradients stay the zeros that they start from."""
+    assert "nbg_product_tn" not in _backward(monkeypatch, 20, 4, 0, 3, True)

@@ -135,3 +135,13 @@ def test_recorded_gradients_by_segment(monkeypatch, smooth):
     assert all(g.abs().sum() > 0 for g in out[0][:3])
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("smooth", [False, True])
+def test_a_run_without_steps(smooth):
+    from neuronbridge_gb300.adjoint import RecurrentLIF
+
+    model = RecurrentLIF(n_in=30, n_rec=150, n_out=5, seed=11, smooth=smooth, use_graphs=False)
+    y = model(torch.zeros(0, 4, 30, device="cuda"))
+    y.sum().backward()
+    assert not y.any() and all(not q.grad.any() for q in model.parameters())
