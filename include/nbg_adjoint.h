@@ -175,6 +175,14 @@ nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0
                                  const float *alpha, const float *theta, const nbg_lif_grad_params *p, int steps, int t0,
                                  int B, int N, void *dT_hi, void *dT_lo, int64_t k_off, int64_t k_cols, float *work,
                                  int *err, void *stream);
+/* The same for the steps that end a run: its last step has no recurrent term
+ * (whatever d_hi/lo hold, which the other reads). */
+nbg_status nbg_lif_adjoint_sweep_end(const void *w_hi, const void *w_lo, void *d_hi0, void *d_lo0, void *d_hi1, void *d_lo1,
+                                 const float *g_read, const float *coef, const float *u, const float *s,
+                                 const uint8_t *m, const float *vprev, float *lam_v, float *g_theta, float *g_alpha,
+                                 const float *alpha, const float *theta, const nbg_lif_grad_params *p, int steps, int t0,
+                                 int B, int N, void *dT_hi, void *dT_lo, int64_t k_off, int64_t k_cols, float *work,
+                                 int *err, void *stream);
 
 /* The recurrent weight gradient of a checkpoint segment on the tensor cores,
  * dW_rec += sum over its L steps of S_{t-1}^T dI_t, in three calls:

@@ -75,6 +75,8 @@ _SIG = {
     "nbg_lif_adjoint_sweep_work": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int]),
     "nbg_lif_adjoint_sweep": (ctypes.c_int, [_vp] * 17 + [ctypes.POINTER(GradParams)] + [ctypes.c_int] * 4 + [_vp, _vp] +
                               [ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp]),
+    "nbg_lif_adjoint_sweep_end": (ctypes.c_int, [_vp] * 17 + [ctypes.POINTER(GradParams)] + [ctypes.c_int] * 4 +
+                                  [_vp, _vp] + [ctypes.c_int64, ctypes.c_int64, _vp, _vp, _vp]),
     "nbg_adjoint_blocked_t": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp, _vp,
                                              _vp]),
     "nbg_small_gemm": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp, ctypes.c_int, ctypes.c_int, _vp,
@@ -474,7 +476,8 @@ def _backward_body(lib, gy, x, w_in, w_rec, w_out, alpha, theta, z, ck_v, ck_ref
         dI = None if fused else dI_all[t0:t1] if whole else dI_all
         if tc and sweep:
             k_off, k_cols = (t0 * B, T * B) if whole else (0, L * B)
-            _lib.check(lib.nbg_lif_adjoint_sweep(
+            run_sweep = lib.nbg_lif_adjoint_sweep_end if t1 == T else lib.nbg_lif_adjoint_sweep
+            _lib.check(run_sweep(
                 _ptr(w_hi), _ptr(w_lo), _ptr(d_hi[0]), _ptr(d_lo[0]), _ptr(d_hi[1]), _ptr(d_lo[1]), _ptr(g_read),
                 _ptr(coef_dev[t0:]), _ptr(U), _ptr(S[1:]), _ptr(M), _ptr(VP), _ptr(lam_v), _ptr(g_theta),
                 _ptr(g_alpha), _ptr(alpha), _ptr(theta), ctypes.byref(p), L, t0, B, N, _ptr(dT_hi), _ptr(dT_lo), k_off,

@@ -613,8 +613,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
     const float *__restrict__ coef, const float *__restrict__ u, const float *__restrict__ s,
     const unsigned char *__restrict__ m, const float *__restrict__ vprev, float *__restrict__ lam_v,
     float *__restrict__ g_theta, float *__restrict__ g_alpha, const float *__restrict__ alpha,
-    const float *__restrict__ theta, nbg_lif_grad_params p, int n, int steps, int t0, __nv_bfloat16 *__restrict__ dT_hi,
-    __nv_bfloat16 *__restrict__ dT_lo, long long k_off, long long k_cols, int *ready,
+    const float *__restrict__ theta, nbg_lif_grad_params p, int n, int steps, int t0, int ends_run,
+    __nv_bfloat16 *__restrict__ dT_hi, __nv_bfloat16 *__restrict__ dT_lo, long long k_off, long long k_cols, int *ready,
     int *__restrict__ err) {
     constexpr int kStages = kSweepStages, kRows = 4;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -834,7 +834,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1) k_adj_sweep_umma(
 #pragma unroll
                 for (int c = 1; c < kAdjCluster; ++c)
                     if (c < ranges) ge = ge + x[c][r];
-                const float gs = gs0[r] + ge;
+                // a run's last step has no recurrent term; the product of its zero operand is NaN where W is not finite
+                const float gs = j == 0 && ends_run ? gs0[r] : gs0[r] + ge;
                 const float gu = gs * ds[r] + gu0[r];
                 const float gm = keep[r] ? gu : 0.0f;
                 const size_t o = blocked_index(b0 + r, i, n);
@@ -1245,7 +1246,7 @@ int64_t nbg_lif_adjoint_sweep_work(int B, int N) {
     return clusters >= tiles ? tiles * kReadyStride : 0;
 }
 
-nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0, void *d_lo0, void *d_hi1, void *d_lo1,
+static nbg_status adj_sweep(const char *name, bool ends_run, const void *w_hi, const void *w_lo, void *d_hi0, void *d_lo0, void *d_hi1, void *d_lo1,
                                  const float *g_read, const float *coef, const float *u, const float *s,
                                  const uint8_t *m, const float *vprev, float *lam_v, float *g_theta, float *g_alpha,
                                  const float *alpha, const float *theta, const nbg_lif_grad_params *p, int steps, int t0,
@@ -1255,10 +1256,10 @@ nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0
         !g_theta || !g_alpha || !alpha || !theta || !p || !dT_hi || !dT_lo || !work || !err || steps <= 0 || t0 < 0 ||
         d_hi0 == d_hi1 || d_lo0 == d_lo1 || k_off < 0 || k_off % kAdjN || k_cols % kKChunk ||
         k_off + (int64_t)steps * B > k_cols || k_cols > 0x7fffffff || steps > 0x7fffffff / kAdjCluster)
-        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_sweep: bad arguments");
+        return nbg_fail(NBG_ERR_INVALID, "%s: bad arguments", name);
     if (!nbg_lif_adjoint_sweep_work(B, N))
-        return nbg_fail(NBG_ERR_INVALID, "nbg_lif_adjoint_sweep: B must be %d, N a multiple of %d and not more than the "
-                        "device holds at once", kAdjN, kAdjM);
+        return nbg_fail(NBG_ERR_INVALID, "%s: B must be %d, N a multiple of %d and not more than the "
+                        "device holds at once", name, kAdjN, kAdjM);
     int *ready = (int *)work;
     NBG_CUDA(cudaMemsetAsync(ready, 0, (size_t)(N / kAdjM * kSweepParts) * kReadyStride * sizeof(int), (cudaStream_t)stream));
     cudaLaunchConfig_t cfg;
@@ -1267,10 +1268,30 @@ nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0
     NBG_CUDA(cudaLaunchKernelEx(&cfg, k_adj_sweep_umma, (const __nv_bfloat16 *)w_hi, (const __nv_bfloat16 *)w_lo,
                                 (__nv_bfloat16 *)d_hi0, (__nv_bfloat16 *)d_lo0, (__nv_bfloat16 *)d_hi1,
                                 (__nv_bfloat16 *)d_lo1, g_read, coef, u, s, (const unsigned char *)m, vprev, lam_v, g_theta,
-                                g_alpha, alpha, theta, *p, N, steps, t0, (__nv_bfloat16 *)dT_hi, (__nv_bfloat16 *)dT_lo,
+                                g_alpha, alpha, theta, *p, N, steps, t0, ends_run ? 1 : 0, (__nv_bfloat16 *)dT_hi, (__nv_bfloat16 *)dT_lo,
                                 (long long)k_off, (long long)k_cols, ready, err));
     NBG_CUDA(cudaGetLastError());
     return NBG_OK;
+}
+
+nbg_status nbg_lif_adjoint_sweep(const void *w_hi, const void *w_lo, void *d_hi0, void *d_lo0, void *d_hi1, void *d_lo1,
+                                 const float *g_read, const float *coef, const float *u, const float *s,
+                                 const uint8_t *m, const float *vprev, float *lam_v, float *g_theta, float *g_alpha,
+                                 const float *alpha, const float *theta, const nbg_lif_grad_params *p, int steps, int t0,
+                                 int B, int N, void *dT_hi, void *dT_lo, int64_t k_off, int64_t k_cols, float *work,
+                                 int *err, void *stream) {
+    return adj_sweep("nbg_lif_adjoint_sweep", false, w_hi, w_lo, d_hi0, d_lo0, d_hi1, d_lo1, g_read, coef, u, s, m, vprev, lam_v, g_theta, g_alpha, alpha,
+                     theta, p, steps, t0, B, N, dT_hi, dT_lo, k_off, k_cols, work, err, stream);
+}
+
+nbg_status nbg_lif_adjoint_sweep_end(const void *w_hi, const void *w_lo, void *d_hi0, void *d_lo0, void *d_hi1, void *d_lo1,
+                                 const float *g_read, const float *coef, const float *u, const float *s,
+                                 const uint8_t *m, const float *vprev, float *lam_v, float *g_theta, float *g_alpha,
+                                 const float *alpha, const float *theta, const nbg_lif_grad_params *p, int steps, int t0,
+                                 int B, int N, void *dT_hi, void *dT_lo, int64_t k_off, int64_t k_cols, float *work,
+                                 int *err, void *stream) {
+    return adj_sweep("nbg_lif_adjoint_sweep_end", true, w_hi, w_lo, d_hi0, d_lo0, d_hi1, d_lo1, g_read, coef, u, s, m, vprev, lam_v, g_theta, g_alpha, alpha,
+                     theta, p, steps, t0, B, N, dT_hi, dT_lo, k_off, k_cols, work, err, stream);
 }
 
 nbg_status nbg_adjoint_blocked_t(const float *src, int L, int B, int R, int R_pad, void *hi, void *lo,

@@ -145,3 +145,30 @@ def test_a_run_without_steps(smooth):
     y = model(torch.zeros(0, 4, 30, device="cuda"))
     y.sum().backward()
     assert not y.any() and all(not q.grad.any() for q in model.parameters())
+
+
+@pytest.mark.parametrize("n,steps", [(128, 1), (384, 1), (1024, 1), (256, 30)])
+def test_a_sweep_has_no_recurrent_term_at_the_last_step(monkeypatch, n, steps):
+    """The sweep's product at the last step runs on a zero operand: with a weight that is not finite it counts as little as in
+    the separate steps, which have none.  (One step: finite gradients.  More: NaN in the same places.)"""
+    from neuronbridge_gb300 import adjoint
+    from neuronbridge_gb300.adjoint import RecurrentLIF, poisson_inputs
+
+    model = RecurrentLIF(n_in=40, n_rec=n, n_out=5, checkpoint=20, seed=11, weight_scale=20.0, use_graphs=False)
+    with torch.no_grad():
+        model.w_rec[3, 5] = float("inf")
+    x = poisson_inputs(torch.linspace(50.0, 400.0, 40), steps, 128, dt=1.0, seed=3)
+    labels = torch.arange(128, device="cuda") % 5
+    out = []
+    for sweep in (True, False):
+        monkeypatch.setattr(adjoint, "SWEEP", sweep)
+        monkeypatch.setattr(adjoint, "FUSED_STEP", sweep)
+        model.zero_grad(set_to_none=True)
+        torch.nn.functional.cross_entropy(model(x), labels).backward()
+        out.append([q.grad for q in model.parameters()])
+    if steps == 1:
+        assert all(torch.isfinite(g).all() for g in out[0])
+        for a, b in zip(*out):
+            assert torch.equal(a, b)
+    for a, b in zip(*out):
+        assert torch.equal(torch.isnan(a), torch.isnan(b))
